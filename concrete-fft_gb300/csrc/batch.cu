@@ -63,8 +63,8 @@ __device__ void run_unit(double2* __restrict__ data, const SizeClass& C, const u
     }
     __syncthreads();
     double2* r = x;
-    if (fwd) r = unordered_smem<true, 0, ALGO>(C.L, 0, U.count, x, y, C.w, tid, nth);
-    if (inv) r = unordered_smem<false, 0, ALGO>(C.L, 0, U.count, r, r == x ? y : x, C.winv, tid, nth);
+    if (fwd) r = unordered_smem<true, kAddsBatch, ALGO>(C.L, 0, U.count, x, y, C.w, tid, nth);
+    if (inv) r = unordered_smem<false, kAddsBatch, ALGO>(C.L, 0, U.count, r, r == x ? y : x, C.winv, tid, nth);
     for (int t = 0; t < U.count; ++t) {
       double2* g = data + offs[U.first + t];
       for (int i = tid; i < n; i += nth) g[i] = r[(t << log2n) + i];
@@ -76,7 +76,7 @@ __device__ void run_unit(double2* __restrict__ data, const SizeClass& C, const u
   double2* g = data + offs[U.first];
   if (fwd) {
     for (int l = 0; l < C.d0; ++l) {
-      outer_level<true, 0>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), g, C.w + C.L.w_off[l], tid, nth);
+      outer_level<true, kAddsBatch>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), g, C.w + C.L.w_off[l], tid, nth);
       __syncthreads();
     }
   }
@@ -86,14 +86,14 @@ __device__ void run_unit(double2* __restrict__ data, const SizeClass& C, const u
     for (int i = tid; i < m; i += nth) x[i] = gc[i];
     __syncthreads();
     double2* r = x;
-    if (fwd) r = unordered_smem<true, 0, ALGO>(C.L, C.d0, 1, x, y, C.w, tid, nth);
-    if (inv) r = unordered_smem<false, 0, ALGO>(C.L, C.d0, 1, r, r == x ? y : x, C.winv, tid, nth);
+    if (fwd) r = unordered_smem<true, kAddsBatch, ALGO>(C.L, C.d0, 1, x, y, C.w, tid, nth);
+    if (inv) r = unordered_smem<false, kAddsBatch, ALGO>(C.L, C.d0, 1, r, r == x ? y : x, C.winv, tid, nth);
     for (int i = tid; i < m; i += nth) gc[i] = r[i];
     __syncthreads();
   }
   if (inv) {
     for (int l = C.d0 - 1; l >= 0; --l) {
-      outer_level<false, 0>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), g, C.winv + C.L.winv_off[l], tid,
+      outer_level<false, kAddsBatch>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), g, C.winv + C.L.winv_off[l], tid,
                             nth);
       __syncthreads();
     }
@@ -311,7 +311,6 @@ cfft_status tune_class(cfft_batch* b, size_t ci, double seconds) {
   const size_t count = std::max<size_t>(b->grid * 2, (size_t(1) << 21) >> log2n);  // >= 2 units per CTA
   double2* buf = nullptr;
   CFFT_CUDA_TRY(cudaMalloc(&buf, count * n * sizeof(double2)));
-  CFFT_CUDA_TRY(cudaMemset(buf, 0, count * n * sizeof(double2)));
   cfft_batch tb;
   tb.grid = b->grid;
   CFFT_CUDA_TRY(cudaMalloc(&tb.d_head, sizeof(unsigned int)));
@@ -333,10 +332,14 @@ cfft_status tune_class(cfft_batch* b, size_t ci, double seconds) {
     tb.classes.push_back(t);
     st = finalize(&tb);
     if (st != CFFT_OK) break;
+    // forward and inverse grow the data by log2 n bits each
+    const int most = timing_reps_max((c.key.dir == 3 ? 2 : 1) * log2n);
+    fill_timing_doubles((double*)buf, 2 * count * n, kTimingScale, s);
     launch_batch(&tb, buf, s);
     int reps = 1;
     double per = 0;
     for (;;) {
+      fill_timing_doubles((double*)buf, 2 * count * n, kTimingScale, s);
       cudaEventRecord(e0, s);
       for (int r = 0; r < reps; ++r) launch_batch(&tb, buf, s);
       cudaEventRecord(e1, s);
@@ -344,8 +347,8 @@ cfft_status tune_class(cfft_batch* b, size_t ci, double seconds) {
       float ms = 0;
       cudaEventElapsedTime(&ms, e0, e1);
       per = ms / reps;
-      if (ms * 1e-3 >= std::max(seconds, 5e-4) || reps >= 64) break;
-      reps *= 2;
+      if (ms * 1e-3 >= std::max(seconds, 5e-4) || reps >= std::min(64, most)) break;
+      reps = std::min(2 * reps, most);
     }
     free_tables(tb.classes[0]);
     times.push_back(per);

@@ -29,9 +29,9 @@ __global__ void __launch_bounds__(256) c64_level_kernel(double2* data, long tota
   for (long g = (long)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (long)gridDim.x * blockDim.x) {
     double2* zc = data + ((g >> lm) << log2nl);
     const int i = (int)(g & ((1L << lm) - 1));
-    if (log2r == 1) outer_group<2, FWD, 0>(zc, lm, i, wl);
-    else if (log2r == 2) outer_group<4, FWD, 0>(zc, lm, i, wl);
-    else outer_group<8, FWD, 0>(zc, lm, i, wl);
+    if (log2r == 1) outer_group<2, FWD, kAddsBatch>(zc, lm, i, wl);
+    else if (log2r == 2) outer_group<4, FWD, kAddsBatch>(zc, lm, i, wl);
+    else outer_group<8, FWD, kAddsBatch>(zc, lm, i, wl);
   }
 }
 
@@ -199,7 +199,7 @@ cfft_status launch_smem(const C64Plan& p, bool fwd, int blocks, size_t smem, cud
   DevLevels L = p.dlv;
   int tpc = p.tpc, d0 = p.d0;
   void* args[] = {&data, &nsub, &tpc, &L, &d0, (void*)&w};
-  const void* fn = c64_kernel(p.base_algo, p.emu, fwd);
+  const void* fn = c64_kernel(p.base_algo, fwd);
   return launch_kernel(fn, blocks, p.threads, args, spread_smem(fn, blocks, p.threads, 1, smem), stream, true);
 }
 
@@ -321,9 +321,11 @@ cfft_status launch_split(const C64Plan& p, bool fwd, int ls, int mode, long nsub
   const size_t part = p.n >> ls;
   const size_t smem = 2 * part * sizeof(double2);
   // one thread per butterfly of a pass over the part (more would idle at the barriers);
-  // two for the DIF algorithms, whose passes split each butterfly into halves
+  // two for the DIF algorithms in small launches, whose passes split each butterfly into
+  // halves (radix 16 at every size: a whole butterfly takes 126 registers, and one warp
+  // per CTA was slower, 84 against 70 us for 1024 transforms of 1024 points on 2 CTAs)
   const int R = algo_radix(p.base_algo);
-  const bool halves = (p.base_algo & 1) == 0;
+  const bool halves = (p.base_algo & 1) == 0 && (R == 16 || half_butterflies(nsub << ls, part / (size_t)R));
   const int threads = (int)std::min<size_t>(256, std::max<size_t>(32, (halves ? 2 : 1) * part / (size_t)R));
   DevLevels L = p.dlv;
   const double2* w = fwd ? p.d_w : p.d_winv;
@@ -529,18 +531,27 @@ double time_forward(const C64Plan& p, double2* scratch, size_t batch, double sec
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
+  const int most = timing_reps_max(p.lv.log2n[0]);
+  fill_timing_doubles((double*)scratch, 2 * batch * p.n, kTimingScale, s);
   run_plan(p, (double*)scratch, batch, true, s);  // warm-up
   int reps = 1;
   double per = 0.0;
   for (;;) {
-    cudaEventRecord(e0, s);
-    for (int i = 0; i < reps; ++i) run_plan(p, (double*)scratch, batch, true, s);
-    cudaEventRecord(e1, s);
-    cudaEventSynchronize(e1);
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    per = ms * 1e-3 / reps;
-    if (ms * 1e-3 >= std::max(seconds, 1e-3) || reps >= (1 << 20)) break;
+    double sec = 0.0;
+    for (int done = 0; done < reps;) {
+      const int now = std::min(reps - done, most);
+      fill_timing_doubles((double*)scratch, 2 * batch * p.n, kTimingScale, s);
+      cudaEventRecord(e0, s);
+      for (int i = 0; i < now; ++i) run_plan(p, (double*)scratch, batch, true, s);
+      cudaEventRecord(e1, s);
+      cudaEventSynchronize(e1);
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, e0, e1);
+      sec += ms * 1e-3;
+      done += now;
+    }
+    per = sec / reps;
+    if (sec >= std::max(seconds, 1e-3) || reps >= (1 << 20)) break;
     reps *= 2;
   }
   cudaEventDestroy(e0);
@@ -593,7 +604,6 @@ cfft_status measure_ordered(size_t n, double seconds, double2* scratch, size_t b
 cfft_status alloc_measure_scratch(size_t n, double2** scratch, size_t* batch) {
   *batch = std::max<size_t>(1, (size_t(1) << 22) / n);  // 64 MiB of c64
   CFFT_CUDA_TRY(cudaMalloc((void**)scratch, *batch * n * sizeof(double2)));
-  CFFT_CUDA_TRY(cudaMemset(*scratch, 0, *batch * n * sizeof(double2)));
   return CFFT_OK;
 }
 
@@ -621,18 +631,6 @@ void tune_launch(C64Plan& p, double2* scratch, size_t batch, double seconds) {
   }
   p.threads = bt;
   p.tpc = bp;
-  int be = p.emu;
-  for (int e : kEmuLevels) {
-    if (emu_level_for(p.base_algo, e) != e) continue;
-    C64Plan q = p;
-    q.emu = e;
-    const double t = time_forward(q, scratch, batch, seconds);
-    if (t < best) {
-      best = t;
-      be = e;
-    }
-  }
-  p.emu = be;
 }
 
 bool valid_algo(int a) { return a >= 0 && a <= 7; }

@@ -1,7 +1,7 @@
 // c64_kernels.cuh -- kernel templates of the c64 transforms and the u64 product.
 //
-// Each kernel is instantiated per (ordered base algorithm, integer-add level)
-// so that it carries exactly one algorithm's code; the instantiations live in
+// Each kernel is instantiated per ordered base algorithm so that it carries
+// exactly one algorithm's code; the instantiations live in
 // the kinst_*.cu translation units (compiled in parallel) and are reached
 // through the pointer tables declared at the end of this file.
 #pragma once
@@ -12,7 +12,7 @@ namespace cfft {
 // Sub-transforms of 2^log2n_{d0} points, `tpc` per CTA: load to shared memory,
 // run the unordered transform from level d0 (ordered plans have no levels),
 // store back.
-template <int ALGO, int E, bool FWD>
+template <int ALGO, bool FWD>
 __global__ void __launch_bounds__(256) c64_smem_kernel(double2* data, int count, int tpc, DevLevels L, int d0,
                                                        const double2* __restrict__ w) {
   extern __shared__ double2 smem[];
@@ -27,14 +27,14 @@ __global__ void __launch_bounds__(256) c64_smem_kernel(double2* data, int count,
   const int tid = threadIdx.x, nth = blockDim.x;
   for (int i = tid; i < npts; i += nth) x[i] = g[i];
   __syncthreads();
-  const double2* r = unordered_smem<FWD, E, ALGO>(L, d0, nch, x, y, w, tid, nth);
+  const double2* r = unordered_smem<FWD, kAddsBatch, ALGO>(L, d0, nch, x, y, w, tid, nth);
   for (int i = tid; i < npts; i += nth) g[i] = r[i];
 }
 
 // Fused negacyclic u64 product (see product_u64.cu for the pipeline): one
 // product per CTA at a time, grid-stride over the batch.
-template <int ALGO, int E, int THREADS>
-__global__ void __launch_bounds__(THREADS) u64_product_kernel(const uint64_t* __restrict__ a,
+template <int ALGO, int THREADS>
+__global__ void __launch_bounds__(THREADS, 6) u64_product_kernel(const uint64_t* __restrict__ a,
                                                              const double2* __restrict__ bhat, long bhat_stride,
                                                              uint64_t* __restrict__ out, long count, DevLevels L,
                                                              const double2* __restrict__ w,
@@ -60,14 +60,14 @@ __global__ void __launch_bounds__(THREADS) u64_product_kernel(const uint64_t* __
       st(x + j, cmul(ldg(tw + jj), v));
     }
     __syncthreads();
-    double2* r = unordered_smem<true, E, ALGO>(L, 0, np, x, y, w, tid, THREADS);
+    double2* r = unordered_smem<true, kAddsBatch, ALGO>(L, 0, np, x, y, w, tid, THREADS);
     for (int k = tid; k < pts; k += THREADS) {
       const double2* bp = bhat + (first + (k >> log2n)) * bhat_stride;
       st(r + k, cmul(ldg(bp + (k & (n - 1))), ld(r + k)));
     }
     __syncthreads();
     double2* o = (r == x) ? y : x;
-    double2* s = unordered_smem<false, E, ALGO>(L, 0, np, r, o, winv, tid, THREADS);
+    double2* s = unordered_smem<false, kAddsBatch, ALGO>(L, 0, np, r, o, winv, tid, THREADS);
     for (int j = tid; j < pts; j += THREADS) {
       const int jj = j & (n - 1);
       uint64_t* op = out + ((first + (j >> log2n)) << (log2n + 1));
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(THREADS) u64_product_sum_kernel(const uint64_t
         st(x + j, cmul(ldg(tw + j), v));
       }
       __syncthreads();
-      const double2* r = unordered_smem<true, 0, ALGO>(L, 0, 1, x, y, w, tid, THREADS);
+      const double2* r = unordered_smem<true, kAddsBatch, ALGO>(L, 0, 1, x, y, w, tid, THREADS);
       const double2* bp = bhat + (term << log2n);
       if (ACC > 0) {
 #pragma unroll
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(THREADS) u64_product_sum_kernel(const uint64_t
       __syncthreads();
       src = y;
     }
-    const double2* s = unordered_smem<false, 0, ALGO>(L, 0, 1, src, x, winv, tid, THREADS);
+    const double2* s = unordered_smem<false, kAddsBatch, ALGO>(L, 0, 1, src, x, winv, tid, THREADS);
     uint64_t* op = out + (g << (log2n + 1));
     for (int j = tid; j < n; j += THREADS) {
       const c64 v = cmul(ldg(itw + j), ld(s + j));
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(THREADS) u64_prepare_kernel(const int64_t* __r
       st(x + j, cmul(ldg(tw + j), v));
     }
     __syncthreads();
-    const double2* r = unordered_smem<true, 0, ALGO>(L, 0, 1, x, y, w, tid, THREADS);
+    const double2* r = unordered_smem<true, kAddsBatch, ALGO>(L, 0, 1, x, y, w, tid, THREADS);
     double2* op = bhat + (prod << log2n);
     for (int k = tid; k < n; k += THREADS) op[k] = r[k];
     __syncthreads();
@@ -186,22 +186,11 @@ __global__ void __launch_bounds__(THREADS) u64_prepare_kernel(const int64_t* __r
 constexpr int kProdThreads = 128;
 
 // Kernel-pointer tables (nullptr when the combination is not instantiated).
-const void* c64_kernel_e0(int algo, bool fwd);
+const void* c64_kernel(int algo, bool fwd);
 // one transform over 2^ls CTAs (split.cuh); mode 0 no outer levels, 1 with levels
 const void* c64_split_kernel_ptr(int algo, bool fwd, int ls, int mode);
-const void* c64_kernel_emu(int algo, int e, bool fwd);
-const void* u64_product_kernel_e0(int algo);
-const void* u64_product_kernel_emu(int algo, int e);
+const void* u64_product_kernel_ptr(int algo);
 const void* u64_prepare_kernel_ptr(int algo);
 const void* u64_product_sum_kernel_ptr(int algo, bool reg_acc);
-
-inline const void* c64_kernel(int algo, int e, bool fwd) {
-  const int lvl = emu_level_for(algo, e);
-  return lvl == 0 ? c64_kernel_e0(algo, fwd) : c64_kernel_emu(algo, lvl, fwd);
-}
-inline const void* u64_product_kernel_ptr(int algo, int e) {
-  const int lvl = emu_level_for(algo, e);
-  return lvl == 0 ? u64_product_kernel_e0(algo) : u64_product_kernel_emu(algo, lvl);
-}
 
 }  // namespace cfft

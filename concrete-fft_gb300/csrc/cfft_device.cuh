@@ -49,27 +49,26 @@ __device__ __forceinline__ c64 cmul(c64 ab, c64 xy) {
 }
 __device__ __forceinline__ c64 real_mul(double r, c64 v) { return {__dmul_rn(r, v.re), __dmul_rn(r, v.im)}; }
 
-// Selectable adders.  E (0..8) is the number of eighths of the butterfly's
-// real additions that run on the integer pipe (dadd_int, bit-identical to the
-// FP64 add); I is the complex operation's index inside its butterfly, so the
-// choice is made at compile time and spread evenly over the butterfly.
-template <int E, int I>
-__device__ __forceinline__ double sel_add(double a, double b) {
-  if constexpr ((I % 8) < E) return dadd_int(a, b);
-  else return __dadd_rn(a, b);
+// A butterfly's additions come in pairs, a sum and a difference of the same two
+// values.  E is the number of eighths of these pairs that run on the integer
+// pipes (int_fp64.cuh, the same bits): 8 all of them, 4 every other complex
+// pair, 0 none.
+// s0 = a0 + b0, d0 = a0 - b0, s1 = a1 + b1, d1 = a1 - b1.
+template <int E>
+__device__ __forceinline__ void sum_diff2(c64 a0, c64 b0, c64 a1, c64 b1, c64& s0, c64& d0, c64& s1, c64& d1) {
+  const double a[4] = {a0.re, a0.im, a1.re, a1.im}, b[4] = {b0.re, b0.im, b1.re, b1.im};
+  double s[4], d[4];
+  sum_diff<4, (1 << (E / 2)) - 1>(a, b, s, d);
+  s0 = {s[0], s[1]}, s1 = {s[2], s[3]};
+  d0 = {d[0], d[1]}, d1 = {d[2], d[3]};
 }
-template <int E, int I>
-__device__ __forceinline__ double sel_sub(double a, double b) {
-  if constexpr ((I % 8) < E) return dsub_int(a, b);
-  else return __dsub_rn(a, b);
-}
-template <int E, int I>
-__device__ __forceinline__ c64 cadd_e(c64 a, c64 b) {
-  return {sel_add<E, 2 * I>(a.re, b.re), sel_add<E, 2 * I + 1>(a.im, b.im)};
-}
-template <int E, int I>
-__device__ __forceinline__ c64 csub_e(c64 a, c64 b) {
-  return {sel_sub<E, 2 * I>(a.re, b.re), sel_sub<E, 2 * I + 1>(a.im, b.im)};
+template <int E>
+__device__ __forceinline__ void sum_diff1(c64 a0, c64 b0, c64& s0, c64& d0) {
+  const double a[2] = {a0.re, a0.im}, b[2] = {b0.re, b0.im};
+  double s[2], d[2];
+  sum_diff<2, (E >= 6 ? 3 : E >= 2 ? 1 : 0)>(a, b, s, d);
+  s0 = {s[0], s[1]};
+  d0 = {d[0], d[1]};
 }
 // src/fft_simd.rs:106-119: multiplication by -i (forward) or +i (inverse) is a
 // swap plus a sign flip, both exact.
@@ -78,18 +77,42 @@ __device__ __forceinline__ c64 mul_j(c64 v) {
   return FWD ? c64{-v.im, v.re} : c64{v.im, -v.re};
 }
 
+// E of the kernels.  All pairs leave the FP64 pipe idle between the products, none leaves
+// the integer pipes idle: with 3 pairs in 4 both are busy (one launch of 8192 products of
+// N = 2048 on Dif4: none 1182 us, 2 in 4 875, 3 in 4 770, all 817).
+constexpr int kAddsBatch = 6;
+// Kernels that split a transform over a cluster.  A whole radix-16 butterfly there is one
+// warp per CTA or less and stays on the FP64 pipe (126 registers against 110, slower).
+template <int R>
+constexpr int kAddsSplit = R == 16 ? 0 : 6;
+
 constexpr double kFrac1Sqrt2 = 0.70710678118654752440;
 constexpr double kH1X = 0.9238795325112867;    // cos(-pi/8)
 constexpr double kH1Y = -0.38268343236508984;  // sin(-pi/8)
 
 // src/fft_simd.rs:121-160
-template <bool FWD, int E = 0, int I = 0>
+template <bool FWD>
 __device__ __forceinline__ c64 mul_exp_pi_over_8(c64 v) {
-  return real_mul(kFrac1Sqrt2, cadd_e<E, I>(v, mul_j<FWD>(v)));
+  return real_mul(kFrac1Sqrt2, cadd(v, mul_j<FWD>(v)));
 }
-template <bool FWD, int E = 0, int I = 0>
+template <bool FWD>
 __device__ __forceinline__ c64 mul_exp_neg_pi_over_8(c64 v) {
-  return mul_exp_pi_over_8<!FWD, E, I>(v);
+  return mul_exp_pi_over_8<!FWD>(v);
+}
+// w = mul_exp_neg_pi_over_8(a) and v = mul_exp_pi_over_8(b).  v + mul_j<true>(v) is
+// (re - im, im + re) and v + mul_j<false>(v) is (re + im, im - re): the sum and the
+// difference of re and im, each operation as above (im - re is computed as such, not as
+// the negated re - im, so that the sign of a zero is the same).
+template <bool FWD, int E>
+__device__ __forceinline__ void mul_exp_pi_over_8_pair(c64 a, c64 b, c64& w, c64& v) {
+  // x: the operand of the (re + im, im - re) form, y: of the (re - im, im + re) form
+  const c64 x = FWD ? a : b, y = FWD ? b : a;
+  const double p[2] = {x.im, y.re}, q[2] = {x.re, y.im};
+  double s[2], d[2];
+  sum_diff<2, (E >= 6 ? 3 : E >= 2 ? 1 : 0)>(p, q, s, d);
+  const c64 rx = real_mul(kFrac1Sqrt2, c64{s[0], d[0]}), ry = real_mul(kFrac1Sqrt2, c64{d[1], s[1]});
+  w = FWD ? rx : ry;
+  v = FWD ? ry : rx;
 }
 template <bool FWD>
 __device__ __forceinline__ c64 mul_exp_pi_over_16(c64 v) {
@@ -104,136 +127,79 @@ __device__ __forceinline__ c64 mul_exp_17pi_over_16(c64 v) {
 // Radix-R DFT cores (the "last_butterfly" of each reference file).  The DIF
 // passes multiply output k by w_k afterwards, the DIT passes multiply input k
 // by w_k beforehand, the end passes use the core alone.
-template <int R, bool FWD, int E = 0>
+template <int R, bool FWD, int E>
 struct Core;
 
 template <bool FWD, int E>
 struct Core<2, FWD, E> {  // src/dif2.rs:108-115
-  __device__ __forceinline__ static void run(c64* x) {
-    const c64 a = x[0], b = x[1];
-    x[0] = cadd_e<E, 0>(a, b);
-    x[1] = csub_e<E, 1>(a, b);
-  }
+  __device__ __forceinline__ static void run(c64* x) { sum_diff1<E>(x[0], x[1], x[0], x[1]); }
 };
 
 template <bool FWD, int E>
 struct Core<4, FWD, E> {  // src/dif4.rs:171-192
   __device__ __forceinline__ static void run(c64* x) {
-    const c64 apc = cadd_e<E, 0>(x[0], x[2]);
-    const c64 amc = csub_e<E, 1>(x[0], x[2]);
-    const c64 bpd = cadd_e<E, 2>(x[1], x[3]);
-    const c64 jbmd = mul_j<FWD>(csub_e<E, 3>(x[1], x[3]));
-    x[0] = cadd_e<E, 4>(apc, bpd);
-    x[1] = csub_e<E, 5>(amc, jbmd);
-    x[2] = csub_e<E, 6>(apc, bpd);
-    x[3] = cadd_e<E, 7>(amc, jbmd);
+    c64 apc, amc, bpd, bmd;
+    sum_diff2<E>(x[0], x[2], x[1], x[3], apc, amc, bpd, bmd);
+    sum_diff2<E>(apc, bpd, amc, mul_j<FWD>(bmd), x[0], x[2], x[3], x[1]);
   }
 };
 
 template <bool FWD, int E>
 struct Core<8, FWD, E> {  // src/dif8.rs:311-352
   __device__ __forceinline__ static void run(c64* x) {
-    const c64 a04 = cadd_e<E, 0>(x[0], x[4]);
-    const c64 s04 = csub_e<E, 1>(x[0], x[4]);
-    const c64 a26 = cadd_e<E, 2>(x[2], x[6]);
-    const c64 js26 = mul_j<FWD>(csub_e<E, 3>(x[2], x[6]));
-    const c64 a15 = cadd_e<E, 4>(x[1], x[5]);
-    const c64 s15 = csub_e<E, 5>(x[1], x[5]);
-    const c64 a37 = cadd_e<E, 6>(x[3], x[7]);
-    const c64 js37 = mul_j<FWD>(csub_e<E, 7>(x[3], x[7]));
-    const c64 a04_p1_a26 = cadd_e<E, 8>(a04, a26);
-    const c64 s04_mj_s26 = csub_e<E, 9>(s04, js26);
-    const c64 a04_m1_a26 = csub_e<E, 10>(a04, a26);
-    const c64 s04_pj_s26 = cadd_e<E, 11>(s04, js26);
-    const c64 a15_p1_a37 = cadd_e<E, 12>(a15, a37);
-    const c64 w8_s15_mj_s37 = mul_exp_neg_pi_over_8<FWD, E, 24>(csub_e<E, 13>(s15, js37));
-    const c64 j_a15_m1_a37 = mul_j<FWD>(csub_e<E, 14>(a15, a37));
-    const c64 v8_s15_pj_s37 = mul_exp_pi_over_8<FWD, E, 25>(cadd_e<E, 15>(s15, js37));
-    x[0] = cadd_e<E, 16>(a04_p1_a26, a15_p1_a37);
-    x[1] = cadd_e<E, 17>(s04_mj_s26, w8_s15_mj_s37);
-    x[2] = csub_e<E, 18>(a04_m1_a26, j_a15_m1_a37);
-    x[3] = csub_e<E, 19>(s04_pj_s26, v8_s15_pj_s37);
-    x[4] = csub_e<E, 20>(a04_p1_a26, a15_p1_a37);
-    x[5] = csub_e<E, 21>(s04_mj_s26, w8_s15_mj_s37);
-    x[6] = cadd_e<E, 22>(a04_m1_a26, j_a15_m1_a37);
-    x[7] = cadd_e<E, 23>(s04_pj_s26, v8_s15_pj_s37);
+    c64 a04, s04, a26, s26, a15, s15, a37, s37;
+    sum_diff2<E>(x[0], x[4], x[2], x[6], a04, s04, a26, s26);
+    sum_diff2<E>(x[1], x[5], x[3], x[7], a15, s15, a37, s37);
+    c64 a04_p1_a26, a04_m1_a26, s04_pj_s26, s04_mj_s26, a15_p1_a37, a15_m1_a37, s15_pj_s37, s15_mj_s37;
+    sum_diff2<E>(a04, a26, s04, mul_j<FWD>(s26), a04_p1_a26, a04_m1_a26, s04_pj_s26, s04_mj_s26);
+    sum_diff2<E>(a15, a37, s15, mul_j<FWD>(s37), a15_p1_a37, a15_m1_a37, s15_pj_s37, s15_mj_s37);
+    c64 w8_s15_mj_s37, v8_s15_pj_s37;
+    mul_exp_pi_over_8_pair<FWD, E>(s15_mj_s37, s15_pj_s37, w8_s15_mj_s37, v8_s15_pj_s37);
+    sum_diff2<E>(a04_p1_a26, a15_p1_a37, s04_mj_s26, w8_s15_mj_s37, x[0], x[4], x[1], x[5]);
+    sum_diff2<E>(a04_m1_a26, mul_j<FWD>(a15_m1_a37), s04_pj_s26, v8_s15_pj_s37, x[6], x[2], x[7], x[3]);
   }
 };
 
 template <bool FWD, int E>
 struct Core<16, FWD, E> {  // src/dif16.rs:650-779
   __device__ __forceinline__ static void run(c64* x) {
-    const c64 a08 = cadd_e<E, 0>(x[0], x[8]), s08 = csub_e<E, 1>(x[0], x[8]);
-    const c64 a4c = cadd_e<E, 2>(x[4], x[12]), s4c = csub_e<E, 3>(x[4], x[12]);
-    const c64 a2a = cadd_e<E, 4>(x[2], x[10]), s2a = csub_e<E, 5>(x[2], x[10]);
-    const c64 a6e = cadd_e<E, 6>(x[6], x[14]), s6e = csub_e<E, 7>(x[6], x[14]);
-    const c64 a19 = cadd_e<E, 8>(x[1], x[9]), s19 = csub_e<E, 9>(x[1], x[9]);
-    const c64 a5d = cadd_e<E, 10>(x[5], x[13]), s5d = csub_e<E, 11>(x[5], x[13]);
-    const c64 a3b = cadd_e<E, 12>(x[3], x[11]), s3b = csub_e<E, 13>(x[3], x[11]);
-    const c64 a7f = cadd_e<E, 14>(x[7], x[15]), s7f = csub_e<E, 15>(x[7], x[15]);
+    c64 a08, s08, a4c, s4c, a2a, s2a, a6e, s6e, a19, s19, a5d, s5d, a3b, s3b, a7f, s7f;
+    sum_diff2<E>(x[0], x[8], x[4], x[12], a08, s08, a4c, s4c);
+    sum_diff2<E>(x[2], x[10], x[6], x[14], a2a, s2a, a6e, s6e);
+    sum_diff2<E>(x[1], x[9], x[5], x[13], a19, s19, a5d, s5d);
+    sum_diff2<E>(x[3], x[11], x[7], x[15], a3b, s3b, a7f, s7f);
 
-    const c64 js4c = mul_j<FWD>(s4c), js6e = mul_j<FWD>(s6e);
-    const c64 js5d = mul_j<FWD>(s5d), js7f = mul_j<FWD>(s7f);
+    c64 a08p1a4c, a08m1a4c, s08pjs4c, s08mjs4c, a2ap1a6e, a2am1a6e, s2apjs6e, s2amjs6e;
+    c64 a19p1a5d, a19m1a5d, s19pjs5d, s19mjs5d, a3bp1a7f, a3bm1a7f, s3bpjs7f, s3bmjs7f;
+    sum_diff2<E>(a08, a4c, s08, mul_j<FWD>(s4c), a08p1a4c, a08m1a4c, s08pjs4c, s08mjs4c);
+    sum_diff2<E>(a2a, a6e, s2a, mul_j<FWD>(s6e), a2ap1a6e, a2am1a6e, s2apjs6e, s2amjs6e);
+    sum_diff2<E>(a19, a5d, s19, mul_j<FWD>(s5d), a19p1a5d, a19m1a5d, s19pjs5d, s19mjs5d);
+    sum_diff2<E>(a3b, a7f, s3b, mul_j<FWD>(s7f), a3bp1a7f, a3bm1a7f, s3bpjs7f, s3bmjs7f);
 
-    const c64 a08p1a4c = cadd_e<E, 16>(a08, a4c), s08mjs4c = csub_e<E, 17>(s08, js4c);
-    const c64 a08m1a4c = csub_e<E, 18>(a08, a4c), s08pjs4c = cadd_e<E, 19>(s08, js4c);
-    const c64 a2ap1a6e = cadd_e<E, 20>(a2a, a6e), s2amjs6e = csub_e<E, 21>(s2a, js6e);
-    const c64 a2am1a6e = csub_e<E, 22>(a2a, a6e), s2apjs6e = cadd_e<E, 23>(s2a, js6e);
-    const c64 a19p1a5d = cadd_e<E, 24>(a19, a5d), s19mjs5d = csub_e<E, 25>(s19, js5d);
-    const c64 a19m1a5d = csub_e<E, 26>(a19, a5d), s19pjs5d = cadd_e<E, 27>(s19, js5d);
-    const c64 a3bp1a7f = cadd_e<E, 28>(a3b, a7f), s3bmjs7f = csub_e<E, 29>(s3b, js7f);
-    const c64 a3bm1a7f = csub_e<E, 30>(a3b, a7f), s3bpjs7f = cadd_e<E, 31>(s3b, js7f);
+    c64 w8_s2amjs6e, v8_s2apjs6e;
+    mul_exp_pi_over_8_pair<FWD, E>(s2amjs6e, s2apjs6e, w8_s2amjs6e, v8_s2apjs6e);
+    c64 e0, e1, e2, e3, e4, e5, e6, e7;
+    sum_diff2<E>(a08p1a4c, a2ap1a6e, s08mjs4c, w8_s2amjs6e, e0, e4, e1, e5);
+    sum_diff2<E>(a08m1a4c, mul_j<FWD>(a2am1a6e), s08pjs4c, v8_s2apjs6e, e6, e2, e7, e3);
 
-    const c64 w8_s2amjs6e = mul_exp_neg_pi_over_8<FWD, E, 64>(s2amjs6e);
-    const c64 j_a2am1a6e = mul_j<FWD>(a2am1a6e);
-    const c64 v8_s2apjs6e = mul_exp_pi_over_8<FWD, E, 65>(s2apjs6e);
-
-    const c64 e0 = cadd_e<E, 32>(a08p1a4c, a2ap1a6e);
-    const c64 e1 = cadd_e<E, 33>(s08mjs4c, w8_s2amjs6e);
-    const c64 e2 = csub_e<E, 34>(a08m1a4c, j_a2am1a6e);
-    const c64 e3 = csub_e<E, 35>(s08pjs4c, v8_s2apjs6e);
-    const c64 e4 = csub_e<E, 36>(a08p1a4c, a2ap1a6e);
-    const c64 e5 = csub_e<E, 37>(s08mjs4c, w8_s2amjs6e);
-    const c64 e6 = cadd_e<E, 38>(a08m1a4c, j_a2am1a6e);
-    const c64 e7 = cadd_e<E, 39>(s08pjs4c, v8_s2apjs6e);
-
-    const c64 w8_s3bmjs7f = mul_exp_neg_pi_over_8<FWD, E, 66>(s3bmjs7f);
-    const c64 j_a3bm1a7f = mul_j<FWD>(a3bm1a7f);
-    const c64 v8_s3bpjs7f = mul_exp_pi_over_8<FWD, E, 67>(s3bpjs7f);
-
-    const c64 f0 = cadd_e<E, 40>(a19p1a5d, a3bp1a7f);
-    const c64 f1 = cadd_e<E, 41>(s19mjs5d, w8_s3bmjs7f);
-    const c64 f2 = csub_e<E, 42>(a19m1a5d, j_a3bm1a7f);
-    const c64 f3 = csub_e<E, 43>(s19pjs5d, v8_s3bpjs7f);
-    const c64 f4 = csub_e<E, 44>(a19p1a5d, a3bp1a7f);
-    const c64 f5 = csub_e<E, 45>(s19mjs5d, w8_s3bmjs7f);
-    const c64 f6 = cadd_e<E, 46>(a19m1a5d, j_a3bm1a7f);
-    const c64 f7 = cadd_e<E, 47>(s19pjs5d, v8_s3bpjs7f);
+    c64 w8_s3bmjs7f, v8_s3bpjs7f;
+    mul_exp_pi_over_8_pair<FWD, E>(s3bmjs7f, s3bpjs7f, w8_s3bmjs7f, v8_s3bpjs7f);
+    c64 f0, f1, f2, f3, f4, f5, f6, f7;
+    sum_diff2<E>(a19p1a5d, a3bp1a7f, s19mjs5d, w8_s3bmjs7f, f0, f4, f1, f5);
+    sum_diff2<E>(a19m1a5d, mul_j<FWD>(a3bm1a7f), s19pjs5d, v8_s3bpjs7f, f6, f2, f7, f3);
 
     const c64 h1 = mul_exp_pi_over_16<FWD>(f1);
-    const c64 w8 = mul_exp_neg_pi_over_8<FWD, E, 68>(f2);
     const c64 h3 = mul_exp_17pi_over_16<FWD>(f3);
     const c64 j4 = mul_j<FWD>(f4);
     const c64 hd = mul_exp_17pi_over_16<!FWD>(f5);
-    const c64 v8 = mul_exp_pi_over_8<FWD, E, 69>(f6);
     const c64 hf = mul_exp_pi_over_16<!FWD>(f7);
+    c64 w8, v8;
+    mul_exp_pi_over_8_pair<FWD, E>(f2, f6, w8, v8);
 
-    x[0] = cadd_e<E, 48>(e0, f0);
-    x[1] = cadd_e<E, 49>(e1, h1);
-    x[2] = cadd_e<E, 50>(e2, w8);
-    x[3] = cadd_e<E, 51>(e3, h3);
-    x[4] = csub_e<E, 52>(e4, j4);
-    x[5] = csub_e<E, 53>(e5, hd);
-    x[6] = csub_e<E, 54>(e6, v8);
-    x[7] = csub_e<E, 55>(e7, hf);
-    x[8] = csub_e<E, 56>(e0, f0);
-    x[9] = csub_e<E, 57>(e1, h1);
-    x[10] = csub_e<E, 58>(e2, w8);
-    x[11] = csub_e<E, 59>(e3, h3);
-    x[12] = cadd_e<E, 60>(e4, j4);
-    x[13] = cadd_e<E, 61>(e5, hd);
-    x[14] = cadd_e<E, 62>(e6, v8);
-    x[15] = cadd_e<E, 63>(e7, hf);
+    sum_diff2<E>(e0, f0, e1, h1, x[0], x[8], x[1], x[9]);
+    sum_diff2<E>(e2, w8, e3, h3, x[2], x[10], x[3], x[11]);
+    sum_diff2<E>(e4, j4, e5, hd, x[12], x[4], x[13], x[5]);
+    sum_diff2<E>(e6, v8, e7, hf, x[14], x[6], x[15], x[7]);
   }
 };
 

@@ -56,10 +56,10 @@ __device__ void engine_product(const EngClass& C, const cfft_product_item& it, d
       st(x + j, cmul(ldg(C.tw + j), v));
     }
     __syncthreads();
-    double2* r = unordered_smem<true, 0, ALGO>(C.L, 0, 1, x, y, C.w, tid, nth);
+    double2* r = unordered_smem<true, kAddsBatch, ALGO>(C.L, 0, 1, x, y, C.w, tid, nth);
     for (int k = tid; k < n; k += nth) st(r + k, cmul(ldg(bh + k), ld(r + k)));
     __syncthreads();
-    double2* s = unordered_smem<false, 0, ALGO>(C.L, 0, 1, r, r == x ? y : x, C.winv, tid, nth);
+    double2* s = unordered_smem<false, kAddsBatch, ALGO>(C.L, 0, 1, r, r == x ? y : x, C.winv, tid, nth);
     for (int j = tid; j < n; j += nth) {
       const c64 t = cmul(ldg(C.itw + j), ld(s + j));
       __stcs(out + j, round_half_up_mod64(t.re));
@@ -74,7 +74,7 @@ __device__ void engine_product(const EngClass& C, const cfft_product_item& it, d
   }
   __syncthreads();
   for (int l = 0; l < C.d0; ++l) {
-    outer_level<true, 0>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), ws, C.w + C.L.w_off[l], tid, nth);
+    outer_level<true, kAddsBatch>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), ws, C.w + C.L.w_off[l], tid, nth);
     __syncthreads();
   }
   const int log2sub = C.L.log2n[C.d0], m = 1 << log2sub;
@@ -82,16 +82,16 @@ __device__ void engine_product(const EngClass& C, const cfft_product_item& it, d
     double2* gc = ws + ((long)c << log2sub);
     for (int i = tid; i < m; i += nth) x[i] = gc[i];
     __syncthreads();
-    double2* r = unordered_smem<true, 0, ALGO>(C.L, C.d0, 1, x, y, C.w, tid, nth);
+    double2* r = unordered_smem<true, kAddsBatch, ALGO>(C.L, C.d0, 1, x, y, C.w, tid, nth);
     const double2* bc = bh + ((long)c << log2sub);
     for (int k = tid; k < m; k += nth) st(r + k, cmul(ldg(bc + k), ld(r + k)));
     __syncthreads();
-    double2* s = unordered_smem<false, 0, ALGO>(C.L, C.d0, 1, r, r == x ? y : x, C.winv, tid, nth);
+    double2* s = unordered_smem<false, kAddsBatch, ALGO>(C.L, C.d0, 1, r, r == x ? y : x, C.winv, tid, nth);
     for (int i = tid; i < m; i += nth) gc[i] = s[i];
     __syncthreads();
   }
   for (int l = C.d0 - 1; l >= 0; --l) {
-    outer_level<false, 0>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), ws, C.winv + C.L.winv_off[l], tid,
+    outer_level<false, kAddsBatch>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), ws, C.winv + C.L.winv_off[l], tid,
                           nth);
     __syncthreads();
   }

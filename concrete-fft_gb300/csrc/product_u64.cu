@@ -172,7 +172,7 @@ cfft_status product_sum_unfused(const cfft_u64_product_plan* plan, const uint64_
 
 cfft_status launch_product(const cfft_u64_product_plan* plan, const uint64_t* a, const double* bhat,
                            size_t bhat_stride, uint64_t* out, size_t count, cudaStream_t stream) {
-  const void* fn = u64_product_kernel_ptr(plan->base_algo, plan->emu);
+  const void* fn = u64_product_kernel_ptr(plan->base_algo);
   // N <= 128: 512 points per CTA iteration (one product of n = 32 would give a radix-4
   // pass 8 butterflies, a quarter warp: 122 vs 375 M products/s possible at N = 64)
   int log2p = 0;
@@ -250,6 +250,19 @@ int split0_log2(const cfft_u64_product_plan* p, bool fast = true) {
   return ls;
 }
 
+// Threads per CTA of the class-split product kernels (`ctas` CTAs of `part` points).  DIF:
+// two threads per butterfly of a pass (half butterflies) in small launches, DIT: one; at
+// least a thread per two points for the elementwise steps (radix 16 has few butterflies per
+// pass).  Larger DIF launches take one thread per butterfly, which is how the kernel tells
+// them apart; not the sums, whose accumulator registers are sized for part / 2 threads.
+int split_product_threads(int algo, size_t part, long ctas, bool sum) {
+  const size_t radix = size_t(2) << (algo / 2);
+  const size_t full = part / radix;
+  size_t want = std::max(((algo & 1) ? 1 : 2) * full, part / 2);
+  if (!(algo & 1) && radix < 16 && !sum && !half_butterflies(ctas, full)) want = full;
+  return (int)std::min<size_t>(256, std::max<size_t>(32, want));
+}
+
 cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, const uint64_t* a, const double* bhat,
                                   size_t bhat_stride, uint64_t* out, size_t count, cudaStream_t stream,
                                   const cfft_product_item* items = nullptr, int terms = 1) {
@@ -258,12 +271,7 @@ cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, con
   if (!fn) return fail(CFFT_ERR_INVALID_SIZE, "no cluster product kernel for this base and cluster size");
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   const size_t part = plan->n >> ls;
-  const size_t radix = size_t(2) << (algo / 2);
-  // DIF: two threads per butterfly of a pass (half butterflies), DIT: one; at
-  // least a thread per two points for the elementwise steps (radix 16 has few
-  // butterflies per pass)
-  const size_t pass_threads = ((algo & 1) ? 1 : 2) * part / radix;
-  const int threads = (int)std::min<size_t>(256, std::max<size_t>(32, std::max(pass_threads, part / 2)));
+  const int threads = split_product_threads(algo, part, (long)(count << ls), terms > 1);
   const size_t smem = 3 * part * sizeof(double2);
   const int grid = (int)(count << ls);
   DevLevels L = plan->dlv;
@@ -278,10 +286,9 @@ cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, con
 
 // Launch shape of u64_product_split2_kernel with 2^ls1 classes: threads per CTA
 // and shared memory (three buffers of the CTA's part of the base).
-void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, int* threads, size_t* smem) {
+void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, bool sum, int* threads, size_t* smem) {
   const size_t part = p->base_n >> ls1;
-  const size_t radix = size_t(2) << (p->base_algo / 2);
-  *threads = (int)std::min<size_t>(256, std::max<size_t>(32, std::max(2 * part / radix, part / 2)));
+  *threads = split_product_threads(p->base_algo, part, ctas, sum);
   *smem = 3 * part * sizeof(double2);
 }
 
@@ -309,7 +316,7 @@ bool split2_shape(const cfft_u64_product_plan* p, size_t count, int* ls0, int* l
     if (l0 + l1 > 3) {  // every product's 16-CTA cluster resident at once, one CTA per SM
       int threads = 0;
       size_t smem = 0;
-      split2_launch_shape(p, l1, &threads, &smem);
+      split2_launch_shape(p, l1, (long)(count << (l0 + l1)), sum, &threads, &smem);
       if ((long)count > (long)spread_clusters(fn, threads, 16)) continue;
     }
     *ls0 = l0;
@@ -328,7 +335,7 @@ cfft_status launch_split2_product(const cfft_u64_product_plan* plan, int ls0, in
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   int threads = 0;
   size_t smem = 0;
-  split2_launch_shape(plan, ls1, &threads, &smem);
+  split2_launch_shape(plan, ls1, (long)(count << ls), terms > 1, &threads, &smem);
   const int grid = (int)(count << ls);
   DevLevels L = plan->dlv;
   long stride = (long)bhat_stride;
@@ -650,10 +657,11 @@ cfft_status cfft_u64_product_plan_create_measure(size_t N, double seconds, cfft_
   CFFT_CUDA_TRY(cudaMalloc(&da, count * N * sizeof(uint64_t)));
   CFFT_CUDA_TRY(cudaMalloc(&dout, count * N * sizeof(uint64_t)));
   CFFT_CUDA_TRY(cudaMalloc(&dbhat, count * n * sizeof(double2)));
-  CFFT_CUDA_TRY(cudaMemset(da, 0, count * N * sizeof(uint64_t)));
-  CFFT_CUDA_TRY(cudaMemset(dbhat, 0, count * n * sizeof(double2)));
   cudaStream_t s;
   CFFT_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  // torus words and the spectra of 8-bit digits
+  fill_timing_words(da, count * N, s);
+  fill_timing_doubles(dbhat, 2 * count * n, 0x1p12, s);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -713,41 +721,7 @@ cfft_status cfft_u64_product_plan_create_measure(size_t N, double seconds, cfft_
   if (st != CFFT_OK) return st;
   st = cfft_u64_product_plan_create(N, (cfft_algo)best_algo, best_base, out);
   if (st != CFFT_OK) return st;
-  // integer-pipe share of the additions for the winning algorithm
-  CFFT_CUDA_TRY(cudaMalloc(&da, count * N * sizeof(uint64_t)));
-  CFFT_CUDA_TRY(cudaMalloc(&dout, count * N * sizeof(uint64_t)));
-  CFFT_CUDA_TRY(cudaMalloc(&dbhat, count * n * sizeof(double2)));
-  CFFT_CUDA_TRY(cudaMemset(da, 0, count * N * sizeof(uint64_t)));
-  CFFT_CUDA_TRY(cudaMemset(dbhat, 0, count * n * sizeof(double2)));
-  CFFT_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  double best_e = 1e30;
-  int be = (*out)->emu;
-  for (int e : kEmuLevels) {
-    if (emu_level_for(best_algo, e) != e) continue;
-    (*out)->emu = e;
-    cfft_u64_product(*out, da, dbhat, n, dout, count, s);
-    cudaEventRecord(e0, s);
-    const int reps = 8;
-    for (int r = 0; r < reps; ++r) cfft_u64_product(*out, da, dbhat, n, dout, count, s);
-    cudaEventRecord(e1, s);
-    cudaEventSynchronize(e1);
-    float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    if (ms < best_e) {
-      best_e = ms;
-      be = e;
-    }
-  }
-  (*out)->emu = be;
-  tune_store(2, N, TuneVal{best_algo, best_base, kProdThreads, 1, be});
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaStreamDestroy(s);
-  cudaFree(da);
-  cudaFree(dout);
-  cudaFree(dbhat);
+  tune_store(2, N, TuneVal{best_algo, best_base, kProdThreads, 1, 0});
   return CFFT_OK;
 }
 

@@ -572,6 +572,16 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
   return z ^ (z >> 31);
 }
 
+__global__ void timing_fill_kernel(uint64_t* p, size_t count, double scale) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
+    const uint64_t r = mix64(i);
+    // scale 0: the word itself; else 1.mantissa - 1.5 in [-0.5, 0.5), times 2 scale
+    p[i] = scale == 0.0 ? r
+                        : (uint64_t)__double_as_longlong(
+                              (__longlong_as_double((long long)((r >> 12) | 0x3ff0000000000000ull)) - 1.5) * (2.0 * scale));
+  }
+}
+
 __device__ void make_pair(uint64_t i, uint64_t seed, double& x, double& y) {
   const uint64_t r0 = mix64(seed ^ (i * 4 + 0)), r1 = mix64(seed ^ (i * 4 + 1)), r2 = mix64(seed ^ (i * 4 + 2));
   const int mode = (int)(i & 3);
@@ -606,10 +616,12 @@ __global__ void dadd_check_kernel(uint64_t count, uint64_t seed, unsigned long l
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
     double x, y;
     make_pair(i, seed, x, y);
-    const double a = cfft::dadd_int(x, y);
-    const double b = __dadd_rn(x, y);
-    const bool nan_both = (a != a) && (b != b);
-    if (!nan_both && __double_as_longlong(a) != __double_as_longlong(b)) {
+    double s, d;
+    cfft::sum_diff<1, 1>(&x, &y, &s, &d);
+    const double s0 = __dadd_rn(x, y), d0 = __dsub_rn(x, y);
+    const bool s_ok = (s != s && s0 != s0) || __double_as_longlong(s) == __double_as_longlong(s0);
+    const bool d_ok = (d != d && d0 != d0) || __double_as_longlong(d) == __double_as_longlong(d0);
+    if (!s_ok || !d_ok) {
       if (atomicAdd(bad, 1ull) == 0) {
         first[0] = (unsigned long long)__double_as_longlong(x);
         first[1] = (unsigned long long)__double_as_longlong(y);
@@ -623,14 +635,28 @@ __global__ void dadd_int_rate_kernel(double* out, double seed) {
   double a[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) a[i] = seed + threadIdx.x * 1e-3 + i;
-  const double c = 1.0000000001e-3;
-  for (int it = 0; it < kIntIters; ++it) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = cfft::dadd_int(a[i], c);
+  for (int it = 0; it < kIntIters; it += 2) {
+    // x + y and x - y, whose own sum and difference are 2x and 2y: the values only double
+    double s[2], d[2];
+    cfft::sum_diff<2, 3>(a, a + 2, s, d);
+    cfft::sum_diff<2, 3>(s, d, a, a + 2);
   }
   out[(size_t)blockIdx.x * blockDim.x + threadIdx.x] = a[0] + a[1] + a[2] + a[3];
 }
 }  // namespace
+
+namespace cfft {
+cfft_status fill_timing_words(uint64_t* p, size_t count, cudaStream_t stream) {
+  timing_fill_kernel<<<sm_count() * 8, 256, 0, stream>>>(p, count, 0.0);
+  CFFT_CHECK_LAUNCH();
+  return CFFT_OK;
+}
+cfft_status fill_timing_doubles(double* p, size_t count, double scale, cudaStream_t stream) {
+  timing_fill_kernel<<<sm_count() * 8, 256, 0, stream>>>((uint64_t*)p, count, scale);
+  CFFT_CHECK_LAUNCH();
+  return CFFT_OK;
+}
+}  // namespace cfft
 
 extern "C" cfft_status cfft_diag_dadd_check(uint64_t count, uint64_t seed, uint64_t* mismatches, uint64_t* bad_pair) {
   if (!mismatches) return cfft::fail(CFFT_ERR_INVALID_ARGUMENT, "null output pointer");

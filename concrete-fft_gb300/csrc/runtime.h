@@ -43,6 +43,15 @@ cfft_status upload(const T* host, size_t count, T** dev) {
 }
 
 int sm_count();
+// Whether a launch of `ctas` CTAs, whose passes have `butterflies` butterflies each, runs
+// them as half butterflies, two threads each, with every addition on the FP64 pipe.  With
+// about one warp per SM sub-partition a pass is one warp's dependent chain: halves shorten
+// it (one 1024-point forward on Dif4, 4 CTAs: 5.3 us against 7.4 with whole butterflies).
+// With more warps the pipes bind, and whole butterflies with most additions on the integer
+// pipes win (batch 96: 9.1 us against 9.9; batch 256: 14.8 against 19.4).
+inline bool half_butterflies(long ctas, size_t butterflies) {
+  return ctas * (long)((butterflies + 31) / 32) * 4 < 5L * 4 * sm_count();
+}
 
 // Launch a kernel through its pointer, raising its dynamic shared-memory limit
 // the first time it is used with more than 48 KiB.  `pdl`: programmatic stream
@@ -119,6 +128,16 @@ HostChunks host_chunks();
 // (pageable memory, device memory).  Kernels then write results there
 // directly: on a Grace host they cross NVLink-C2C as the kernel stores them.
 void* mapped_host_range(const void* p, size_t bytes);
+// Input for timing candidates (Method::Measure, the batch tuner): 64-bit words, uniform as
+// integers, or doubles uniform in [-scale, scale).  Zeros would not do: the butterflies'
+// integer path (int_fp64.cuh) leaves them to the FP64 pipe.
+cfft_status fill_timing_words(uint64_t* p, size_t count, cudaStream_t stream);
+cfft_status fill_timing_doubles(double* p, size_t count, double scale, cudaStream_t stream);
+// Transforms are unnormalised, so repeated in-place calls grow their data.  A timed run of
+// `bits` bits of growth per call starts at kTimingScale and lasts at most timing_reps_max
+// calls, then the data are filled again.
+constexpr double kTimingScale = 0x1p-900;
+inline int timing_reps_max(int bits) { return 1800 / (bits < 1 ? 1 : bits); }
 // Makes the current device's primary context current on the calling thread.
 void bind_device_context();
 

@@ -53,13 +53,13 @@ __device__ __forceinline__ FlatBuf dif_after_first(int log2n, int ls, FlatBuf x,
   const int log2c = log2n - ls;
   FlatBuf cur = x, oth = y;
   for (int i = 1; i < npass; ++i) {
-    stockham_pass<R, FWD, false, 0, true>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
+    stockham_pass<R, FWD, false, kAddsSplit<R>, true>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
     __syncthreads();
     const FlatBuf t = cur;
     cur = oth;
     oth = t;
   }
-  end_dispatch<R, FWD, 0, true>(lm, log2c, 1, cur, tid, nth);
+  end_dispatch<R, FWD, kAddsSplit<R>, true>(lm, log2c, 1, cur, tid, nth);
   __syncthreads();
   return cur;
 }
@@ -77,10 +77,10 @@ __device__ __forceinline__ FlatBuf dit_before_last(int log2n, int ls, FlatBuf x,
   }
   const int log2c = log2n - ls;
   FlatBuf cur = x, oth = y;
-  end_dispatch<R, FWD, 0>(lm, log2c, 1, cur, tid, nth);
+  end_dispatch<R, FWD, kAddsSplit<R>>(lm, log2c, 1, cur, tid, nth);
   __syncthreads();
   for (int i = npass - 1; i >= 1; --i) {
-    stockham_pass<R, FWD, true, 0>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
+    stockham_pass<R, FWD, true, kAddsSplit<R>>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
     __syncthreads();
     const FlatBuf t = cur;
     cur = oth;
@@ -101,7 +101,7 @@ __device__ __forceinline__ void level0_scatter(double2* const* src, double2* con
     c64 v[R0];
 #pragma unroll
     for (int k = 0; k < R0; ++k) v[k] = ld(src[k / SL] + ((k % SL) << lm) + i);
-    Core<R0, true, 0>::run(v);
+    Core<R0, true, kAddsSplit<R0>>::run(v);
     const double2* tw = wl + (R0 - 1) * i - 1;
 #pragma unroll
     for (int k = 0; k < R0; ++k) {
@@ -128,7 +128,7 @@ __device__ __forceinline__ void level0_last(double2* g, int lm, double2* const* 
       const int sl = slot<R0>(k);
       v[k] = cmul(ldg(tw + k), ld(peer[sl >> (LR0 - LS)] + ((sl & ((R0 >> LS) - 1)) << lm) + i));
     }
-    Core<R0, false, 0>::run(v);
+    Core<R0, false, kAddsSplit<R0>>::run(v);
 #pragma unroll
     for (int k = 0; k < R0; ++k) st(g + (k << lm) + i, v[k]);
   }
@@ -185,7 +185,7 @@ __device__ __forceinline__ void first_pass_scatter(Load load, int per, int p0, i
     c64 v[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) v[k] = load(k, b, p);
-    Core<R, FWD, 0>::run(v);
+    Core<R, FWD, kAddsSplit<R>>::run(v);
     const double2* tw = wb + (p << LR);
 #pragma unroll
     for (int k = 0; k < R; ++k) {
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(tw + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, FWD, 0>::run(v);
+      Core<R, FWD, kAddsSplit<R>>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) st(g + (k << lper) + p, v[k]);
     }
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
       level0_scatter<8, LS>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     }
     cl.sync();  // every part's xs is complete, and every peer is done reading this CTA's ys
-    const FlatBuf r = unordered_t<true, 0, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
+    const FlatBuf r = unordered_t<true, kAddsSplit<AlgoInfo<ALGO>::R>, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
     double2* gw = g + ((long)c << log2c);
     for (int j = tid; j < (1 << log2c); j += nth) gw[j] = r.p[j];
   } else {
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     __syncthreads();
     const int lr0 = L.log2r[0];
     const int lm = log2n - lr0;
-    const FlatBuf r = unordered_t<false, 0, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
+    const FlatBuf r = unordered_t<false, kAddsSplit<AlgoInfo<ALGO>::R>, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
     double2* peer[S];
 #pragma unroll
     for (int j = 0; j < S; ++j) peer[j] = cl.map_shared_rank(r.p, (unsigned)j);
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
       c64 v[R0];
 #pragma unroll
       for (int k = 0; k < R0; ++k) v[k] = b == tid ? v0[k] : ld(g + (k << log2m) + i);
-      Core<R0, true, 0>::run(v);
+      Core<R0, true, kAddsSplit<R0>>::run(v);
       const double2* twl = wl + (R0 - 1) * i - 1;
       const int p = i & ((1 << lq) - 1);
       const int dst = ((i >> lq) << lpp) + (p & (pp - 1));
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
 #pragma unroll
       for (int k = 1; k < R0; ++k)
         v[k] = cmul(ldg(twl + k), ld(cl.map_shared_rank(sv.p, (unsigned)((slot<R0>(k) << LS1) + cls)) + at));
-      Core<R0, false, 0>::run(v);
+      Core<R0, false, kAddsSplit<R0>>::run(v);
 #pragma unroll
       for (int k = 0; k < R0; ++k) st(g + (k << log2m) + i, v[k]);
     }
@@ -492,5 +492,16 @@ const void* split_ptr(bool fwd, int ls, int mode) {
     default: return nullptr;
   }
 }
+
+#ifndef CFFT_KERNEL_INSTANCE  // instantiated in kinst_split_<A>.cu, one unit per algorithm
+extern template const void* split_ptr<0>(bool, int, int);
+extern template const void* split_ptr<1>(bool, int, int);
+extern template const void* split_ptr<2>(bool, int, int);
+extern template const void* split_ptr<3>(bool, int, int);
+extern template const void* split_ptr<4>(bool, int, int);
+extern template const void* split_ptr<5>(bool, int, int);
+extern template const void* split_ptr<6>(bool, int, int);
+extern template const void* split_ptr<7>(bool, int, int);
+#endif
 
 }  // namespace cfft

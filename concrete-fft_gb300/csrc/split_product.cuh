@@ -57,7 +57,7 @@ __device__ __forceinline__ void level0_inv_untwist(double2* const* src, int lm, 
       const int sl = slot<R0>(k);
       v[k] = cmul(ldg(tw + k), ld(src[sl >> (LR0 - LS)] + ((sl & (SL - 1)) << lm) + i));
     }
-    Core<R0, false, 0>::run(v);
+    Core<R0, false, kAddsSplit<R0>>::run(v);
 #pragma unroll
     for (int k = 0; k < R0; ++k) {
       const int j = (k << lm) + i;
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
 
     // 3. the slices forward, the pointwise product added into the accumulator
     // (a single term: stored in place, the inverse starts from it)
-    const FlatBuf r = unordered_t<true, 0, ALGO>(L, 1, nsl, FlatBuf{x}, FlatBuf{y}, w, tid, nth);
+    const FlatBuf r = unordered_t<true, kAddsSplit<AlgoInfo<ALGO>::R>, ALGO>(L, 1, nsl, FlatBuf{x}, FlatBuf{y}, w, tid, nth);
     const double2* bp = bprod + base;
 #pragma unroll
     for (int k = 0; k < kSplitAcc; ++k) {
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
     }
     __syncthreads();
   }
-  const FlatBuf s = unordered_t<false, 0, ALGO>(L, 1, nsl, FlatBuf{src}, FlatBuf{src == x ? y : x}, winv, tid, nth);
+  const FlatBuf s = unordered_t<false, kAddsSplit<AlgoInfo<ALGO>::R>, ALGO>(L, 1, nsl, FlatBuf{src}, FlatBuf{src == x ? y : x}, winv, tid, nth);
   double2* peer_s[1 << LS];
 #pragma unroll
   for (int j = 0; j < (1 << LS); ++j) peer_s[j] = cl.map_shared_rank(s.p, (unsigned)j);
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(twp + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, true, 0>::run(v);
+      Core<R, true, kAddsSplit<R>>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) st(z + (k << lpc) + b, cmul(ldg(bp + (k << lper) + p), v[k]));
     }
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(twp + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, false, 0>::run(v);
+      Core<R, false, kAddsSplit<R>>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         const int jg = (k << lper) + p;
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
     } else {
       load_l0(i, v);
     }
-    Core<R0, true, 0>::run(v);
+    Core<R0, true, kAddsSplit<R0>>::run(v);
     const double2* twl = wl + (R0 - 1) * i - 1;
     const int p = i & ((1 << lq) - 1);
     const int dst = (((i >> lq) << lpp) + (p & (pp - 1)));
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
 #pragma unroll
     for (int k = 1; k < R0; ++k)
       v[k] = cmul(ldg(twl + k), ld(cl.map_shared_rank(sv.p, (unsigned)((slot<R0>(k) << LS1) + cls)) + at));
-    Core<R0, false, 0>::run(v);
+    Core<R0, false, kAddsSplit<R0>>::run(v);
 #pragma unroll
     for (int k = 0; k < R0; ++k) {
       const int j = (k << log2m) + i;
@@ -548,42 +548,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
   cl.sync();  // no CTA exits while a peer reads its shared memory
 }
 
-// kernel pointers by base algorithm (kinst_split_prod_*.cu, one unit per pair)
-// (big: the 512-thread variant, for parts of 4096 points)
-const void* u64_product_split_ptr_01(int algo, int ls, bool big);
-const void* u64_product_split_ptr_23(int algo, int ls, bool big);
-const void* u64_product_split_ptr_45(int algo, int ls, bool big);
-const void* u64_product_split_ptr_67(int algo, int ls, bool big);
-inline const void* u64_product_split_ptr(int algo, int ls, bool big) {
-  return algo < 2 ? u64_product_split_ptr_01(algo, ls, big)
-                  : algo < 4 ? u64_product_split_ptr_23(algo, ls, big)
-                             : algo < 6 ? u64_product_split_ptr_45(algo, ls, big) : u64_product_split_ptr_67(algo, ls, big);
-}
-// the kernel for plans without an outer level (sum: its Fourier-domain sum
-// variant); nullptr where S = 2^ls exceeds the radix, or a sum on a DIT base
-const void* u64_product_split0_ptr_01(int algo, int ls, bool sum);
-const void* u64_product_split0_ptr_23(int algo, int ls, bool sum);
-const void* u64_product_split0_ptr_45(int algo, int ls, bool sum);
-const void* u64_product_split0_ptr_67(int algo, int ls, bool sum);
-// the one-level kernel (DIF bases only; sum: its Fourier-domain sum variant);
-// nullptr where the shape is not instantiated
-const void* u64_product_split2_ptr_01(int algo, int ls0, int ls1, bool sum);
-const void* u64_product_split2_ptr_23(int algo, int ls0, int ls1, bool sum);
-const void* u64_product_split2_ptr_45(int algo, int ls0, int ls1, bool sum);
-const void* u64_product_split2_ptr_67(int algo, int ls0, int ls1, bool sum);
-inline const void* u64_product_split2_ptr(int algo, int ls0, int ls1, bool sum) {
-  return algo < 2 ? u64_product_split2_ptr_01(algo, ls0, ls1, sum)
-                  : algo < 4 ? u64_product_split2_ptr_23(algo, ls0, ls1, sum)
-                             : algo < 6 ? u64_product_split2_ptr_45(algo, ls0, ls1, sum)
-                                        : u64_product_split2_ptr_67(algo, ls0, ls1, sum);
-}
-inline const void* u64_product_split0_ptr(int algo, int ls, bool sum) {
-  return algo < 2 ? u64_product_split0_ptr_01(algo, ls, sum)
-                  : algo < 4 ? u64_product_split0_ptr_23(algo, ls, sum)
-                             : algo < 6 ? u64_product_split0_ptr_45(algo, ls, sum)
-                                        : u64_product_split0_ptr_67(algo, ls, sum);
-}
-
+// Kernel pointers of base algorithm A (big: the 512-thread variant, for parts of 4096 points).
 template <int A>
 const void* split_product_ptr(int ls, bool big) {
   if (big) {
@@ -643,5 +608,44 @@ template <int A>
 const void* split2_product_ptr(int ls0, int ls1, bool sum) {
   return sum ? split2_product_ptr_t<A, true>(ls0, ls1) : split2_product_ptr_t<A, false>(ls0, ls1);
 }
+
+#ifndef CFFT_KERNEL_INSTANCE  // instantiated in kinst_split_prod_<A>.cu, one unit per algorithm
+#define CFFT_EXTERN_SPLIT_PRODUCT(A)                              \
+  extern template const void* split_product_ptr<A>(int, bool);    \
+  extern template const void* split0_product_ptr<A>(int, bool);   \
+  extern template const void* split2_product_ptr<A>(int, int, bool);
+CFFT_EXTERN_SPLIT_PRODUCT(0)
+CFFT_EXTERN_SPLIT_PRODUCT(1)
+CFFT_EXTERN_SPLIT_PRODUCT(2)
+CFFT_EXTERN_SPLIT_PRODUCT(3)
+CFFT_EXTERN_SPLIT_PRODUCT(4)
+CFFT_EXTERN_SPLIT_PRODUCT(5)
+CFFT_EXTERN_SPLIT_PRODUCT(6)
+CFFT_EXTERN_SPLIT_PRODUCT(7)
+#undef CFFT_EXTERN_SPLIT_PRODUCT
+
+inline const void* u64_product_split_ptr(int algo, int ls, bool big) {
+  const void* (*const of[8])(int, bool) = {split_product_ptr<0>, split_product_ptr<1>, split_product_ptr<2>,
+                                           split_product_ptr<3>, split_product_ptr<4>, split_product_ptr<5>,
+                                           split_product_ptr<6>, split_product_ptr<7>};
+  return of[algo](ls, big);
+}
+// the kernel for plans without an outer level (sum: its Fourier-domain sum
+// variant); nullptr where S = 2^ls exceeds the radix, or a sum on a DIT base
+inline const void* u64_product_split0_ptr(int algo, int ls, bool sum) {
+  const void* (*const of[8])(int, bool) = {split0_product_ptr<0>, split0_product_ptr<1>, split0_product_ptr<2>,
+                                           split0_product_ptr<3>, split0_product_ptr<4>, split0_product_ptr<5>,
+                                           split0_product_ptr<6>, split0_product_ptr<7>};
+  return of[algo](ls, sum);
+}
+// the one-level kernel (DIF bases only; sum: its Fourier-domain sum variant);
+// nullptr where the shape is not instantiated
+inline const void* u64_product_split2_ptr(int algo, int ls0, int ls1, bool sum) {
+  const void* (*const of[8])(int, int, bool) = {split2_product_ptr<0>, split2_product_ptr<1>, split2_product_ptr<2>,
+                                                split2_product_ptr<3>, split2_product_ptr<4>, split2_product_ptr<5>,
+                                                split2_product_ptr<6>, split2_product_ptr<7>};
+  return of[algo](ls0, ls1, sum);
+}
+#endif
 
 }  // namespace cfft

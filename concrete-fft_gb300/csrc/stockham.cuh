@@ -66,7 +66,7 @@ __device__ __forceinline__ void stockham_pass(int log2n, int log2s, int nchunks,
   const int lper = log2n - LR;  // log2(n / R): butterflies per chunk
   const int total = nchunks << lper;
   const int smask = (1 << log2s) - 1;
-  if constexpr (HALF && !DIT && E == 0) {
+  if constexpr (HALF && !DIT) {
     if (nth >= 2 * total && (total & 31) == 0) {
       if (tid < 2 * total) {
         const int h = tid >= total ? 1 : 0;
@@ -132,7 +132,7 @@ __device__ __forceinline__ void end_pass(int log2n, int nchunks, B x, int tid, i
   const int log2s = log2n - LM;
   const int total = nchunks << log2s;
   const int smask = (1 << log2s) - 1;
-  if constexpr (HALF && E == 0) {
+  if constexpr (HALF) {
     if (nth >= 2 * total && (total & 31) == 0) {
       const bool act = tid < 2 * total;
       const int h = tid >= total ? 1 : 0;

@@ -33,3 +33,48 @@ def test_fp64_rates(cfft_lib):
     p = ctypes.c_double()
     cf.check(cfft_lib.cfft_diag_fp64_peak(ctypes.byref(p)))
     assert p.value > 0.9 * max(rates)
+
+
+def _edge_data(kind, batch, n):
+    """Inputs that leave the integer additions' range: each pair then takes the FP64 pipe."""
+    import numpy as np
+    rng = np.random.default_rng(n + batch)
+    x = rng.uniform(-1, 1, (batch, n)) + 1j * rng.uniform(-1, 1, (batch, n))
+    if kind == "zeros":
+        x[:] = 0
+    elif kind == "impulses":
+        x[:] = 0
+        x[np.arange(batch), np.arange(batch) % n] = 1.5 - 0.25j
+    elif kind == "constant":  # every difference cancels exactly
+        x[:] = 0.75 + 0.5j
+    elif kind == "real":
+        x.imag = 0
+    elif kind == "small_integers":  # exact halves: ties in every rounding
+        x = (rng.integers(-3, 4, (batch, n)) + 1j * rng.integers(-3, 4, (batch, n))).astype(np.complex128)
+    elif kind == "spread":  # exponents up to 1200 apart, neighbours too
+        x = x * np.exp2(rng.integers(-600, 600, (batch, n)))
+    elif kind == "near_limits":  # gaps of 8 to 13 bits around the 10 that are exact
+        x = x * np.exp2(rng.integers(8, 14, (batch, n)) * rng.integers(0, 2, (batch, n)))
+    elif kind == "subnormal":
+        x = x * 2.0 ** -1060
+    return x
+
+
+@pytest.mark.parametrize("kind", ["zeros", "impulses", "constant", "real", "small_integers", "spread", "near_limits",
+                                  "subnormal"])
+@pytest.mark.parametrize("algo", range(8))
+def test_transforms_outside_the_integer_range(cuda, oracle, algo, kind):
+    """Split (half and whole butterflies) and one-CTA kernels on inputs that the integer additions leave
+    to the FP64 pipe, bit for bit."""
+    import concrete_fft as cf
+    import numpy as np
+    torch = cuda
+    for n, batch in ((256, 1), (1024, 3), (1024, 200), (512, 700)):
+        x = _edge_data(kind, batch, n)
+        plan = cf.ordered.Plan(n, cf.ordered.Method.UserProvided(algo))
+        d = torch.from_numpy(x.copy()).cuda()
+        plan.fwd(d)
+        f = oracle.ordered_fwd(algo, x)
+        assert np.array_equal(d.cpu().numpy().view(np.uint64), f.view(np.uint64)), (n, batch, "fwd")
+        plan.inv(d)
+        assert np.array_equal(d.cpu().numpy().view(np.uint64), oracle.ordered_inv(algo, f).view(np.uint64)), (n, batch)
