@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256) u128_product_kernel(const uint64_t* __res
     const double* bp = bhat + prod * bhat_stride;
     for (int k = tid; k < n; k += nth) {
       f128 pr, pi;
-      cplx_mul(f128{s.re0[k], s.re1[k]}, f128{s.im0[k], s.im1[k]}, f128{__ldg(bp + k), __ldg(bp + n + k)},
+      cplx_mul<false>(f128{s.re0[k], s.re1[k]}, f128{s.im0[k], s.im1[k]}, f128{__ldg(bp + k), __ldg(bp + n + k)},
                f128{__ldg(bp + 2 * n + k), __ldg(bp + 3 * n + k)}, pr, pi);
       s.re0[k] = __dmul_rn(pr.hi, factor);
       s.re1[k] = __dmul_rn(pr.lo, factor);
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(256) u128_product_cluster_kernel(const uint64_
   const double* bp = bhat + prod * bhat_stride + ((long)c << lnp);
   for (int q = tid; q < np; q += nth) {
     f128 pr, pi;
-    cplx_mul(f128{B.re0[q], B.re1[q]}, f128{B.im0[q], B.im1[q]}, f128{__ldg(bp + q), __ldg(bp + n + q)},
+    cplx_mul<false>(f128{B.re0[q], B.re1[q]}, f128{B.im0[q], B.im1[q]}, f128{__ldg(bp + q), __ldg(bp + n + q)},
              f128{__ldg(bp + 2 * n + q), __ldg(bp + 3 * n + q)}, pr, pi);
     B.re0[q] = __dmul_rn(pr.hi, factor);
     B.re1[q] = __dmul_rn(pr.lo, factor);
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(256) u128_pointwise_kernel(F128Arrays z, const
     const long p = g >> log2n, k = g & (n - 1);
     const double* bp = bhat + p * bhat_stride;
     f128 pr, pi;
-    cplx_mul(f128{z.re0[g], z.re1[g]}, f128{z.im0[g], z.im1[g]}, f128{__ldg(bp + k), __ldg(bp + n + k)},
+    cplx_mul<false>(f128{z.re0[g], z.re1[g]}, f128{z.im0[g], z.im1[g]}, f128{__ldg(bp + k), __ldg(bp + n + k)},
              f128{__ldg(bp + 2 * n + k), __ldg(bp + 3 * n + k)}, pr, pi);
     z.re0[g] = __dmul_rn(pr.hi, factor);
     z.re1[g] = __dmul_rn(pr.lo, factor);

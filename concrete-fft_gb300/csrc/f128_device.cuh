@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "cfft_device.cuh"
+#include "int_f128.cuh"
 
 namespace cfft {
 
@@ -31,45 +32,156 @@ __device__ __forceinline__ void two_diff(double a, double b, double& s, double& 
   e = __dsub_rn(__dsub_rn(a, __dsub_rn(s, bb)), __dadd_rn(b, bb));
 }
 
-// src/fft128/f128_ops.rs:314-320
-__device__ __forceinline__ f128 add_est(f128 a, f128 b) {
-  double s, e;
-  two_sum(a.hi, b.hi, s, e);
-  e = __dadd_rn(e, __dadd_rn(a.lo, b.lo));
-  f128 r;
-  quick_two_sum(s, e, r.hi, r.lo);
-  return r;
+// N of these at once on the integer pipes (int_f128.cuh, the same bits), with
+// the ones outside its range redone on the FP64 pipe one by one, in a loop
+// (as sum_diff in int_fp64.cuh, and for its reason).
+template <int N, class Redo>
+__device__ __forceinline__ void redo_each(uint32_t bits, Redo redo) {
+  asm volatile("" : "+r"(bits));
+  while (bits) {
+    const int i = 31 - __clz((int)bits);
+    bits &= ~(1u << i);
+    redo(i);
+  }
 }
-// src/fft128/f128_ops.rs:360-367
-__device__ __forceinline__ f128 sub_est(f128 a, f128 b) {
-  double s, e;
-  two_diff(a.hi, b.hi, s, e);
-  e = __dadd_rn(e, a.lo);
-  e = __dsub_rn(e, b.lo);
-  f128 r;
-  quick_two_sum(s, e, r.hi, r.lo);
-  return r;
+template <int N>
+__device__ __forceinline__ double pick(const double* v, int i) {
+  double x = v[0];
+#pragma unroll
+  for (int j = 1; j < N; ++j)
+    if (i == j) x = v[j];
+  return x;
 }
-// src/fft128/f128_ops.rs:395-400 (TwoProd by FMA, src/fft128/f128_ops.rs:37-40)
-__device__ __forceinline__ f128 mul(f128 a, f128 b) {
-  const double p = __dmul_rn(a.hi, b.hi);
-  double e = __fma_rn(a.hi, b.hi, -p);
-  e = __dadd_rn(e, __dadd_rn(__dmul_rn(a.hi, b.lo), __dmul_rn(a.lo, b.hi)));
-  f128 r;
-  quick_two_sum(p, e, r.hi, r.lo);
-  return r;
+template <int N>
+__device__ __forceinline__ void put(double* v, int i, double x) {
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    if (i == j) v[j] = x;
 }
 
-// src/fft128/mod.rs:310-346 (Scalar backend: add/sub are the estimate variants)
-__device__ __forceinline__ void cplx_mul(f128 ar, f128 ai, f128 br, f128 bi, f128& orr, f128& oi) {
-  const f128 rr = mul(ar, br), ri = mul(ar, bi), ir = mul(ai, br), ii = mul(ai, bi);
-  orr = sub_est(rr, ii);
-  oi = add_est(ir, ri);
+template <int N>
+__device__ __forceinline__ void quick_two_sums(const double* s, const double* e, double* hi, double* lo) {
+  uint32_t bits = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    if (!quick_two_sum_int(s[j], e[j], hi[j], lo[j])) bits += 1u << j;
+  redo_each<N>(bits, [&](int i) {
+    double h, l;
+    quick_two_sum(pick<N>(s, i), pick<N>(e, i), h, l);
+    put<N>(hi, i, h);
+    put<N>(lo, i, l);
+  });
 }
-__device__ __forceinline__ void cplx_mul_conj(f128 ar, f128 ai, f128 br, f128 bi, f128& orr, f128& oi) {
-  const f128 rr = mul(ar, br), ri = mul(ar, bi), ir = mul(ai, br), ii = mul(ai, bi);
-  orr = add_est(rr, ii);
-  oi = sub_est(ir, ri);
+template <int N>
+__device__ __forceinline__ void two_sums(const double* a, const double* b, double* s, double* e) {
+  uint32_t bits = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    if (!two_sum_int(a[j], b[j], s[j], e[j])) bits += 1u << j;
+  redo_each<N>(bits, [&](int i) {
+    double h, l;
+    two_sum(pick<N>(a, i), pick<N>(b, i), h, l);
+    put<N>(s, i, h);
+    put<N>(e, i, l);
+  });
+}
+// s + es = a + b, d + ed = a - b
+template <int N>
+__device__ __forceinline__ void two_sum_diffs(const double* a, const double* b, double* s, double* es, double* d,
+                                              double* ed) {
+  uint32_t bits = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    if (!two_sum_diff_int(a[j], b[j], s[j], es[j], d[j], ed[j])) bits += 1u << j;
+  redo_each<N>(bits, [&](int i) {
+    const double x = pick<N>(a, i), y = pick<N>(b, i);
+    double h, l;
+    two_sum(x, y, h, l);
+    put<N>(s, i, h);
+    put<N>(es, i, l);
+    two_diff(x, y, h, l);
+    put<N>(d, i, h);
+    put<N>(ed, i, l);
+  });
+}
+
+// p[j] = w[j] * b[j], rounded to nearest
+template <int N>
+__device__ __forceinline__ void products(const double* w, const double* b, double* p) {
+  uint32_t bits = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    if (!mul_int(w[j], b[j], p[j])) bits += 1u << j;
+  redo_each<N>(bits, [&](int i) { put<N>(p, i, __dmul_rn(pick<N>(w, i), pick<N>(b, i))); });
+}
+
+// r[j] = a[j] * b[j]: src/fft128/f128_ops.rs:395-400 (TwoProd by FMA, src/fft128/f128_ops.rs:37-40)
+template <int N>
+__device__ __forceinline__ void muls(const f128* a, const f128* b, f128* r) {
+  double p[N], e[N], hi[N], lo[N], w[2 * N], v[2 * N], x[2 * N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    w[j] = b[j].lo, v[j] = a[j].hi;
+    w[N + j] = b[j].hi, v[N + j] = a[j].lo;
+    p[j] = __dmul_rn(a[j].hi, b[j].hi);
+    e[j] = __fma_rn(a[j].hi, b[j].hi, -p[j]);
+  }
+  products<2 * N>(w, v, x);
+#pragma unroll
+  for (int j = 0; j < N; ++j) e[j] = __dadd_rn(e[j], __dadd_rn(x[j], x[N + j]));
+  quick_two_sums<N>(p, e, hi, lo);
+#pragma unroll
+  for (int j = 0; j < N; ++j) r[j] = f128{hi[j], lo[j]};
+}
+
+// r[j] = a[j] + b[j] (add[j]) or a[j] - b[j] by the estimate variants,
+// src/fft128/f128_ops.rs:314-320 and :360-367.  two_diff(a, b) is two_sum(a, -b).
+template <int N>
+__device__ __forceinline__ void ests(const f128* a, const f128* b, const bool* add, f128* r) {
+  double x[N], y[N], s[N], e[N], hi[N], lo[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = a[j].hi, y[j] = add[j] ? b[j].hi : -b[j].hi;
+  two_sums<N>(x, y, s, e);
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    // e + (a.lo + b.lo) or (e + a.lo) - b.lo, by selected operands: a runtime add[j] must not
+    // make both (an FP64 instruction that is predicated off takes its time all the same)
+    const double t = __dadd_rn(add[j] ? b[j].lo : e[j], a[j].lo);
+    e[j] = __dadd_rn(t, add[j] ? e[j] : -b[j].lo);
+  }
+  quick_two_sums<N>(s, e, hi, lo);
+#pragma unroll
+  for (int j = 0; j < N; ++j) r[j] = f128{hi[j], lo[j]};
+}
+// u[j] = a[j] + b[j] and v[j] = a[j] - b[j] by the estimate variants
+template <int N>
+__device__ __forceinline__ void est_pairs(const f128* a, const f128* b, f128* u, f128* v) {
+  double x[N], y[N], s[2 * N], e[2 * N], hi[2 * N], lo[2 * N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = a[j].hi, y[j] = b[j].hi;
+  two_sum_diffs<N>(x, y, s, e, s + N, e + N);
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    e[j] = __dadd_rn(e[j], __dadd_rn(a[j].lo, b[j].lo));
+    e[N + j] = __dsub_rn(__dadd_rn(e[N + j], a[j].lo), b[j].lo);
+  }
+  quick_two_sums<2 * N>(s, e, hi, lo);
+#pragma unroll
+  for (int j = 0; j < N; ++j) u[j] = f128{hi[j], lo[j]}, v[j] = f128{hi[N + j], lo[N + j]};
+}
+
+// src/fft128/mod.rs:310-346 (Scalar backend: add/sub are the estimate variants);
+// CONJ: times the conjugate of (br, bi)
+template <bool CONJ>
+__device__ __forceinline__ void cplx_mul(f128 ar, f128 ai, f128 br, f128 bi, f128& orr, f128& oi) {
+  const f128 a[4] = {ar, ai, ai, ar}, b[4] = {br, br, bi, bi};
+  f128 m[4];  // rr, ir, ii, ri
+  muls<4>(a, b, m);
+  const bool add[2] = {CONJ, !CONJ};
+  f128 o[2];
+  ests<2>(m, m + 2, add, o);
+  orr = o[0];
+  oi = o[1];
 }
 
 // Split-array views: four f64 arrays (re0, re1, im0, im1).
@@ -92,18 +204,18 @@ __device__ __forceinline__ void f128_fwd_bfly(F128Arrays d, long j, long t, cons
   const f128 wi{__ldg(tw.im0 + widx), __ldg(tw.im1 + widx)};
   const f128 z0r{d.re0[j], d.re1[j]}, z0i{d.im0[j], d.im1[j]};
   const f128 z1r{d.re0[j + t], d.re1[j + t]}, z1i{d.im0[j + t], d.im1[j + t]};
-  f128 zr, zi;
-  cplx_mul(z1r, z1i, wr, wi, zr, zi);
-  const f128 ar = add_est(z0r, zr), ai = add_est(z0i, zi);
-  const f128 sr = sub_est(z0r, zr), si = sub_est(z0i, zi);
-  d.re0[j] = ar.hi;
-  d.re1[j] = ar.lo;
-  d.im0[j] = ai.hi;
-  d.im1[j] = ai.lo;
-  d.re0[j + t] = sr.hi;
-  d.re1[j + t] = sr.lo;
-  d.im0[j + t] = si.hi;
-  d.im1[j + t] = si.lo;
+  const f128 z0[2] = {z0r, z0i};
+  f128 z[2], u[2], v[2];
+  cplx_mul<false>(z1r, z1i, wr, wi, z[0], z[1]);
+  est_pairs<2>(z0, z, u, v);
+  d.re0[j] = u[0].hi;
+  d.re1[j] = u[0].lo;
+  d.im0[j] = u[1].hi;
+  d.im1[j] = u[1].lo;
+  d.re0[j + t] = v[0].hi;
+  d.re1[j + t] = v[0].lo;
+  d.im0[j + t] = v[1].hi;
+  d.im1[j + t] = v[1].lo;
 }
 
 // Inverse radix-2 butterfly of src/fft128/mod.rs:1131-1150.
@@ -112,14 +224,14 @@ __device__ __forceinline__ void f128_inv_bfly(F128Arrays d, long j, long t, cons
   const f128 wi{__ldg(tw.im0 + widx), __ldg(tw.im1 + widx)};
   const f128 z0r{d.re0[j], d.re1[j]}, z0i{d.im0[j], d.im1[j]};
   const f128 z1r{d.re0[j + t], d.re1[j + t]}, z1i{d.im0[j + t], d.im1[j + t]};
-  const f128 dr = sub_est(z0r, z1r), di = sub_est(z0i, z1i);
-  const f128 ar = add_est(z0r, z1r), ai = add_est(z0i, z1i);
-  f128 mr, mi;
-  cplx_mul_conj(dr, di, wr, wi, mr, mi);
-  d.re0[j] = ar.hi;
-  d.re1[j] = ar.lo;
-  d.im0[j] = ai.hi;
-  d.im1[j] = ai.lo;
+  const f128 z0[2] = {z0r, z0i}, z1[2] = {z1r, z1i};
+  f128 u[2], dd[2], mr, mi;
+  est_pairs<2>(z0, z1, u, dd);
+  cplx_mul<true>(dd[0], dd[1], wr, wi, mr, mi);
+  d.re0[j] = u[0].hi;
+  d.re1[j] = u[0].lo;
+  d.im0[j] = u[1].hi;
+  d.im1[j] = u[1].lo;
   d.re0[j + t] = mr.hi;
   d.re1[j + t] = mr.lo;
   d.im0[j + t] = mi.hi;
@@ -159,13 +271,15 @@ __device__ __forceinline__ void f128_half_stage(F128Arrays s, double* xs, int nb
       if (FWD) {
         const f128 z1r{s.re0[qb], s.re1[qb]}, z1i{s.im0[qb], s.im1[qb]};
         // real: mul(z1r, wr) - mul(z1i, wi); imaginary: mul(z1i, wr) + mul(z1r, wi)
-        const f128 z = h ? add_est(mul(z1i, wr), mul(z1r, wi)) : sub_est(mul(z1r, wr), mul(z1i, wi));
-        u = add_est(z0, z);
-        v = sub_est(z0, z);
+        const f128 a[2] = {h ? z1i : z1r, h ? z1r : z1i}, b[2] = {wr, wi};
+        f128 m[2], z;
+        muls<2>(a, b, m);
+        const bool add = h != 0;
+        ests<1>(m, m + 1, &add, &z);
+        est_pairs<1>(&z0, &z, &u, &v);
       } else {
         const f128 z1{d0[qb], d1[qb]};
-        dd = sub_est(z0, z1);  // dr (h = 0) or di (h = 1)
-        u = add_est(z0, z1);
+        est_pairs<1>(&z0, &z1, &u, &dd);  // dd: dr (h = 0) or di (h = 1)
         double* x = xs + (((b - b0) << 1) + h) * 2;
         x[0] = dd.hi;
         x[1] = dd.lo;
@@ -177,7 +291,11 @@ __device__ __forceinline__ void f128_half_stage(F128Arrays s, double* xs, int nb
         const double* x = xs + (((b - b0) << 1) + (h ^ 1)) * 2;
         const f128 od{x[0], x[1]};
         // real: mul(dr, wr) + mul(di, wi); imaginary: mul(di, wr) - mul(dr, wi)
-        v = h ? sub_est(mul(dd, wr), mul(od, wi)) : add_est(mul(dd, wr), mul(od, wi));
+        const f128 a[2] = {dd, od}, b[2] = {wr, wi};
+        f128 m[2];
+        muls<2>(a, b, m);
+        const bool add = h == 0;
+        ests<1>(m, m + 1, &add, &v);
       }
       d0[qa] = u.hi;
       d1[qa] = u.lo;

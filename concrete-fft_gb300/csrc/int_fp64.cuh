@@ -82,6 +82,33 @@ __device__ __forceinline__ bool sum_diff_int(double a, double b, double& s, doub
   return ok;
 }
 
+// w * b, rounded to nearest even, where w and b are normal and so is the
+// product (false otherwise).  The significands' 106-bit product comes from four
+// 32 x 32 multiplications on the FMA pipe, w's shifted so that the product's
+// leading one is at bit 52 or 51 of the upper 64 bits (one w serves several b).
+__device__ __forceinline__ bool mul_int(double w, double b, double& p) {
+  const uint32_t wh = (uint32_t)__double2hiint(w), wl = (uint32_t)__double2loint(w);
+  const uint32_t bh = (uint32_t)__double2hiint(b), bl = (uint32_t)__double2loint(b);
+  const uint32_t xw = wh & 0x7ff00000u, xb = bh & 0x7ff00000u;
+  const uint32_t mw = (wh & 0xfffffu) | 0x100000u, mb = (bh & 0xfffffu) | 0x100000u;
+  const uint32_t Wh = __funnelshift_l(wl, mw, 11), Wl = wl << 11;
+  const uint64_t p00 = (uint64_t)Wl * bl;
+  const uint64_t p01 = (uint64_t)Wl * mb + (p00 >> 32);
+  const uint64_t p10 = (uint64_t)Wh * bl + (uint32_t)p01;
+  const uint64_t P = (uint64_t)Wh * mb + (p01 >> 32) + (p10 >> 32);
+  const uint32_t Ph = (uint32_t)(P >> 32), Pl = (uint32_t)P, R1 = (uint32_t)p10, R0 = (uint32_t)p00;
+  // bring the leading one from bit 51 to bit 52 where it is there
+  const uint32_t c = Ph >> 20, f = c ^ 1u;
+  uint32_t ph = __funnelshift_l(Pl, Ph, f), pl = __funnelshift_l(R1, Pl, f);
+  const uint32_t u = __funnelshift_l(R0, R1, f) | min(R0, 1u) | (pl & 1u);
+  // biased exponent of the result less one (the hidden bit adds it back), in place
+  const uint32_t x = xw + xb + (c << 20) - (1023u << 20);
+  const bool ok = min(xw, xb) >= (1u << 20) && max(xw, xb) < (0x7ffu << 20) && x - (64u << 20) < (0x77eu << 20);
+  round_and_pack(ph, pl, x - (1u << 20) + ((wh ^ bh) & 0x80000000u), u);
+  p = __hiloint2double((int)ph, (int)pl);
+  return ok;
+}
+
 // N sums and differences s[j] = a[j] + b[j], d[j] = a[j] - b[j]; the pairs in
 // MASK run on the integer pipes, the others on the FP64 pipe.  Pairs outside
 // sum_diff_int's range are redone on the FP64 pipe one by one in a loop: a

@@ -116,3 +116,52 @@ def test_f128_invalid_size(cuda):
     import concrete_fft as cf
     with pytest.raises(cf.CfftError):
         cf.fft128.Plan(16)
+
+
+def _edge_arrays(kind, batch, n):
+    """Double-doubles at and outside the range of the integer error-free sums (the FP64 pipe takes the rest)."""
+    rng = np.random.default_rng(n + batch)
+    hi = rng.uniform(-1, 1, (2, batch, n))
+    lo = rng.uniform(-1, 1, (2, batch, n)) * np.spacing(np.abs(hi)) / 2
+    if kind == "zeros":
+        hi[:], lo[:] = 0, 0
+    elif kind == "impulses":
+        hi[:, :, 1:], lo[:] = 0, 0
+    elif kind == "integers":  # no low words; exact sums and ties
+        hi, lo = rng.integers(-5, 6, (2, batch, n)).astype(np.float64), np.zeros((2, batch, n))
+    elif kind == "powers":  # significands at the low end of a binade, low words of half a unit
+        hi = np.exp2(rng.integers(-3, 4, (2, batch, n)).astype(np.float64)) * rng.choice([-1.0, 1.0], (2, batch, n))
+        lo = rng.choice([-0.25, 0.25, -0.125, 0.0], (2, batch, n)) * np.spacing(np.abs(hi))
+    elif kind == "spread":
+        f = np.exp2(rng.integers(-300, 300, (2, batch, n)).astype(np.float64))
+        hi, lo = hi * f, lo * f
+    elif kind == "near_limits":  # high words 8 to 13 bits apart
+        f = np.exp2((rng.integers(8, 14, (2, batch, n)) * rng.integers(0, 2, (2, batch, n))).astype(np.float64))
+        hi, lo = hi * f, lo * f
+    elif kind == "tiny":  # low words below the normal range
+        hi, lo = hi * 2.0 ** -960, lo * 2.0 ** -960
+    return [np.ascontiguousarray(v) for v in (hi[0], lo[0], hi[1], lo[1])]
+
+
+@pytest.mark.parametrize("kind", ["random", "zeros", "impulses", "integers", "powers", "spread", "near_limits", "tiny"])
+@pytest.mark.parametrize("n,batch", [(32, 5), (64, 1), (512, 1), (512, 400), (2048, 1), (4096, 1), (4096, 200)])
+def test_f128_outside_the_integer_range(cuda, oracle, kind, n, batch):
+    """Every kernel of the double-double transforms (packed, block, cluster, global and half stages), bit for bit."""
+    import concrete_fft as cf
+    torch = cuda
+    x = _edge_arrays(kind, batch, n)
+    plan = cf.fft128.Plan(n)
+    d = [torch.from_numpy(v.copy()).cuda() for v in x]
+    check = range(batch) if batch < 8 else (0, 1, batch - 1)
+    plan.fwd(*d)
+    f = [v.cpu().numpy() for v in d]
+    for b in check:
+        want = oracle.f128_fwd(*[v[b] for v in x])
+        for k in range(4):
+            assert np.array_equal(f[k][b].view(np.uint64), np.asarray(want[k]).view(np.uint64)), ("fwd", b, k)
+    plan.inv(*d)
+    g = [v.cpu().numpy() for v in d]
+    for b in check:
+        want = oracle.f128_inv(*[v[b] for v in f])
+        for k in range(4):
+            assert np.array_equal(g[k][b].view(np.uint64), np.asarray(want[k]).view(np.uint64)), ("inv", b, k)
