@@ -23,6 +23,7 @@ namespace cfft {
 
 constexpr int kF128SmemLog2 = 12;  // 4096 points x 32 B = 128 KiB
 constexpr int kF128BlockLog2Auto = 9;
+constexpr int kF128ClassStages = 5;  // rows of at least 16 points (128 bytes) in a tile of 512
 
 // Blocks of 2^log2c points; 2^log2t consecutive blocks per CTA iteration (whole
 // transforms of fewer than 128 points are packed so that a stage's butterflies
@@ -189,45 +190,96 @@ __global__ void __launch_bounds__(256) f128_cluster_kernel(F128Arrays g, int log
   }
 }
 
-// One stage (half-size 2^log2t) over every transform of the batch, in global memory.
+// The stages of half-size 2^hi .. 2^lo over every transform of the batch, on
+// tiles in shared memory.  These stages split a transform into blocks of
+// 2^(hi+1) points and each block into its residue classes mod 2^lo, of
+// 2^(hi+1-lo) points; a tile is 2^lq neighbouring classes (a row of it is
+// contiguous in memory), 2^log2tile points in all.  One launch and one trip
+// through memory take the place of one per stage.
 template <bool FWD>
-__global__ void __launch_bounds__(256) f128_stage_kernel(F128Arrays g, int log2n, int log2t, long total, F128Tw tw) {
-  const long m = 1L << (log2n - 1 - log2t);
+__global__ void __launch_bounds__(256) f128_class_kernel(F128Arrays g, int log2n, int hi, int lo, int log2tile,
+                                                         long ntiles, F128Tw tw) {
+  extern __shared__ double sm[];
+  const int points = 1 << log2tile;
+  const F128Arrays s{sm, sm + points, sm + 2 * points, sm + 3 * points};
+  const int lp = hi + 1 - lo;      // stages, and log2 of the points of a class
+  const int lq = log2tile - lp;    // log2 of the classes in a tile
+  const int tid = threadIdx.x, nth = blockDim.x;
   grid_dependency_wait();
-  for (long b = (long)blockIdx.x * blockDim.x + threadIdx.x; b < total; b += (long)gridDim.x * blockDim.x) {
-    const long tr = b >> (log2n - 1);                 // transform index
-    const long bb = b & ((1L << (log2n - 1)) - 1);    // butterfly within transform
-    const long i = bb >> log2t;
-    const long j = (tr << log2n) + (i << (log2t + 1)) + (bb & ((1L << log2t) - 1));
-    if (FWD) f128_fwd_bfly(g, j, 1L << log2t, tw, m + i);
-    else f128_inv_bfly(g, j, 1L << log2t, tw, m + i);
+  for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const long blk = tile >> (lo - lq);  // block of 2^(hi+1) points in the batch
+    const long base = (blk << (hi + 1)) + ((tile & ((1L << (lo - lq)) - 1)) << lq);
+    const long first = blk & ((1L << (log2n - 1 - hi)) - 1);  // the block's index in its transform
+    for (int i = tid; i < points; i += nth) {
+      const long p = base + ((long)(i >> lq) << lo) + (i & ((1 << lq) - 1));
+      s.re0[i] = g.re0[p];
+      s.re1[i] = g.re1[p];
+      s.im0[i] = g.im0[p];
+      s.im1[i] = g.im1[p];
+    }
+    __syncthreads();
+    for (int st = 0; st < lp; ++st) {
+      const int l = FWD ? lp - 1 - st : st;  // half-size 2^(lo + l)
+      const long m = (1L << (log2n - 1 - lo - l)) + (first << (lp - 1 - l));
+      for (int b = tid; b < points / 2; b += nth) {
+        const int k = b >> lq;  // butterfly of a class, b's low bits the class
+        const long a = ((long)(((k >> l) << (l + 1)) + (k & ((1 << l) - 1))) << lq) + (b & ((1 << lq) - 1));
+        if (FWD) f128_fwd_bfly(s, a, 1L << (l + lq), tw, m + (k >> l));
+        else f128_inv_bfly(s, a, 1L << (l + lq), tw, m + (k >> l));
+      }
+      __syncthreads();
+    }
+    for (int i = tid; i < points; i += nth) {
+      const long p = base + ((long)(i >> lq) << lo) + (i & ((1 << lq) - 1));
+      g.re0[p] = s.re0[i];
+      g.re1[p] = s.re1[i];
+      g.im0[p] = s.im0[i];
+      g.im1[p] = s.im1[i];
+    }
+    __syncthreads();
   }
 }
 
-// Small batches: one stage over every transform of the batch in global memory with
-// two warps per 32 butterflies (real and imaginary halves, f128_half_stage), 32
-// butterflies per 64-thread CTA, so that a stage of a few thousand butterflies
-// keeps twice as many SM sub-partitions' FP64 pipes busy as one thread per
-// butterfly.  The butterflies and twiddles of f128_stage_kernel; total < 2^31
-// points in the batch.
+// Small batches: every stage of half-size 2^lo and more, one residue class mod
+// 2^lo of a transform (2^(log2n - lo) <= 256 points) per CTA in shared memory,
+// two warps per 32 butterflies (real and imaginary halves, f128_half_stage), so
+// that a few transforms keep every SM sub-partition busy.  With the block
+// kernel below, a transform is two launches (one 16384-point forward, stage by
+// stage in eight launches: 61.6 us from Python, 32.3 on the device).
 template <bool FWD>
-__global__ void __launch_bounds__(64) f128_half_stage_kernel(F128Arrays g, int log2n, int log2t, long total,
-                                                             F128Tw tw) {
-  __shared__ double xs[128];  // the inverse's differences: 4 doubles per butterfly
-  const long m = 1L << (log2n - 1 - log2t);
-  const long first = (long)blockIdx.x * 32;
-  const int nb = (int)(total - first < 32 ? total - first : 32);
+__global__ void __launch_bounds__(256) f128_class_half_kernel(F128Arrays g, int log2n, int lo, F128Tw tw) {
+  __shared__ double sm[4 * 256 + 2 * 256];
+  const int lp = log2n - lo;
+  const int np = 1 << lp;
+  const F128Arrays s{sm, sm + np, sm + 2 * np, sm + 3 * np};
+  double* xs = sm + 4 * np;
+  const int tid = threadIdx.x, nth = blockDim.x;
+  const long base = ((long)(blockIdx.x >> lo) << log2n) + (blockIdx.x & ((1 << lo) - 1));
   grid_dependency_wait();
-  f128_half_stage<FWD>(g, xs, nb, [&](int b, int& qa, int& qb, long& widx) {
-    const long gb = first + b;
-    const long tr = gb >> (log2n - 1);               // transform index
-    const long bb = gb & ((1L << (log2n - 1)) - 1);  // butterfly within transform
-    const long i = bb >> log2t;
-    const long j = (tr << log2n) + (i << (log2t + 1)) + (bb & ((1L << log2t) - 1));
-    qa = (int)j;
-    qb = (int)(j + (1L << log2t));
-    widx = m + i;
-  }, tw, threadIdx.x, 64);
+  for (int i = tid; i < np; i += nth) {
+    const long p = base + ((long)i << lo);
+    s.re0[i] = g.re0[p];
+    s.re1[i] = g.re1[p];
+    s.im0[i] = g.im0[p];
+    s.im1[i] = g.im1[p];
+  }
+  __syncthreads();
+  for (int st = 0; st < lp; ++st) {
+    const int l = FWD ? lp - 1 - st : st;
+    const long m = 1L << (lp - 1 - l);
+    f128_half_stage<FWD>(s, xs, np / 2, [&](int b, int& qa, int& qb, long& widx) {
+      qa = ((b >> l) << (l + 1)) + (b & ((1 << l) - 1));
+      qb = qa + (1 << l);
+      widx = m + (b >> l);
+    }, tw, tid, nth);
+  }
+  for (int i = tid; i < np; i += nth) {
+    const long p = base + ((long)i << lo);
+    g.re0[p] = s.re0[i];
+    g.re1[p] = s.re1[i];
+    g.im0[p] = s.im0[i];
+    g.im1[p] = s.im1[i];
+  }
 }
 
 // Small batches: the stages of one sub-block of 2^log2c points (log2c <= 8) per CTA
@@ -620,9 +672,9 @@ cfft_status run_f128_tw(size_t n, const F128Tw& tw, double* re0, double* re1, do
     }
   }
   // a small batch of larger transforms (or more transforms than the cluster rule above
-  // takes): every stage above 128- or 256-point blocks in global memory, then the
-  // blocks in shared memory, one per CTA, all with two warps per 32 butterflies
-  // (f128_half_stage_kernel, f128_smem_half_kernel), at most one block per SM
+  // takes): every stage above 128- or 256-point blocks on the residue classes mod the
+  // block size, then the blocks, one class or block per CTA, all with two warps per 32
+  // butterflies (f128_class_half_kernel, f128_smem_half_kernel), at most one block per SM
   if (!one_kernel && block_log2 == 0 && log2n >= 8 && ((long)batch << log2n) < (1L << 31)) {
     int log2c = 7;
     while (log2c < 8 && ((long)batch << (log2n - log2c)) > (long)sm_count()) ++log2c;
@@ -630,24 +682,19 @@ cfft_status run_f128_tw(size_t n, const F128Tw& tw, double* re0, double* re1, do
       F128Arrays g{re0, re1, im0, im1};
       F128Tw t = tw;
       int ln = log2n, lc = log2c;
-      long total = (long)batch << (log2n - 1);
-      const int sgrid = (int)((total + 31) / 32);
       const int bgrid = (int)((long)batch << (log2n - log2c));
-      const void* sfn = fwd ? (const void*)f128_half_stage_kernel<true> : (const void*)f128_half_stage_kernel<false>;
+      const int lp = log2n - log2c;  // stages above the blocks: 2^log2c classes of 2^lp points
+      const int cgrid = (int)((long)batch << log2c);
+      const int cthreads = std::min(256, std::max(64, 1 << lp));
+      const void* cfn = fwd ? (const void*)f128_class_half_kernel<true> : (const void*)f128_class_half_kernel<false>;
       const void* bfn = fwd ? (const void*)f128_smem_half_kernel<true> : (const void*)f128_smem_half_kernel<false>;
-      auto stage = [&](int lt) {
-        void* args[] = {&g, &ln, &lt, &total, &t};
-        return launch_kernel(sfn, sgrid, 64, args, 0, stream, true);
-      };
       void* bargs[] = {&g, &ln, &lc, &t};
-      cfft_status st = CFFT_OK;
-      if (fwd) {
-        for (int lt = log2n - 1; lt >= log2c && st == CFFT_OK; --lt) st = stage(lt);
-        if (st == CFFT_OK) st = launch_kernel(bfn, bgrid, 1 << log2c, bargs, 0, stream, true);
-      } else {
-        st = launch_kernel(bfn, bgrid, 1 << log2c, bargs, 0, stream, true);
-        for (int lt = log2c; lt <= log2n - 1 && st == CFFT_OK; ++lt) st = stage(lt);
-      }
+      auto classes = [&]() {
+        return lp == 0 ? CFFT_OK : launch_kernel(cfn, cgrid, cthreads, bargs, 0, stream, true);
+      };
+      auto blocks = [&]() { return launch_kernel(bfn, bgrid, 1 << log2c, bargs, 0, stream, true); };
+      cfft_status st = fwd ? classes() : blocks();
+      if (st == CFFT_OK) st = fwd ? blocks() : classes();
       return st;
     }
   }
@@ -673,30 +720,34 @@ cfft_status run_f128_tw(size_t n, const F128Tw& tw, double* re0, double* re1, do
   const size_t smem = (size_t)4 * (size_t(1) << (log2c + log2t)) * sizeof(double);
   const int grid = product_grid(fwd ? (const void*)f128_smem_kernel<true> : (const void*)f128_smem_kernel<false>,
                                 threads, smem, (nblocks + (1L << log2t) - 1) >> log2t);
-  const long total = (long)batch << (log2n - 1);
-  // global stages: 256-thread CTAs; a stage of fewer butterflies than one such CTA per SM
-  // takes 128-thread CTAs, so that its warps land on twice as many SM sub-partitions (a
-  // warp issues FP64 on one sub-partition, and one butterfly is ~100 dependent FP64 steps)
-  const int sthreads = total < 256L * sm_count() ? 128 : 256;
-  const int sgrid = (int)std::min<long>((total + sthreads - 1) / sthreads, (long)sm_count() * 16);
   // programmatic dependent launches: each kernel is launched as the previous one's CTAs exit
   F128Tw t = tw;
-  long tot = total, nb = nblocks;
+  long nb = nblocks;
   int ln = log2n, lc = log2c;
-  auto stage = [&](int lt) {
-    void* args[] = {&g, &ln, &lt, &tot, &t};
-    return launch_kernel(fwd ? (const void*)f128_stage_kernel<true> : (const void*)f128_stage_kernel<false>, sgrid,
-                         sthreads, args, 0, stream, true);
+  // The stages above the blocks, up to kF128ClassStages per launch on tiles of 512 points.
+  // Fewer tiles than 4 CTAs per SM take more threads each.
+  const int above = log2n - log2c;
+  const int groups = (above + kF128ClassStages - 1) / kF128ClassStages;
+  const int log2tile = kF128BlockLog2Auto;
+  long ntiles = ((long)batch << log2n) >> log2tile;
+  const int cthreads = ntiles < 2L * sm_count() ? 256 : ntiles < 4L * sm_count() ? 128 : 64;
+  const void* cfn = fwd ? (const void*)f128_class_kernel<true> : (const void*)f128_class_kernel<false>;
+  const size_t csmem = (size_t)4 * (size_t(1) << log2tile) * sizeof(double);
+  auto classes = [&](int k) {  // group k of the stages, from the largest
+    int hi = log2n - 1 - above * k / groups, lo = log2n - above * (k + 1) / groups;
+    int ltile = log2tile;
+    void* args[] = {&g, &ln, &hi, &lo, &ltile, &ntiles, &t};
+    return launch_kernel(cfn, (int)std::min<long>(ntiles, 0x7fffffffL), cthreads, args, csmem, stream, true);
   };
   void* sargs[] = {&g, &ln, &lc, &nb, &t, &log2t};
   const void* sfn = fwd ? (const void*)f128_smem_kernel<true> : (const void*)f128_smem_kernel<false>;
   cfft_status st = CFFT_OK;
   if (fwd) {
-    for (int lt = log2n - 1; lt >= log2c && st == CFFT_OK; --lt) st = stage(lt);
+    for (int k = 0; k < groups && st == CFFT_OK; ++k) st = classes(k);
     if (st == CFFT_OK) st = launch_kernel(sfn, grid, threads, sargs, smem, stream, true);
   } else {
     st = launch_kernel(sfn, grid, threads, sargs, smem, stream, true);
-    for (int lt = log2c; lt <= log2n - 1 && st == CFFT_OK; ++lt) st = stage(lt);
+    for (int k = groups - 1; k >= 0 && st == CFFT_OK; --k) st = classes(k);
   }
   return st;
 }

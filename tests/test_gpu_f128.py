@@ -165,3 +165,26 @@ def test_f128_outside_the_integer_range(cuda, oracle, kind, n, batch):
         want = oracle.f128_inv(*[v[b] for v in f])
         for k in range(4):
             assert np.array_equal(g[k][b].view(np.uint64), np.asarray(want[k]).view(np.uint64)), ("inv", b, k)
+
+
+@pytest.mark.parametrize("n,batch,block", [(4096, 3, 0), (8192, 1, 0), (16384, 2, 0), (32768, 1, 0), (16384, 13, 0),
+                                           (1024, 301, 0), (1 << 17, 2, 0), (4096, 40, 256), (1 << 16, 1, 256)])
+def test_f128_stages_on_classes(cuda, oracle, n, batch, block):
+    """Stages above the blocks on residue classes: half butterflies, tiles of 1 to 5 stages, several groups."""
+    import concrete_fft as cf
+    torch = cuda
+    x = _edge_arrays("random", batch, n)
+    plan = cf.fft128.Plan(n)
+    if block:
+        plan.set_block_points(block)
+    d = [torch.from_numpy(v.copy()).cuda() for v in x]
+    plan.fwd(*d)
+    f = [v.cpu().numpy() for v in d]
+    plan.inv(*d)
+    g = [v.cpu().numpy() for v in d]
+    for b in {0, batch - 1}:
+        wf = oracle.f128_fwd(*[v[b] for v in x])
+        wi = oracle.f128_inv(*wf)
+        for k in range(4):
+            assert np.array_equal(f[k][b].view(np.uint64), np.asarray(wf[k]).view(np.uint64)), ("fwd", b, k)
+            assert np.array_equal(g[k][b].view(np.uint64), np.asarray(wi[k]).view(np.uint64)), ("inv", b, k)
