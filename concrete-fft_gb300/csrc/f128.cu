@@ -320,24 +320,12 @@ __global__ void __launch_bounds__(256) f128_smem_half_kernel(F128Arrays g, int l
   }
 }
 
-// One u128 coefficient (lo, hi, read as i128) -> f128: hi = the nearest double, lo =
-// the nearest double to the remainder (src/fft128/mod.rs:2006-2016 pattern).
-__device__ __forceinline__ void u128_to_f128(uint64_t lo, uint64_t hi, double& xh, double& xl) {
-  xh = i128_to_f64_rne(lo, hi);
-  uint64_t tl, th;
-  double fr;
-  trunc_mod128(xh, tl, th, fr);
-  const uint64_t rl = lo - tl;
-  const uint64_t rh = hi - th - (lo < tl ? 1 : 0);
-  xl = i128_to_f64_rne(rl, rh);
-}
-
 // u128 product: the fft128 pipeline of src/fft128/mod.rs:1998-2058 fused.
 // a, out: N coefficients as (lo, hi) u64 pairs; bhat: 4 arrays of n = N/2 f64.
 __global__ void __launch_bounds__(256) u128_product_kernel(const uint64_t* __restrict__ a,
                                                           const double* __restrict__ bhat, long bhat_stride,
                                                           uint64_t* __restrict__ out, long count, int log2n,
-                                                          F128Tw tw, double factor) {
+                                                          F128Tw tw) {
   extern __shared__ double sm[];
   const int n = 1 << log2n;
   F128Arrays s{sm, sm + n, sm + 2 * n, sm + 3 * n};
@@ -363,10 +351,12 @@ __global__ void __launch_bounds__(256) u128_product_kernel(const uint64_t* __res
       f128 pr, pi;
       cplx_mul<false>(f128{s.re0[k], s.re1[k]}, f128{s.im0[k], s.im1[k]}, f128{__ldg(bp + k), __ldg(bp + n + k)},
                f128{__ldg(bp + 2 * n + k), __ldg(bp + 3 * n + k)}, pr, pi);
-      s.re0[k] = __dmul_rn(pr.hi, factor);
-      s.re1[k] = __dmul_rn(pr.lo, factor);
-      s.im0[k] = __dmul_rn(pi.hi, factor);
-      s.im1[k] = __dmul_rn(pi.lo, factor);
+      double x[4] = {pr.hi, pr.lo, pi.hi, pi.lo};
+      scale_down<4>(x, log2n);  // 2/N
+      s.re0[k] = x[0];
+      s.re1[k] = x[1];
+      s.im0[k] = x[2];
+      s.im1[k] = x[3];
     }
     __syncthreads();
     f128_stages_smem<false>(s, log2n, log2n, 0, tw, tid, nth);
@@ -393,8 +383,7 @@ __global__ void __launch_bounds__(256) u128_product_kernel(const uint64_t* __res
 template <int LS>
 __global__ void __launch_bounds__(256) u128_product_cluster_kernel(const uint64_t* __restrict__ a,
                                                                   const double* __restrict__ bhat, long bhat_stride,
-                                                                  uint64_t* __restrict__ out, int log2n, F128Tw tw,
-                                                                  double factor) {
+                                                                  uint64_t* __restrict__ out, int log2n, F128Tw tw) {
   constexpr int S = 1 << LS;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -435,10 +424,12 @@ __global__ void __launch_bounds__(256) u128_product_cluster_kernel(const uint64_
     f128 pr, pi;
     cplx_mul<false>(f128{B.re0[q], B.re1[q]}, f128{B.im0[q], B.im1[q]}, f128{__ldg(bp + q), __ldg(bp + n + q)},
              f128{__ldg(bp + 2 * n + q), __ldg(bp + 3 * n + q)}, pr, pi);
-    B.re0[q] = __dmul_rn(pr.hi, factor);
-    B.re1[q] = __dmul_rn(pr.lo, factor);
-    B.im0[q] = __dmul_rn(pi.hi, factor);
-    B.im1[q] = __dmul_rn(pi.lo, factor);
+    double x[4] = {pr.hi, pr.lo, pi.hi, pi.lo};
+    scale_down<4>(x, log2n);  // 2/N
+    B.re0[q] = x[0];
+    B.re1[q] = x[1];
+    B.im0[q] = x[2];
+    B.im1[q] = x[3];
   }
   __syncthreads();
   for (int lt = 0; lt < LS; ++lt) f128_narrow_stage<false, LS>(B, xs, log2n, c, lt, tw, tid, nth);
@@ -511,9 +502,9 @@ __global__ void __launch_bounds__(256) u128_fold_kernel(const uint64_t* __restri
   }
 }
 
-// z <- (z * bhat) * factor, the fused kernel's double-double pointwise step.
+// z <- (z * bhat) * 2/N, the fused kernel's double-double pointwise step.
 __global__ void __launch_bounds__(256) u128_pointwise_kernel(F128Arrays z, const double* __restrict__ bhat,
-                                                            long bhat_stride, long count, int log2n, double factor) {
+                                                            long bhat_stride, long count, int log2n) {
   grid_dependency_wait();
   const long n = 1L << log2n;
   const long total = count << log2n;
@@ -523,10 +514,12 @@ __global__ void __launch_bounds__(256) u128_pointwise_kernel(F128Arrays z, const
     f128 pr, pi;
     cplx_mul<false>(f128{z.re0[g], z.re1[g]}, f128{z.im0[g], z.im1[g]}, f128{__ldg(bp + k), __ldg(bp + n + k)},
              f128{__ldg(bp + 2 * n + k), __ldg(bp + 3 * n + k)}, pr, pi);
-    z.re0[g] = __dmul_rn(pr.hi, factor);
-    z.re1[g] = __dmul_rn(pr.lo, factor);
-    z.im0[g] = __dmul_rn(pi.hi, factor);
-    z.im1[g] = __dmul_rn(pi.lo, factor);
+    double x[4] = {pr.hi, pr.lo, pi.hi, pi.lo};
+    scale_down<4>(x, log2n);  // 2/N
+    z.re0[g] = x[0];
+    z.re1[g] = x[1];
+    z.im0[g] = x[2];
+    z.im1[g] = x[3];
   }
 }
 
@@ -708,8 +701,12 @@ cfft_status run_f128_tw(size_t n, const F128Tw& tw, double* re0, double* re1, do
   while (!one_kernel && log2c > 8 && ((long)batch << (log2n - log2c)) < (long)sm_count() / 2) --log2c;
   F128Arrays g{re0, re1, im0, im1};
   const long nblocks = (long)batch << (log2n - log2c);
-  // few blocks: a thread per butterfly of a stage (latency); many: fewer threads, more CTAs per SM
+  // few blocks: a thread per butterfly of a stage (latency); fewer than 9 per SM: two
+  // butterflies per thread; many: fewer threads, more CTAs per SM (512-point blocks,
+  // forward: 600 blocks 117 us on 64 threads, 103 on 128; 1000 blocks 188 and 164; 2000
+  // blocks 309 and 326)
   int threads = few ? std::min(256, 1 << (log2c - 1)) : f128_threads(log2c);
+  if (!few && nblocks < 9L * sm_count()) threads = std::min(256, std::max(threads, 1 << (log2c - 2)));
   // whole transforms of fewer than 128 points: 128 points per CTA iteration, 64 threads,
   // one butterfly per thread and stage (n = 32 alone would fill half a warp)
   int log2t = 0;
@@ -1041,48 +1038,59 @@ cfft_status cfft_u128_product(const cfft_u128_product_plan* p, const uint64_t* a
       long stride = (long)bhat_stride;
       int ln = log2n;
       F128Tw t = p->f.tw();
-      double factor = 2.0 / (double)p->N;
-      void* args[] = {(void*)&a, (void*)&bhat4, &stride, (void*)&out, &ln, &t, &factor};
+      void* args[] = {(void*)&a, (void*)&bhat4, &stride, (void*)&out, &ln, &t};
       return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),
                                    (cudaStream_t)stream);
     }
   }
-  // Above N = 8192, and for a few products of N >= 1024 (their transforms then spread
+  // From N = 4096, and for a few products of N >= 1024 (their transforms then spread
   // over many SMs instead of one CTA each): fold, forward, pointwise, inverse, round
-  // as five launches around the plan's transform.  Bit-identical to the fused kernel.
-  if (ilog2(p->f.n) > kF128SmemLog2 || (few && p->f.n >= 512)) {
+  // as five launches around the plan's transform.  Bit-identical to the fused kernel,
+  // whose CTA of 2048 points and more leaves 8 to 24 warps per SM (512 products of
+  // N = 4096: 1001 us fused, 908 as five launches; 200 of N = 8192: 1272 and 790; 1024
+  // of N = 2048: 838 and 853).  The workspace is at most 1 GiB: larger batches go
+  // through it in parts.
+  if (p->f.n >= 2048 || (few && p->f.n >= 512)) {
     cudaStream_t s = (cudaStream_t)stream;
     const int log2n = ilog2(p->f.n);
+    const size_t part = std::min(count, std::max<size_t>(1, (size_t(1) << 30) / (32 * p->f.n)));
     F128Arrays z;
-    cfft_status st = workspace_alloc(count, p->f.n, s, &z);
+    cfft_status st = workspace_alloc(part, p->f.n, s, &z);
     if (st != CFFT_OK) return st;
-    const long total = (long)count << log2n;
-    CFFT_CUDA_TRY(launch_dependent(u128_fold_kernel, elementwise_grid(2 * total), 256, 0, s, a, z, (long)count, log2n));
-    st = run_f128_tw(p->f.n, p->f.tw(), z.re0, z.re1, z.im0, z.im1, count, true, s, p->f.block_log2);
-    if (st == CFFT_OK) {
-      st = launch_dependent(u128_pointwise_kernel, elementwise_grid(total), 256, 0, s, z, bhat4, (long)bhat_stride,
-                            (long)count, log2n, 2.0 / (double)p->N) == cudaSuccess
-               ? CFFT_OK
-               : fail(CFFT_ERR_CUDA, "pointwise launch");
-    }
-    if (st == CFFT_OK)
-      st = run_f128_tw(p->f.n, p->f.tw(), z.re0, z.re1, z.im0, z.im1, count, false, s, p->f.block_log2);
-    if (st == CFFT_OK) {
-      st = launch_dependent(u128_round_kernel, elementwise_grid(2 * total), 256, 0, s, z, out, (long)count, log2n) ==
-                   cudaSuccess
-               ? CFFT_OK
-               : fail(CFFT_ERR_CUDA, "round launch");
+    for (size_t first = 0; first < count && st == CFFT_OK; first += part) {
+      const size_t c = std::min(part, count - first);
+      const long total = (long)c << log2n;
+      const uint64_t* pa = a + first * 2 * p->N;
+      uint64_t* po = out + first * 2 * p->N;
+      if (launch_dependent(u128_fold_kernel, elementwise_grid(2 * total), 256, 0, s, pa, z, (long)c, log2n) != cudaSuccess)
+        st = fail(CFFT_ERR_CUDA, "fold launch");
+      if (st == CFFT_OK)
+        st = run_f128_tw(p->f.n, p->f.tw(), z.re0, z.re1, z.im0, z.im1, c, true, s, p->f.block_log2);
+      if (st == CFFT_OK)
+        st = launch_dependent(u128_pointwise_kernel, elementwise_grid(total), 256, 0, s, z,
+                              bhat4 + first * bhat_stride, (long)bhat_stride, (long)c, log2n) == cudaSuccess
+                 ? CFFT_OK
+                 : fail(CFFT_ERR_CUDA, "pointwise launch");
+      if (st == CFFT_OK)
+        st = run_f128_tw(p->f.n, p->f.tw(), z.re0, z.re1, z.im0, z.im1, c, false, s, p->f.block_log2);
+      if (st == CFFT_OK)
+        st = launch_dependent(u128_round_kernel, elementwise_grid(2 * total), 256, 0, s, z, po, (long)c, log2n) ==
+                     cudaSuccess
+                 ? CFFT_OK
+                 : fail(CFFT_ERR_CUDA, "round launch");
     }
     cudaFreeAsync(z.re0, s);
     return st;
   }
   const int log2n = ilog2(p->f.n);
-  // few products: a thread per butterfly (latency); many: fewer threads, more CTAs per SM
-  const int threads = few ? std::min(256, 1 << (log2n - 1)) : f128_threads(log2n);
+  // a thread per butterfly of a stage, up to 256: the integer pipes need the warps, and
+  // larger CTAs leave a shorter last wave (N = 1024, 2048 products: 811 us on 64 threads,
+  // 756 on 256; 400 products: 250 and 172)
+  const int threads = std::min(256, std::max(64, 1 << (log2n - 1)));
   const size_t smem = 4 * p->f.n * sizeof(double);
   const int grid = product_grid((const void*)u128_product_kernel, threads, smem, (long)count);
   u128_product_kernel<<<grid, threads, smem, (cudaStream_t)stream>>>(
-      a, bhat4, (long)bhat_stride, out, (long)count, log2n, p->f.tw(), 2.0 / (double)p->N);
+      a, bhat4, (long)bhat_stride, out, (long)count, log2n, p->f.tw());
   CFFT_CHECK_LAUNCH();
   return CFFT_OK;
 }

@@ -367,6 +367,83 @@ __device__ __forceinline__ double i128_to_f64_rne(uint64_t lo, uint64_t hi) {
   return __longlong_as_double((long long)((neg ? 0x8000000000000000ull : 0ull) | (e << 52) | (m & 0xfffffffffffffull)));
 }
 
+// One u128 coefficient (lo, hi, read as i128) -> f128: xh = the nearest double, xl =
+// the nearest double to the remainder (src/fft128/mod.rs:2006-2016 pattern), without
+// going back from xh to an integer: the remainder is the bits that xh's rounding
+// drops, less 2^75 of its unit where it rounds up.
+__device__ __forceinline__ void u128_to_f128(uint64_t lo, uint64_t hi, double& xh, double& xl) {
+  const uint64_t neg = hi >> 63;
+  if (neg) {
+    lo = 0 - lo;
+    hi = ~hi + (lo == 0 ? 1 : 0);
+  }
+  if ((hi | lo) == 0) {
+    xh = xl = 0.0;
+    return;
+  }
+  const int lz = hi != 0 ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+  if (lz >= 64) {
+    hi = lo;
+    lo = 0;
+  }
+  const int sh = lz & 63;
+  if (sh != 0) {
+    hi = (hi << sh) | (lo >> (64 - sh));
+    lo <<= sh;
+  }
+  // leading one at bit 127: 53 bits kept, 75 dropped
+  const uint64_t top = hi >> 11;
+  const uint64_t dh = hi & 0x7ff;
+  const uint64_t half = 0x400;
+  const bool up = dh > half || (dh == half && (lo != 0 || (top & 1) != 0));
+  xh = __longlong_as_double((long long)((neg << 63) | (((uint64_t)(1023 + 126 - lz) << 52) + top + (up ? 1 : 0))));
+  // the remainder's magnitude: 76 bits (rh:rl)
+  uint64_t rh = dh, rl = lo;
+  if (up) {
+    rl = 0 - lo;
+    rh = 0x800 - dh - (lo != 0 ? 1 : 0);
+  }
+  if ((rh | rl) == 0) {
+    xl = 0.0;
+    return;
+  }
+  uint64_t th = (rh << 52) | (rl >> 12), tl = rl << 52;  // left-aligned in 128 bits
+  const int l2 = th != 0 ? __clzll((long long)th) : 64 + __clzll((long long)tl);
+  if (l2 >= 64) {
+    th = tl;
+    tl = 0;
+  }
+  const int s2 = l2 & 63;
+  if (s2 != 0) {
+    th = (th << s2) | (tl >> (64 - s2));
+    tl <<= s2;
+  }
+  const uint64_t m = th >> 11;
+  const uint64_t r = th & 0x7ff;
+  const bool up2 = r > half || (r == half && (tl != 0 || (m & 1) != 0));
+  const uint64_t sign = (neg ^ (up ? 1 : 0)) << 63;
+  xl = __longlong_as_double((long long)(sign | (((uint64_t)(1023 + 74 - l2 - lz) << 52) + m + (up2 ? 1 : 0))));
+}
+
+// x[j] *= 2^-k, 0 <= k < 64: on the exponent field, or by an FP64 product outside
+// the normal range.
+template <int N>
+__device__ __forceinline__ void scale_down(double* x, int k) {
+  uint32_t bits = 0;
+  double y[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const uint32_t h = (uint32_t)__double2hiint(x[j]);
+    if ((h & 0x7ff00000u) - (64u << 20) >= (0x7bfu << 20)) bits += 1u << j;
+    y[j] = __hiloint2double((int)(h - ((uint32_t)k << 20)), __double2loint(x[j]));
+  }
+  redo_each<N>(bits, [&](int i) {
+    put<N>(y, i, __dmul_rn(pick<N>(x, i), __hiloint2double((int)((1023u - (uint32_t)k) << 20), 0)));
+  });
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = y[j];
+}
+
 // trunc(x) as an integer mod 2^128 (lo, hi words), and x - trunc(x).
 __device__ __forceinline__ void trunc_mod128(double x, uint64_t& lo, uint64_t& hi, double& frac) {
   const double t = trunc(x);
@@ -397,8 +474,40 @@ __device__ __forceinline__ void trunc_mod128(double x, uint64_t& lo, uint64_t& h
   }
 }
 
+// m * 2^e mod 2^128, 0 <= e
+__device__ __forceinline__ void shift_left_mod128(uint64_t m, int e, uint64_t& lo, uint64_t& hi) {
+  lo = e < 64 ? m << (e & 63) : 0;
+  hi = e >= 128 ? 0 : e >= 64 ? m << (e & 63) : e == 0 ? 0 : m >> (64 - e);
+}
+
 // floor(hi + lo + 1/2) mod 2^128 for a double-double, exact.
 __device__ __forceinline__ void round_half_up_mod128(double xhi, double xlo, uint64_t& rlo, uint64_t& rhi) {
+  const uint64_t hb = (uint64_t)__double_as_longlong(xhi), lb = (uint64_t)__double_as_longlong(xlo);
+  const int he = (int)((hb >> 52) & 0x7ff) - 1075, le = (int)((lb >> 52) & 0x7ff) - 1075;
+  if (he >= 0 && he < 0x7ff - 1075 && le < 0x7ff - 1075) {
+    // the high word is an integer: itself plus floor(lo + 1/2), in integers
+    uint64_t al, ah, bl, bh;
+    shift_left_mod128((hb & 0xfffffffffffffull) | (1ull << 52), he, al, ah);
+    const uint64_t m = (lb & 0xfffffffffffffull) | (1ull << 52);
+    const uint64_t lneg = lb >> 63;
+    if (le >= 0) {
+      shift_left_mod128(m, le, bl, bh);
+    } else {
+      // |lo| < 2^53: floor(m 2^-k + 1/2), or of -m 2^-k minus floor((m + half - 1) 2^-k); 0 below 1/4
+      const int k = -le;
+      bl = k > 54 ? 0 : (m + (1ull << ((k - 1) & 63)) - lneg) >> (k & 63);
+      bh = 0;
+    }
+    // two's complement: xor with the sign, the carries below
+    const uint64_t hs = 0 - (hb >> 63), ls = 0 - lneg;
+    al = (al ^ hs) - hs;
+    ah = (ah ^ hs) + (hs & (al == 0 ? 1 : 0));
+    bl = (bl ^ ls) - ls;
+    bh = (bh ^ ls) + (ls & (bl == 0 ? 1 : 0));
+    rlo = al + bl;
+    rhi = ah + bh + (rlo < al ? 1 : 0);
+    return;
+  }
   uint64_t hl, hh, ll, lh;
   double fh, fl;
   trunc_mod128(xhi, hl, hh, fh);
