@@ -1,16 +1,20 @@
-// batch.cu -- mixed-size c64 transforms in one persistent launch.
+// batch.cu -- mixed-size c64 transforms in a few persistent launches.
 //
 // A batch is a list of transforms of different power-of-two sizes and kinds
 // (ordered n <= 1024, unordered n <= 65536) living anywhere in one device
 // buffer.  At creation the host groups the items by (kind, size, direction)
 // into work units of `tpc` same-size transforms, orders the units longest
 // first, and picks each size class's schedule (base algorithm, base size,
-// transforms per unit) by timing candidates on the device.  A run is a single
-// persistent kernel: every CTA takes the next unit from a device counter
-// (atomicAdd, no waiting on other CTAs), transforms it -- in shared memory up
-// to 2048 points, with the unordered top levels in global memory above that --
-// and takes the next, until the queue is empty.  Runs on a user stream are
-// replayed from a CUDA graph captured on the first run.
+// transforms per unit) by timing candidates on the device.  Transforms above
+// 2048 points are cut up: their outer levels into units of 4096 points of
+// butterflies in global memory, the sub-transforms below into units of 2048
+// points like the small transforms.  A run is one persistent kernel per phase
+// (forward levels, one launch each; everything that fits shared memory; inverse
+// levels): every CTA takes the next unit from a device counter (atomicAdd, no
+// waiting on other CTAs) until the queue is empty.  So a batch takes the time of
+// its work and not that of its largest transform on one CTA (300 items of 256 to
+// 65536 points, forward and inverse: 2578 us with a unit per item).  Runs on a
+// user stream are replayed from a CUDA graph captured on the first run.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -42,65 +46,54 @@ struct SizeClass {
 };
 
 struct Unit {
-  int cls;
-  int first;  // index into the sorted item-offset array
-  int count;  // transforms in this unit (<= tpc of the class)
-  int dir;    // 1 forward, 2 inverse, 3 forward then inverse
+  uint16_t cls;
+  uint8_t count;  // transforms in this unit (<= tpc of the class), or sub-transforms of one
+  uint8_t dir;    // 1 forward, 2 inverse, 3 forward then inverse
+  int first;      // index into the sorted item-offset array
+  int level;      // outer level in global memory, or -1: transforms in shared memory
+  int part;       // which part of the level, or the first sub-transform
 };
+constexpr int kLevelUnitLog2 = 12;  // points of an outer level per unit
+
+// Butterflies [part, part + 1) * 2^kLevelUnitLog2 / r of outer level l of the transform at g.
+template <bool FWD>
+__device__ void run_level(double2* g, const SizeClass& C, int l, int part, int tid, int nth) {
+  const int log2r = C.L.log2r[l], lm = C.L.log2n[l] - log2r;
+  const double2* wl = FWD ? C.w + C.L.w_off[l] : C.winv + C.L.winv_off[l];
+  const int per = 1 << (min(kLevelUnitLog2, C.log2n) - log2r);
+  for (int b = part * per + tid; b < (part + 1) * per; b += nth) {
+    double2* zc = g + ((long)(b >> lm) << C.L.log2n[l]);
+    const int i = b & ((1 << lm) - 1);
+    if (log2r == 1) outer_group<2, FWD, kAddsBatch>(zc, lm, i, wl);
+    else if (log2r == 2) outer_group<4, FWD, kAddsBatch>(zc, lm, i, wl);
+    else outer_group<8, FWD, kAddsBatch>(zc, lm, i, wl);
+  }
+}
 
 template <int ALGO>
 __device__ void run_unit(double2* __restrict__ data, const SizeClass& C, const uint64_t* __restrict__ offs,
                          const Unit& U, double2* x, double2* y, int tid, int nth) {
-  const int log2n = C.log2n;
   const int log2sub = C.L.log2n[C.d0];
   const bool fwd = U.dir & 1, inv = (U.dir & 2) != 0;
-  if (C.d0 == 0) {
-    // whole transforms in shared memory, U.count of them back to back
-    const int n = 1 << log2n;
-    for (int t = 0; t < U.count; ++t) {
-      const double2* g = data + offs[U.first + t];
-      for (int i = tid; i < n; i += nth) x[(t << log2n) + i] = g[i];
-    }
-    __syncthreads();
-    double2* r = x;
-    if (fwd) r = unordered_smem<true, kAddsBatch, ALGO>(C.L, 0, U.count, x, y, C.w, tid, nth);
-    if (inv) r = unordered_smem<false, kAddsBatch, ALGO>(C.L, 0, U.count, r, r == x ? y : x, C.winv, tid, nth);
-    for (int t = 0; t < U.count; ++t) {
-      double2* g = data + offs[U.first + t];
-      for (int i = tid; i < n; i += nth) g[i] = r[(t << log2n) + i];
-    }
-    __syncthreads();
-    return;
+  const int n = 1 << log2sub;
+  // whole transforms (d0 = 0), or consecutive sub-transforms of one, back to back
+  const long step = C.d0 == 0 ? 0 : 1;
+  for (int t = 0; t < U.count; ++t) {
+    const double2* g = data + offs[U.first + (step ? 0 : t)] + ((long)(step ? U.part + t : 0) << log2sub);
+    for (int i = tid; i < n; i += nth) x[(t << log2sub) + i] = g[i];
   }
-  // one large transform: top levels in global memory, sub-transforms in shared memory
-  double2* g = data + offs[U.first];
-  if (fwd) {
-    for (int l = 0; l < C.d0; ++l) {
-      outer_level<true, kAddsBatch>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), g, C.w + C.L.w_off[l], tid, nth);
-      __syncthreads();
-    }
+  __syncthreads();
+  double2* r = x;
+  if (fwd) r = unordered_smem<true, kAddsBatch, ALGO>(C.L, C.d0, U.count, x, y, C.w, tid, nth);
+  if (inv) r = unordered_smem<false, kAddsBatch, ALGO>(C.L, C.d0, U.count, r, r == x ? y : x, C.winv, tid, nth);
+  for (int t = 0; t < U.count; ++t) {
+    double2* g = data + offs[U.first + (step ? 0 : t)] + ((long)(step ? U.part + t : 0) << log2sub);
+    for (int i = tid; i < n; i += nth) g[i] = r[(t << log2sub) + i];
   }
-  const int nsub = 1 << (log2n - log2sub), m = 1 << log2sub;
-  for (int c = 0; c < nsub; ++c) {
-    double2* gc = g + ((long)c << log2sub);
-    for (int i = tid; i < m; i += nth) x[i] = gc[i];
-    __syncthreads();
-    double2* r = x;
-    if (fwd) r = unordered_smem<true, kAddsBatch, ALGO>(C.L, C.d0, 1, x, y, C.w, tid, nth);
-    if (inv) r = unordered_smem<false, kAddsBatch, ALGO>(C.L, C.d0, 1, r, r == x ? y : x, C.winv, tid, nth);
-    for (int i = tid; i < m; i += nth) gc[i] = r[i];
-    __syncthreads();
-  }
-  if (inv) {
-    for (int l = C.d0 - 1; l >= 0; --l) {
-      outer_level<false, kAddsBatch>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), g, C.winv + C.L.winv_off[l], tid,
-                            nth);
-      __syncthreads();
-    }
-  }
+  __syncthreads();
 }
 
-__global__ void __launch_bounds__(kBatchThreads, 2) batch_kernel(double2* __restrict__ data,
+__global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(double2* __restrict__ data,
                                                              const SizeClass* __restrict__ classes,
                                                              const uint64_t* __restrict__ offs,
                                                              const Unit* __restrict__ units, int nunits,
@@ -118,7 +111,11 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_kernel(double2* __rest
     if (u >= nunits) break;
     const Unit U = units[u];
     const SizeClass C = classes[U.cls];
-    if (C.algo == 2) run_unit<2>(data, C, offs, U, x, y, tid, nth);
+    if (U.level >= 0) {
+      double2* g = data + offs[U.first];
+      if (U.dir == 1) run_level<true>(g, C, U.level, U.part, tid, nth);
+      else run_level<false>(g, C, U.level, U.part, tid, nth);
+    } else if (C.algo == 2) run_unit<2>(data, C, offs, U, x, y, tid, nth);
     else run_unit<4>(data, C, offs, U, x, y, tid, nth);
   }
 }
@@ -179,9 +176,64 @@ SizeClass device_class(const ClassHost& c) {
   return d;
 }
 
-// Relative cost of one unit (FP64 work ~ n log n), for longest-first ordering.
-double unit_cost(int log2n, int count, int dir) {
-  return (double)count * (double)(1L << log2n) * log2n * ((dir == 3) ? 2 : 1);
+// The units of one launch of each phase of a run: forward levels 0, 1, ..., the
+// transforms in shared memory, inverse levels ..., 1, 0.
+struct Phases {
+  std::vector<Unit> units;   // of all phases, in order
+  std::vector<int> count;    // units per phase
+};
+constexpr int kMaxPhases = 2 * kMaxLevels + 1;
+
+// The units of one class in one phase, all of about the same cost (relative work of one).
+struct UnitGroup {
+  double cost;
+  std::vector<Unit> units;
+};
+using PhaseGroups = std::vector<UnitGroup>[kMaxPhases];
+
+// Adds the units of one class whose items are offs[first .. first + items).
+void add_units(const ClassHost& c, const SizeClass& d, int cls, int first, size_t items, PhaseGroups& per) {
+  const int log2sub = d.L.log2n[d.d0];
+  const double passes = c.key.dir == 3 ? 2 : 1;
+  const uint16_t cl = (uint16_t)cls;
+  const uint8_t dir = (uint8_t)c.key.dir;
+  if (d.d0 == 0) {
+    UnitGroup g{(double)c.tpc * (double)(1L << log2sub) * log2sub * passes, {}};
+    g.units.reserve(items / (size_t)c.tpc + 1);
+    for (size_t k = 0; k < items; k += (size_t)c.tpc)
+      g.units.push_back(Unit{cl, (uint8_t)std::min<size_t>(c.tpc, items - k), dir, first + (int)k, -1, 0});
+    per[kMaxLevels].push_back(std::move(g));
+    return;
+  }
+  const int nsub = 1 << (d.log2n - log2sub), group = std::min(nsub, 1 << (kBatchSmemLog2 - log2sub));
+  const int parts = 1 << std::max(0, d.log2n - kLevelUnitLog2);
+  UnitGroup g{(double)group * (double)(1L << log2sub) * log2sub * passes, {}};
+  g.units.reserve(items * (size_t)(nsub / group));
+  for (size_t k = 0; k < items; ++k)
+    for (int t = 0; t < nsub; t += group) g.units.push_back(Unit{cl, (uint8_t)group, dir, first + (int)k, -1, t});
+  per[kMaxLevels].push_back(std::move(g));
+  for (int l = 0; l < d.d0; ++l)
+    for (int way : {1, 2}) {
+      if (!(c.key.dir & way)) continue;
+      UnitGroup lg{(double)d.L.log2r[l], {}};
+      lg.units.reserve(items * (size_t)parts);
+      for (size_t k = 0; k < items; ++k)
+        for (int p = 0; p < parts; ++p) lg.units.push_back(Unit{cl, 1, (uint8_t)way, first + (int)k, l, p});
+      per[way == 1 ? l : 2 * kMaxLevels - l].push_back(std::move(lg));
+    }
+}
+
+// Longest units first in each phase.
+Phases order_units(PhaseGroups& per) {
+  Phases ph;
+  for (auto& groups : per) {
+    if (groups.empty()) continue;
+    std::stable_sort(groups.begin(), groups.end(), [](const UnitGroup& x, const UnitGroup& y) { return x.cost > y.cost; });
+    const size_t before = ph.units.size();
+    for (const UnitGroup& g : groups) ph.units.insert(ph.units.end(), g.units.begin(), g.units.end());
+    ph.count.push_back((int)(ph.units.size() - before));
+  }
+  return ph;
 }
 
 cfft_status batch_attr() {
@@ -192,11 +244,12 @@ cfft_status batch_attr() {
 
 struct cfft_batch {
   std::vector<ClassHost> classes;
-  std::vector<Unit> units;
+  size_t units = 0;
+  std::vector<int> phase;  // units of each launch
   SizeClass* d_classes = nullptr;
   uint64_t* d_offs = nullptr;
   Unit* d_units = nullptr;
-  unsigned int* d_head = nullptr;
+  unsigned int* d_head = nullptr;  // one counter per phase
   int grid = 0;
   size_t total_points = 0;
   // graph cache: one captured launch per (stream, data pointer)
@@ -210,7 +263,7 @@ struct cfft_batch {
     uint64_t lo = 0, hi = 0;  // point range [lo, hi) covered by the chunk's items
     uint64_t* d_offs = nullptr;
     Unit* d_units = nullptr;
-    int nunits = 0;
+    std::vector<int> phase;
   };
   std::vector<cfft_batch_item> items;
   std::vector<Chunk> chunks;
@@ -221,13 +274,20 @@ struct cfft_batch {
 
 namespace {
 
-cfft_status launch_batch(cfft_batch* b, double2* data, cudaStream_t s) {
-  CFFT_CUDA_TRY(cudaMemsetAsync(b->d_head, 0, sizeof(unsigned int), s));
+cfft_status launch_phases(cfft_batch* b, double2* data, const uint64_t* offs, const Unit* units,
+                          const std::vector<int>& phase, unsigned int* heads, cudaStream_t s) {
+  CFFT_CUDA_TRY(cudaMemsetAsync(heads, 0, kMaxPhases * sizeof(unsigned int), s));
   const size_t smem = 2 * (1 << kBatchSmemLog2) * sizeof(double2);
-  batch_kernel<<<b->grid, kBatchThreads, smem, s>>>(data, b->d_classes, b->d_offs, b->d_units, (int)b->units.size(),
-                                                     b->d_head);
+  for (size_t p = 0; p < phase.size(); ++p) {
+    batch_kernel<<<std::min(b->grid, phase[p]), kBatchThreads, smem, s>>>(data, b->d_classes, offs, units, phase[p],
+                                                                         heads + p);
+    units += phase[p];
+  }
   CFFT_CHECK_LAUNCH();
   return CFFT_OK;
+}
+cfft_status launch_batch(cfft_batch* b, double2* data, cudaStream_t s) {
+  return launch_phases(b, data, b->d_offs, b->d_units, b->phase, b->d_head, s);
 }
 
 void free_batch_device(cfft_batch* b) {
@@ -242,26 +302,22 @@ void free_batch_device(cfft_batch* b) {
 // Builds units and uploads class descriptors, offsets and units.
 cfft_status finalize(cfft_batch* b) {
   free_batch_device(b);
-  b->units.clear();
   std::vector<uint64_t> offs;
   std::vector<SizeClass> dcls;
-  std::vector<std::pair<double, Unit>> u;
+  PhaseGroups per;
   for (size_t ci = 0; ci < b->classes.size(); ++ci) {
     ClassHost& c = b->classes[ci];
     dcls.push_back(device_class(c));
     const int first = (int)offs.size();
     offs.insert(offs.end(), c.items.begin(), c.items.end());
-    const int tpc = dcls.back().d0 == 0 ? c.tpc : 1;
-    for (size_t k = 0; k < c.items.size(); k += (size_t)tpc) {
-      Unit un{(int)ci, first + (int)k, (int)std::min<size_t>(tpc, c.items.size() - k), c.key.dir};
-      u.push_back({unit_cost(c.key.log2n, un.count, un.dir), un});
-    }
+    add_units(c, dcls.back(), (int)ci, first, c.items.size(), per);
   }
-  std::stable_sort(u.begin(), u.end(), [](const auto& a, const auto& bb) { return a.first > bb.first; });
-  for (auto& p : u) b->units.push_back(p.second);
+  const Phases ph = order_units(per);
+  b->units = ph.units.size();
+  b->phase = ph.count;
   cfft_status st = upload(dcls.data(), dcls.size(), &b->d_classes);
   if (st == CFFT_OK) st = upload(offs.data(), offs.size(), &b->d_offs);
-  if (st == CFFT_OK) st = upload(b->units.data(), b->units.size(), &b->d_units);
+  if (st == CFFT_OK) st = upload(ph.units.data(), ph.units.size(), &b->d_units);
   return st;
 }
 
@@ -313,7 +369,7 @@ cfft_status tune_class(cfft_batch* b, size_t ci, double seconds) {
   CFFT_CUDA_TRY(cudaMalloc(&buf, count * n * sizeof(double2)));
   cfft_batch tb;
   tb.grid = b->grid;
-  CFFT_CUDA_TRY(cudaMalloc(&tb.d_head, sizeof(unsigned int)));
+  CFFT_CUDA_TRY(cudaMalloc(&tb.d_head, kMaxPhases * sizeof(unsigned int)));
   cudaStream_t s;
   CFFT_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   cudaEvent_t e0, e1;
@@ -419,29 +475,23 @@ cfft_status build_chunks(cfft_batch* b) {
       per[cls[ClassKey{(int)it.kind, (int)it.log2n, (int)it.direction}]].push_back(it.offset);
     }
     std::vector<uint64_t> offs;
-    std::vector<std::pair<double, Unit>> u;
+    PhaseGroups by_phase;
     for (size_t ci = 0; ci < per.size(); ++ci) {
       if (per[ci].empty()) continue;
-      const ClassHost& c = b->classes[ci];
       const int first = (int)offs.size();
       offs.insert(offs.end(), per[ci].begin(), per[ci].end());
-      const int tpc = device_class(c).d0 == 0 ? c.tpc : 1;
-      for (size_t k = 0; k < per[ci].size(); k += (size_t)tpc) {
-        Unit un{(int)ci, first + (int)k, (int)std::min<size_t>(tpc, per[ci].size() - k), c.key.dir};
-        u.push_back({unit_cost(c.key.log2n, un.count, un.dir), un});
-      }
+      add_units(b->classes[ci], device_class(b->classes[ci]), (int)ci, first, per[ci].size(), by_phase);
     }
-    std::stable_sort(u.begin(), u.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-    std::vector<Unit> units;
-    for (auto& pu : u) units.push_back(pu.second);
-    ch.nunits = (int)units.size();
+    const Phases ph = order_units(by_phase);
+    const std::vector<Unit>& units = ph.units;
+    ch.phase = ph.count;
     b->chunks.push_back(ch);
     cfft_status st = upload(offs.data(), offs.size(), &b->chunks.back().d_offs);
     if (st == CFFT_OK) st = upload(units.data(), units.size(), &b->chunks.back().d_units);
     if (st != CFFT_OK) return st;
     i = j;
   }
-  CFFT_CUDA_TRY(cudaMalloc(&b->d_heads, b->chunks.size() * sizeof(unsigned int)));
+  CFFT_CUDA_TRY(cudaMalloc(&b->d_heads, b->chunks.size() * kMaxPhases * sizeof(unsigned int)));
   for (cudaStream_t& st : b->pstream) CFFT_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   for (cudaEvent_t& ev : b->pevent) CFFT_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   return CFFT_OK;
@@ -475,7 +525,7 @@ cfft_status cfft_batch_create(const cfft_batch_item* items, size_t count, double
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, kBatchThreads,
                                                 2 * (1 << kBatchSmemLog2) * sizeof(double2));
   b->grid = sm_count() * std::max(per_sm, 1);
-  st = cudaMalloc(&b->d_head, sizeof(unsigned int)) == cudaSuccess ? CFFT_OK : CFFT_ERR_OUT_OF_MEMORY;
+  st = cudaMalloc(&b->d_head, kMaxPhases * sizeof(unsigned int)) == cudaSuccess ? CFFT_OK : CFFT_ERR_OUT_OF_MEMORY;
   for (auto& g : groups) {
     if (st != CFFT_OK) break;
     ClassHost c;
@@ -502,7 +552,7 @@ cfft_status cfft_batch_create(const cfft_batch_item* items, size_t count, double
 
 void cfft_batch_destroy(cfft_batch* batch) { destroy_batch(batch); }
 
-size_t cfft_batch_units(const cfft_batch* batch) { return batch ? batch->units.size() : 0; }
+size_t cfft_batch_units(const cfft_batch* batch) { return batch ? batch->units : 0; }
 
 cfft_status cfft_batch_schedule(const cfft_batch* batch, uint32_t kind, uint32_t log2n, uint32_t direction,
                                 cfft_algo* base_algo, size_t* base_n, uint32_t* per_unit) {
@@ -519,7 +569,7 @@ cfft_status cfft_batch_schedule(const cfft_batch* batch, uint32_t kind, uint32_t
 
 cfft_status cfft_batch_run(cfft_batch* b, double* data, void* stream) {
   if (!b || !data) return fail(CFFT_ERR_INVALID_ARGUMENT, "null argument");
-  if (b->units.empty()) return CFFT_OK;
+  if (b->units == 0) return CFFT_OK;
   cudaStream_t s = (cudaStream_t)stream;
   if (s == nullptr) return launch_batch(b, (double2*)data, s);  // the legacy stream cannot be captured
   std::lock_guard<std::mutex> lk(b->mu);
@@ -546,7 +596,7 @@ cfft_status cfft_batch_run(cfft_batch* b, double* data, void* stream) {
 
 cfft_status cfft_batch_run_host(cfft_batch* b, double* host, double* dev, void* stream) {
   if (!b || !host || !dev) return fail(CFFT_ERR_INVALID_ARGUMENT, "null argument");
-  if (b->units.empty()) return CFFT_OK;
+  if (b->units == 0) return CFFT_OK;
   std::lock_guard<std::mutex> lk(b->mu);
   if (b->chunks.empty()) {
     cfft_status st = build_chunks(b);
@@ -555,7 +605,6 @@ cfft_status cfft_batch_run_host(cfft_batch* b, double* host, double* dev, void* 
   cudaStream_t s = (cudaStream_t)stream;
   CFFT_CUDA_TRY(cudaEventRecord(b->pevent[3], s));
   for (cudaStream_t ps : b->pstream) CFFT_CUDA_TRY(cudaStreamWaitEvent(ps, b->pevent[3], 0));
-  const size_t smem = 2 * (1 << kBatchSmemLog2) * sizeof(double2);
   for (size_t k = 0; k < b->chunks.size(); ++k) {
     const cfft_batch::Chunk& c = b->chunks[k];
     cudaStream_t ps = b->pstream[k % 3];
@@ -563,10 +612,9 @@ cfft_status cfft_batch_run_host(cfft_batch* b, double* host, double* dev, void* 
     double* hp = host + 2 * c.lo;
     double* dp = dev + 2 * c.lo;
     CFFT_CUDA_TRY(cudaMemcpyAsync(dp, hp, bytes, cudaMemcpyHostToDevice, ps));
-    CFFT_CUDA_TRY(cudaMemsetAsync(b->d_heads + k, 0, sizeof(unsigned int), ps));
-    batch_kernel<<<b->grid, kBatchThreads, smem, ps>>>((double2*)dev, b->d_classes, c.d_offs, c.d_units, c.nunits,
-                                                        b->d_heads + k);
-    CFFT_CHECK_LAUNCH();
+    const cfft_status st =
+        launch_phases(b, (double2*)dev, c.d_offs, c.d_units, c.phase, b->d_heads + k * kMaxPhases, ps);
+    if (st != CFFT_OK) return st;
     CFFT_CUDA_TRY(cudaMemcpyAsync(hp, dp, bytes, cudaMemcpyDeviceToHost, ps));
   }
   for (int i = 0; i < 3; ++i) {

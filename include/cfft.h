@@ -480,7 +480,7 @@ cfft_status cfft_u128_product_host(const cfft_u128_product_plan* plan, const uin
                                    size_t bhat_stride, uint64_t* out, size_t count);
 
 /* ============================================ mixed-size batch (persistent) ====
- * Many c64 transforms of different sizes and kinds in one persistent kernel
+ * Many c64 transforms of different sizes and kinds in a few persistent kernels
  * launch (no counterpart in the reference, whose plans transform one buffer of
  * one size per call).  Items live anywhere in one device buffer; each is the
  * transform the matching ordered::Plan / unordered::Plan would compute, with

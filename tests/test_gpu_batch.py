@@ -110,3 +110,21 @@ def test_batch_rejects_bad_items(cuda):
         cf.batch.Batch([(0, 17, 1, 1)])
     with pytest.raises(cf.CfftError):
         cf.batch.Batch([(0, 4, 1, 0)])
+
+
+@pytest.mark.parametrize("direction", [1, 2, 3])
+@pytest.mark.parametrize("sizes", [(11, 12), (13,), (14, 14, 15), (16, 1, 10), (12, 13, 14, 15, 16, 5)])
+def test_large_items_in_parts(cuda, oracle, sizes, direction):
+    """Transforms above 2048 points as level units and sub-transform units, alone and beside small ones."""
+    import concrete_fft as cf
+    torch = cuda
+    rng = np.random.default_rng(sum(sizes) + direction)
+    items, off = [], 3
+    for k in sizes:
+        items.append((off, k, 1, direction))
+        off += (1 << k) + 5
+    data = rng.uniform(-1, 1, off) + 1j * rng.uniform(-1, 1, off)
+    b = cf.batch.Batch(items)
+    d = torch.from_numpy(data.copy()).cuda()
+    b.run(d)
+    assert np.array_equal(bits(d.cpu().numpy()), bits(expected(oracle, b, items, data)))
