@@ -85,6 +85,20 @@ constexpr int kAddsBatch = 6;
 // warp per CTA or less and stays on the FP64 pipe (126 registers against 110, slower).
 template <int R>
 constexpr int kAddsSplit = R == 16 ? 0 : 6;
+// With about one warp per SM sub-partition there is nothing to overlap, and the integer
+// additions of a butterfly of radix 8, or of the outer level of a one-level kernel, are a
+// longer chain than its FP64 ones (one N = 16384 product on Dif4/1024: 30.2 us, 27.5 with
+// the radix-8 level on the FP64 pipe; 512 points x 64 on Dit8: 13.0 and 11.0).  kAddsFew is
+// for the DIT passes; core_split chooses by the launch's kind (half butterflies: few).
+template <int R>
+constexpr int kAddsFew = R >= 8 ? 0 : 6;
+template <int R, bool FWD, int E>
+struct Core;
+template <int R, bool FWD>
+__device__ __forceinline__ void core_split(c64* v, bool few) {
+  if (few) Core<R, FWD, 0>::run(v);
+  else Core<R, FWD, kAddsSplit<R>>::run(v);
+}
 
 constexpr double kFrac1Sqrt2 = 0.70710678118654752440;
 constexpr double kH1X = 0.9238795325112867;    // cos(-pi/8)
@@ -127,9 +141,6 @@ __device__ __forceinline__ c64 mul_exp_17pi_over_16(c64 v) {
 // Radix-R DFT cores (the "last_butterfly" of each reference file).  The DIF
 // passes multiply output k by w_k afterwards, the DIT passes multiply input k
 // by w_k beforehand, the end passes use the core alone.
-template <int R, bool FWD, int E>
-struct Core;
-
 template <bool FWD, int E>
 struct Core<2, FWD, E> {  // src/dif2.rs:108-115
   __device__ __forceinline__ static void run(c64* x) { sum_diff1<E>(x[0], x[1], x[0], x[1]); }

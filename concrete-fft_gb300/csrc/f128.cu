@@ -581,6 +581,7 @@ struct cfft_f128_plan {
 
 struct cfft_u128_product_plan {
   size_t N = 0;
+  WorkspaceUser workspace;
   cfft_f128_plan f;
 };
 
@@ -755,10 +756,10 @@ int elementwise_grid(long total) {
 
 // Four arrays of count x n f64 from the stream-ordered allocator (no device
 // synchronisation; calls on different streams get different blocks).
-cfft_status workspace_alloc(size_t count, size_t n, cudaStream_t s, F128Arrays* z) {
+cfft_status workspace_alloc(const WorkspaceUser& w, size_t count, size_t n, cudaStream_t s, F128Arrays* z) {
   void* ptr = nullptr;
   const size_t per = count * n;
-  if (cudaMallocAsync(&ptr, 4 * per * sizeof(double), s) != cudaSuccess)
+  if (w.alloc(&ptr, 4 * per * sizeof(double), s) != cudaSuccess)
     return fail(CFFT_ERR_OUT_OF_MEMORY, "u128 product workspace");
   double* d = (double*)ptr;
   *z = F128Arrays{d, d + per, d + 2 * per, d + 3 * per};
@@ -986,7 +987,7 @@ cfft_status cfft_u128_prepare_operand(const cfft_u128_product_plan* p, const int
     cudaStream_t s = (cudaStream_t)stream;
     const int log2n = ilog2(p->f.n);
     F128Arrays z;
-    cfft_status st = workspace_alloc(count, p->f.n, s, &z);
+    cfft_status st = workspace_alloc(p->workspace, count, p->f.n, s, &z);
     if (st != CFFT_OK) return st;
     const long total = (long)count << log2n;
     CFFT_CUDA_TRY(launch_dependent(u128_prepare_fold_kernel, elementwise_grid(total), 256, 0, s, b, z, (long)count,
@@ -1055,7 +1056,7 @@ cfft_status cfft_u128_product(const cfft_u128_product_plan* p, const uint64_t* a
     const int log2n = ilog2(p->f.n);
     const size_t part = std::min(count, std::max<size_t>(1, (size_t(1) << 30) / (32 * p->f.n)));
     F128Arrays z;
-    cfft_status st = workspace_alloc(part, p->f.n, s, &z);
+    cfft_status st = workspace_alloc(p->workspace, part, p->f.n, s, &z);
     if (st != CFFT_OK) return st;
     for (size_t first = 0; first < count && st == CFFT_OK; first += part) {
       const size_t c = std::min(part, count - first);

@@ -31,6 +31,7 @@
 using namespace cfft;
 
 struct cfft_u64_product_plan {
+  WorkspaceUser workspace;
   size_t N = 0, n = 0, base_n = 0;
   cfft_unordered_plan* fft = nullptr;  // the plan's transform, for the unfused entry points
   int base_algo = 0;
@@ -147,7 +148,7 @@ cfft_status product_sum_unfused(const cfft_u64_product_plan* plan, const uint64_
   const size_t n = plan->n, per_group = (terms + 1) * n * sizeof(double2);
   const size_t chunk = std::min(count, std::max<size_t>(1, (size_t(1) << 30) / per_group));
   void* ws = nullptr;
-  if (cudaMallocAsync(&ws, chunk * per_group, s) != cudaSuccess)
+  if (plan->workspace.alloc((void**)&ws, chunk * per_group, s) != cudaSuccess)
     return fail(CFFT_ERR_OUT_OF_MEMORY, "product sum workspace");
   double2* z = (double2*)ws;
   double2* acc = z + chunk * terms * n;
@@ -254,41 +255,44 @@ int split0_log2(const cfft_u64_product_plan* p, bool fast = true) {
 // two threads per butterfly of a pass (half butterflies) in small launches, DIT: one; at
 // least a thread per two points for the elementwise steps (radix 16 has few butterflies per
 // pass).  Larger DIF launches take one thread per butterfly, which is how the kernel tells
-// them apart; not the sums, whose accumulator registers are sized for part / 2 threads.
-int split_product_threads(int algo, size_t part, long ctas, bool sum) {
+// them apart.
+int split_product_threads(int algo, size_t part, long ctas) {
   const size_t radix = size_t(2) << (algo / 2);
   const size_t full = part / radix;
   size_t want = std::max(((algo & 1) ? 1 : 2) * full, part / 2);
-  if (!(algo & 1) && radix < 16 && !sum && !half_butterflies(ctas, full)) want = full;
+  if (!(algo & 1) && radix < 16 && !half_butterflies(ctas, full)) want = full;
   return (int)std::min<size_t>(256, std::max<size_t>(32, want));
 }
 
+// phase kForward: `count` terms into ws; kInverse: `count` outputs of `terms` terms each
+// from ws; kWhole: `count` products.
 cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, const uint64_t* a, const double* bhat,
                                   size_t bhat_stride, uint64_t* out, size_t count, cudaStream_t stream,
-                                  const cfft_product_item* items = nullptr, int terms = 1) {
+                                  const cfft_product_item* items = nullptr, int phase = kWhole, int terms = 1,
+                                  double2* ws = nullptr) {
   const int algo = plan->base_algo;
-  const void* fn = u64_product_split0_ptr(algo, ls, terms > 1);
+  const void* fn = u64_product_split0_ptr(algo, ls, phase);
   if (!fn) return fail(CFFT_ERR_INVALID_SIZE, "no cluster product kernel for this base and cluster size");
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   const size_t part = plan->n >> ls;
-  const int threads = split_product_threads(algo, part, (long)(count << ls), terms > 1);
+  const int threads = split_product_threads(algo, part, (long)(count << ls));
   const size_t smem = 3 * part * sizeof(double2);
   const int grid = (int)(count << ls);
   DevLevels L = plan->dlv;
   long stride = (long)bhat_stride;
   const double2* bh = (const double2*)bhat;
   void* args[] = {(void*)&a, (void*)&bh, &stride, (void*)&out, &terms, (void*)&items, &L, (void*)&plan->d_w,
-                  (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw};
+                  (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw, (void*)&ws};
   // a few products: every CTA on an SM of its own
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),
-                               stream);
+                               stream, phase != kWhole);
 }
 
 // Launch shape of u64_product_split2_kernel with 2^ls1 classes: threads per CTA
 // and shared memory (three buffers of the CTA's part of the base).
-void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, bool sum, int* threads, size_t* smem) {
+void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, int* threads, size_t* smem) {
   const size_t part = p->base_n >> ls1;
-  *threads = split_product_threads(p->base_algo, part, ctas, sum);
+  *threads = split_product_threads(p->base_algo, part, ctas);
   *smem = 3 * part * sizeof(double2);
 }
 
@@ -300,24 +304,26 @@ void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, boo
 // are resident at once with one CTA per SM; else at most 8.  Not for a radix-2 base under a radix-4 level: N = 4096
 // on Dif2/512 measured slower than the five launches from 16 products (29.7
 // against 24.9 us).  false when the plan has another shape.
-bool split2_shape(const cfft_u64_product_plan* p, size_t count, int* ls0, int* ls1, bool sum = false,
+bool split2_shape(const cfft_u64_product_plan* p, size_t count, int* ls0, int* ls1, int phase = kWhole,
                   bool allow16 = true) {
   if (p->lv.nlevels != 1 || (p->base_algo & 1) || p->lv.log2r[0] > 3) return false;
   const int lr = p->base_algo / 2 + 1;
   if (lr == 1 && p->lv.log2r[0] > 1) return false;
   const int log2m = ilog2(p->base_n);
   const int l0 = p->lv.log2r[0];
-  for (int max_ls = allow16 && (count << 4) <= (size_t)sm_count() ? 4 : 3; max_ls >= 3; --max_ls) {
+  for (int max_ls = allow16 && (count << 4) <= (size_t)sm_count() * (phase == kForward ? 2 : 1) ? 4 : 3; max_ls >= 3; --max_ls) {
     int l1 = std::min(max_ls - l0, lr);
     while (l1 > 0 && (log2m - l1 < 6 || log2m - l1 - lr < 5)) --l1;
     if (l1 < 1) return false;
-    const void* fn = u64_product_split2_ptr(p->base_algo, l0, l1, sum);
+    const void* fn = u64_product_split2_ptr(p->base_algo, l0, l1, phase);
     if (!fn) continue;
     if (l0 + l1 > 3) {  // every product's 16-CTA cluster resident at once, one CTA per SM
       int threads = 0;
       size_t smem = 0;
-      split2_launch_shape(p, l1, (long)(count << (l0 + l1)), sum, &threads, &smem);
-      if ((long)count > (long)spread_clusters(fn, threads, 16)) continue;
+      split2_launch_shape(p, l1, (long)(count << (l0 + l1)), &threads, &smem);
+      // the terms of a sum may take two rounds of clusters: two outputs of 4 terms, N = 16384
+      const long rounds = phase == kForward ? 2 : 1;
+      if ((long)count > rounds * spread_clusters(fn, threads, 16)) continue;
     }
     *ls0 = l0;
     *ls1 = l1;
@@ -328,22 +334,23 @@ bool split2_shape(const cfft_u64_product_plan* p, size_t count, int* ls0, int* l
 
 cfft_status launch_split2_product(const cfft_u64_product_plan* plan, int ls0, int ls1, const uint64_t* a,
                                   const double* bhat, size_t bhat_stride, uint64_t* out, size_t count,
-                                  cudaStream_t stream, const cfft_product_item* items = nullptr, int terms = 1) {
-  const void* fn = u64_product_split2_ptr(plan->base_algo, ls0, ls1, terms > 1);
+                                  cudaStream_t stream, const cfft_product_item* items = nullptr, int phase = kWhole,
+                                  int terms = 1, double2* ws = nullptr) {
+  const void* fn = u64_product_split2_ptr(plan->base_algo, ls0, ls1, phase);
   if (!fn) return fail(CFFT_ERR_INVALID_SIZE, "no one-level cluster product kernel for this shape");
   const int ls = ls0 + ls1;
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   int threads = 0;
   size_t smem = 0;
-  split2_launch_shape(plan, ls1, (long)(count << ls), terms > 1, &threads, &smem);
+  split2_launch_shape(plan, ls1, (long)(count << ls), &threads, &smem);
   const int grid = (int)(count << ls);
   DevLevels L = plan->dlv;
   long stride = (long)bhat_stride;
   const double2* bh = (const double2*)bhat;
   void* args[] = {(void*)&a, (void*)&bh, &stride, (void*)&out, &terms, (void*)&items, &L, (void*)&plan->d_w,
-                  (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw};
+                  (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw, (void*)&ws};
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),
-                               stream);
+                               stream, phase != kWhole);
 }
 
 }  // namespace
@@ -367,7 +374,7 @@ cfft_status cfft::u64_product_split_items(const cfft_u64_product_plan* plan, con
   // At most 8 CTAs per product here: the serving loop and the work queue keep several
   // launches in flight, and a 16-CTA cluster waits for 16 free SMs of one GPC
   int ls0 = 0, ls1 = 0;
-  if (split2_shape(plan, count, &ls0, &ls1, false, false))
+  if (split2_shape(plan, count, &ls0, &ls1, kWhole, false))
     return launch_split2_product(plan, ls0, ls1, nullptr, nullptr, 0, nullptr, count, (cudaStream_t)stream, items);
   const int max_ls = std::min(3, plan->lv.log2r[0]);
   return launch_split_product(plan, max_ls, nullptr, nullptr, 0, nullptr, count, (cudaStream_t)stream, items);
@@ -423,7 +430,7 @@ cfft_status cfft_u64_fourier_mul_monomial(const cfft_u64_product_plan* plan, uns
   // product with every polynomial: the same bits as preparing X^degree and multiplying
   void* ws = nullptr;
   const size_t digit_bytes = plan->N * sizeof(int64_t);
-  if (cudaMallocAsync(&ws, digit_bytes + plan->n * sizeof(double2), s) != cudaSuccess)
+  if (plan->workspace.alloc((void**)&ws, digit_bytes + plan->n * sizeof(double2), s) != cudaSuccess)
     return fail(CFFT_ERR_OUT_OF_MEMORY, "monomial workspace");
   int64_t* digits = (int64_t*)ws;
   double* mono = (double*)((char*)ws + digit_bytes);
@@ -441,13 +448,39 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
                                  size_t terms, uint64_t* out, size_t count, void* stream) {
   if (!plan || !a || !bhat || !out) return fail(CFFT_ERR_INVALID_ARGUMENT, "null argument");
   if (terms == 0 || terms > 0x7fffffff) return fail(CFFT_ERR_INVALID_ARGUMENT, "terms must be at least 1");
-  // a few outputs of a plan with one outer level of radix 2 or 4 over a DIF base: one
-  // cluster of level-0 slices times base classes per output, as the products
-  int l0 = 0, l1 = 0;
-  if (count > 0 && (long)count < (long)sm_count() / 2 && plan->cluster == 0 &&
-      split2_shape(plan, count, &l0, &l1, terms > 1))
-    return launch_split2_product(plan, l0, l1, a, bhat, plan->n, out, count, (cudaStream_t)stream, nullptr,
-                                 (int)terms);
+  // A few outputs of a plan on a DIF base without an outer level, or with one of radix 2,
+  // 4 or 8 (the external product of a blind-rotation step): every term's forward on a
+  // cluster of its own, then every output's sum and inverse on one, in two launches
+  // around a workspace of the terms' products.  Below SMs/2 outputs and within the
+  // workspace pool; more outputs fill the SMs with one CTA or cluster each.
+  const size_t all = count * terms;
+  if (count > 0 && (long)count < (long)sm_count() / 2 && plan->cluster == 0 && !(plan->base_algo & 1) &&
+      all <= kWorkspaceKeep / (plan->n * sizeof(double2))) {
+    const int s0 = split0_log2(plan);
+    int f0 = 0, f1 = 0, i0 = 0, i1 = 0;
+    const bool level = split2_shape(plan, all, &f0, &f1, kForward) && split2_shape(plan, count, &i0, &i1, kInverse);
+    cudaStream_t s = (cudaStream_t)stream;
+    if (terms == 1 && s0 >= 1) return launch_split0_product(plan, s0, a, bhat, plan->n, out, count, s);
+    if (terms == 1 && split2_shape(plan, count, &f0, &f1))
+      return launch_split2_product(plan, f0, f1, a, bhat, plan->n, out, count, s);
+    if (terms > 1 && (s0 >= 1 || level)) {
+      void* ws = nullptr;
+      if (plan->workspace.alloc(&ws, all * plan->n * sizeof(double2), s) != cudaSuccess)
+        return fail(CFFT_ERR_OUT_OF_MEMORY, "product sum workspace");
+      const int tr = (int)terms;
+      cfft_status st =
+          s0 >= 1 ? launch_split0_product(plan, s0, a, bhat, plan->n, nullptr, all, s, nullptr, kForward, 1, (double2*)ws)
+                  : launch_split2_product(plan, f0, f1, a, bhat, plan->n, nullptr, all, s, nullptr, kForward, 1,
+                                          (double2*)ws);
+      if (st == CFFT_OK)
+        st = s0 >= 1 ? launch_split0_product(plan, s0, nullptr, nullptr, 0, out, count, s, nullptr, kInverse, tr,
+                                             (double2*)ws)
+                     : launch_split2_product(plan, i0, i1, nullptr, nullptr, 0, out, count, s, nullptr, kInverse, tr,
+                                             (double2*)ws);
+      cudaFreeAsync(ws, s);
+      return st;
+    }
+  }
   if (plan->N > (size_t(2) << kBlockLog2Auto)) {  // one output per thread-block cluster (N = 8192: by default)
     bool ok = true;
     const int ls = product_split_log2(plan, count, &ok);
@@ -460,12 +493,6 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
                                   (int)terms);
   }
   if (count == 0) return CFFT_OK;
-  // a few outputs of a plan without an outer level on a DIF base (the external
-  // product of a blind-rotation step): one cluster per output, as the products
-  const int ls0 = split0_log2(plan);
-  if (ls0 >= 1 && !(plan->base_algo & 1) && (long)count < (long)sm_count() / 2 && plan->cluster == 0 &&
-      (plan->n >> ls0) <= (size_t)kSplit0Acc * 256)
-    return launch_split0_product(plan, ls0, a, bhat, plan->n, out, count, (cudaStream_t)stream, nullptr, (int)terms);
   const bool reg_acc = plan->n <= (size_t)(kSumRegAcc * kProdThreads);
   const void* fn = u64_product_sum_kernel_ptr(plan->base_algo, reg_acc);
   const size_t smem = (reg_acc ? 2 : 3) * plan->n * sizeof(double2);
@@ -608,7 +635,7 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
   if (!ok || (plan->N >= 32768 && plan->cluster == 0) || few_unsplit || few_mid) {
     cudaStream_t s = (cudaStream_t)stream;
     void* z = nullptr;
-    if (cudaMallocAsync(&z, count * plan->n * sizeof(double2), s) != cudaSuccess)
+    if (plan->workspace.alloc((void**)&z, count * plan->n * sizeof(double2), s) != cudaSuccess)
       return fail(CFFT_ERR_OUT_OF_MEMORY, "u64 product workspace");
     cfft_status st = cfft_u64_fold_twist(plan, a, (double*)z, count, stream);
     if (st == CFFT_OK) st = cfft_unordered_fwd(plan->fft, (double*)z, count, stream);

@@ -288,6 +288,53 @@ cfft_status launch_kernel_cluster(const void* fn, int grid, int block, int clust
   return CFFT_OK;
 }
 
+namespace {
+struct DevicePool {
+  int dev;
+  cudaMemPool_t pool;
+};
+struct WorkspacePools {
+  std::mutex mu;
+  std::vector<DevicePool> pools;
+  size_t users = 0;
+};
+WorkspacePools& workspace_pools() {
+  static WorkspacePools* p = new WorkspacePools();  // outlives plans destroyed at exit
+  return *p;
+}
+}  // namespace
+
+WorkspaceUser::WorkspaceUser() {
+  WorkspacePools& w = workspace_pools();
+  std::lock_guard<std::mutex> lk(w.mu);
+  ++w.users;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  for (const DevicePool& p : w.pools)
+    if (p.dev == dev) {
+      pool = p.pool;
+      return;
+    }
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    pool = nullptr;
+    return;
+  }
+  unsigned long long keep = kWorkspaceKeep;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  w.pools.push_back({dev, pool});
+}
+WorkspaceUser::~WorkspaceUser() {
+  WorkspacePools& w = workspace_pools();
+  std::lock_guard<std::mutex> lk(w.mu);
+  if (--w.users == 0)
+    for (const DevicePool& p : w.pools) cudaMemPoolTrimTo(p.pool, 0);
+}
+
 cfft_status ensure_smem(const void* fn, size_t smem) { return ensure_smem_attr(fn, smem); }
 
 int max_blocks_per_sm(const void* fn, int block, size_t smem) {

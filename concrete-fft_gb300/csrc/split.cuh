@@ -77,10 +77,10 @@ __device__ __forceinline__ FlatBuf dit_before_last(int log2n, int ls, FlatBuf x,
   }
   const int log2c = log2n - ls;
   FlatBuf cur = x, oth = y;
-  end_dispatch<R, FWD, kAddsSplit<R>>(lm, log2c, 1, cur, tid, nth);
+  end_dispatch<R, FWD, kAddsFew<R>>(lm, log2c, 1, cur, tid, nth);
   __syncthreads();
   for (int i = npass - 1; i >= 1; --i) {
-    stockham_pass<R, FWD, true, kAddsSplit<R>>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
+    stockham_pass<R, FWD, true, kAddsFew<R>>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
     __syncthreads();
     const FlatBuf t = cur;
     cur = oth;
@@ -92,7 +92,7 @@ __device__ __forceinline__ FlatBuf dit_before_last(int log2n, int ls, FlatBuf x,
 // Forward unordered level 0 of radix R0 for butterflies [i0, i1): inputs from
 // the parts `src[j]` (part j holds slices [j*R0/S, (j+1)*R0/S)), each output
 // stored into the part that owns its slot (`dst[j]`).
-template <int R0, int LS>
+template <int R0, int LS, int E>
 __device__ __forceinline__ void level0_scatter(double2* const* src, double2* const* dst, int lm, int i0, int i1,
                                                const double2* __restrict__ wl, int tid, int nth) {
   constexpr int LR0 = Log2<R0>::v;
@@ -101,7 +101,7 @@ __device__ __forceinline__ void level0_scatter(double2* const* src, double2* con
     c64 v[R0];
 #pragma unroll
     for (int k = 0; k < R0; ++k) v[k] = ld(src[k / SL] + ((k % SL) << lm) + i);
-    Core<R0, true, kAddsSplit<R0>>::run(v);
+    Core<R0, true, E>::run(v);
     const double2* tw = wl + (R0 - 1) * i - 1;
 #pragma unroll
     for (int k = 0; k < R0; ++k) {
@@ -115,7 +115,7 @@ __device__ __forceinline__ void level0_scatter(double2* const* src, double2* con
 // Inverse unordered level 0 of radix R0 for butterflies [i0, i1): inputs from
 // the cluster's parts (part j holds slots [j*R0/S, (j+1)*R0/S) at `peer[j]`),
 // outputs to global g.
-template <int R0, int LS>
+template <int R0, int LS, int E>
 __device__ __forceinline__ void level0_last(double2* g, int lm, double2* const* peer, int i0, int i1,
                                             const double2* __restrict__ wl, int tid, int nth) {
   constexpr int LR0 = Log2<R0>::v;
@@ -128,7 +128,7 @@ __device__ __forceinline__ void level0_last(double2* g, int lm, double2* const* 
       const int sl = slot<R0>(k);
       v[k] = cmul(ldg(tw + k), ld(peer[sl >> (LR0 - LS)] + ((sl & ((R0 >> LS) - 1)) << lm) + i));
     }
-    Core<R0, false, kAddsSplit<R0>>::run(v);
+    Core<R0, false, E>::run(v);
 #pragma unroll
     for (int k = 0; k < R0; ++k) st(g + (k << lm) + i, v[k]);
   }
@@ -218,6 +218,9 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
   constexpr int LR = Log2<R>::v;
   constexpr int S = 1 << LS;
   constexpr bool LAST = MODE == 0 ? AlgoInfo<ALGO>::DIT : !FWD;
+  // the DIT algorithms have no other kernel for small batches with levels
+  constexpr bool DIT = AlgoInfo<ALGO>::DIT;
+  constexpr int kAddsLevels = DIT ? kAddsFew<R> : kAddsSplit<R>;
   extern __shared__ double2 smem[];
   grid_dependency_wait();
   const int log2n = L.log2n[0];
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(tw + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, FWD, kAddsSplit<R>>::run(v);
+      Core<R, FWD, kAddsFew<R>>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) st(g + (k << lper) + p, v[k]);
     }
@@ -295,14 +298,14 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     const double2* wl = w + L.w_off[0];
     const int per = (1 << lm) >> LS;
     if (lr0 == 1) {
-      if constexpr (LS <= 1) level0_scatter<2, LS>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 1) level0_scatter<2, LS, DIT ? kAddsFew<2> : kAddsSplit<2>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     } else if (lr0 == 2) {
-      if constexpr (LS <= 2) level0_scatter<4, LS>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 2) level0_scatter<4, LS, DIT ? kAddsFew<4> : kAddsSplit<4>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     } else {
-      level0_scatter<8, LS>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      level0_scatter<8, LS, DIT ? kAddsFew<8> : kAddsSplit<8>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     }
     cl.sync();  // every part's xs is complete, and every peer is done reading this CTA's ys
-    const FlatBuf r = unordered_t<true, kAddsSplit<AlgoInfo<ALGO>::R>, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
+    const FlatBuf r = unordered_t<true, kAddsLevels, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
     double2* gw = g + ((long)c << log2c);
     for (int j = tid; j < (1 << log2c); j += nth) gw[j] = r.p[j];
   } else {
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     __syncthreads();
     const int lr0 = L.log2r[0];
     const int lm = log2n - lr0;
-    const FlatBuf r = unordered_t<false, kAddsSplit<AlgoInfo<ALGO>::R>, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
+    const FlatBuf r = unordered_t<false, kAddsLevels, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
     double2* peer[S];
 #pragma unroll
     for (int j = 0; j < S; ++j) peer[j] = cl.map_shared_rank(r.p, (unsigned)j);
@@ -323,11 +326,11 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     const double2* wl = w + L.winv_off[0];
     const int per = (1 << lm) >> LS;
     if (lr0 == 1) {
-      if constexpr (LS <= 1) level0_last<2, LS>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 1) level0_last<2, LS, DIT ? kAddsFew<2> : kAddsSplit<2>>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
     } else if (lr0 == 2) {
-      if constexpr (LS <= 2) level0_last<4, LS>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 2) level0_last<4, LS, DIT ? kAddsFew<4> : kAddsSplit<4>>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
     } else {
-      level0_last<8, LS>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
+      level0_last<8, LS, DIT ? kAddsFew<8> : kAddsSplit<8>>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
     }
     cl.sync();
   }
@@ -376,6 +379,7 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
   const int lpp = lq - LS1;
   const int pp = 1 << lpp;
   const int cnt = m >> LS;  // level-0 butterflies per CTA
+  const bool few = nth >= 2 * pp;  // a small launch, in half butterflies
   const int i0 = c * cnt;
   double2* part[S1];
   if constexpr (FWD) {
@@ -395,7 +399,7 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
       c64 v[R0];
 #pragma unroll
       for (int k = 0; k < R0; ++k) v[k] = b == tid ? v0[k] : ld(g + (k << log2m) + i);
-      Core<R0, true, kAddsSplit<R0>>::run(v);
+      core_split<R0, true>(v, few);
       const double2* twl = wl + (R0 - 1) * i - 1;
       const int p = i & ((1 << lq) - 1);
       const int dst = ((i >> lq) << lpp) + (p & (pp - 1));
@@ -438,7 +442,7 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
 #pragma unroll
       for (int k = 1; k < R0; ++k)
         v[k] = cmul(ldg(twl + k), ld(cl.map_shared_rank(sv.p, (unsigned)((slot<R0>(k) << LS1) + cls)) + at));
-      Core<R0, false, kAddsSplit<R0>>::run(v);
+      core_split<R0, false>(v, few);
 #pragma unroll
       for (int k = 0; k < R0; ++k) st(g + (k << log2m) + i, v[k]);
     }

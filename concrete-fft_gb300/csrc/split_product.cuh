@@ -73,7 +73,6 @@ __device__ __forceinline__ void level0_inv_untwist(double2* const* src, int lm, 
 constexpr int kSplitAcc = 8;
 // The same for u64_product_split0_kernel, whose launches give at least one
 // thread per two points of a part.
-constexpr int kSplit0Acc = 2;
 
 // One output per cluster of S CTAs (blockIdx.x >> LS): the sum over `terms`
 // products a_t * B_t, accumulated in the Fourier domain in term order, then
@@ -131,11 +130,11 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
     // 2. level 0 forward: 1/S of the butterflies, each output into its owner's x
     const double2* wl = w + L.w_off[0];
     if (lr0 == 1) {
-      if constexpr (LS <= 1) level0_scatter<2, LS>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 1) level0_scatter<2, LS, kAddsSplit<2>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     } else if (lr0 == 2) {
-      if constexpr (LS <= 2) level0_scatter<4, LS>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 2) level0_scatter<4, LS, kAddsSplit<4>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     } else {
-      level0_scatter<8, LS>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      level0_scatter<8, LS, kAddsSplit<8>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     }
     cl.sync();  // every part's x is complete and every peer has read this CTA's y
 
@@ -204,24 +203,31 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
 // class c: the pointwise product is applied as they are stored into z.  Every
 // inverse pass but the last is local; the last reads every part and its
 // outputs are untwisted, rounded and stored.
-// SUM (DIF bases): one output is the Fourier-domain sum of `terms` products:
-// each term runs the forward steps and is multiplied and added into a register
-// accumulator in term order, as in u64_product_sum_kernel, then one inverse.
+// PHASE (DIF bases): a Fourier-domain sum of products is two launches.  Forward
+// (kForward): every term runs the forward steps on a cluster of its own and
+// stores its pointwise product into ws, in the operand's order.  Inverse
+// (kInverse): the cluster of an output adds its `terms` products in term order,
+// as u64_product_sum_kernel does, and runs the inverse steps once.  The terms
+// thus take the time of one (2 outputs of 4 terms, N = 2048 on Dif4: 28.6 us
+// with the terms one after another on the output's cluster).
 // Every butterfly and elementwise step does the operations of the one-CTA
 // product kernel on the same values, so results are bit-identical to it.
 // Shared memory: three buffers of n/S points.  Requires L.nlevels == 0,
-// S <= R, n >= R*S and, for SUM, n/S <= kSplit0Acc x blockDim.x.
-template <int ALGO, int LS, bool SUM>
+// S <= R and n >= R*S.
+enum ProductPhase { kWhole = 0, kForward = 1, kInverse = 2 };
+template <int ALGO, int LS, int PHASE>
 __global__ void __launch_bounds__(256) u64_product_split0_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
     int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
-    const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw) {
+    const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw,
+    double2* __restrict__ ws) {
   constexpr int R = AlgoInfo<ALGO>::R;
   constexpr int LR = Log2<R>::v;
   constexpr int S = 1 << LS;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ double2 smem[];
+  if constexpr (PHASE != kWhole) grid_dependency_wait();
   const int log2n = L.log2n[0];
   const int log2c = log2n - LS;
   const int n = 1 << log2n;
@@ -248,25 +254,14 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       peer_x[j] = cl.map_shared_rank(x, (unsigned)j);
       peer_z[j] = cl.map_shared_rank(z, (unsigned)j);
     }
-    // SUM: a sum of `terms` products (terms of an output consecutive in a and bhat,
-    // bhat at stride bhat_stride): each term forward and multiplied, added into
-    // registers in term order, one inverse.  Otherwise one product (terms = 1).
-    c64 acc[SUM ? kSplit0Acc : 1];
-    const double2* src = x;  // input of the inverse's first pass
-    const int nterms = SUM ? terms : 1;
-#pragma unroll 1
-    for (int t = 0; t < nterms; ++t) {
-      const long term = g * nterms + t;
-      const uint64_t* tap = SUM ? a + (term << (log2n + 1)) : ap;
-      const double2* tbp = SUM ? bhat + term * bhat_stride : bp;
-      // every CTA runs, and is done with its x from the previous term, before a peer
-      // writes its x
-      auto token = cl.barrier_arrive();
-      if (t > 0) __syncthreads();  // this CTA is done with y
+    // every CTA runs before a peer's memory is written
+    auto token = cl.barrier_arrive();
+    const double2* src = y;  // input of the inverse's first pass
+    if constexpr (PHASE != kInverse) {
       // input k of first-pass butterfly c*per + b, folded and twisted, at y[k*per + b]
       for (int q = tid; q < (R << lpc); q += nth) {
         const int j = ((q >> lpc) << lper) + c * per + (q & (per - 1));
-        const c64 v{i64_to_f64_rne((int64_t)__ldcs(tap + j)), i64_to_f64_rne((int64_t)__ldcs(tap + j + n))};
+        const c64 v{i64_to_f64_rne((int64_t)__ldcs(ap + j)), i64_to_f64_rne((int64_t)__ldcs(ap + j + n))};
         st(y + q, cmul(ldg(tw + j), v));
       }
       __syncthreads();
@@ -275,28 +270,21 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
                                       peer_x, wf, tid, nth);
       cl.sync();  // every part's x is complete
       const FlatBuf r = dif_after_first<R, true>(log2n, LS, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
-      if constexpr (!SUM) {
-        for (int j = tid; j < (1 << log2c); j += nth) st(r.p + j, cmul(ldg(tbp + (j << LS) + c), ld(r.p + j)));
-        src = r.p;
-      } else {
-#pragma unroll
-        for (int k = 0; k < kSplit0Acc; ++k) {
-          const int j = tid + k * nth;
-          if (j < (1 << log2c)) {
-            const c64 p = cmul(ldg(tbp + (j << LS) + c), ld(r.p + j));
-            acc[k] = t == 0 ? p : cadd(acc[k], p);
-          }
-        }
+      if constexpr (PHASE == kForward) {
+        double2* o = ws + (g << log2n) + c;
+        for (int j = tid; j < (1 << log2c); j += nth) st(o + (j << LS), cmul(ldg(bp + (j << LS) + c), ld(r.p + j)));
+        return;  // no peer touches this CTA's memory after the last barrier
       }
-    }
-    if constexpr (SUM) {
-      __syncthreads();  // every read of the last term's buffers is done
-#pragma unroll
-      for (int k = 0; k < kSplit0Acc; ++k) {
-        const int j = tid + k * nth;
-        if (j < (1 << log2c)) st(y + j, acc[k]);
+      for (int j = tid; j < (1 << log2c); j += nth) st(r.p + j, cmul(ldg(bp + (j << LS) + c), ld(r.p + j)));
+      src = r.p;
+    } else {
+      const double2* p = ws + ((g * terms) << log2n) + c;
+      for (int j = tid; j < (1 << log2c); j += nth) {
+        c64 acc = ld(p + (j << LS));
+        for (int t = 1; t < terms; ++t) acc = cadd(acc, ld(p + ((long)t << log2n) + (j << LS)));
+        st(y + j, acc);
       }
-      src = y;
+      cl.barrier_wait(std::move(token));
     }
     __syncthreads();
     first_pass_scatter<R, false, LS>([&](int k, int b, int) { return ld(src + (k << lpc) + b); }, per, c, S, peer_z,
@@ -331,7 +319,7 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(twp + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, true, kAddsSplit<R>>::run(v);
+      Core<R, true, kAddsFew<R>>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) st(z + (k << lpc) + b, cmul(ldg(bp + (k << lper) + p), v[k]));
     }
@@ -348,7 +336,7 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(twp + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, false, kAddsSplit<R>>::run(v);
+      Core<R, false, kAddsFew<R>>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         const int jg = (k << lper) + p;
@@ -386,16 +374,15 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
 //      cluster barrier keeps every CTA alive while a peer reads its memory.
 // Every butterfly and elementwise step does the operations of the one-CTA
 // product kernel on the same values, so results are bit-identical to it.
-// SUM: one output is the Fourier-domain sum of `terms` products (steps 1-3 per
-// term, added into a register accumulator in term order, then one inverse).
-// Shared memory: three buffers of m/S1 points.  Requires L.nlevels == 1,
-// 2^L.log2r[0] == R0, S1 <= the base radix R, m >= R*S1 and, for SUM,
-// m/S1 <= kSplit0Acc x blockDim.x.
-template <int ALGO, int LS0, int LS1, bool SUM>
+// PHASE: a Fourier-domain sum as two launches, steps 1-3 per term and the rest
+// per output, as u64_product_split0_kernel.  Requires L.nlevels == 1,
+// 2^L.log2r[0] == R0, S1 <= the base radix R and m >= R*S1.
+template <int ALGO, int LS0, int LS1, int PHASE>
 __global__ void __launch_bounds__(256) u64_product_split2_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
     int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
-    const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw) {
+    const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw,
+    double2* __restrict__ ws) {
   constexpr int R = AlgoInfo<ALGO>::R;
   constexpr int LR = Log2<R>::v;
   constexpr int R0 = 1 << LS0;
@@ -406,6 +393,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ double2 smem[];
+  if constexpr (PHASE != kWhole) grid_dependency_wait();
   const int log2n = L.log2n[0];
   const int log2m = L.log2n[1];
   const int n = 1 << log2n, m = 1 << log2m;
@@ -435,28 +423,18 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
     peer_z[j] = cl.map_shared_rank(z, (unsigned)((s0 << LS1) + j));
   }
   const int cnt = m >> LS;
+  const bool few = nth >= 2 * pp;  // a small launch, in half butterflies
   const int i0 = c * cnt;
-  // SUM: a sum of `terms` products (terms of an output consecutive in a and bhat,
-  // bhat at stride bhat_stride), steps 1-3 per term, each product added into a
-  // register accumulator in term order, one inverse.  Otherwise one product.
-  c64 acc[SUM ? kSplit0Acc : 1];
-  const double2* src = nullptr;  // input of the inverse's first pass
-  const int nterms = SUM ? terms : 1;
-#pragma unroll 1
-  for (int t = 0; t < nterms; ++t) {
-  const long term = g * nterms + t;
-  const uint64_t* tap = SUM ? a + (term << (log2n + 1)) : ap;
-  const double2* tbp = SUM ? bhat + term * bhat_stride : bp;
-  // every CTA runs, and is done with its buffers of the previous term, before a
-  // peer writes them
+  // every CTA runs before a peer's memory is written
   auto token = cl.barrier_arrive();
-
+  const double2* src = y;  // input of the inverse's first pass
+  if constexpr (PHASE != kInverse) {
   // 1. level 0 forward on butterflies [c*m/S, (c+1)*m/S)
   auto load_l0 = [&](int i, c64* v) {
 #pragma unroll
     for (int k = 0; k < R0; ++k) {
       const int j = (k << log2m) + i;
-      const c64 u{i64_to_f64_rne((int64_t)__ldcs(tap + j)), i64_to_f64_rne((int64_t)__ldcs(tap + j + n))};
+      const c64 u{i64_to_f64_rne((int64_t)__ldcs(ap + j)), i64_to_f64_rne((int64_t)__ldcs(ap + j + n))};
       v[k] = cmul(ldg(tw + j), u);
     }
   };
@@ -472,7 +450,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
     } else {
       load_l0(i, v);
     }
-    Core<R0, true, kAddsSplit<R0>>::run(v);
+    core_split<R0, true>(v, few);
     const double2* twl = wl + (R0 - 1) * i - 1;
     const int p = i & ((1 << lq) - 1);
     const int dst = (((i >> lq) << lpp) + (p & (pp - 1)));
@@ -492,29 +470,22 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
 
   // 3. the later passes, the pointwise product, the inverse's first pass
   const FlatBuf r = dif_after_first<R, true>(log2m, LS1, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
-  const double2* bs = tbp + ((long)s0 << log2m) + c1;
-  if constexpr (!SUM) {
-    for (int j = tid; j < (1 << log2c); j += nth) st(r.p + j, cmul(ldg(bs + (j << LS1)), ld(r.p + j)));
-    src = r.p;
+  const double2* bs = bp + ((long)s0 << log2m) + c1;
+  if constexpr (PHASE == kForward) {
+    double2* o = ws + (g << log2n) + ((long)s0 << log2m) + c1;
+    for (int j = tid; j < (1 << log2c); j += nth) st(o + (j << LS1), cmul(ldg(bs + (j << LS1)), ld(r.p + j)));
+    return;  // no peer touches this CTA's memory after the last barrier
+  }
+  for (int j = tid; j < (1 << log2c); j += nth) st(r.p + j, cmul(ldg(bs + (j << LS1)), ld(r.p + j)));
+  src = r.p;
   } else {
-#pragma unroll
-    for (int k = 0; k < kSplit0Acc; ++k) {
-      const int j = tid + k * nth;
-      if (j < (1 << log2c)) {
-        const c64 p = cmul(ldg(bs + (j << LS1)), ld(r.p + j));
-        acc[k] = t == 0 ? p : cadd(acc[k], p);
-      }
+    const double2* p = ws + ((g * terms) << log2n) + ((long)s0 << log2m) + c1;
+    for (int j = tid; j < (1 << log2c); j += nth) {
+      c64 acc = ld(p + (j << LS1));
+      for (int t = 1; t < terms; ++t) acc = cadd(acc, ld(p + ((long)t << log2n) + (j << LS1)));
+      st(y + j, acc);
     }
-  }
-  }
-  if constexpr (SUM) {
-    __syncthreads();  // every read of the last term's buffers is done
-#pragma unroll
-    for (int k = 0; k < kSplit0Acc; ++k) {
-      const int j = tid + k * nth;
-      if (j < (1 << log2c)) st(y + j, acc[k]);
-    }
-    src = y;
+    cl.barrier_wait(std::move(token));
   }
   __syncthreads();
   first_pass_scatter<R, false, LS1>([&](int k, int b, int) { return ld(src + (k << lpp) + b); }, pp, c1, S1, peer_z,
@@ -536,7 +507,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
 #pragma unroll
     for (int k = 1; k < R0; ++k)
       v[k] = cmul(ldg(twl + k), ld(cl.map_shared_rank(sv.p, (unsigned)((slot<R0>(k) << LS1) + cls)) + at));
-    Core<R0, false, kAddsSplit<R0>>::run(v);
+    core_split<R0, false>(v, few);
 #pragma unroll
     for (int k = 0; k < R0; ++k) {
       const int j = (k << log2m) + i;
@@ -567,53 +538,54 @@ const void* split_product_ptr(int ls, bool big) {
   }
 }
 
-template <int A, bool SUM>
+template <int A, int PHASE>
 const void* split0_product_ptr_t(int ls) {
   constexpr int LRA = Log2<AlgoInfo<A>::R>::v;
   switch (ls) {
-    case 1: return (const void*)u64_product_split0_kernel<A, 1, SUM>;
-    case 2: if constexpr (LRA >= 2) return (const void*)u64_product_split0_kernel<A, 2, SUM>; else return nullptr;
-    case 3: if constexpr (LRA >= 3) return (const void*)u64_product_split0_kernel<A, 3, SUM>; else return nullptr;
+    case 1: return (const void*)u64_product_split0_kernel<A, 1, PHASE>;
+    case 2: if constexpr (LRA >= 2) return (const void*)u64_product_split0_kernel<A, 2, PHASE>; else return nullptr;
+    case 3: if constexpr (LRA >= 3) return (const void*)u64_product_split0_kernel<A, 3, PHASE>; else return nullptr;
     default: return nullptr;
   }
 }
-// sum: the Fourier-domain sum variant (DIF bases only)
+// phase: kWhole, or a phase of a sum (DIF bases only)
 template <int A>
-const void* split0_product_ptr(int ls, bool sum) {
-  if (!sum) return split0_product_ptr_t<A, false>(ls);
+const void* split0_product_ptr(int ls, int phase) {
+  if (phase == kWhole) return split0_product_ptr_t<A, kWhole>(ls);
   if constexpr (AlgoInfo<A>::DIT) return nullptr;
-  else return split0_product_ptr_t<A, true>(ls);
+  else return phase == kForward ? split0_product_ptr_t<A, kForward>(ls) : split0_product_ptr_t<A, kInverse>(ls);
 }
 
 // (R0, S1) = (2, 2), (2, 4), (4, 2) for DIF bases with S1 <= R
-template <int A, bool SUM>
+template <int A, int PHASE>
 const void* split2_product_ptr_t(int ls0, int ls1) {
   if constexpr (AlgoInfo<A>::DIT) {
     return nullptr;
   } else {
     constexpr int LRA = Log2<AlgoInfo<A>::R>::v;
-    if (ls0 == 1 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 1, 1, SUM>;
-    if (ls0 == 2 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 2, 1, SUM>;
+    if (ls0 == 1 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 1, 1, PHASE>;
+    if (ls0 == 2 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 2, 1, PHASE>;
     if constexpr (LRA >= 2) {
-      if (ls0 == 1 && ls1 == 2) return (const void*)u64_product_split2_kernel<A, 1, 2, SUM>;
+      if (ls0 == 1 && ls1 == 2) return (const void*)u64_product_split2_kernel<A, 1, 2, PHASE>;
       // 16-CTA clusters
-      if (ls0 == 2 && ls1 == 2) return (const void*)u64_product_split2_kernel<A, 2, 2, SUM>;
-      if (ls0 == 3 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 3, 1, SUM>;
+      if (ls0 == 2 && ls1 == 2) return (const void*)u64_product_split2_kernel<A, 2, 2, PHASE>;
+      if (ls0 == 3 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 3, 1, PHASE>;
     }
     return nullptr;
   }
 }
-// sum: the Fourier-domain sum variant
 template <int A>
-const void* split2_product_ptr(int ls0, int ls1, bool sum) {
-  return sum ? split2_product_ptr_t<A, true>(ls0, ls1) : split2_product_ptr_t<A, false>(ls0, ls1);
+const void* split2_product_ptr(int ls0, int ls1, int phase) {
+  return phase == kWhole     ? split2_product_ptr_t<A, kWhole>(ls0, ls1)
+         : phase == kForward ? split2_product_ptr_t<A, kForward>(ls0, ls1)
+                             : split2_product_ptr_t<A, kInverse>(ls0, ls1);
 }
 
 #ifndef CFFT_KERNEL_INSTANCE  // instantiated in kinst_split_prod_<A>.cu, one unit per algorithm
 #define CFFT_EXTERN_SPLIT_PRODUCT(A)                              \
   extern template const void* split_product_ptr<A>(int, bool);    \
-  extern template const void* split0_product_ptr<A>(int, bool);   \
-  extern template const void* split2_product_ptr<A>(int, int, bool);
+  extern template const void* split0_product_ptr<A>(int, int);    \
+  extern template const void* split2_product_ptr<A>(int, int, int);
 CFFT_EXTERN_SPLIT_PRODUCT(0)
 CFFT_EXTERN_SPLIT_PRODUCT(1)
 CFFT_EXTERN_SPLIT_PRODUCT(2)
@@ -630,21 +602,20 @@ inline const void* u64_product_split_ptr(int algo, int ls, bool big) {
                                            split_product_ptr<6>, split_product_ptr<7>};
   return of[algo](ls, big);
 }
-// the kernel for plans without an outer level (sum: its Fourier-domain sum
-// variant); nullptr where S = 2^ls exceeds the radix, or a sum on a DIT base
-inline const void* u64_product_split0_ptr(int algo, int ls, bool sum) {
-  const void* (*const of[8])(int, bool) = {split0_product_ptr<0>, split0_product_ptr<1>, split0_product_ptr<2>,
-                                           split0_product_ptr<3>, split0_product_ptr<4>, split0_product_ptr<5>,
-                                           split0_product_ptr<6>, split0_product_ptr<7>};
-  return of[algo](ls, sum);
+// the kernel for plans without an outer level; nullptr where S = 2^ls exceeds the
+// radix, or a phase of a sum on a DIT base
+inline const void* u64_product_split0_ptr(int algo, int ls, int phase) {
+  const void* (*const of[8])(int, int) = {split0_product_ptr<0>, split0_product_ptr<1>, split0_product_ptr<2>,
+                                          split0_product_ptr<3>, split0_product_ptr<4>, split0_product_ptr<5>,
+                                          split0_product_ptr<6>, split0_product_ptr<7>};
+  return of[algo](ls, phase);
 }
-// the one-level kernel (DIF bases only; sum: its Fourier-domain sum variant);
-// nullptr where the shape is not instantiated
-inline const void* u64_product_split2_ptr(int algo, int ls0, int ls1, bool sum) {
-  const void* (*const of[8])(int, int, bool) = {split2_product_ptr<0>, split2_product_ptr<1>, split2_product_ptr<2>,
-                                                split2_product_ptr<3>, split2_product_ptr<4>, split2_product_ptr<5>,
-                                                split2_product_ptr<6>, split2_product_ptr<7>};
-  return of[algo](ls0, ls1, sum);
+// the one-level kernel (DIF bases only); nullptr where the shape is not instantiated
+inline const void* u64_product_split2_ptr(int algo, int ls0, int ls1, int phase) {
+  const void* (*const of[8])(int, int, int) = {split2_product_ptr<0>, split2_product_ptr<1>, split2_product_ptr<2>,
+                                               split2_product_ptr<3>, split2_product_ptr<4>, split2_product_ptr<5>,
+                                               split2_product_ptr<6>, split2_product_ptr<7>};
+  return of[algo](ls0, ls1, phase);
 }
 #endif
 
