@@ -240,24 +240,27 @@ __global__ void __launch_bounds__(256) f128_class_kernel(F128Arrays g, int log2n
   }
 }
 
-// Small batches: every stage of half-size 2^lo and more, one residue class mod
-// 2^lo of a transform (2^(log2n - lo) <= 256 points) per CTA in shared memory,
-// two warps per 32 butterflies (real and imaginary halves, f128_half_stage), so
-// that a few transforms keep every SM sub-partition busy.  With the block
-// kernel below, a transform is two launches (one 16384-point forward, stage by
-// stage in eight launches: 61.6 us from Python, 32.3 on the device).
+// Small batches: every stage of half-size 2^lo and more on residue classes mod 2^lo of a
+// transform, 2^lq neighbouring classes of 2^(log2n - lo) points per CTA in shared memory
+// (at most 256 points), two warps per 32 butterflies (real and imaginary halves,
+// f128_half_stage), so that a few transforms keep every SM sub-partition busy.  With the
+// block kernel below, a transform is two launches (one 16384-point forward, stage by
+// stage in eight launches: 61.6 us from Python, 32.3 on the device).  A class of fewer than
+// 64 points shares its CTA with its neighbours, to fill the two warps (30 transforms of 512
+// points: 44.0 us with one class of 4 points per CTA).
 template <bool FWD>
-__global__ void __launch_bounds__(256) f128_class_half_kernel(F128Arrays g, int log2n, int lo, F128Tw tw) {
+__global__ void __launch_bounds__(256) f128_class_half_kernel(F128Arrays g, int log2n, int lo, F128Tw tw, int lq) {
   __shared__ double sm[4 * 256 + 2 * 256];
   const int lp = log2n - lo;
-  const int np = 1 << lp;
+  const int np = 1 << (lp + lq);
   const F128Arrays s{sm, sm + np, sm + 2 * np, sm + 3 * np};
   double* xs = sm + 4 * np;
   const int tid = threadIdx.x, nth = blockDim.x;
-  const long base = ((long)(blockIdx.x >> lo) << log2n) + (blockIdx.x & ((1 << lo) - 1));
+  const int col = (1 << lq) - 1;
+  const long base = ((long)(blockIdx.x >> (lo - lq)) << log2n) + ((blockIdx.x & ((1 << (lo - lq)) - 1)) << lq);
   grid_dependency_wait();
   for (int i = tid; i < np; i += nth) {
-    const long p = base + ((long)i << lo);
+    const long p = base + ((long)(i >> lq) << lo) + (i & col);
     s.re0[i] = g.re0[p];
     s.re1[i] = g.re1[p];
     s.im0[i] = g.im0[p];
@@ -268,13 +271,14 @@ __global__ void __launch_bounds__(256) f128_class_half_kernel(F128Arrays g, int 
     const int l = FWD ? lp - 1 - st : st;
     const long m = 1L << (lp - 1 - l);
     f128_half_stage<FWD>(s, xs, np / 2, [&](int b, int& qa, int& qb, long& widx) {
-      qa = ((b >> l) << (l + 1)) + (b & ((1 << l) - 1));
-      qb = qa + (1 << l);
-      widx = m + (b >> l);
+      const int k = b >> lq;  // butterfly of a class, b's low bits the class
+      qa = ((((k >> l) << (l + 1)) + (k & ((1 << l) - 1))) << lq) + (b & col);
+      qb = qa + (1 << (l + lq));
+      widx = m + (k >> l);
     }, tw, tid, nth);
   }
   for (int i = tid; i < np; i += nth) {
-    const long p = base + ((long)i << lo);
+    const long p = base + ((long)(i >> lq) << lo) + (i & col);
     g.re0[p] = s.re0[i];
     g.re1[p] = s.re1[i];
     g.im0[p] = s.im0[i];
@@ -678,11 +682,12 @@ cfft_status run_f128_tw(size_t n, const F128Tw& tw, double* re0, double* re1, do
       int ln = log2n, lc = log2c;
       const int bgrid = (int)((long)batch << (log2n - log2c));
       const int lp = log2n - log2c;  // stages above the blocks: 2^log2c classes of 2^lp points
-      const int cgrid = (int)((long)batch << log2c);
-      const int cthreads = std::min(256, std::max(64, 1 << lp));
+      int lq = std::max(0, 6 - lp);  // neighbouring classes per CTA: at least 64 points
+      const int cgrid = (int)((long)batch << (log2c - lq));
+      const int cthreads = std::min(256, 1 << (lp + lq));
       const void* cfn = fwd ? (const void*)f128_class_half_kernel<true> : (const void*)f128_class_half_kernel<false>;
       const void* bfn = fwd ? (const void*)f128_smem_half_kernel<true> : (const void*)f128_smem_half_kernel<false>;
-      void* bargs[] = {&g, &ln, &lc, &t};
+      void* bargs[] = {&g, &ln, &lc, &t, &lq};  // the block kernel takes the first four
       auto classes = [&]() {
         return lp == 0 ? CFFT_OK : launch_kernel(cfn, cgrid, cthreads, bargs, 0, stream, true);
       };

@@ -188,3 +188,23 @@ def test_f128_stages_on_classes(cuda, oracle, n, batch, block):
         for k in range(4):
             assert np.array_equal(f[k][b].view(np.uint64), np.asarray(wf[k]).view(np.uint64)), ("fwd", b, k)
             assert np.array_equal(g[k][b].view(np.uint64), np.asarray(wi[k]).view(np.uint64)), ("inv", b, k)
+
+
+@pytest.mark.parametrize("n,batch", [(256, 76), (512, 30), (512, 38), (1024, 10), (1024, 38), (2048, 19), (4096, 9),
+                                     (8192, 2)])
+def test_f128_neighbouring_classes_share_a_cta(cuda, oracle, n, batch):
+    """Small batches whose stages above the blocks are few: several classes of 2 to 64 points per CTA."""
+    import concrete_fft as cf
+    torch = cuda
+    x = _edge_arrays("random", batch, n)
+    plan = cf.fft128.Plan(n)
+    d = [torch.from_numpy(v.copy()).cuda() for v in x]
+    plan.fwd(*d)
+    f = [v.cpu().numpy() for v in d]
+    plan.inv(*d)
+    for b in {0, batch // 2, batch - 1}:
+        wf = oracle.f128_fwd(*[v[b] for v in x])
+        wi = oracle.f128_inv(*wf)
+        for k in range(4):
+            assert np.array_equal(f[k][b].view(np.uint64), np.asarray(wf[k]).view(np.uint64)), ("fwd", b, k)
+            assert np.array_equal(d[k][b].cpu().numpy().view(np.uint64), np.asarray(wi[k]).view(np.uint64)), ("inv", b, k)
