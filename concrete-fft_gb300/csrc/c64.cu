@@ -200,7 +200,8 @@ cfft_status launch_smem(const C64Plan& p, bool fwd, int blocks, size_t smem, cud
   DevLevels L = p.dlv;
   int tpc = p.tpc, d0 = p.d0;
   void* args[] = {&data, &nsub, &tpc, &L, &d0, (void*)&w};
-  const void* fn = c64_kernel(p.base_algo, fwd);
+  const size_t pass = ((size_t)p.tpc << p.lv.log2n[p.d0]) / (size_t)algo_radix(p.base_algo);  // butterflies per CTA
+  const void* fn = c64_kernel(p.base_algo, fwd, half_butterflies(blocks, std::min(pass, (size_t)p.threads)));
   return launch_kernel(fn, blocks, p.threads, args, spread_smem(fn, blocks, p.threads, 1, smem), stream, true);
 }
 
@@ -326,11 +327,12 @@ cfft_status launch_split(const C64Plan& p, bool fwd, int ls, int mode, long nsub
   // halves (radix 16 at every size: a whole butterfly takes 126 registers, and one warp
   // per CTA was slower, 84 against 70 us for 1024 transforms of 1024 points on 2 CTAs)
   const int R = algo_radix(p.base_algo);
-  const bool halves = (p.base_algo & 1) == 0 && (R == 16 || half_butterflies(nsub << ls, part / (size_t)R));
+  int few = half_butterflies(nsub << ls, part / (size_t)R);
+  const bool halves = (p.base_algo & 1) == 0 && (R == 16 || few);
   const int threads = (int)std::min<size_t>(256, std::max<size_t>(32, (halves ? 2 : 1) * part / (size_t)R));
   DevLevels L = p.dlv;
   const double2* w = fwd ? p.d_w : p.d_winv;
-  void* args[] = {&data, &L, (void*)&w};
+  void* args[] = {&data, &L, (void*)&w, &few};
   if ((nsub << ls) > 0x7fffffffL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   const int grid = (int)(nsub << ls);
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),

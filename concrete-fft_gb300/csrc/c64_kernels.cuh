@@ -12,7 +12,7 @@ namespace cfft {
 // Sub-transforms of 2^log2n_{d0} points, `tpc` per CTA: load to shared memory,
 // run the unordered transform from level d0 (ordered plans have no levels),
 // store back.
-template <int ALGO, bool FWD>
+template <int ALGO, int E, bool FWD>
 __global__ void __launch_bounds__(256) c64_smem_kernel(double2* data, int count, int tpc, DevLevels L, int d0,
                                                        const double2* __restrict__ w) {
   extern __shared__ double2 smem[];
@@ -27,20 +27,20 @@ __global__ void __launch_bounds__(256) c64_smem_kernel(double2* data, int count,
   const int tid = threadIdx.x, nth = blockDim.x;
   for (int i = tid; i < npts; i += nth) x[i] = g[i];
   __syncthreads();
-  const double2* r = unordered_smem<FWD, kAddsBatch, ALGO>(L, d0, nch, x, y, w, tid, nth);
+  const double2* r = unordered_smem<FWD, E, ALGO>(L, d0, nch, x, y, w, tid, nth);
   for (int i = tid; i < npts; i += nth) g[i] = r[i];
 }
 
 // Fused negacyclic u64 product (see product_u64.cu for the pipeline): one
 // product per CTA at a time, grid-stride over the batch.
-template <int ALGO, int THREADS>
-__global__ void __launch_bounds__(THREADS, 6) u64_product_kernel(const uint64_t* __restrict__ a,
-                                                             const double2* __restrict__ bhat, long bhat_stride,
-                                                             uint64_t* __restrict__ out, long count, DevLevels L,
-                                                             const double2* __restrict__ w,
-                                                             const double2* __restrict__ winv,
-                                                             const double2* __restrict__ tw,
-                                                             const double2* __restrict__ itw, int log2p) {
+// E > 0: 6 CTAs per SM by registers (5 for radix 16, whose butterflies spill 2.8 KB in 80
+// registers: 8192 products of N = 2048 on Dif16 take 1866 us at 6, 962 at 5).
+template <int ALGO, int E, int THREADS>
+__global__ void __launch_bounds__(THREADS, E == 0 ? 1 : AlgoInfo<ALGO>::R == 16 ? 5 : 6)
+    u64_product_kernel(const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride,
+                       uint64_t* __restrict__ out, long count, DevLevels L, const double2* __restrict__ w,
+                       const double2* __restrict__ winv, const double2* __restrict__ tw,
+                       const double2* __restrict__ itw, int log2p) {
   // 2^log2p products per CTA iteration, back to back in shared memory (small N: a pass's
   // butterflies then fill whole warps; the products stay independent, so the bits do not
   // depend on the packing)
@@ -60,14 +60,14 @@ __global__ void __launch_bounds__(THREADS, 6) u64_product_kernel(const uint64_t*
       st(x + j, cmul(ldg(tw + jj), v));
     }
     __syncthreads();
-    double2* r = unordered_smem<true, kAddsBatch, ALGO>(L, 0, np, x, y, w, tid, THREADS);
+    double2* r = unordered_smem<true, E, ALGO>(L, 0, np, x, y, w, tid, THREADS);
     for (int k = tid; k < pts; k += THREADS) {
       const double2* bp = bhat + (first + (k >> log2n)) * bhat_stride;
       st(r + k, cmul(ldg(bp + (k & (n - 1))), ld(r + k)));
     }
     __syncthreads();
     double2* o = (r == x) ? y : x;
-    double2* s = unordered_smem<false, kAddsBatch, ALGO>(L, 0, np, r, o, winv, tid, THREADS);
+    double2* s = unordered_smem<false, E, ALGO>(L, 0, np, r, o, winv, tid, THREADS);
     for (int j = tid; j < pts; j += THREADS) {
       const int jj = j & (n - 1);
       uint64_t* op = out + ((first + (j >> log2n)) << (log2n + 1));
@@ -88,14 +88,15 @@ __global__ void __launch_bounds__(THREADS, 6) u64_product_kernel(const uint64_t*
 // entries k = tid + j x THREADS it multiplies in registers, so shared memory
 // is the 2 x N/2 ping-pong pair and more CTAs fit on an SM; the additions and
 // their order are the same.
-template <int ALGO, int THREADS, int ACC>
-__global__ void __launch_bounds__(THREADS) u64_product_sum_kernel(const uint64_t* __restrict__ a,
-                                                                 const double2* __restrict__ bhat, int terms,
-                                                                 uint64_t* __restrict__ out, long count, DevLevels L,
-                                                                 const double2* __restrict__ w,
-                                                                 const double2* __restrict__ winv,
-                                                                 const double2* __restrict__ tw,
-                                                                 const double2* __restrict__ itw) {
+// E > 0: 4 CTAs per SM by registers; the integer additions are bound by warps in flight (8192
+// terms of N = 2048 in groups of 8 on Dif4: 628 us at 3 CTAs, 557 at 4, 567 at 5, 809 with
+// all additions on the FP64 pipe).
+template <int ALGO, int E, int THREADS, int ACC>
+__global__ void __launch_bounds__(THREADS, E == 0 ? 1 : 4)
+    u64_product_sum_kernel(const uint64_t* __restrict__ a, const double2* __restrict__ bhat, int terms,
+                           uint64_t* __restrict__ out, long count, DevLevels L, const double2* __restrict__ w,
+                           const double2* __restrict__ winv, const double2* __restrict__ tw,
+                           const double2* __restrict__ itw) {
   extern __shared__ double2 smem[];
   const int log2n = L.log2n[0];
   const int n = 1 << log2n;
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(THREADS) u64_product_sum_kernel(const uint64_t
         st(x + j, cmul(ldg(tw + j), v));
       }
       __syncthreads();
-      const double2* r = unordered_smem<true, kAddsBatch, ALGO>(L, 0, 1, x, y, w, tid, THREADS);
+      const double2* r = unordered_smem<true, E, ALGO>(L, 0, 1, x, y, w, tid, THREADS);
       const double2* bp = bhat + (term << log2n);
       if (ACC > 0) {
 #pragma unroll
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(THREADS) u64_product_sum_kernel(const uint64_t
       __syncthreads();
       src = y;
     }
-    const double2* s = unordered_smem<false, kAddsBatch, ALGO>(L, 0, 1, src, x, winv, tid, THREADS);
+    const double2* s = unordered_smem<false, E, ALGO>(L, 0, 1, src, x, winv, tid, THREADS);
     uint64_t* op = out + (g << (log2n + 1));
     for (int j = tid; j < n; j += THREADS) {
       const c64 v = cmul(ldg(itw + j), ld(s + j));
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(THREADS) u64_product_sum_kernel(const uint64_t
 constexpr int kSumRegAcc = 8;
 
 // Bhat = fwd(tau^j * (b_j + i b_{j+N/2})) for small signed digits b.
-template <int ALGO, int THREADS>
+template <int ALGO, int E, int THREADS>
 __global__ void __launch_bounds__(THREADS) u64_prepare_kernel(const int64_t* __restrict__ b,
                                                              double2* __restrict__ bhat, long count, DevLevels L,
                                                              const double2* __restrict__ w,
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(THREADS) u64_prepare_kernel(const int64_t* __r
       st(x + j, cmul(ldg(tw + j), v));
     }
     __syncthreads();
-    const double2* r = unordered_smem<true, kAddsBatch, ALGO>(L, 0, 1, x, y, w, tid, THREADS);
+    const double2* r = unordered_smem<true, E, ALGO>(L, 0, 1, x, y, w, tid, THREADS);
     double2* op = bhat + (prod << log2n);
     for (int k = tid; k < n; k += THREADS) op[k] = r[k];
     __syncthreads();
@@ -186,11 +187,14 @@ __global__ void __launch_bounds__(THREADS) u64_prepare_kernel(const int64_t* __r
 constexpr int kProdThreads = 128;
 
 // Kernel-pointer tables (nullptr when the combination is not instantiated).
-const void* c64_kernel(int algo, bool fwd);
+// few: the launch has about one warp per SM sub-partition (half_butterflies), where the
+// radix-8 and radix-16 algorithms keep their additions on the FP64 pipe (269 products of
+// N = 256 on Dif16: 49 us on the integer pipes, 25; one of N = 1024 on Dit8: 37 and 25).
+const void* c64_kernel(int algo, bool fwd, bool few);
 // one transform over 2^ls CTAs (split.cuh); mode 0 no outer levels, 1 with levels
 const void* c64_split_kernel_ptr(int algo, bool fwd, int ls, int mode);
-const void* u64_product_kernel_ptr(int algo);
-const void* u64_prepare_kernel_ptr(int algo);
-const void* u64_product_sum_kernel_ptr(int algo, bool reg_acc);
+const void* u64_product_kernel_ptr(int algo, bool few);
+const void* u64_prepare_kernel_ptr(int algo, bool few);
+const void* u64_product_sum_kernel_ptr(int algo, bool reg_acc, bool few);
 
 }  // namespace cfft

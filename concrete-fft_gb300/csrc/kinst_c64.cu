@@ -3,20 +3,20 @@
 #include "split.cuh"
 
 namespace cfft {
-template <int A>
+template <int A, int E>
 static const void* pick(bool fwd) {
-  return fwd ? (const void*)c64_smem_kernel<A, true> : (const void*)c64_smem_kernel<A, false>;
+  return fwd ? (const void*)c64_smem_kernel<A, E, true> : (const void*)c64_smem_kernel<A, E, false>;
 }
-const void* c64_kernel(int algo, bool fwd) {
+const void* c64_kernel(int algo, bool fwd, bool few) {
   switch (algo) {
-    case 0: return pick<0>(fwd);
-    case 1: return pick<1>(fwd);
-    case 2: return pick<2>(fwd);
-    case 3: return pick<3>(fwd);
-    case 4: return pick<4>(fwd);
-    case 5: return pick<5>(fwd);
-    case 6: return pick<6>(fwd);
-    case 7: return pick<7>(fwd);
+    case 0: return few ? pick<0, 0>(fwd) : pick<0, kAddsBatch>(fwd);
+    case 1: return few ? pick<1, 0>(fwd) : pick<1, kAddsBatch>(fwd);
+    case 2: return few ? pick<2, 0>(fwd) : pick<2, kAddsBatch>(fwd);
+    case 3: return few ? pick<3, 0>(fwd) : pick<3, kAddsBatch>(fwd);
+    case 4: return few ? pick<4, 0>(fwd) : pick<4, kAddsBatch>(fwd);
+    case 5: return few ? pick<5, 0>(fwd) : pick<5, kAddsBatch>(fwd);
+    case 6: return few ? pick<6, 0>(fwd) : pick<6, kAddsBatch>(fwd);
+    case 7: return few ? pick<7, 0>(fwd) : pick<7, kAddsBatch>(fwd);
     default: return nullptr;
   }
 }

@@ -2,21 +2,21 @@
 #include "c64_kernels.cuh"
 
 namespace cfft {
-template <int A>
-static const void* pick_sum(bool reg_acc) {
-  return reg_acc ? (const void*)u64_product_sum_kernel<A, kProdThreads, kSumRegAcc>
-                 : (const void*)u64_product_sum_kernel<A, kProdThreads, 0>;
+template <int A, int E>
+static const void* pick(bool reg_acc) {
+  return reg_acc ? (const void*)u64_product_sum_kernel<A, E, kProdThreads, kSumRegAcc>
+                 : (const void*)u64_product_sum_kernel<A, E, kProdThreads, 0>;
 }
-const void* u64_product_sum_kernel_ptr(int algo, bool reg_acc) {
+const void* u64_product_sum_kernel_ptr(int algo, bool reg_acc, bool few) {
   switch (algo) {
-    case 0: return pick_sum<0>(reg_acc);
-    case 1: return pick_sum<1>(reg_acc);
-    case 2: return pick_sum<2>(reg_acc);
-    case 3: return pick_sum<3>(reg_acc);
-    case 4: return pick_sum<4>(reg_acc);
-    case 5: return pick_sum<5>(reg_acc);
-    case 6: return pick_sum<6>(reg_acc);
-    case 7: return pick_sum<7>(reg_acc);
+    case 0: return few ? pick<0, 0>(reg_acc) : pick<0, kAddsBatch>(reg_acc);
+    case 1: return few ? pick<1, 0>(reg_acc) : pick<1, kAddsBatch>(reg_acc);
+    case 2: return few ? pick<2, 0>(reg_acc) : pick<2, kAddsBatch>(reg_acc);
+    case 3: return few ? pick<3, 0>(reg_acc) : pick<3, kAddsBatch>(reg_acc);
+    case 4: return few ? pick<4, 0>(reg_acc) : pick<4, kAddsBatch>(reg_acc);
+    case 5: return few ? pick<5, 0>(reg_acc) : pick<5, kAddsBatch>(reg_acc);
+    case 6: return few ? pick<6, 0>(reg_acc) : pick<6, kAddsBatch>(reg_acc);
+    case 7: return few ? pick<7, 0>(reg_acc) : pick<7, kAddsBatch>(reg_acc);
     default: return nullptr;
   }
 }

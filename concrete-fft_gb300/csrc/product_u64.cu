@@ -171,13 +171,31 @@ cfft_status product_sum_unfused(const cfft_u64_product_plan* plan, const uint64_
   return st;
 }
 
+// Whether a launch of `ctas` one-CTA kernels of `points` points each has about one busy
+// warp per SM sub-partition in a pass of the base, counting the CTAs that shared memory
+// lets run at once (300 operands of 4096 points on Dit2, one per SM: 159 us on the integer
+// pipes, 150).  A radix-16 pass of less than a warp of butterflies counts as such: what its
+// idle lanes leave of an integer addition costs more than the FP64 one (1500 products of
+// N = 256 on Dit16: 78.6 us, 66.8; of N = 1024, a full warp: 110 and 121).
+bool few_warps(const cfft_u64_product_plan* plan, long ctas, size_t points) {
+  const size_t radix = (size_t)algo_radix(plan->base_algo), pass = std::min<size_t>(kProdThreads, points / radix);
+  if (radix == 16 && pass < 32) return true;
+  const long per_sm = std::max<long>(1, (long)((size_t(227) << 10) / (2 * points * sizeof(double2))));
+  return half_butterflies(std::min(ctas, (long)sm_count() * per_sm), pass);
+}
+
 cfft_status launch_product(const cfft_u64_product_plan* plan, const uint64_t* a, const double* bhat,
                            size_t bhat_stride, uint64_t* out, size_t count, cudaStream_t stream) {
-  const void* fn = u64_product_kernel_ptr(plan->base_algo);
   // N <= 128: 512 points per CTA iteration (one product of n = 32 would give a radix-4
   // pass 8 butterflies, a quarter warp: 122 vs 375 M products/s possible at N = 64)
   int log2p = 0;
   while ((plan->n << log2p) < 512 && plan->n <= 64) ++log2p;
+  // likewise a radix whose pass over one product is less than a warp, while two CTAs per SM
+  // remain (1500 products of N = 256: 74 us on Dif16, 67 on Dit16 with one per CTA)
+  while ((plan->n << log2p) < 32 * (size_t)algo_radix(plan->base_algo) && (long)(count >> (log2p + 1)) >= 2L * sm_count())
+    ++log2p;
+  const void* fn = u64_product_kernel_ptr(
+      plan->base_algo, few_warps(plan, ((long)count + (1L << log2p) - 1) >> log2p, plan->n << log2p));
   const size_t smem = 2 * (plan->n << log2p) * sizeof(double2);
   const int grid = grid_for(fn, kProdThreads, smem, ((long)count + (1L << log2p) - 1) >> log2p);
   DevLevels L = plan->dlv;
@@ -224,12 +242,13 @@ cfft_status launch_split_product(const cfft_u64_product_plan* plan, int ls, cons
   DevLevels L = plan->dlv;
   long stride = (long)bhat_stride;
   const double2* bh = (const double2*)bhat;
-  void* args[] = {(void*)&a, (void*)&bh, &stride, (void*)&out, &terms, (void*)&items, &L, (void*)&plan->d_w,
-                  (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw};
   // 128 threads (several CTAs per SM) for parts up to 1024 points, 256 for 2048
   // (shared memory allows 3 CTAs per SM), 512 for 4096 (one CTA per SM)
   const int threads = part <= 1024 ? 128 : (part <= 2048 ? kSplitProdThreads : kSplitProdThreadsBig);
   const int grid = (int)(count << ls);
+  int few = half_butterflies(grid, std::min<size_t>((size_t)threads, part / (size_t)algo_radix(plan->base_algo)));
+  void* args[] = {(void*)&a, (void*)&bh, &stride, (void*)&out, &terms, (void*)&items, &L, (void*)&plan->d_w,
+                  (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw, &few};
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),
                                stream);
 }
@@ -494,7 +513,7 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   }
   if (count == 0) return CFFT_OK;
   const bool reg_acc = plan->n <= (size_t)(kSumRegAcc * kProdThreads);
-  const void* fn = u64_product_sum_kernel_ptr(plan->base_algo, reg_acc);
+  const void* fn = u64_product_sum_kernel_ptr(plan->base_algo, reg_acc, few_warps(plan, (long)count, plan->n));
   const size_t smem = (reg_acc ? 2 : 3) * plan->n * sizeof(double2);
   const int grid = grid_for(fn, kProdThreads, smem, (long)count);
   DevLevels L = plan->dlv;
@@ -581,7 +600,7 @@ cfft_status cfft_u64_prepare_operand(const cfft_u64_product_plan* plan, const in
     return cfft_unordered_fwd(plan->fft, bhat, count, stream);
   }
   const size_t smem = 2 * plan->n * sizeof(double2);
-  const void* fn = u64_prepare_kernel_ptr(plan->base_algo);
+  const void* fn = u64_prepare_kernel_ptr(plan->base_algo, few_warps(plan, (long)count, plan->n));
   const int grid = grid_for(fn, kProdThreads, smem, (long)count);
   DevLevels L = plan->dlv;
   long cnt = (long)count;

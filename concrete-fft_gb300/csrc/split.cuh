@@ -41,7 +41,7 @@ namespace cfft {
 
 // Passes 1 .. npass-1 and the end butterfly of a DIF transform of 2^log2n
 // points, run on one residue class mod 2^LS compacted to 2^(log2n - LS) points.
-template <int R, bool FWD>
+template <int R, bool FWD, int E = kAddsSplit<R>>
 __device__ __forceinline__ FlatBuf dif_after_first(int log2n, int ls, FlatBuf x, FlatBuf y,
                                                    const double2* __restrict__ wb, int tid, int nth) {
   constexpr int LR = Log2<R>::v;
@@ -53,20 +53,20 @@ __device__ __forceinline__ FlatBuf dif_after_first(int log2n, int ls, FlatBuf x,
   const int log2c = log2n - ls;
   FlatBuf cur = x, oth = y;
   for (int i = 1; i < npass; ++i) {
-    stockham_pass<R, FWD, false, kAddsSplit<R>, true>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
+    stockham_pass<R, FWD, false, E, true>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
     __syncthreads();
     const FlatBuf t = cur;
     cur = oth;
     oth = t;
   }
-  end_dispatch<R, FWD, kAddsSplit<R>, true>(lm, log2c, 1, cur, tid, nth);
+  end_dispatch<R, FWD, E, true>(lm, log2c, 1, cur, tid, nth);
   __syncthreads();
   return cur;
 }
 
 // The end butterfly and passes npass-1 .. 1 of a DIT transform, on one
 // residue class mod 2^LS (compacted), i.e. everything but the s = 1 pass.
-template <int R, bool FWD>
+template <int R, bool FWD, int E = kAddsFew<R>>
 __device__ __forceinline__ FlatBuf dit_before_last(int log2n, int ls, FlatBuf x, FlatBuf y,
                                                    const double2* __restrict__ wb, int tid, int nth) {
   constexpr int LR = Log2<R>::v;
@@ -77,10 +77,10 @@ __device__ __forceinline__ FlatBuf dit_before_last(int log2n, int ls, FlatBuf x,
   }
   const int log2c = log2n - ls;
   FlatBuf cur = x, oth = y;
-  end_dispatch<R, FWD, kAddsFew<R>>(lm, log2c, 1, cur, tid, nth);
+  end_dispatch<R, FWD, E>(lm, log2c, 1, cur, tid, nth);
   __syncthreads();
   for (int i = npass - 1; i >= 1; --i) {
-    stockham_pass<R, FWD, true, kAddsFew<R>>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
+    stockham_pass<R, FWD, true, E>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
     __syncthreads();
     const FlatBuf t = cur;
     cur = oth;
@@ -145,7 +145,7 @@ __device__ __forceinline__ void level0_last(double2* g, int lm, double2* const* 
 struct NoWait {
   __device__ void operator()() const {}
 };
-template <int R, bool FWD, int LS, class Load, class Wait = NoWait>
+template <int R, bool FWD, int LS, int E = kAddsSplit<R>, class Load, class Wait = NoWait>
 __device__ __forceinline__ void first_pass_scatter(Load load, int per, int p0, int pstep, double2* const* part,
                                                    const double2* __restrict__ wb, int tid, int nth,
                                                    Wait before_store = Wait{}) {
@@ -185,7 +185,7 @@ __device__ __forceinline__ void first_pass_scatter(Load load, int per, int p0, i
     c64 v[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) v[k] = load(k, b, p);
-    Core<R, FWD, kAddsSplit<R>>::run(v);
+    Core<R, FWD, E>::run(v);
     const double2* tw = wb + (p << LR);
 #pragma unroll
     for (int k = 0; k < R; ++k) {
@@ -198,12 +198,12 @@ __device__ __forceinline__ void first_pass_scatter(Load load, int per, int p0, i
 // The first pass of a DIF transform held in global memory: CTA c takes the
 // butterflies [c*per, (c+1)*per) in full -- no output is computed twice --
 // reading their inputs from g.
-template <int R, bool FWD, int LS, class Wait>
+template <int R, bool FWD, int LS, int E, class Wait>
 __device__ __forceinline__ void dif_first_scatter(const double2* g, int lper, int c, double2* const* part,
                                                   const double2* __restrict__ wb, int tid, int nth,
                                                   Wait before_store) {
   const int per = (1 << lper) >> LS;
-  first_pass_scatter<R, FWD, LS>([&](int k, int, int p) { return ld(g + (k << lper) + p); }, per, c * per, 1, part,
+  first_pass_scatter<R, FWD, LS, E>([&](int k, int, int p) { return ld(g + (k << lper) + p); }, per, c * per, 1, part,
                                  wb, tid, nth, before_store);
 }
 
@@ -212,15 +212,17 @@ __device__ __forceinline__ void dif_first_scatter(const double2* g, int lper, in
 // MODE 1: unordered with outer levels (forward: first, inverse: last).
 // One transform per S consecutive CTAs; w is the plan's forward table
 // (forward) or inverse table (inverse).
-template <int ALGO, bool FWD, int LS, int MODE>
-__global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels L, const double2* __restrict__ w) {
+template <int ALGO, bool FWD, int LS, int MODE, bool FEW>
+__device__ __forceinline__ void c64_split(double2* data, const DevLevels& L, const double2* __restrict__ w) {
   constexpr int R = AlgoInfo<ALGO>::R;
   constexpr int LR = Log2<R>::v;
   constexpr int S = 1 << LS;
   constexpr bool LAST = MODE == 0 ? AlgoInfo<ALGO>::DIT : !FWD;
   // the DIT algorithms have no other kernel for small batches with levels
   constexpr bool DIT = AlgoInfo<ALGO>::DIT;
-  constexpr int kAddsLevels = DIT ? kAddsFew<R> : kAddsSplit<R>;
+  constexpr int E = FEW ? 0 : DIT ? kAddsFew<R> : kAddsSplit<R>;
+  constexpr int E0 = FEW ? 0 : kAddsSplit<2>;                // level 0 of radix 2 or 4
+  constexpr int E8 = FEW || DIT ? 0 : kAddsSplit<8>;  // of radix 8
   extern __shared__ double2 smem[];
   grid_dependency_wait();
   const int log2n = L.log2n[0];
@@ -245,10 +247,10 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     // every CTA of the cluster runs before its shared memory is written: the barrier's
     // wait comes after the first pass's loads
     auto token = cl.barrier_arrive();
-    dif_first_scatter<R, FWD, LS>(g, log2n - LR, c, part, wb, tid, nth,
+    dif_first_scatter<R, FWD, LS, E>(g, log2n - LR, c, part, wb, tid, nth,
                                   [&] { cl.barrier_wait(std::move(token)); });
     cl.sync();  // every part is complete, and every read of the transform in global memory is done
-    const FlatBuf r = dif_after_first<R, FWD>(log2n, LS, FlatBuf{xs}, FlatBuf{ys}, wb, tid, nth);
+    const FlatBuf r = dif_after_first<R, FWD, E>(log2n, LS, FlatBuf{xs}, FlatBuf{ys}, wb, tid, nth);
     for (int j = tid; j < (1 << log2c); j += nth) g[(j << LS) + c] = r.p[j];
   } else if constexpr (MODE == 0 && LAST) {
     // DIT: own residue class through every pass but the last, then the s = 1
@@ -257,7 +259,7 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     cg::cluster_group cl = cg::this_cluster();
     for (int j = tid; j < (1 << log2c); j += nth) xs[j] = g[(j << LS) + c];
     __syncthreads();
-    const FlatBuf r = dit_before_last<R, FWD>(log2n, LS, FlatBuf{xs}, FlatBuf{ys}, wb, tid, nth);
+    const FlatBuf r = dit_before_last<R, FWD, E>(log2n, LS, FlatBuf{xs}, FlatBuf{ys}, wb, tid, nth);
     double2* peer[S];
 #pragma unroll
     for (int j = 0; j < S; ++j) peer[j] = cl.map_shared_rank(r.p, (unsigned)j);
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(tw + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, FWD, kAddsFew<R>>::run(v);
+      Core<R, FWD, E>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) st(g + (k << lper) + p, v[k]);
     }
@@ -298,14 +300,14 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     const double2* wl = w + L.w_off[0];
     const int per = (1 << lm) >> LS;
     if (lr0 == 1) {
-      if constexpr (LS <= 1) level0_scatter<2, LS, DIT ? kAddsFew<2> : kAddsSplit<2>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 1) level0_scatter<2, LS, E0>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     } else if (lr0 == 2) {
-      if constexpr (LS <= 2) level0_scatter<4, LS, DIT ? kAddsFew<4> : kAddsSplit<4>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 2) level0_scatter<4, LS, E0>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     } else {
-      level0_scatter<8, LS, DIT ? kAddsFew<8> : kAddsSplit<8>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      level0_scatter<8, LS, E8>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     }
     cl.sync();  // every part's xs is complete, and every peer is done reading this CTA's ys
-    const FlatBuf r = unordered_t<true, kAddsLevels, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
+    const FlatBuf r = unordered_t<true, E, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
     double2* gw = g + ((long)c << log2c);
     for (int j = tid; j < (1 << log2c); j += nth) gw[j] = r.p[j];
   } else {
@@ -318,7 +320,7 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     __syncthreads();
     const int lr0 = L.log2r[0];
     const int lm = log2n - lr0;
-    const FlatBuf r = unordered_t<false, kAddsLevels, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
+    const FlatBuf r = unordered_t<false, E, ALGO>(L, 1, 1 << (lr0 - LS), FlatBuf{xs}, FlatBuf{ys}, w, tid, nth);
     double2* peer[S];
 #pragma unroll
     for (int j = 0; j < S; ++j) peer[j] = cl.map_shared_rank(r.p, (unsigned)j);
@@ -326,14 +328,25 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
     const double2* wl = w + L.winv_off[0];
     const int per = (1 << lm) >> LS;
     if (lr0 == 1) {
-      if constexpr (LS <= 1) level0_last<2, LS, DIT ? kAddsFew<2> : kAddsSplit<2>>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 1) level0_last<2, LS, E0>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
     } else if (lr0 == 2) {
-      if constexpr (LS <= 2) level0_last<4, LS, DIT ? kAddsFew<4> : kAddsSplit<4>>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 2) level0_last<4, LS, E0>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
     } else {
-      level0_last<8, LS, DIT ? kAddsFew<8> : kAddsSplit<8>>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
+      level0_last<8, LS, E8>(g, lm, peer, c * per, (c + 1) * per, wl, tid, nth);
     }
     cl.sync();
   }
+}
+// few: about one warp per SM sub-partition (half_butterflies), where the additions stay on
+// the FP64 pipe (one forward of 16384 points on Dit2/1024: 27.4 us on the integer pipes, 24.1;
+// one of 256 points on Dif8, too few butterflies for halves: 11.0 and 10.2).
+template <int ALGO, bool FWD, int LS, int MODE>
+__global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels L, const double2* __restrict__ w,
+                                                        int few) {
+  constexpr int R = AlgoInfo<ALGO>::R;
+  constexpr bool kSame = MODE == 0 && (R == 16 || (AlgoInfo<ALGO>::DIT && R == 8));  // FP64 pipe in both
+  if (kSame || few) c64_split<ALGO, FWD, LS, MODE, true>(data, L, w);
+  else c64_split<ALGO, FWD, LS, MODE, false>(data, L, w);
 }
 
 // An unordered transform with exactly one outer level, of radix R0 = 2^LS0 <= 4,

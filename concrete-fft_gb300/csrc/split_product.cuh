@@ -82,14 +82,15 @@ constexpr int kSplitAcc = 8;
 // all); out: N u64 per output.  When `items` is not null (terms = 1), product
 // p takes its three pointers from items[p] instead.  Requires L.nlevels >= 1,
 // 2^L.log2r[0] >= S and n/S <= kSplitAcc x blockDim.x.
-template <int ALGO, int LS, int MAXT>
-__global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
+template <int ALGO, int LS, bool FEW>
+__device__ __forceinline__ void u64_product_split(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
-    int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
+    int terms, const cfft_product_item* __restrict__ items, const DevLevels& L, const double2* __restrict__ w,
     const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ double2 smem[];
+  constexpr int E = FEW ? 0 : kAddsSplit<AlgoInfo<ALGO>::R>;
   const int log2n = L.log2n[0];
   const int log2c = log2n - LS;  // points per part
   const int c = (int)(blockIdx.x & ((1 << LS) - 1));
@@ -130,17 +131,17 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
     // 2. level 0 forward: 1/S of the butterflies, each output into its owner's x
     const double2* wl = w + L.w_off[0];
     if (lr0 == 1) {
-      if constexpr (LS <= 1) level0_scatter<2, LS, kAddsSplit<2>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 1) level0_scatter<2, LS, FEW ? 0 : kAddsSplit<2>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     } else if (lr0 == 2) {
-      if constexpr (LS <= 2) level0_scatter<4, LS, kAddsSplit<4>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      if constexpr (LS <= 2) level0_scatter<4, LS, FEW ? 0 : kAddsSplit<4>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     } else {
-      level0_scatter<8, LS, kAddsSplit<8>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
+      level0_scatter<8, LS, FEW ? 0 : kAddsSplit<8>>(peer_y, peer_x, lm, c * per, (c + 1) * per, wl, tid, nth);
     }
     cl.sync();  // every part's x is complete and every peer has read this CTA's y
 
     // 3. the slices forward, the pointwise product added into the accumulator
     // (a single term: stored in place, the inverse starts from it)
-    const FlatBuf r = unordered_t<true, kAddsSplit<AlgoInfo<ALGO>::R>, ALGO>(L, 1, nsl, FlatBuf{x}, FlatBuf{y}, w, tid, nth);
+    const FlatBuf r = unordered_t<true, E, ALGO>(L, 1, nsl, FlatBuf{x}, FlatBuf{y}, w, tid, nth);
     const double2* bp = bprod + base;
 #pragma unroll
     for (int k = 0; k < kSplitAcc; ++k) {
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
     }
     __syncthreads();
   }
-  const FlatBuf s = unordered_t<false, kAddsSplit<AlgoInfo<ALGO>::R>, ALGO>(L, 1, nsl, FlatBuf{src}, FlatBuf{src == x ? y : x}, winv, tid, nth);
+  const FlatBuf s = unordered_t<false, E, ALGO>(L, 1, nsl, FlatBuf{src}, FlatBuf{src == x ? y : x}, winv, tid, nth);
   double2* peer_s[1 << LS];
 #pragma unroll
   for (int j = 0; j < (1 << LS); ++j) peer_s[j] = cl.map_shared_rank(s.p, (unsigned)j);
@@ -180,6 +181,17 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
     level0_inv_untwist<8, LS>(peer_s, lm, log2n, c * per, (c + 1) * per, wli, itw, op, tid, nth);
   }
   cl.sync();  // no CTA exits while a peer reads its shared memory
+}
+// few: about one warp per SM sub-partition (half_butterflies), where the additions stay on
+// the FP64 pipe (one N = 2048 product on Dit8/512: 39.4 us on the integer pipes, 26.4).
+template <int ALGO, int LS, int MAXT>
+__global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
+    const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
+    int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
+    const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw, int few) {
+  // (parts of 4096 points, one CTA of 16 warps per SM, are not told apart)
+  if (MAXT == kSplitProdThreads && few) u64_product_split<ALGO, LS, true>(a, bhat, bhat_stride, out, terms, items, L, w, winv, tw, itw);
+  else u64_product_split<ALGO, LS, false>(a, bhat, bhat_stride, out, terms, items, L, w, winv, tw, itw);
 }
 
 // One product per cluster of S = 2^LS CTAs (S <= the base radix R) when the
@@ -298,13 +310,16 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       __stcs(op + jg + n, round_half_up_mod64(t.im));
     }
   } else {
+    // up to one product per SM, two warps per CTA from radix 4 (one of N = 1024 on Dit4:
+    // 17.2 us on the integer pipes, 16.4; on Dit2, of more warps: 13.8 and 14.7)
+    constexpr int ED = R == 2 ? kAddsFew<R> : 0;
     for (int j = tid; j < (1 << log2c); j += nth) {
       const int jg = (j << LS) + c;
       const c64 v{i64_to_f64_rne((int64_t)__ldcs(ap + jg)), i64_to_f64_rne((int64_t)__ldcs(ap + jg + n))};
       st(x + j, cmul(ldg(tw + jg), v));
     }
     __syncthreads();
-    const FlatBuf r = dit_before_last<R, true>(log2n, LS, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
+    const FlatBuf r = dit_before_last<R, true, ED>(log2n, LS, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
     double2* peer[S];
 #pragma unroll
     for (int j = 0; j < S; ++j) peer[j] = cl.map_shared_rank(r.p, (unsigned)j);
@@ -319,13 +334,13 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(twp + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, true, kAddsFew<R>>::run(v);
+      Core<R, true, ED>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) st(z + (k << lpc) + b, cmul(ldg(bp + (k << lper) + p), v[k]));
     }
     __syncthreads();
     // the inverse ping-pongs between z and the buffer that no peer reads
-    const FlatBuf s = dit_before_last<R, false>(log2n, LS, FlatBuf{z}, FlatBuf{r.p == x ? y : x}, wi, tid, nth);
+    const FlatBuf s = dit_before_last<R, false, ED>(log2n, LS, FlatBuf{z}, FlatBuf{r.p == x ? y : x}, wi, tid, nth);
 #pragma unroll
     for (int j = 0; j < S; ++j) peer[j] = cl.map_shared_rank(s.p, (unsigned)j);
     cl.sync();  // every part's inverse passes are done
@@ -336,7 +351,7 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       v[0] = ld(peer[0] + lo);
 #pragma unroll
       for (int k = 1; k < R; ++k) v[k] = cmul(ldg(twp + k), ld(peer[k & (S - 1)] + lo + (k >> LS)));
-      Core<R, false, kAddsFew<R>>::run(v);
+      Core<R, false, ED>::run(v);
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         const int jg = (k << lper) + p;

@@ -167,6 +167,15 @@ __device__ __forceinline__ void end_pass(int log2n, int nchunks, B x, int tid, i
 
 template <int R, bool FWD, int E, bool HALF = false, class B>
 __device__ __forceinline__ void end_dispatch(int lm, int log2n, int nchunks, B x, int tid, int nth) {
+  // two threads per butterfly of the passes: a small launch, whose whole end butterflies
+  // (more than half as many as threads) stay on the FP64 pipe too (one N = 8192 product on
+  // Dif8/1024, a radix-2 end: 22.3 us on the integer pipes, 20.9)
+  if constexpr (HALF && E != 0) {
+    if ((nth << Log2<R>::v) >= (2 * nchunks << log2n)) {
+      end_dispatch<R, FWD, 0, HALF>(lm, log2n, nchunks, x, tid, nth);
+      return;
+    }
+  }
   if (lm == 1) end_pass<2, FWD, E, HALF>(log2n, nchunks, x, tid, nth);
   if constexpr (R >= 4) {
     if (lm == 2) end_pass<4, FWD, E, HALF>(log2n, nchunks, x, tid, nth);
@@ -187,6 +196,10 @@ __device__ __forceinline__ void end_dispatch(int lm, int log2n, int nchunks, B x
 template <int R, bool FWD, bool DIT, int E, class B = FlatBuf, class S = CtaSync>
 __device__ B stockham_t(int log2n, int nchunks, B x, B y, const double2* __restrict__ w, int tid, int nth) {
   constexpr int LR = Log2<R>::v;
+  // a radix-16 butterfly has 28 pairs and more registers than any other: half of the pairs
+  // on the integer pipes is the fastest there (8192 products of N = 2048 on Dif16: none
+  // 1266 us, half 962, three quarters 1045)
+  constexpr int EB = R == 16 && E > 4 ? 4 : E;
   const S sync{};
   if (log2n == 0) return x;
   int lm = log2n, npass = 0;
@@ -198,19 +211,19 @@ __device__ B stockham_t(int log2n, int nchunks, B x, B y, const double2* __restr
   B oth = y;
   if (!DIT) {
     for (int i = 0; i < npass; ++i) {
-      stockham_pass<R, FWD, false, E>(log2n, i * LR, nchunks, cur, oth, w, tid, nth);
+      stockham_pass<R, FWD, false, EB>(log2n, i * LR, nchunks, cur, oth, w, tid, nth);
       sync();
       const B t = cur;
       cur = oth;
       oth = t;
     }
-    end_dispatch<R, FWD, E>(lm, log2n, nchunks, cur, tid, nth);
+    end_dispatch<R, FWD, EB>(lm, log2n, nchunks, cur, tid, nth);
     sync();
   } else {
-    end_dispatch<R, FWD, E>(lm, log2n, nchunks, cur, tid, nth);
+    end_dispatch<R, FWD, EB>(lm, log2n, nchunks, cur, tid, nth);
     sync();
     for (int i = npass - 1; i >= 0; --i) {
-      stockham_pass<R, FWD, true, E>(log2n, i * LR, nchunks, cur, oth, w, tid, nth);
+      stockham_pass<R, FWD, true, EB>(log2n, i * LR, nchunks, cur, oth, w, tid, nth);
       sync();
       const B t = cur;
       cur = oth;

@@ -78,3 +78,38 @@ def test_transforms_outside_the_integer_range(cuda, oracle, algo, kind):
         assert np.array_equal(d.cpu().numpy().view(np.uint64), f.view(np.uint64)), (n, batch, "fwd")
         plan.inv(d)
         assert np.array_equal(d.cpu().numpy().view(np.uint64), oracle.ordered_inv(algo, f).view(np.uint64)), (n, batch)
+
+
+@pytest.mark.parametrize("algo", [4, 5, 6, 7])
+@pytest.mark.parametrize("N", [64, 128, 512, 1024, 2048])
+def test_one_cta_kernels_with_few_and_many_warps(cuda, oracle, algo, N):
+    """Radix 8 and 16: launches of about a warp per SM sub-partition keep their additions on the FP64
+    pipe, larger ones move them; counts on both sides of the line, bit for bit."""
+    import concrete_fft as cf
+    import numpy as np
+    torch = cuda
+    n = N // 2
+    rng = np.random.default_rng(N + algo)
+    plan = cf.product.U64ProductPlan(N, algo, n)
+    fft = cf.ordered.Plan(n, cf.ordered.Method.UserProvided(algo))
+    warps = -(-min(128, max(1, n >> (algo // 2 + 1))) // 32)
+    line = 5 * torch.cuda.get_device_properties(0).multi_processor_count // warps  # first count that is not few
+    for count in (1, 3, line - 1, line, 2 * line + 5):
+        a = rng.integers(0, 1 << 64, (count, N), dtype=np.uint64)
+        b = rng.integers(-512, 512, (count, N), dtype=np.int64)
+        bhat = torch.empty((count, n), dtype=torch.complex128, device="cuda")
+        plan.prepare_operand(torch.from_numpy(b).cuda(), bhat)
+        want_bhat = oracle.u64_prepare(N, algo, n, b)
+        assert np.array_equal(bhat.cpu().numpy().view(np.uint64), want_bhat.view(np.uint64)), count
+        da = torch.from_numpy(a.view(np.int64)).cuda()
+        out = torch.empty_like(da)
+        plan.product(da, bhat, out)
+        want = oracle.u64_product(N, algo, n, a, want_bhat, nthreads=0)
+        assert np.array_equal(out.cpu().numpy().view(np.uint64), want), count
+        plan.product_sum(da.reshape(count, 1, N), bhat.reshape(count, 1, n), out)
+        want = oracle.u64_product_sum(N, algo, n, a.reshape(count, 1, N), want_bhat.reshape(count, 1, n), nthreads=0)
+        assert np.array_equal(out.cpu().numpy().view(np.uint64), want), (count, "sum")
+        x = rng.uniform(-1, 1, (count, n)) + 1j * rng.uniform(-1, 1, (count, n))
+        d = torch.from_numpy(x.copy()).cuda()
+        fft.fwd(d)
+        assert np.array_equal(d.cpu().numpy().view(np.uint64), oracle.ordered_fwd(algo, x).view(np.uint64)), count

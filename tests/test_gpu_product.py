@@ -462,3 +462,22 @@ def test_u64_product_sum_unfused_chunks(cuda, oracle):
     assert np.array_equal(bhat[sel].cpu().numpy().view(np.uint64), want_bhat.view(np.uint64))
     want = oracle.u64_product_sum(N, 2, 1024, a[sel], want_bhat, nthreads=0)
     assert np.array_equal(out.cpu().numpy().view(np.uint64)[sel], want)
+
+
+@pytest.mark.parametrize("N,algo", [(256, 6), (256, 7), (512, 6), (256, 4), (128, 7)])
+@pytest.mark.parametrize("count", [607, 608, 1217, 1500])
+def test_u64_product_packed_to_a_warp(cuda, oracle, N, algo, count):
+    """Several small products per CTA where a pass over one has less than a warp of butterflies, last CTA ragged."""
+    import concrete_fft as cf
+    torch = cuda
+    rng = np.random.default_rng(N + count)
+    plan = cf.product.U64ProductPlan(N, algo, N // 2)
+    a = rng.integers(0, 2 ** 64, (count, N), dtype=np.uint64)
+    b = rng.integers(-2 ** 7, 2 ** 7, (count, N))
+    bhat = torch.empty((count, N // 2), dtype=torch.complex128, device="cuda")
+    plan.prepare_operand(torch.from_numpy(b).cuda(), bhat)
+    da = torch.from_numpy(a.view(np.int64)).cuda()
+    out = torch.empty_like(da)
+    plan.product(da, bhat, out)
+    want = oracle.u64_product(N, algo, N // 2, a, oracle.u64_prepare(N, algo, N // 2, b), nthreads=0)
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
