@@ -139,7 +139,7 @@ int grid_for(const void* kernel, int threads, size_t smem, long count) {
   return (int)((long)sm_count() * max_blocks_per_sm(kernel, threads, smem));
 }
 
-// Sums of products too large for a cluster (N > 65536), unfused: fold and twist
+// Sums of products that no cluster holds (N > 65536) or too few to fill the SMs, unfused: fold and twist
 // every term, the plan's forward transforms, the Fourier-domain sum per group,
 // one inverse per group, untwist and round.  Groups run in chunks whose
 // workspace (terms + 1 transforms per group) stays within 1 GiB.
@@ -473,15 +473,20 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   // around a workspace of the terms' products.  Below SMs/2 outputs and within the
   // workspace pool; more outputs fill the SMs with one CTA or cluster each.
   const size_t all = count * terms;
+  const long fill = plan->n > (size_t(1) << kBlockLog2Auto) ? (long)sm_count() / 2 : 2L * sm_count();
+  // One term is a product, except where a cluster per product beats the five launches that a
+  // product takes (one of N = 8192 on Dit16/512: 48 us and 58).
+  int p0 = 0, p1 = 0;
+  const bool cluster16 = plan->lv.nlevels > 0 && algo_radix(plan->base_algo) == 16 && plan->N == 8192 &&
+                         !split2_shape(plan, count, &p0, &p1);
+  if (terms == 1 && plan->cluster == 0 && (long)count < fill && !cluster16)
+    return cfft_u64_product(plan, a, bhat, plan->n, out, count, stream);
   if (count > 0 && (long)count < (long)sm_count() / 2 && plan->cluster == 0 && !(plan->base_algo & 1) &&
       all <= kWorkspaceKeep / (plan->n * sizeof(double2))) {
     const int s0 = split0_log2(plan);
     int f0 = 0, f1 = 0, i0 = 0, i1 = 0;
     const bool level = split2_shape(plan, all, &f0, &f1, kForward) && split2_shape(plan, count, &i0, &i1, kInverse);
     cudaStream_t s = (cudaStream_t)stream;
-    if (terms == 1 && s0 >= 1) return launch_split0_product(plan, s0, a, bhat, plan->n, out, count, s);
-    if (terms == 1 && split2_shape(plan, count, &f0, &f1))
-      return launch_split2_product(plan, f0, f1, a, bhat, plan->n, out, count, s);
     if (terms > 1 && (s0 >= 1 || level)) {
       void* ws = nullptr;
       if (plan->workspace.alloc(&ws, all * plan->n * sizeof(double2), s) != cudaSuccess)
@@ -500,6 +505,13 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
       return st;
     }
   }
+  // Otherwise, while the outputs do not fill the SMs, five launches over all terms at once:
+  // one CTA or cluster per output runs its terms one after the other (N = 2048 on Dit4: two
+  // outputs of 8 terms 137 us, five launches 24; 75 of 6 108 and 44; 300 of 4, two CTAs per
+  // SM, 106 and 93; N = 8192 on Dit8/1024: 40 of 3 101 and 90, 75 of 6 186 and 207).
+  if (count > 0 && terms > 1 && plan->cluster == 0 && (long)count < fill &&
+      all + count <= kWorkspaceKeep / (plan->n * sizeof(double2)))
+    return product_sum_unfused(plan, a, bhat, terms, out, count, (cudaStream_t)stream);
   if (plan->N > (size_t(2) << kBlockLog2Auto)) {  // one output per thread-block cluster (N = 8192: by default)
     bool ok = true;
     const int ls = product_split_log2(plan, count, &ok);

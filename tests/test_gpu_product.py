@@ -464,6 +464,33 @@ def test_u64_product_sum_unfused_chunks(cuda, oracle):
     assert np.array_equal(out.cpu().numpy().view(np.uint64)[sel], want)
 
 
+@pytest.mark.parametrize("N,algo,base,count,terms", [(64, 1, 32, 5, 3), (2048, 3, 1024, 2, 8), (2048, 0, 1024, 90, 2),
+                                                     (2048, 7, 1024, 303, 2), (4096, 5, 512, 7, 2),
+                                                     (8192, 4, 512, 2, 8), (8192, 2, 512, 75, 2), (8192, 7, 512, 1, 1),
+                                                     (16384, 2, 1024, 2, 8), (1024, 5, 512, 9, 1)])
+def test_u64_product_sum_of_few_outputs(cuda, oracle, N, algo, base, count, terms):
+    """Sums whose outputs do not fill the SMs: all terms at once, with the bits of the plan forced to one CTA
+    or cluster per output, and of the oracle."""
+    import concrete_fft as cf
+    torch = cuda
+    plan = cf.product.U64ProductPlan(N, algo, base)
+    rng = np.random.default_rng(N + count)
+    a = rng.integers(0, 2 ** 64, (count, terms, N), dtype=np.uint64)
+    b = rng.integers(-2 ** 7, 2 ** 7, (count * terms, N))
+    bhat = torch.empty((count, terms, N // 2), dtype=torch.complex128, device="cuda")
+    plan.prepare_operand(torch.from_numpy(b).cuda(), bhat)
+    da = torch.from_numpy(a.view(np.int64)).cuda()
+    out = torch.empty((count, N), dtype=torch.int64, device="cuda")
+    plan.product_sum(da, bhat, out)
+    want = oracle.u64_product_sum(N, algo, base, a, oracle.u64_prepare(N, algo, base, b).reshape(count, terms, N // 2),
+                                  nthreads=0)
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
+    plan.set_cluster_size(1)
+    other = torch.empty_like(out)
+    plan.product_sum(da, bhat, other)
+    assert torch.equal(out, other)
+
+
 @pytest.mark.parametrize("N,algo", [(256, 6), (256, 7), (512, 6), (256, 4), (128, 7)])
 @pytest.mark.parametrize("count", [607, 608, 1217, 1500])
 def test_u64_product_packed_to_a_warp(cuda, oracle, N, algo, count):
