@@ -470,7 +470,8 @@ def run_gb300(args):
                      "fp64": {"achieved_ops_per_s": fp64_achieved, "peak_ops_per_s": fp64_peak,
                               "frac": fp64_achieved / fp64_peak, "ops_per_product": fp64_ops,
                               "microbenchmark_rates": rates,
-                              "note": "binding roof: FP64 pipe (best DFMA/DADD/DMUL/mix issue rate, measured live)"}},
+                              "note": "the algorithm's FP64 operations against the best DFMA/DADD/DMUL/mix issue rate, "
+                                      "measured live; three additions in four run on the integer pipes, so above 1"}},
         "plain_path": plain,
         "cpu_baseline": cpu,
         "accuracy": accuracy,
@@ -502,29 +503,41 @@ def gpu_setup():
     return torch, cf, rank, world, local
 
 
-def timed(torch, fn, steps, warmup, local, world):
-    """CUDA-event time of `steps` calls of fn (after warm-up), max over ranks, with clocks."""
+def timed(torch, fn, steps, warmup, local, world, restore=None, every=0):
+    """CUDA-event time of `steps` calls of fn (after warm-up), max over ranks, with clocks.
+
+    The transforms are unnormalised, so an in-place forward and inverse multiplies its data by n and a
+    few hundred steps in a row would time infinities and NaN.  `restore` puts the inputs back: after the
+    warm-up and, outside the event pairs that are summed, between every `every` steps."""
     stream = torch.cuda.current_stream()
-    e0 = torch.cuda.Event(enable_timing=True)
-    e1 = torch.cuda.Event(enable_timing=True)
+    every = every if restore is not None else steps
+    pairs = []
     with ClockSampler(local) as clk:
         time.sleep(0.5)
         for _ in range(warmup):
             fn()
+        if restore is not None:
+            restore()
         torch.cuda.synchronize()
         if world > 1:
             torch.distributed.barrier()
         t0 = time.time()
-        e0.record(stream)
-        for _ in range(steps):
-            fn()
-        e1.record(stream)
+        for first in range(0, steps, every):
+            if first:
+                restore()
+            e0 = torch.cuda.Event(enable_timing=True)
+            e1 = torch.cuda.Event(enable_timing=True)
+            e0.record(stream)
+            for _ in range(min(every, steps - first)):
+                fn()
+            e1.record(stream)
+            pairs.append((e0, e1))
         torch.cuda.synchronize()
         if world > 1:
             torch.distributed.barrier()
         clk.mark(t0, time.time())
     from concrete_fft import replicas
-    return replicas.max_over_ranks(e0.elapsed_time(e1), "cuda"), clk.summary()
+    return replicas.max_over_ranks(sum(e0.elapsed_time(e1) for e0, e1 in pairs), "cuda"), clk.summary()
 
 
 def graph_device_us(torch, call, calls=20, replays=10):
@@ -695,8 +708,8 @@ def measure_ordered(torch, cf, steps, warmup, local, world, full=False, cpu_seco
                 "rel_l2_fwd_vs_numpy_fft": rel_l2(got_f, np.fft.fft(x, axis=-1)),
                 "roundtrip_rel_l2": rel_l2(got_i / 1024, x),
                 "bound": "c64 relative L2 <= 1e-13 against the reference (the oracle: same algorithm, same bits)"}
-    d.copy_(torch.from_numpy(x))  # fwd+inv multiplies by n each step: start from the inputs
-    one = d[:1].clone()
+    x0 = torch.from_numpy(x).cuda()
+    one = x0[:1].clone()
 
     def step256():
         plan.fwd(d)
@@ -706,16 +719,20 @@ def measure_ordered(torch, cf, steps, warmup, local, world, full=False, cpu_seco
         plan.fwd(one)
         plan.inv(one)
 
-    ms256, clocks = timed(torch, step256, steps, warmup, local, world)
-    d.copy_(torch.from_numpy(x))
-    ms1, _ = timed(torch, step1, steps, warmup, local, world)
+    def restore1():
+        one.copy_(x0[:1])
+
+    # 2^10 per step: 64 steps stay far below the largest double
+    ms256, clocks = timed(torch, step256, steps, warmup, local, world, lambda: d.copy_(x0), 64)
+    restore1()
+    ms1, _ = timed(torch, step1, steps, warmup, local, world, restore1, 64)
     # device-side batch-1 latency: 20 fwd+inv pairs in one CUDA graph (no host call between)
     graph20 = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph20):
         for _ in range(20):
             step1()
     reps20 = max(5, steps // 10)
-    ms1g20, _ = timed(torch, graph20.replay, reps20, warmup, local, world)
+    ms1g20, _ = timed(torch, graph20.replay, reps20, min(warmup, 4), local, world, restore1, 4)
     per = ms256 * 1e-3 / steps
     ops = 256 * 2 * fp64_ops_ordered(1024, int(algo))
     peak = fp64_peak(cf)
@@ -747,13 +764,15 @@ def measure_ordered(torch, cf, steps, warmup, local, world, full=False, cpu_seco
                      "algorithmic_bytes_per_launch": 256 * 32768,
                      "fp64": {"achieved_ops_per_s": ops / per, "peak_ops_per_s": peak, "frac": ops / per / peak,
                               "ops_per_transform": fp64_ops_ordered(1024, int(algo)),
-                              "note": "binding roof: FP64 pipe"}},
+                              "note": "the algorithm's operations; additions also run on the integer pipes"}},
         "e2e": {"value": e2e, "unit": "transforms/s", "h2d_bytes_per_step": 2 * 256 * 1024 * 16,
                 "d2h_bytes_per_step": 2 * 256 * 1024 * 16, "steps": e2e_steps,
                 "path": "cfft_ordered_fwd_host / _inv_host on a page-locked buffer, in place"},
         "accuracy": accuracy, "clocks": clocks, "gpu_launches": 2 * steps,
     }
     if full:
+        d.copy_(x0)
+        restore1()
         entry["config"].update(ordered_sweeps(torch, cf, plan, d, one, step1, steps, warmup, local, world, rng))
     if cpu and world == 1:
         threads = host_threads()
@@ -787,11 +806,13 @@ def ordered_sweeps(torch, cf, plan, d, one, step1, steps, warmup, local, world, 
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         step1()
-    ms1g, _ = timed(torch, graph.replay, steps, warmup, local, world)
+    one0 = one.clone()
+    ms1g, _ = timed(torch, graph.replay, steps, warmup, local, world, lambda: one.copy_(one0), 64)
     large = {}
     for lgn in (12, 13, 14, 15):
         up = cf.unordered.Plan(1 << lgn, cf.unordered.Method.UserProvided(cf.FftAlgo.Dif4, 1024))
         u1 = torch.from_numpy(rng.uniform(-1, 1, (1, 1 << lgn)) + 0j).cuda()
+        u0 = u1.clone()
 
         def stepu():
             up.fwd(u1)
@@ -799,7 +820,7 @@ def ordered_sweeps(torch, cf, plan, d, one, step1, steps, warmup, local, world, 
         row = {}
         for ctas, name in ((0, "split"), (1, "one_cta_or_levels")):
             up.set_cluster_size(ctas)
-            msu, _ = timed(torch, stepu, max(10, steps // 4), warmup, local, world)
+            msu, _ = timed(torch, stepu, max(10, steps // 4), warmup, local, world, lambda: u1.copy_(u0), 48)
             row[name] = round(msu * 1e3 / max(10, steps // 4), 2)
         large[1 << lgn] = row
     sweep = {}
@@ -815,7 +836,8 @@ def ordered_sweeps(torch, cf, plan, d, one, step1, steps, warmup, local, world, 
             row = {}
             for ctas in (0, 1, 2, 4, 8):
                 sp.set_cluster_size(ctas)
-                ms_b, _ = timed(torch, step_b, max(10, steps // 4), warmup, local, world)
+                ms_b, _ = timed(torch, step_b, max(10, steps // 4), warmup, local, world,
+                                lambda: sub.copy_(d[:len(sub)]), 64)
                 row["auto" if ctas == 0 else ctas] = round(ms_b * 1e3 / max(10, steps // 4), 2)
             sweep[aname][batch] = row
     # the same at batch 256 without spreading one-wave grids over every SM (cfft_diag_set_spread)
@@ -833,7 +855,8 @@ def ordered_sweeps(torch, cf, plan, d, one, step1, steps, warmup, local, world, 
             row = {}
             for ctas in (0, 1, 2, 4, 8):
                 sp.set_cluster_size(ctas)
-                ms_b, _ = timed(torch, step_b, max(10, steps // 4), warmup, local, world)
+                ms_b, _ = timed(torch, step_b, max(10, steps // 4), warmup, local, world,
+                                lambda: sub.copy_(d[:len(sub)]), 64)
                 row["auto" if ctas == 0 else ctas] = round(ms_b * 1e3 / max(10, steps // 4), 2)
             no_spread[aname] = row
     finally:
@@ -876,7 +899,11 @@ def measure_mixed(torch, cf, steps, warmup, local, world, count=100000, tune_sec
     saved = {int(i): data[int(offs[i]):int(offs[i]) + int(sizes[i])].clone() for i in sample}
     stream = torch.cuda.Stream()
     with torch.cuda.stream(stream):
-        ms, clocks = timed(torch, lambda: b.run(data), steps, warmup, local, world)
+        def restore():
+            g.manual_seed(seed)
+            data.copy_(torch.rand((total, 2), dtype=torch.float64, device="cuda", generator=g) * 2 - 1)
+
+        ms, clocks = timed(torch, lambda: b.run(data), steps, warmup, local, world, restore, 48)  # 2^16 per step
         # accuracy: the sampled items from their inputs again, one launch, against the oracle
         for i, v in saved.items():
             data[int(offs[i]):int(offs[i]) + int(sizes[i])].copy_(v)
@@ -941,7 +968,7 @@ def measure_mixed(torch, cf, steps, warmup, local, world, count=100000, tune_sec
                      "traffic": (prof.get("dram_bytes_per_point") * total) if prof.get("dram_bytes_per_point") else None,
                      "algorithmic_bytes_per_launch": bytes_alg,
                      "fp64": {"achieved_ops_per_s": ops / per_launch, "peak_ops_per_s": peak,
-                              "frac": ops / per_launch / peak, "note": "binding roof: FP64 pipe"}},
+                              "frac": ops / per_launch / peak, "note": "the algorithm's operations; additions also run on the integer pipes"}},
         "e2e": {"value": world * transforms * e2e_steps / e2e_s, "unit": "transforms/s",
                 "h2d_bytes_per_step": total * 16, "d2h_bytes_per_step": total * 16, "steps": e2e_steps,
                 "path": "cfft_batch_run_host from page-locked host memory, 16 pipelined chunks"},
@@ -1075,8 +1102,8 @@ def measure_u128(torch, cf, steps, warmup, local, world, full=False, cpu_seconds
         ach = prof["fp64_thread_inst_per_product"] * v
         fp64 = {"achieved_ops_per_s": ach, "peak_ops_per_s": peak, "frac": ach / peak,
                 "ops_per_product": prof["fp64_thread_inst_per_product"],
-                "note": "DADD/DFMA/DMUL per product counted by ncu (N=1024); the FP64 pipe also issues the "
-                        "double-double code's comparisons and conversions"}
+                "note": "DADD/DFMA/DMUL of the algorithm per product (N=1024); its error-free sums and cross "
+                        "products run on the integer pipes, so above 1"}
     # fft128::Plan itself at n = 512 (batch 4096 and batch 1), GPU and the host's restatement
     plans128 = {}
     for n, batch in (((512, 4096), (2048, 1024), (4096, 512), (16384, 128)) if full else ((512, 4096),)):
@@ -1087,13 +1114,22 @@ def measure_u128(torch, cf, steps, warmup, local, world, full=False, cpu_seconds
             fp.fwd(*bufs)
             fp.inv(*bufs)
         s128 = max(5, steps)
-        ms128, _ = timed(torch, step128, s128, warmup, local, world)
-        one = [bb[:1].clone() for bb in bufs]
+        bufs0 = [bb.clone() for bb in bufs]
+
+        def restore128():
+            for bb, b0 in zip(bufs, bufs0):
+                bb.copy_(b0)
+        ms128, _ = timed(torch, step128, s128, warmup, local, world, restore128, 64)
+        one = [b0[:1].clone() for b0 in bufs0]
 
         def step1():
             fp.fwd(*one)
             fp.inv(*one)
-        ms1, _ = timed(torch, step1, max(10, steps), warmup, local, world)
+
+        def restore1():
+            for o, b0 in zip(one, bufs0):
+                o.copy_(b0[:1])
+        ms1, _ = timed(torch, step1, max(10, steps), warmup, local, world, restore1, 64)
         row = {"transforms_per_s": world * 2 * batch * s128 / (ms128 * 1e-3), "batch": batch,
                "batch1_us_per_fwd_inv": round(ms1 * 1e3 / max(10, steps), 2)}
         if cpu and world == 1 and n == 512:
@@ -1130,7 +1166,7 @@ def measure_u128(torch, cf, steps, warmup, local, world, full=False, cpu_seconds
                      "frac": v * 49152 / 1e9 / peaks["hbm_gbs"], "peak_kind": peak_kind,
                      "traffic": prof.get("dram_bytes_per_launch"),
                      "algorithmic_bytes_per_launch": 49152 * count, "fp64": fp64,
-                     "note": "N=1024: 49,152 algorithmic bytes per product; bound by the FP64 pipe"},
+                     "note": "N=1024: 49,152 algorithmic bytes per product; bound by the FP64 and integer pipes"},
         "e2e": e2e,
         "accuracy": {"N%d" % N: r["accuracy"] for N, r in by_n.items()},
         "clocks": clocks, "gpu_launches": 4 * steps,
@@ -1173,14 +1209,26 @@ def reference_case_tables(torch, cf, local, world, cpu=True, cpu_seconds=0.04):
         torch.cuda.synchronize()
         return e0.elapsed_time(e1)
 
-    def device_us(call):
+    def device_us(call, data):
+        saved = [t.clone() for t in data]
         call()  # first call outside the capture (one-time kernel attributes and launch shapes)
         torch.cuda.synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             for _ in range(20):
                 call()
-        return events_ms(graph.replay, 10, 2) * 1e3 / 200
+        pairs = []
+        for _ in range(12):  # each replay from the inputs: 20 unnormalised transforms in a row
+            for t, v in zip(data, saved):
+                t.copy_(v)
+            e0 = torch.cuda.Event(enable_timing=True)
+            e1 = torch.cuda.Event(enable_timing=True)
+            e0.record(stream)
+            graph.replay()
+            e1.record(stream)
+            pairs.append((e0, e1))
+        torch.cuda.synchronize()
+        return sum(a.elapsed_time(b) for a, b in pairs[2:]) * 1e3 / 200
 
     def host_us(call, reps=20):
         call()
@@ -1210,7 +1258,7 @@ def reference_case_tables(torch, cf, local, world, cpu=True, cpu_seconds=0.04):
             row["gpu_ordered_plan"] = op.algo().name
             cases.insert(0, ("ordered_fwd", lambda b: op.fwd(b)))
         for name, fn in cases:
-            r = {"gpu_device_us": round(device_us(lambda: fn(one)), 3),
+            r = {"gpu_device_us": round(device_us(lambda: fn(one), [one]), 3),
                  "host_slice_api_us": round(host_us(lambda: fn(host)), 2)}
             if name != "fwd_monomial":
                 r["gpu_batched_transforms_per_s"] = batched_per_s(lambda: fn(many), batch)
@@ -1237,7 +1285,7 @@ def reference_case_tables(torch, cf, local, world, cpu=True, cpu_seconds=0.04):
         host = [np.random.default_rng(k).uniform(-1, 1, (1, n)) for _ in range(4)]
         row = {}
         for name, fn in (("fwd", fp.fwd), ("inv", fp.inv)):
-            row[name] = {"gpu_device_us": round(device_us(lambda: fn(*one)), 3),
+            row[name] = {"gpu_device_us": round(device_us(lambda: fn(*one), one), 3),
                          "host_slice_api_us": round(host_us(lambda: fn(*host)), 2),
                          "gpu_batched_transforms_per_s": batched_per_s(lambda: fn(*many), batch)}
             if cpu and world == 1:
@@ -1257,7 +1305,7 @@ def measure_reference_cases(torch, cf, local, world, cpu=True, cpu_seconds=0.04)
     return {"c64": rows, "fft128": f128rows, "clocks": clk.summary(),
             "cpu": "restated reference, one host thread, scalar (the reference's own Scalar backend on this Arm "
                    "host), each call timed in a loop in C as criterion does",
-            "gpu_device": "20 calls of one transform in a CUDA graph, replayed 10 times, CUDA events",
+            "gpu_device": "20 calls of one transform in a CUDA graph, replayed 10 times from the inputs, CUDA events",
             "host_slice_api": "cfft_*_fwd_host / _inv_host / fwd_monomial_host on a pageable numpy buffer, from "
                               "Python (staged copies in and out)"}
 
@@ -1661,7 +1709,7 @@ def measure_latency(torch, cf, local, world, cpu=True, cpu_seconds=0.5, profile_
             rows["u128_product_N%d" % N] = row
         clk.mark(t0, time.time())
     return {"rows": rows, "clocks": clk.summary(),
-            "gpu": "device time per call: 20 calls captured in a CUDA graph, replayed 10 times, CUDA events",
+            "gpu": "device time per call: 20 calls captured in a CUDA graph, replayed 10 times from the inputs, CUDA events",
             "cpu": "the restated reference pipeline on one host core with the plan's algorithm, per product over "
                    "calls of 32 products (8 for u128), so that the plan's set-up is spread as for a prepared plan"}
 

@@ -28,7 +28,7 @@ class U64ProductPlan:
             self._h = None
 
     def set_int_adds(self, eighths):
-        """Share (in eighths) of butterfly additions issued on the integer pipe; results are unchanged."""
+        """Kept with the plan (0..8): the kernels choose the integer-pipe share of the additions themselves."""
         check(self._lib.cfft_u64_product_set_int_adds(self._h, int(eighths)))
 
     def int_adds(self):

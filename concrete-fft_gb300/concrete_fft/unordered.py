@@ -49,7 +49,7 @@ class Plan:
         return FftAlgo(a.value), b.value
 
     def set_int_adds(self, eighths):
-        """Share (in eighths) of butterfly additions issued on the integer pipe; results are unchanged."""
+        """Kept with the plan (0..8): the kernels choose the integer-pipe share of the additions themselves."""
         check(self._lib.cfft_unordered_set_int_adds(self._h, int(eighths)))
 
     def set_cluster_size(self, ctas):

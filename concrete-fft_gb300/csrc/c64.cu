@@ -165,7 +165,7 @@ DevLevels to_dev(const LevelDesc& l) {
   return d;
 }
 
-// First level of at most 2048 points (measured, fwd+inv, Dif16 base 1024:
+// First level of at most 2048 points (fwd+inv, Dif16 base 1024, additions on the FP64 pipe:
 // n = 4096 x 4096 transforms 2527 vs 2864 us with 4096-point blocks; n = 32768
 // x 512: 3195 vs 3530 us; n = 2^18 x 64: 3862 vs 4197 us).  Plans whose levels
 // skip from above 4096 points to the base keep the first level of at most 4096.
@@ -298,7 +298,7 @@ int split_log2(const C64Plan& p, long batch, int* mode) {
   if (min_ls > 0) {
     // transforms above one CTA's shared memory: a cluster of 8 SMs beats the global-level
     // path (all SMs, several launches) only up to 8192 points and for small batches
-    // (measured, batch 1 fwd+inv: 37 vs 47 us at 8192, 70 vs 72 at 16384, 131 vs 123 at 32768)
+    // (batch 1 fwd+inv, additions on the FP64 pipe as such launches keep them: 37 vs 47 us at 8192, 70 vs 72 at 16384, 131 vs 123 at 32768)
     if (log2n > 13 || (batch << max_ls) >= target) return 0;
     return max_ls;
   }

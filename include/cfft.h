@@ -99,10 +99,12 @@ cfft_status cfft_ordered_fwd_host(const cfft_ordered_plan* plan, double* buf, si
 cfft_status cfft_ordered_inv_host(const cfft_ordered_plan* plan, double* buf, size_t batch);
 
 /* Integer-pipe share of the butterfly additions (no counterpart in the
- * reference).  GB300 issues FP64 at 1/64 of its integer rate; `eighths` (0..8)
- * of every butterfly's additions run as an exact integer-pipe IEEE add
- * instead, alongside the FP64 pipe.  Results are bit-identical for every
- * value; only the speed changes.  Measure-created plans tune it themselves. */
+ * reference).  GB300 issues FP64 at 1/64 of its integer rate, so the kernels
+ * run three in four of a butterfly's additions as exact IEEE additions on the
+ * integer pipes, and none in launches of about a warp per SM sub-partition.
+ * That share is the kernels' own: `eighths` (0..8, checked) is kept with the
+ * plan and its saved tuning and given back, and changes neither speed nor
+ * results. */
 cfft_status cfft_ordered_set_int_adds(cfft_ordered_plan* plan, int eighths);
 int cfft_ordered_int_adds(const cfft_ordered_plan* plan);
 
@@ -288,12 +290,12 @@ cfft_status cfft_u64_product_host(const cfft_u64_product_plan* plan, const uint6
  * mod (X^N + 1), every term transformed forward, multiplied and accumulated
  * in term order, then one inverse per group instead of one per term.
  * a: count * terms * N u64; bhat: count * terms * N/2 c64; out: count * N u64.
- * N <= 2^29: one output per CTA up to 8192 (fewer than SMs/2 outputs of a plan
- * on a DIF base without an outer level or with one of radix 2, 4 or 8: one
- * thread-block cluster each), per
- * thread-block cluster up to 16384 (65536 with a forced cluster size), and
- * from 32768 the unfused steps on a stream-ordered workspace of at most 1 GiB
- * (groups in chunks). */
+ * N <= 2^29: one output per CTA up to 4096, per thread-block cluster up to
+ * 16384 (65536 with a forced cluster size), and from 32768 the unfused steps on
+ * a stream-ordered workspace of at most 1 GiB (groups in chunks).  Outputs that
+ * do not fill the SMs run all their terms at once, around a workspace of at
+ * most 256 MiB: in two launches (fewer than SMs/2 outputs of a plan on a DIF
+ * base without an outer level or with one of radix 2, 4 or 8) or unfused. */
 cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64_t* a, const double* bhat,
                                  size_t terms, uint64_t* out, size_t count, void* stream);
 
