@@ -663,18 +663,37 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
   // 4096, 37 vs 39 us at 8192; from SMs/4 products of N = 8192 the cluster kernel is faster)
   const bool few_mid = plan->cluster == 0 && plan->N >= 4096 && plan->N <= 8192 &&
                        (long)count < (long)sm_count() / 4;
-  if (!ok || (plan->N >= 32768 && plan->cluster == 0) || few_unsplit || few_mid) {
+  // N = 4096 to 16384 from 4 products per SM (2 at 16384): whole transforms of 2048 points
+  // run 3 CTAs per SM with the additions on the integer pipes, where the product kernels wait
+  // for their clusters and, at N = 4096, for 128 threads per 2048 points.  2000 products,
+  // kernel / five launches: N = 4096 on Dif4/1024 1.07, on Dif8/512 1.13; 8192 1.12 and 1.13;
+  // 16384 1.12 and 1.16.  With fewer both are uneven (300 of N = 8192: 0.95 and 0.82).
+  const long per_sm = (long)count / sm_count();
+  const bool large = plan->cluster == 0 && plan->lv.nlevels > 0 && plan->N >= 4096 && plan->N <= 16384 &&
+                     per_sm >= (plan->N == 16384 ? 2 : 4);
+  if (!ok || (plan->N >= 32768 && plan->cluster == 0) || few_unsplit || few_mid || large) {
     cudaStream_t s = (cudaStream_t)stream;
+    // `large` calls have another route: in equal parts within the workspace the plan keeps
+    const size_t fit = large ? std::max<size_t>(1, kWorkspaceKeep / (plan->n * sizeof(double2))) : count;
+    const size_t parts = (count + fit - 1) / fit, part = (count + parts - 1) / parts;
     void* z = nullptr;
-    if (plan->workspace.alloc((void**)&z, count * plan->n * sizeof(double2), s) != cudaSuccess)
-      return fail(CFFT_ERR_OUT_OF_MEMORY, "u64 product workspace");
-    cfft_status st = cfft_u64_fold_twist(plan, a, (double*)z, count, stream);
-    if (st == CFFT_OK) st = cfft_unordered_fwd(plan->fft, (double*)z, count, stream);
-    if (st == CFFT_OK) st = cfft_c64_pointwise(bhat, bhat_stride, (double*)z, plan->n, count, stream);
-    if (st == CFFT_OK) st = cfft_unordered_inv(plan->fft, (double*)z, count, stream);
-    if (st == CFFT_OK) st = cfft_u64_untwist_round(plan, (const double*)z, out, count, stream);
-    cudaFreeAsync(z, s);
-    return st;
+    const bool got = plan->workspace.alloc((void**)&z, part * plan->n * sizeof(double2), s) == cudaSuccess;
+    if (!got && !large) return fail(CFFT_ERR_OUT_OF_MEMORY, "u64 product workspace");
+    if (got) {
+      cfft_status st = CFFT_OK;
+      for (size_t c0 = 0; c0 < count && st == CFFT_OK; c0 += part) {
+        const size_t c = std::min(part, count - c0);
+        st = cfft_u64_fold_twist(plan, a + c0 * plan->N, (double*)z, c, stream);
+        if (st == CFFT_OK) st = cfft_unordered_fwd(plan->fft, (double*)z, c, stream);
+        if (st == CFFT_OK)
+          st = cfft_c64_pointwise(bhat + 2 * c0 * bhat_stride, bhat_stride, (double*)z, plan->n, c, stream);
+        if (st == CFFT_OK) st = cfft_unordered_inv(plan->fft, (double*)z, c, stream);
+        if (st == CFFT_OK) st = cfft_u64_untwist_round(plan, (const double*)z, out + c0 * plan->N, c, stream);
+      }
+      cudaFreeAsync(z, s);
+      return st;
+    }
+    cudaGetLastError();  // no workspace: the product kernels below need none
   }
   if (ls > 0) return launch_split_product(plan, ls, a, bhat, bhat_stride, out, count, (cudaStream_t)stream);
   return launch_product(plan, a, bhat, bhat_stride, out, count, (cudaStream_t)stream);

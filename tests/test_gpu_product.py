@@ -508,3 +508,34 @@ def test_u64_product_packed_to_a_warp(cuda, oracle, N, algo, count):
     plan.product(da, bhat, out)
     want = oracle.u64_product(N, algo, N // 2, a, oracle.u64_prepare(N, algo, N // 2, b), nthreads=0)
     assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("N,algo,base", [(4096, 2, 1024), (8192, 5, 512), (16384, 4, 1024)])
+@pytest.mark.parametrize("shared", [False, True])
+def test_u64_product_many_large(cuda, oracle, N, algo, base, shared):
+    """N = 4096 to 16384 on both sides of the five launches' line, and in several parts, against the kernels."""
+    import concrete_fft as cf
+    torch = cuda
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    line = sms * (2 if N == 16384 else 4)
+    part = (1 << 28) // (8 * N)
+    plan = cf.product.U64ProductPlan(N, algo, base)
+    g = torch.Generator(device="cuda").manual_seed(N)
+    for count in (line - 1, line, line + 3) + ((2 * part + 5,) if N == 16384 else ()):
+        a = torch.randint(-2 ** 63, 2 ** 63 - 1, (count, N), generator=g, device="cuda")
+        b = torch.randint(-128, 128, (1 if shared else count, N), generator=g, device="cuda")
+        bhat = torch.empty((b.shape[0], N // 2), dtype=torch.complex128, device="cuda")
+        plan.prepare_operand(b, bhat)
+        if shared:
+            bhat = bhat[0]
+        out, other = torch.empty_like(a), torch.empty_like(a)
+        plan.set_cluster_size(0)
+        plan.product(a, bhat, out, shared)
+        plan.set_cluster_size(2)
+        plan.product(a, bhat, other, shared)
+        assert torch.equal(out, other), count
+        ha = a[:2].cpu().numpy().view(np.uint64)
+        hb = oracle.u64_prepare(N, algo, base, b[:1 if shared else 2].cpu().numpy())
+        if shared:
+            hb = np.repeat(hb, 2, axis=0)
+        assert np.array_equal(out[:2].cpu().numpy().view(np.uint64), oracle.u64_product(N, algo, base, ha, hb, nthreads=0))
