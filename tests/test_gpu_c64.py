@@ -459,3 +459,24 @@ def test_invalid_calls_raise(cuda):
     u = cf.unordered.Plan(64, cf.unordered.Method.UserProvided(0, 64))
     with pytest.raises(cf.CfftError):
         u.fwd_monomial(64, torch.zeros(64, dtype=torch.complex128, device="cuda"))
+
+
+@pytest.mark.parametrize("n,base,algo", [(512, 512, 0), (1024, 1024, 2), (1024, 512, 1), (2048, 1024, 3), (2048, 512, 2)])
+def test_four_to_five_transforms_per_sm(cuda, n, base, algo):
+    """Batches around the lines between two CTAs and one per transform give the bits of one CTA each."""
+    import concrete_fft as cf
+    torch = cuda
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    plan = cf.unordered.Plan(n, cf.unordered.Method.UserProvided(algo, base))
+    for batch in (4 * sms - 1, 4 * sms, 4 * sms + 5, 5 * sms - 1, 5 * sms):
+        x = torch.randn(batch, n, dtype=torch.complex128, device="cuda")
+        y, z = x.clone(), x.clone()
+        plan.set_cluster_size(0)
+        plan.fwd(y)
+        plan.set_cluster_size(1)
+        plan.fwd(z)
+        assert torch.equal(torch.view_as_real(y).view(torch.int64), torch.view_as_real(z).view(torch.int64)), batch
+        plan.inv(z)
+        plan.set_cluster_size(0)
+        plan.inv(y)
+        assert torch.equal(torch.view_as_real(y).view(torch.int64), torch.view_as_real(z).view(torch.int64)), batch
