@@ -317,9 +317,11 @@ int split_log2(const C64Plan& p, long batch, int* mode) {
   // 4 to 5 transforms per SM on radix 2 or 4: whole, a fifth on some SMs doubles their last
   // round; two CTAs each halve it (613 forwards of 2048 points on Dif4: 69.0 us, 64.6; of
   // 1024 32.2 and 28.4, on Dif2 36.1 and 31.4).  From 6 per SM the exchange costs as much
-  // (1000 of 2048 points: 94 and 99), at radix 8 from the start (613 of 1024: 32.4 and 36.1),
-  // and at 4096 points one CTA per SM holds half a transform (613: 121 and 132)
-  if (ls == 0 && max_ls >= 1 && p.base_algo < 4 && log2n >= 9 && log2n <= kBlockLog2Auto && batch < 5L * sm_count())
+  // (1000 of 2048 points: 94 and 99), at radix 8 from the start (613 of 1024: 32.4 and 36.1)
+  // but for Dif8 under an outer level (613 of 2048: 71.6 and 61.9 on 1024, 65.9 and 61.6 on
+  // 512), and at 4096 points one CTA per SM holds half a transform (613: 121 and 132)
+  const bool split_wins = p.base_algo < 4 || (p.base_algo == CFFT_DIF8 && p.lv.nlevels > 0 && log2n == kBlockLog2Auto);
+  if (ls == 0 && max_ls >= 1 && split_wins && log2n >= 9 && log2n <= kBlockLog2Auto && batch < 5L * sm_count())
     ls = 1;
   return ls;
 }

@@ -461,7 +461,8 @@ def test_invalid_calls_raise(cuda):
         u.fwd_monomial(64, torch.zeros(64, dtype=torch.complex128, device="cuda"))
 
 
-@pytest.mark.parametrize("n,base,algo", [(512, 512, 0), (1024, 1024, 2), (1024, 512, 1), (2048, 1024, 3), (2048, 512, 2)])
+@pytest.mark.parametrize("n,base,algo", [(512, 512, 0), (1024, 1024, 2), (1024, 512, 1), (2048, 1024, 3), (2048, 512, 2),
+                                         (2048, 512, 4), (2048, 1024, 4)])
 def test_four_to_five_transforms_per_sm(cuda, n, base, algo):
     """Batches around the lines between two CTAs and one per transform give the bits of one CTA each."""
     import concrete_fft as cf
