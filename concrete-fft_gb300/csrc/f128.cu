@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(256) u128_prepare_kernel(const int64_t* __rest
 }
 
 
-// ---- u128 products above N = 8192: the same steps as separate kernels around
+// ---- u128 products from N = 4096, and a few from N = 1024: the same steps as separate kernels around
 // the fft128 plan's transform (global stages + shared-memory blocks), on a
 // workspace of four arrays of count x n f64 (the plan's batch layout).
 
@@ -1055,38 +1055,42 @@ cfft_status cfft_u128_product(const cfft_u128_product_plan* p, const uint64_t* a
   // whose CTA of 2048 points and more leaves 8 to 24 warps per SM (512 products of
   // N = 4096: 1001 us fused, 908 as five launches; 200 of N = 8192: 1272 and 790; 1024
   // of N = 2048: 838 and 853).  The workspace is at most 1 GiB: larger batches go
-  // through it in parts.
+  // through it in parts.  N up to 8192 runs fused where no workspace can be had.
+  const bool fused_fits = p->f.n <= (size_t(1) << kF128SmemLog2);
   if (p->f.n >= 2048 || (few && p->f.n >= 512)) {
     cudaStream_t s = (cudaStream_t)stream;
     const int log2n = ilog2(p->f.n);
     const size_t part = std::min(count, std::max<size_t>(1, (size_t(1) << 30) / (32 * p->f.n)));
     F128Arrays z;
     cfft_status st = workspace_alloc(p->workspace, part, p->f.n, s, &z);
-    if (st != CFFT_OK) return st;
-    for (size_t first = 0; first < count && st == CFFT_OK; first += part) {
-      const size_t c = std::min(part, count - first);
-      const long total = (long)c << log2n;
-      const uint64_t* pa = a + first * 2 * p->N;
-      uint64_t* po = out + first * 2 * p->N;
-      if (launch_dependent(u128_fold_kernel, elementwise_grid(2 * total), 256, 0, s, pa, z, (long)c, log2n) != cudaSuccess)
-        st = fail(CFFT_ERR_CUDA, "fold launch");
-      if (st == CFFT_OK)
-        st = run_f128_tw(p->f.n, p->f.tw(), z.re0, z.re1, z.im0, z.im1, c, true, s, p->f.block_log2);
-      if (st == CFFT_OK)
-        st = launch_dependent(u128_pointwise_kernel, elementwise_grid(total), 256, 0, s, z,
-                              bhat4 + first * bhat_stride, (long)bhat_stride, (long)c, log2n) == cudaSuccess
-                 ? CFFT_OK
-                 : fail(CFFT_ERR_CUDA, "pointwise launch");
-      if (st == CFFT_OK)
-        st = run_f128_tw(p->f.n, p->f.tw(), z.re0, z.re1, z.im0, z.im1, c, false, s, p->f.block_log2);
-      if (st == CFFT_OK)
-        st = launch_dependent(u128_round_kernel, elementwise_grid(2 * total), 256, 0, s, z, po, (long)c, log2n) ==
-                     cudaSuccess
-                 ? CFFT_OK
-                 : fail(CFFT_ERR_CUDA, "round launch");
+    if (st != CFFT_OK && !fused_fits) return st;
+    if (st == CFFT_OK) {
+      for (size_t first = 0; first < count && st == CFFT_OK; first += part) {
+        const size_t c = std::min(part, count - first);
+        const long total = (long)c << log2n;
+        const uint64_t* pa = a + first * 2 * p->N;
+        uint64_t* po = out + first * 2 * p->N;
+        if (launch_dependent(u128_fold_kernel, elementwise_grid(2 * total), 256, 0, s, pa, z, (long)c, log2n) !=
+            cudaSuccess)
+          st = fail(CFFT_ERR_CUDA, "fold launch");
+        if (st == CFFT_OK)
+          st = run_f128_tw(p->f.n, p->f.tw(), z.re0, z.re1, z.im0, z.im1, c, true, s, p->f.block_log2);
+        if (st == CFFT_OK)
+          st = launch_dependent(u128_pointwise_kernel, elementwise_grid(total), 256, 0, s, z,
+                                bhat4 + first * bhat_stride, (long)bhat_stride, (long)c, log2n) == cudaSuccess
+                   ? CFFT_OK
+                   : fail(CFFT_ERR_CUDA, "pointwise launch");
+        if (st == CFFT_OK)
+          st = run_f128_tw(p->f.n, p->f.tw(), z.re0, z.re1, z.im0, z.im1, c, false, s, p->f.block_log2);
+        if (st == CFFT_OK)
+          st = launch_dependent(u128_round_kernel, elementwise_grid(2 * total), 256, 0, s, z, po, (long)c, log2n) ==
+                       cudaSuccess
+                   ? CFFT_OK
+                   : fail(CFFT_ERR_CUDA, "round launch");
+      }
+      cudaFreeAsync(z.re0, s);
+      return st;
     }
-    cudaFreeAsync(z.re0, s);
-    return st;
   }
   const int log2n = ilog2(p->f.n);
   // a thread per butterfly of a stage, up to 256: the integer pipes need the warps, and

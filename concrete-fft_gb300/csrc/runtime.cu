@@ -335,6 +335,17 @@ WorkspaceUser::~WorkspaceUser() {
     for (const DevicePool& p : w.pools) cudaMemPoolTrimTo(p.pool, 0);
 }
 
+namespace {
+thread_local size_t g_workspace_limit = ~size_t(0);  // cfft_diag_set_workspace_limit
+}
+cudaError_t WorkspaceUser::alloc(void** ptr, size_t bytes, cudaStream_t stream) const {
+  // above the limit, CUDA's own refusal of more memory than any device has
+  if (bytes > g_workspace_limit) bytes = size_t(1) << 60;
+  const cudaError_t e = pool ? cudaMallocFromPoolAsync(ptr, bytes, pool, stream) : cudaMallocAsync(ptr, bytes, stream);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 cfft_status ensure_smem(const void* fn, size_t smem) { return ensure_smem_attr(fn, smem); }
 
 int max_blocks_per_sm(const void* fn, int block, size_t smem) {
@@ -704,6 +715,11 @@ cfft_status fill_timing_doubles(double* p, size_t count, double scale, cudaStrea
   return CFFT_OK;
 }
 }  // namespace cfft
+
+extern "C" cfft_status cfft_diag_set_workspace_limit(size_t bytes) {
+  cfft::g_workspace_limit = bytes == 0 ? ~size_t(0) : bytes;
+  return CFFT_OK;
+}
 
 extern "C" cfft_status cfft_diag_dadd_check(uint64_t count, uint64_t seed, uint64_t* mismatches, uint64_t* bad_pair) {
   if (!mismatches) return cfft::fail(CFFT_ERR_INVALID_ARGUMENT, "null output pointer");

@@ -139,9 +139,9 @@ constexpr unsigned long long kWorkspaceKeep = 256ull << 20;
 struct WorkspaceUser {
   WorkspaceUser();  // makes the pool of the current device, the plan's, if there is none
   ~WorkspaceUser();
-  cudaError_t alloc(void** ptr, size_t bytes, cudaStream_t stream) const {
-    return pool ? cudaMallocFromPoolAsync(ptr, bytes, pool, stream) : cudaMallocAsync(ptr, bytes, stream);
-  }
+  // A failure leaves no CUDA error behind: the caller reports it, or runs kernels that need
+  // no workspace, whose launch checks would otherwise find it.
+  cudaError_t alloc(void** ptr, size_t bytes, cudaStream_t stream) const;
   cudaMemPool_t pool = nullptr;
   WorkspaceUser(const WorkspaceUser&) = delete;
   WorkspaceUser& operator=(const WorkspaceUser&) = delete;

@@ -54,6 +54,11 @@ cfft_status cfft_diag_set_spread(int on);
  * Process-wide; for measurement. */
 cfft_status cfft_diag_set_host_chunks(int chunks, int slots, int first, int last);
 
+/* The calling thread's product calls fail to allocate a workspace of more than
+ * `bytes` (0: no limit, the default), as on a full device.  For tests of what
+ * the calls do then. */
+cfft_status cfft_diag_set_workspace_limit(size_t bytes);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,50 @@
+"""Product calls whose workspace cannot be had: the kernels without a workspace run."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+class no_workspace:
+    """The calling thread's product calls find no memory for a workspace (cfft_diag_set_workspace_limit)."""
+
+    def __enter__(self):
+        import concrete_fft as cf
+        cf.check(cf.load().cfft_diag_set_workspace_limit(1))
+
+    def __exit__(self, *exc):
+        import concrete_fft as cf
+        cf.check(cf.load().cfft_diag_set_workspace_limit(0))
+
+
+def u128_case(torch, N, count):
+    import concrete_fft as cf
+    g = torch.Generator(device="cuda").manual_seed(N + count)
+    plan = cf.product.U128ProductPlan(N)
+    a = torch.randint(-(1 << 63), (1 << 63) - 1, (count, N, 2), generator=g, device="cuda")
+    bhat = torch.empty((1, 4, N // 2), dtype=torch.float64, device="cuda")
+    plan.prepare_operand(torch.randint(-128, 128, (1, N), generator=g, device="cuda"), bhat)
+    return plan, lambda out: plan.product(a, bhat, out, shared_operand=True), torch.empty_like(a)
+
+
+@pytest.mark.parametrize("N,count", [(4096, 80), (8192, 78), (8192, 3), (2048, 20)])
+def test_u128_product_without_workspace(cuda, N, count):
+    plan, product, want = u128_case(cuda, N, count)
+    product(want)
+    out = want.clone().fill_(-1)
+    with no_workspace():
+        product(out)
+    assert cuda.equal(out, want)
+
+
+def test_u128_product_that_needs_a_workspace(cuda):
+    """Refused as out of memory, and nothing of that is left for the launch check of the next call."""
+    import concrete_fft as cf
+    plan, product, want = u128_case(cuda, 16384, 3)
+    fused, fused_product, fused_out = u128_case(cuda, 1024, 200)
+    product(want)
+    out = want.clone().fill_(-1)
+    with no_workspace(), pytest.raises(cf.CfftError, match="workspace"):
+        product(out)
+    fused_product(fused_out)
+    product(out)
+    assert cuda.equal(out, want)
