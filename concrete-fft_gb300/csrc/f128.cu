@@ -1055,9 +1055,11 @@ cfft_status cfft_u128_product(const cfft_u128_product_plan* p, const uint64_t* a
   // whose CTA of 2048 points and more leaves 8 to 24 warps per SM (512 products of
   // N = 4096: 1001 us fused, 908 as five launches; 200 of N = 8192: 1272 and 790; 1024
   // of N = 2048: 838 and 853).  The workspace is at most 1 GiB: larger batches go
-  // through it in parts.  N up to 8192 runs fused where no workspace can be had.
+  // through it in parts.  N up to 8192 runs fused where no workspace can be had and, but
+  // for the few, where the stream is captured (stream_capturing).
   const bool fused_fits = p->f.n <= (size_t(1) << kF128SmemLog2);
-  if (p->f.n >= 2048 || (few && p->f.n >= 512)) {
+  if (!fused_fits || (few && p->f.n >= 512) ||
+      (p->f.n >= 2048 && !stream_capturing((cudaStream_t)stream))) {
     cudaStream_t s = (cudaStream_t)stream;
     const int log2n = ilog2(p->f.n);
     const size_t part = std::min(count, std::max<size_t>(1, (size_t(1) << 30) / (32 * p->f.n)));

@@ -345,6 +345,14 @@ cudaError_t WorkspaceUser::alloc(void** ptr, size_t bytes, cudaStream_t stream) 
   if (e != cudaSuccess) cudaGetLastError();
   return e;
 }
+bool stream_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) {  // the legacy stream while another one is captured
+    cudaGetLastError();
+    return false;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
 
 cfft_status ensure_smem(const void* fn, size_t smem) { return ensure_smem_attr(fn, smem); }
 

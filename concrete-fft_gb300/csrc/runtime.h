@@ -146,6 +146,10 @@ struct WorkspaceUser {
   WorkspaceUser(const WorkspaceUser&) = delete;
   WorkspaceUser& operator=(const WorkspaceUser&) = delete;
 };
+// Whether `stream` is being captured.  A workspace allocated there becomes nodes of the
+// graph, and CUDA then allows one instance of it at a time and no child graph of it; a call
+// that also has kernels without a workspace takes those, and its graph stays unrestricted.
+bool stream_capturing(cudaStream_t stream);
 // Input for timing candidates (Method::Measure, the batch tuner): 64-bit words, uniform as
 // integers, or doubles uniform in [-scale, scale).  Zeros would not do: the butterflies'
 // integer path (int_fp64.cuh) leaves them to the FP64 pipe.

@@ -465,7 +465,8 @@ cfft_status cfft_server_run_alone(cfft_server* server, const cfft_serve_config* 
  * N = 1024, five launches around the plan's transform on a stream-ordered
  * workspace (2N f64 per product, at most 1 GiB or one product at a time, freed
  * on the stream).  Up to N = 8192 a call that cannot have its workspace runs the
- * fused kernel.  bhat holds 4 arrays of N/2 f64
+ * fused kernel, as do calls of SMs/2 products and more on a stream under
+ * capture, whose graphs then hold no allocation.  bhat holds 4 arrays of N/2 f64
  * (re0, re1, im0, im1) per operand; bhat_stride is 0 or 2N (doubles). */
 typedef struct cfft_u128_product_plan cfft_u128_product_plan;
 cfft_status cfft_u128_product_plan_create(size_t N, cfft_u128_product_plan** out);

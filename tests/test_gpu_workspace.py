@@ -1,4 +1,6 @@
-"""Product calls whose workspace cannot be had: the kernels without a workspace run."""
+"""Product calls whose workspace cannot be had, or whose stream is captured: the kernels without a workspace run."""
+import ctypes
+
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -14,6 +16,39 @@ class no_workspace:
     def __exit__(self, *exc):
         import concrete_fft as cf
         cf.check(cf.load().cfft_diag_set_workspace_limit(0))
+
+
+def run_two_instances(torch, call, wipe):
+    """Captures call(), makes two instances of the graph and launches each, with wipe() before; a graph with
+    allocation nodes can have one only.  Yields after each launch."""
+    cu = ctypes.CDLL("libcuda.so.1")
+
+    def ok(status, what):
+        assert status == 0, (what, status)
+
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    s, graph = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p()
+    with torch.cuda.stream(stream):
+        call()  # kernel attributes are set once, outside the capture
+        stream.synchronize()
+        ok(cu.cuStreamBeginCapture_v2(s, 1), "begin")
+        try:
+            call()
+        finally:
+            end = cu.cuStreamEndCapture(s, ctypes.byref(graph))
+        ok(end, "end")
+        execs = [ctypes.c_void_p(), ctypes.c_void_p()]
+        for e in execs:
+            ok(cu.cuGraphInstantiateWithFlags(ctypes.byref(e), graph, ctypes.c_ulonglong(0)), "instance")
+        for e in execs:
+            wipe()
+            ok(cu.cuGraphLaunch(e, s), "launch")
+            stream.synchronize()
+            yield
+        for e in execs:
+            ok(cu.cuGraphExecDestroy(e), "destroy")
+        ok(cu.cuGraphDestroy(graph), "destroy")
 
 
 def u128_case(torch, N, count):
@@ -48,3 +83,12 @@ def test_u128_product_that_needs_a_workspace(cuda):
     fused_product(fused_out)
     product(out)
     assert cuda.equal(out, want)
+
+
+@pytest.mark.parametrize("N,count", [(4096, 80), (8192, 78)])
+def test_u128_product_captured_without_allocations(cuda, N, count):
+    plan, product, want = u128_case(cuda, N, count)
+    product(want)
+    out = want.clone()
+    for _ in run_two_instances(cuda, lambda: product(out), lambda: out.fill_(-1)):
+        assert cuda.equal(out, want)
