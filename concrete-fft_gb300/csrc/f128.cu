@@ -1054,15 +1054,15 @@ cfft_status cfft_u128_product(const cfft_u128_product_plan* p, const uint64_t* a
   // as five launches around the plan's transform.  Bit-identical to the fused kernel,
   // whose CTA of 2048 points and more leaves 8 to 24 warps per SM (512 products of
   // N = 4096: 1001 us fused, 908 as five launches; 200 of N = 8192: 1272 and 790; 1024
-  // of N = 2048: 838 and 853).  The workspace is at most 1 GiB: larger batches go
-  // through it in parts.  N up to 8192 runs fused where no workspace can be had and, but
+  // of N = 2048: 838 and 853).  The workspace is at most what the pool keeps: larger
+  // batches go through it in parts.  N up to 8192 runs fused where no workspace can be had and, but
   // for the few, where the stream is captured (stream_capturing).
   const bool fused_fits = p->f.n <= (size_t(1) << kF128SmemLog2);
   if (!fused_fits || (few && p->f.n >= 512) ||
       (p->f.n >= 2048 && !stream_capturing((cudaStream_t)stream))) {
     cudaStream_t s = (cudaStream_t)stream;
     const int log2n = ilog2(p->f.n);
-    const size_t part = std::min(count, std::max<size_t>(1, (size_t(1) << 30) / (32 * p->f.n)));
+    const size_t part = std::min(count, std::max<size_t>(1, kWorkspaceKeep / (32 * p->f.n)));
     F128Arrays z;
     cfft_status st = workspace_alloc(p->workspace, part, p->f.n, s, &z);
     if (st != CFFT_OK && !fused_fits) return st;

@@ -142,11 +142,11 @@ int grid_for(const void* kernel, int threads, size_t smem, long count) {
 // Sums of products that no cluster holds (N > 65536) or too few to fill the SMs, unfused: fold and twist
 // every term, the plan's forward transforms, the Fourier-domain sum per group,
 // one inverse per group, untwist and round.  Groups run in chunks whose
-// workspace (terms + 1 transforms per group) stays within 1 GiB.
+// workspace (terms + 1 transforms per group) stays within what the pool keeps.
 cfft_status product_sum_unfused(const cfft_u64_product_plan* plan, const uint64_t* a, const double* bhat,
                                 size_t terms, uint64_t* out, size_t count, cudaStream_t s) {
   const size_t n = plan->n, per_group = (terms + 1) * n * sizeof(double2);
-  const size_t chunk = std::min(count, std::max<size_t>(1, (size_t(1) << 30) / per_group));
+  const size_t chunk = std::min(count, std::max<size_t>(1, kWorkspaceKeep / per_group));
   void* ws = nullptr;
   if (plan->workspace.alloc((void**)&ws, chunk * per_group, s) != cudaSuccess)
     return fail(CFFT_ERR_OUT_OF_MEMORY, "product sum workspace");
@@ -482,7 +482,7 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   if (terms == 1 && plan->cluster == 0 && (long)count < fill && !cluster16)
     return cfft_u64_product(plan, a, bhat, plan->n, out, count, stream);
   if (count > 0 && (long)count < (long)sm_count() / 2 && plan->cluster == 0 && !(plan->base_algo & 1) &&
-      all <= kWorkspaceKeep / (plan->n * sizeof(double2))) {
+      all <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
     const int s0 = split0_log2(plan);
     int f0 = 0, f1 = 0, i0 = 0, i1 = 0;
     const bool level = split2_shape(plan, all, &f0, &f1, kForward) && split2_shape(plan, count, &i0, &i1, kInverse);
@@ -510,7 +510,7 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   // outputs of 8 terms 137 us, five launches 24; 75 of 6 108 and 44; 300 of 4, two CTAs per
   // SM, 106 and 93; N = 8192 on Dit8/1024: 40 of 3 101 and 90, 75 of 6 186 and 207).
   if (count > 0 && terms > 1 && plan->cluster == 0 && (long)count < fill &&
-      all + count <= kWorkspaceKeep / (plan->n * sizeof(double2)))
+      all + count <= kWorkspaceSmall / (plan->n * sizeof(double2)))
     return product_sum_unfused(plan, a, bhat, terms, out, count, (cudaStream_t)stream);
   if (plan->N > (size_t(2) << kBlockLog2Auto)) {  // one output per thread-block cluster (N = 8192: by default)
     bool ok = true;
@@ -673,8 +673,8 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
                      per_sm >= (plan->N == 16384 ? 2 : 4);
   if (!ok || (plan->N >= 32768 && plan->cluster == 0) || few_unsplit || few_mid || large) {
     cudaStream_t s = (cudaStream_t)stream;
-    // `large` calls have another route: in equal parts within the workspace the plan keeps
-    const size_t fit = large ? std::max<size_t>(1, kWorkspaceKeep / (plan->n * sizeof(double2))) : count;
+    // `large` calls have another route: in equal parts within a small workspace
+    const size_t fit = large ? std::max<size_t>(1, kWorkspaceSmall / (plan->n * sizeof(double2))) : count;
     const size_t parts = (count + fit - 1) / fit, part = (count + parts - 1) / parts;
     void* z = nullptr;
     const bool got = plan->workspace.alloc((void**)&z, part * plan->n * sizeof(double2), s) == cudaSuccess;

@@ -92,3 +92,16 @@ def test_u128_product_captured_without_allocations(cuda, N, count):
     out = want.clone()
     for _ in run_two_instances(cuda, lambda: product(out), lambda: out.fill_(-1)):
         assert cuda.equal(out, want)
+
+
+def test_workspace_parts_stay_in_the_pool(cuda):
+    """A batch beyond one part, waited for and called again, takes no more memory from the device."""
+    N, count = 16384, 4200  # 1050 MiB of f64 in all
+    plan, product, out = u128_case(cuda, N, count)
+    product(out)
+    cuda.cuda.synchronize()
+    before = cuda.cuda.mem_get_info()[0]
+    product(out)
+    after = cuda.cuda.mem_get_info()[0]
+    cuda.cuda.synchronize()
+    assert before - after <= 32 << 20
