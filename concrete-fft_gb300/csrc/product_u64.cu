@@ -274,17 +274,18 @@ int split0_log2(const cfft_u64_product_plan* p, bool fast = true) {
 // two threads per butterfly of a pass (half butterflies) in small launches, DIT: one; at
 // least a thread per two points for the elementwise steps (radix 16 has few butterflies per
 // pass).  Larger DIF launches take one thread per butterfly, which is how the kernel tells
-// them apart.
-int split_product_threads(int algo, size_t part, long ctas) {
+// them apart.  Sums in one launch (kSum) always have a thread per two points, for their
+// accumulators.
+int split_product_threads(int algo, size_t part, long ctas, int phase) {
   const size_t radix = size_t(2) << (algo / 2);
   const size_t full = part / radix;
   size_t want = std::max(((algo & 1) ? 1 : 2) * full, part / 2);
-  if (!(algo & 1) && radix < 16 && !half_butterflies(ctas, full)) want = full;
+  if (!(algo & 1) && radix < 16 && phase != kSum && !half_butterflies(ctas, full)) want = full;
   return (int)std::min<size_t>(256, std::max<size_t>(32, want));
 }
 
 // phase kForward: `count` terms into ws; kInverse: `count` outputs of `terms` terms each
-// from ws; kWhole: `count` products.
+// from ws; kSum: `count` sums of `terms` terms without ws; kWhole: `count` products.
 cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, const uint64_t* a, const double* bhat,
                                   size_t bhat_stride, uint64_t* out, size_t count, cudaStream_t stream,
                                   const cfft_product_item* items = nullptr, int phase = kWhole, int terms = 1,
@@ -294,7 +295,7 @@ cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, con
   if (!fn) return fail(CFFT_ERR_INVALID_SIZE, "no cluster product kernel for this base and cluster size");
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   const size_t part = plan->n >> ls;
-  const int threads = split_product_threads(algo, part, (long)(count << ls));
+  const int threads = split_product_threads(algo, part, (long)(count << ls), phase);
   const size_t smem = 3 * part * sizeof(double2);
   const int grid = (int)(count << ls);
   DevLevels L = plan->dlv;
@@ -304,14 +305,14 @@ cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, con
                   (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw, (void*)&ws};
   // a few products: every CTA on an SM of its own
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),
-                               stream, phase != kWhole);
+                               stream, phase == kForward || phase == kInverse);
 }
 
 // Launch shape of u64_product_split2_kernel with 2^ls1 classes: threads per CTA
 // and shared memory (three buffers of the CTA's part of the base).
-void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, int* threads, size_t* smem) {
+void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, int phase, int* threads, size_t* smem) {
   const size_t part = p->base_n >> ls1;
-  *threads = split_product_threads(p->base_algo, part, ctas);
+  *threads = split_product_threads(p->base_algo, part, ctas, phase);
   *smem = 3 * part * sizeof(double2);
 }
 
@@ -339,7 +340,7 @@ bool split2_shape(const cfft_u64_product_plan* p, size_t count, int* ls0, int* l
     if (l0 + l1 > 3) {  // every product's 16-CTA cluster resident at once, one CTA per SM
       int threads = 0;
       size_t smem = 0;
-      split2_launch_shape(p, l1, (long)(count << (l0 + l1)), &threads, &smem);
+      split2_launch_shape(p, l1, (long)(count << (l0 + l1)), phase, &threads, &smem);
       // the terms of a sum may take two rounds of clusters: two outputs of 4 terms, N = 16384
       const long rounds = phase == kForward ? 2 : 1;
       if ((long)count > rounds * spread_clusters(fn, threads, 16)) continue;
@@ -361,7 +362,7 @@ cfft_status launch_split2_product(const cfft_u64_product_plan* plan, int ls0, in
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   int threads = 0;
   size_t smem = 0;
-  split2_launch_shape(plan, ls1, (long)(count << ls), &threads, &smem);
+  split2_launch_shape(plan, ls1, (long)(count << ls), phase, &threads, &smem);
   const int grid = (int)(count << ls);
   DevLevels L = plan->dlv;
   long stride = (long)bhat_stride;
@@ -369,7 +370,7 @@ cfft_status launch_split2_product(const cfft_u64_product_plan* plan, int ls0, in
   void* args[] = {(void*)&a, (void*)&bh, &stride, (void*)&out, &terms, (void*)&items, &L, (void*)&plan->d_w,
                   (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw, (void*)&ws};
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),
-                               stream, phase != kWhole);
+                               stream, phase == kForward || phase == kInverse);
 }
 
 }  // namespace
@@ -467,30 +468,31 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
                                  size_t terms, uint64_t* out, size_t count, void* stream) {
   if (!plan || !a || !bhat || !out) return fail(CFFT_ERR_INVALID_ARGUMENT, "null argument");
   if (terms == 0 || terms > 0x7fffffff) return fail(CFFT_ERR_INVALID_ARGUMENT, "terms must be at least 1");
-  // A few outputs of a plan on a DIF base without an outer level, or with one of radix 2,
-  // 4 or 8 (the external product of a blind-rotation step): every term's forward on a
-  // cluster of its own, then every output's sum and inverse on one, in two launches
-  // around a workspace of the terms' products.  Below SMs/2 outputs and within the
-  // workspace pool; more outputs fill the SMs with one CTA or cluster each.
+  if (count == 0) return CFFT_OK;
+  cudaStream_t s = (cudaStream_t)stream;
   const size_t all = count * terms;
+  const bool few = plan->cluster == 0 && (long)count < (long)sm_count() / 2;
   const long fill = plan->n > (size_t(1) << kBlockLog2Auto) ? (long)sm_count() / 2 : 2L * sm_count();
+  // outputs that do not fill the SMs
+  const bool fewer = plan->cluster == 0 && (long)count < fill;
   // One term is a product, except where a cluster per product beats the five launches that a
   // product takes (one of N = 8192 on Dit16/512: 48 us and 58).
   int p0 = 0, p1 = 0;
   const bool cluster16 = plan->lv.nlevels > 0 && algo_radix(plan->base_algo) == 16 && plan->N == 8192 &&
                          !split2_shape(plan, count, &p0, &p1);
-  if (terms == 1 && plan->cluster == 0 && (long)count < fill && !cluster16)
-    return cfft_u64_product(plan, a, bhat, plan->n, out, count, stream);
-  if (count > 0 && (long)count < (long)sm_count() / 2 && plan->cluster == 0 && !(plan->base_algo & 1) &&
-      all <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
-    const int s0 = split0_log2(plan);
+  if (terms == 1 && fewer && !cluster16) return cfft_u64_product(plan, a, bhat, plan->n, out, count, stream);
+  // A few outputs of a plan on a DIF base without an outer level, or with one of radix 2,
+  // 4 or 8 (the external product of a blind-rotation step): every term's forward on a
+  // cluster of its own, then every output's sum and inverse on one, in two launches
+  // around a small workspace of the terms' products.  Below SMs/2 outputs; more outputs
+  // fill the SMs with one CTA or cluster each.
+  const bool dif = !(plan->base_algo & 1);
+  const int s0 = dif ? split0_log2(plan) : 0;
+  if (few && dif && terms > 1 && all <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
     int f0 = 0, f1 = 0, i0 = 0, i1 = 0;
     const bool level = split2_shape(plan, all, &f0, &f1, kForward) && split2_shape(plan, count, &i0, &i1, kInverse);
-    cudaStream_t s = (cudaStream_t)stream;
-    if (terms > 1 && (s0 >= 1 || level)) {
-      void* ws = nullptr;
-      if (plan->workspace.alloc(&ws, all * plan->n * sizeof(double2), s) != cudaSuccess)
-        return fail(CFFT_ERR_OUT_OF_MEMORY, "product sum workspace");
+    void* ws = nullptr;
+    if ((s0 >= 1 || level) && plan->workspace.alloc(&ws, all * plan->n * sizeof(double2), s) == cudaSuccess) {
       const int tr = (int)terms;
       cfft_status st =
           s0 >= 1 ? launch_split0_product(plan, s0, a, bhat, plan->n, nullptr, all, s, nullptr, kForward, 1, (double2*)ws)
@@ -509,13 +511,20 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   // one CTA or cluster per output runs its terms one after the other (N = 2048 on Dit4: two
   // outputs of 8 terms 137 us, five launches 24; 75 of 6 108 and 44; 300 of 4, two CTAs per
   // SM, 106 and 93; N = 8192 on Dit8/1024: 40 of 3 101 and 90, 75 of 6 186 and 207).
-  if (count > 0 && terms > 1 && plan->cluster == 0 && (long)count < fill &&
-      all + count <= kWorkspaceSmall / (plan->n * sizeof(double2)))
-    return product_sum_unfused(plan, a, bhat, terms, out, count, (cudaStream_t)stream);
+  if (fewer && terms > 1 && all + count <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
+    const cfft_status st = product_sum_unfused(plan, a, bhat, terms, out, count, s);
+    if (st != CFFT_ERR_OUT_OF_MEMORY) return st;
+  }
+  // Without a workspace, a few outputs on DIF bases run their terms one after another on
+  // the cluster of each output.
+  int l0 = 0, l1 = 0;
+  if (few && dif && terms > 1 && s0 >= 1 && (plan->n >> s0) <= (size_t)kSplit0Acc * 256)
+    return launch_split0_product(plan, s0, a, bhat, plan->n, out, count, s, nullptr, kSum, (int)terms);
+  if (few && dif && terms > 1 && split2_shape(plan, count, &l0, &l1, kSum))
+    return launch_split2_product(plan, l0, l1, a, bhat, plan->n, out, count, s, nullptr, kSum, (int)terms);
   if (plan->N > (size_t(2) << kBlockLog2Auto)) {  // one output per thread-block cluster (N = 8192: by default)
     bool ok = true;
     const int ls = product_split_log2(plan, count, &ok);
-    if (count == 0) return CFFT_OK;
     // from N = 32768 the unfused sum, as the products take five launches there
     if (!ok || (plan->N >= 32768 && plan->cluster == 0))
       return product_sum_unfused(plan, a, bhat, terms, out, count, (cudaStream_t)stream);
@@ -523,7 +532,6 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
       return launch_split_product(plan, ls, a, bhat, plan->n, out, count, (cudaStream_t)stream, nullptr,
                                   (int)terms);
   }
-  if (count == 0) return CFFT_OK;
   const bool reg_acc = plan->n <= (size_t)(kSumRegAcc * kProdThreads);
   const void* fn = u64_product_sum_kernel_ptr(plan->base_algo, reg_acc, few_warps(plan, (long)count, plan->n));
   const size_t smem = (reg_acc ? 2 : 3) * plan->n * sizeof(double2);

@@ -71,8 +71,9 @@ __device__ __forceinline__ void level0_inv_untwist(double2* const* src, int lm, 
 // Accumulator entries per thread: the CTA sizes keep a part at most 8 entries
 // per thread (1024 points / 128 threads, 2048 / 256, 4096 / 512).
 constexpr int kSplitAcc = 8;
-// The same for u64_product_split0_kernel, whose launches give at least one
-// thread per two points of a part.
+// The same for the sums of u64_product_split0_kernel and u64_product_split2_kernel (kSum),
+// whose launches give at least one thread per two points of a part.
+constexpr int kSplit0Acc = 2;
 
 // One output per cluster of S CTAs (blockIdx.x >> LS): the sum over `terms`
 // products a_t * B_t, accumulated in the Fourier domain in term order, then
@@ -220,13 +221,15 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
 // stores its pointwise product into ws, in the operand's order.  Inverse
 // (kInverse): the cluster of an output adds its `terms` products in term order,
 // as u64_product_sum_kernel does, and runs the inverse steps once.  The terms
-// thus take the time of one (2 outputs of 4 terms, N = 2048 on Dif4: 28.6 us
-// with the terms one after another on the output's cluster).
+// thus take the time of one (2 outputs of 4 terms, N = 2048 on Dif4: 14.1 us, 28.6
+// with the terms one after another on the output's cluster).  kSum is the latter,
+// one launch that needs no workspace: every term's product is added into a register
+// accumulator in term order.
 // Every butterfly and elementwise step does the operations of the one-CTA
 // product kernel on the same values, so results are bit-identical to it.
 // Shared memory: three buffers of n/S points.  Requires L.nlevels == 0,
-// S <= R and n >= R*S.
-enum ProductPhase { kWhole = 0, kForward = 1, kInverse = 2 };
+// S <= R, n >= R*S and, for kSum, n/S <= kSplit0Acc x blockDim.x.
+enum ProductPhase { kWhole = 0, kForward = 1, kInverse = 2, kSum = 3 };
 template <int ALGO, int LS, int PHASE>
 __global__ void __launch_bounds__(256) u64_product_split0_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
@@ -239,7 +242,7 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ double2 smem[];
-  if constexpr (PHASE != kWhole) grid_dependency_wait();
+  if constexpr (PHASE == kForward || PHASE == kInverse) grid_dependency_wait();
   const int log2n = L.log2n[0];
   const int log2c = log2n - LS;
   const int n = 1 << log2n;
@@ -266,30 +269,60 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       peer_x[j] = cl.map_shared_rank(x, (unsigned)j);
       peer_z[j] = cl.map_shared_rank(z, (unsigned)j);
     }
-    // every CTA runs before a peer's memory is written
-    auto token = cl.barrier_arrive();
     const double2* src = y;  // input of the inverse's first pass
     if constexpr (PHASE != kInverse) {
-      // input k of first-pass butterfly c*per + b, folded and twisted, at y[k*per + b]
-      for (int q = tid; q < (R << lpc); q += nth) {
-        const int j = ((q >> lpc) << lper) + c * per + (q & (per - 1));
-        const c64 v{i64_to_f64_rne((int64_t)__ldcs(ap + j)), i64_to_f64_rne((int64_t)__ldcs(ap + j + n))};
-        st(y + q, cmul(ldg(tw + j), v));
+      c64 acc[PHASE == kSum ? kSplit0Acc : 1];
+      const int nterms = PHASE == kSum ? terms : 1;
+#pragma unroll 1
+      for (int t = 0; t < nterms; ++t) {
+        const long term = g * nterms + t;
+        const uint64_t* tap = PHASE == kSum ? a + (term << (log2n + 1)) : ap;
+        const double2* tbp = PHASE == kSum ? bhat + term * bhat_stride : bp;
+        // every CTA runs, and is done with its x from the previous term, before a peer
+        // writes its x
+        auto token = cl.barrier_arrive();
+        if (t > 0) __syncthreads();  // this CTA is done with y
+        // input k of first-pass butterfly c*per + b, folded and twisted, at y[k*per + b]
+        for (int q = tid; q < (R << lpc); q += nth) {
+          const int j = ((q >> lpc) << lper) + c * per + (q & (per - 1));
+          const c64 v{i64_to_f64_rne((int64_t)__ldcs(tap + j)), i64_to_f64_rne((int64_t)__ldcs(tap + j + n))};
+          st(y + q, cmul(ldg(tw + j), v));
+        }
+        __syncthreads();
+        cl.barrier_wait(std::move(token));
+        first_pass_scatter<R, true, LS>([&](int k, int b, int) { return ld(y + (k << lpc) + b); }, per, c * per, 1,
+                                        peer_x, wf, tid, nth);
+        cl.sync();  // every part's x is complete
+        const FlatBuf r = dif_after_first<R, true>(log2n, LS, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
+        if constexpr (PHASE == kForward) {
+          double2* o = ws + (g << log2n) + c;
+          for (int j = tid; j < (1 << log2c); j += nth)
+            st(o + (j << LS), cmul(ldg(tbp + (j << LS) + c), ld(r.p + j)));
+          return;  // no peer touches this CTA's memory after the last barrier
+        } else if constexpr (PHASE == kSum) {
+#pragma unroll
+          for (int k = 0; k < kSplit0Acc; ++k) {
+            const int j = tid + k * nth;
+            if (j < (1 << log2c)) {
+              const c64 p = cmul(ldg(tbp + (j << LS) + c), ld(r.p + j));
+              acc[k] = t == 0 ? p : cadd(acc[k], p);
+            }
+          }
+        } else {
+          for (int j = tid; j < (1 << log2c); j += nth) st(r.p + j, cmul(ldg(tbp + (j << LS) + c), ld(r.p + j)));
+          src = r.p;
+        }
       }
-      __syncthreads();
-      cl.barrier_wait(std::move(token));
-      first_pass_scatter<R, true, LS>([&](int k, int b, int) { return ld(y + (k << lpc) + b); }, per, c * per, 1,
-                                      peer_x, wf, tid, nth);
-      cl.sync();  // every part's x is complete
-      const FlatBuf r = dif_after_first<R, true>(log2n, LS, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
-      if constexpr (PHASE == kForward) {
-        double2* o = ws + (g << log2n) + c;
-        for (int j = tid; j < (1 << log2c); j += nth) st(o + (j << LS), cmul(ldg(bp + (j << LS) + c), ld(r.p + j)));
-        return;  // no peer touches this CTA's memory after the last barrier
+      if constexpr (PHASE == kSum) {
+        __syncthreads();  // every read of the last term's buffers is done
+#pragma unroll
+        for (int k = 0; k < kSplit0Acc; ++k) {
+          const int j = tid + k * nth;
+          if (j < (1 << log2c)) st(y + j, acc[k]);
+        }
       }
-      for (int j = tid; j < (1 << log2c); j += nth) st(r.p + j, cmul(ldg(bp + (j << LS) + c), ld(r.p + j)));
-      src = r.p;
     } else {
+      auto token = cl.barrier_arrive();  // every CTA runs before a peer's memory is written
       const double2* p = ws + ((g * terms) << log2n) + c;
       for (int j = tid; j < (1 << log2c); j += nth) {
         c64 acc = ld(p + (j << LS));
@@ -390,8 +423,9 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
 // Every butterfly and elementwise step does the operations of the one-CTA
 // product kernel on the same values, so results are bit-identical to it.
 // PHASE: a Fourier-domain sum as two launches, steps 1-3 per term and the rest
-// per output, as u64_product_split0_kernel.  Requires L.nlevels == 1,
-// 2^L.log2r[0] == R0, S1 <= the base radix R and m >= R*S1.
+// per output, or as one (kSum), as u64_product_split0_kernel.  Requires
+// L.nlevels == 1, 2^L.log2r[0] == R0, S1 <= the base radix R, m >= R*S1 and, for
+// kSum, m/S1 <= kSplit0Acc x blockDim.x.
 template <int ALGO, int LS0, int LS1, int PHASE>
 __global__ void __launch_bounds__(256) u64_product_split2_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
@@ -408,7 +442,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ double2 smem[];
-  if constexpr (PHASE != kWhole) grid_dependency_wait();
+  if constexpr (PHASE == kForward || PHASE == kInverse) grid_dependency_wait();
   const int log2n = L.log2n[0];
   const int log2m = L.log2n[1];
   const int n = 1 << log2n, m = 1 << log2m;
@@ -440,16 +474,24 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
   const int cnt = m >> LS;
   const bool few = nth >= 2 * pp;  // a small launch, in half butterflies
   const int i0 = c * cnt;
-  // every CTA runs before a peer's memory is written
-  auto token = cl.barrier_arrive();
   const double2* src = y;  // input of the inverse's first pass
   if constexpr (PHASE != kInverse) {
+  c64 acc[PHASE == kSum ? kSplit0Acc : 1];
+  const int nterms = PHASE == kSum ? terms : 1;
+#pragma unroll 1
+  for (int t = 0; t < nterms; ++t) {
+  const long term = g * nterms + t;
+  const uint64_t* tap = PHASE == kSum ? a + (term << (log2n + 1)) : ap;
+  const double2* tbp = PHASE == kSum ? bhat + term * bhat_stride : bp;
+  // every CTA runs, and is done with its buffers of the previous term, before a
+  // peer writes them
+  auto token = cl.barrier_arrive();
   // 1. level 0 forward on butterflies [c*m/S, (c+1)*m/S)
   auto load_l0 = [&](int i, c64* v) {
 #pragma unroll
     for (int k = 0; k < R0; ++k) {
       const int j = (k << log2m) + i;
-      const c64 u{i64_to_f64_rne((int64_t)__ldcs(ap + j)), i64_to_f64_rne((int64_t)__ldcs(ap + j + n))};
+      const c64 u{i64_to_f64_rne((int64_t)__ldcs(tap + j)), i64_to_f64_rne((int64_t)__ldcs(tap + j + n))};
       v[k] = cmul(ldg(tw + j), u);
     }
   };
@@ -485,15 +527,35 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
 
   // 3. the later passes, the pointwise product, the inverse's first pass
   const FlatBuf r = dif_after_first<R, true>(log2m, LS1, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
-  const double2* bs = bp + ((long)s0 << log2m) + c1;
+  const double2* bs = tbp + ((long)s0 << log2m) + c1;
   if constexpr (PHASE == kForward) {
     double2* o = ws + (g << log2n) + ((long)s0 << log2m) + c1;
     for (int j = tid; j < (1 << log2c); j += nth) st(o + (j << LS1), cmul(ldg(bs + (j << LS1)), ld(r.p + j)));
     return;  // no peer touches this CTA's memory after the last barrier
-  }
-  for (int j = tid; j < (1 << log2c); j += nth) st(r.p + j, cmul(ldg(bs + (j << LS1)), ld(r.p + j)));
-  src = r.p;
+  } else if constexpr (PHASE == kSum) {
+#pragma unroll
+    for (int k = 0; k < kSplit0Acc; ++k) {
+      const int j = tid + k * nth;
+      if (j < (1 << log2c)) {
+        const c64 p = cmul(ldg(bs + (j << LS1)), ld(r.p + j));
+        acc[k] = t == 0 ? p : cadd(acc[k], p);
+      }
+    }
   } else {
+    for (int j = tid; j < (1 << log2c); j += nth) st(r.p + j, cmul(ldg(bs + (j << LS1)), ld(r.p + j)));
+    src = r.p;
+  }
+  }
+  if constexpr (PHASE == kSum) {
+    __syncthreads();  // every read of the last term's buffers is done
+#pragma unroll
+    for (int k = 0; k < kSplit0Acc; ++k) {
+      const int j = tid + k * nth;
+      if (j < (1 << log2c)) st(y + j, acc[k]);
+    }
+  }
+  } else {
+    auto token = cl.barrier_arrive();  // every CTA runs before a peer's memory is written
     const double2* p = ws + ((g * terms) << log2n) + ((long)s0 << log2m) + c1;
     for (int j = tid; j < (1 << log2c); j += nth) {
       c64 acc = ld(p + (j << LS1));
@@ -568,7 +630,10 @@ template <int A>
 const void* split0_product_ptr(int ls, int phase) {
   if (phase == kWhole) return split0_product_ptr_t<A, kWhole>(ls);
   if constexpr (AlgoInfo<A>::DIT) return nullptr;
-  else return phase == kForward ? split0_product_ptr_t<A, kForward>(ls) : split0_product_ptr_t<A, kInverse>(ls);
+  else
+    return phase == kForward   ? split0_product_ptr_t<A, kForward>(ls)
+           : phase == kInverse ? split0_product_ptr_t<A, kInverse>(ls)
+                               : split0_product_ptr_t<A, kSum>(ls);
 }
 
 // (R0, S1) = (2, 2), (2, 4), (4, 2) for DIF bases with S1 <= R
@@ -593,7 +658,8 @@ template <int A>
 const void* split2_product_ptr(int ls0, int ls1, int phase) {
   return phase == kWhole     ? split2_product_ptr_t<A, kWhole>(ls0, ls1)
          : phase == kForward ? split2_product_ptr_t<A, kForward>(ls0, ls1)
-                             : split2_product_ptr_t<A, kInverse>(ls0, ls1);
+         : phase == kInverse ? split2_product_ptr_t<A, kInverse>(ls0, ls1)
+                             : split2_product_ptr_t<A, kSum>(ls0, ls1);
 }
 
 #ifndef CFFT_KERNEL_INSTANCE  // instantiated in kinst_split_prod_<A>.cu, one unit per algorithm

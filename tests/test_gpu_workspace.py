@@ -105,3 +105,34 @@ def test_workspace_parts_stay_in_the_pool(cuda):
     after = cuda.cuda.mem_get_info()[0]
     cuda.cuda.synchronize()
     assert before - after <= 32 << 20
+
+
+def sum_case(torch, N, algo, base, count, terms):
+    import concrete_fft as cf
+    g = torch.Generator(device="cuda").manual_seed(N + count + terms)
+    plan = cf.product.U64ProductPlan(N, algo, base)
+    a = torch.randint(-(1 << 63), (1 << 63) - 1, (count, terms, N), generator=g, device="cuda")
+    bhat = torch.empty((count, terms, N // 2), dtype=torch.complex128, device="cuda")
+    plan.prepare_operand(torch.randint(-128, 128, (count * terms, N), generator=g, device="cuda"), bhat)
+    want = torch.empty((count, N), dtype=torch.int64, device="cuda")
+    plan.set_cluster_size(1 if N <= 8192 else 2)  # the kernels that need no workspace
+    plan.product_sum(a, bhat, want)
+    plan.set_cluster_size(0)
+    return plan, lambda out: plan.product_sum(a, bhat, out), want
+
+
+SUMS = [(2048, 2, 1024, 2, 4), (1024, 4, 512, 3, 5), (2048, 0, 1024, 75, 2), (4096, 2, 1024, 2, 4), (8192, 4, 1024, 1, 3),
+        (16384, 2, 1024, 2, 3), (8192, 6, 512, 5, 2), (2048, 3, 1024, 4, 3), (2048, 7, 1024, 2, 2), (8192, 5, 1024, 40, 3),
+        (4096, 1, 512, 3, 2), (8192, 7, 512, 1, 2), (64, 1, 32, 5, 3)]
+
+
+@pytest.mark.parametrize("N,algo,base,count,terms", SUMS)
+def test_u64_product_sum_without_workspace(cuda, N, algo, base, count, terms):
+    plan, product_sum, want = sum_case(cuda, N, algo, base, count, terms)
+    out = want.clone().fill_(-1)
+    product_sum(out)
+    assert cuda.equal(out, want)
+    out.fill_(-1)
+    with no_workspace():
+        product_sum(out)
+    assert cuda.equal(out, want)
