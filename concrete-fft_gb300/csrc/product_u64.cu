@@ -373,6 +373,66 @@ cfft_status launch_split2_product(const cfft_u64_product_plan* plan, int ls0, in
                                stream, phase == kForward || phase == kInverse);
 }
 
+// Where the products of a call run.
+struct ProductRoute {
+  enum Kind {
+    kSplit0,  // u64_product_split0_kernel on 2^ls0 CTAs each
+    kSplit2,  // u64_product_split2_kernel on 2^ls0 slices x 2^ls1 classes
+    kFive,    // five launches on a workspace
+    kPlain    // u64_product_split_kernel on 2^ls0 CTAs each, or one CTA (ls0 = 0)
+  } kind;
+  int ls0 = 0, ls1 = 0;
+  bool spare = false;  // of kFive: kPlain with ls0 serves as well
+};
+ProductRoute product_route(const cfft_u64_product_plan* plan, size_t count) {
+  bool ok = true;
+  const int ls = product_split_log2(plan, count, &ok);
+  // The five-launch path on a workspace from the stream-ordered allocator: N > 65536
+  // (no cluster holds it), and N >= 32768 at every batch, where it measured faster
+  // than one cluster per product (Dif8/512, CUDA events: one product 30.5 vs 74.4 us
+  // at 32768, 35.8 vs 142 at 65536; 38 products 134 vs 212 and 274 vs 423; large
+  // batches 304 vs 280 k products/s at 32768, 129 vs 102 k at 65536)
+  const bool many = (long)count >= (long)sm_count() / 2 && plan->cluster == 0;
+  // A few products whose transform has no outer level (n = base_n): one cluster per
+  // product on the base's residue classes (u64_product_split0_kernel), as does a plan
+  // forced to a cluster size.  Device time per call at N = 2048, Dif4, 4
+  // CTAs: 11.7 us for one product (one CTA: 32.2, the five launches: 13.7), 16.7 for
+  // 38 (one CTA: 34.9, five launches: 19.4)
+  if (plan->cluster >= 2 && split0_log2(plan, false) >= 1)
+    return {ProductRoute::kSplit0, std::min(split0_log2(plan, false), ilog2((size_t)plan->cluster))};
+  // Base radix >= 4: up to one product per SM (N = 2048, 152 products: 25.5 us on Dif4
+  // clusters, 33.9 on one CTA each; Dif8 28.9 against 35.0); radix 2 lost there (Dif2,
+  // N = 1024, 152 products: 24.9 against 20.5 us) and keeps the SMs/2 limit.
+  const long split0_max = (plan->base_algo >= 2) ? (long)sm_count() : (long)sm_count() / 2 - 1;
+  if (plan->cluster == 0 && plan->N >= 512 && (long)count <= split0_max && split0_log2(plan) >= 1)
+    return {ProductRoute::kSplit0, split0_log2(plan)};
+  // Likewise a plan with one outer level of radix 2, 4 or 8 over a DIF base: level 0's
+  // slices times classes of the base (u64_product_split2_kernel).  One product, Dif4
+  // on 1024 points: 13.7 us at N = 4096 (five launches 32.1), 20.9 at 8192 (34.2);
+  // 38 products: 23.3 (33.5) and 44.7 (58.8)
+  int ls0 = 0, ls1 = 0;
+  if (plan->cluster == 0 && !many && split2_shape(plan, count, &ls0, &ls1))
+    return {ProductRoute::kSplit2, ls0, ls1};
+  // otherwise (no cluster kernel for the base) the five launches, whose transforms
+  // split over 2-8 CTAs each
+  const bool few_unsplit = ls == 0 && plan->cluster == 0 && plan->N >= 2048 && !many;
+  // Fewer than SMs/4 products of N = 4096 or 8192 as well (one product: 34 vs 37 us at
+  // 4096, 37 vs 39 us at 8192; from SMs/4 products of N = 8192 the cluster kernel is faster)
+  const bool few_mid = plan->cluster == 0 && plan->N >= 4096 && plan->N <= 8192 &&
+                       (long)count < (long)sm_count() / 4;
+  // N = 4096 to 16384 from 4 products per SM (2 at 16384): whole transforms of 2048 points
+  // run 3 CTAs per SM with the additions on the integer pipes, where the product kernels wait
+  // for their clusters and, at N = 4096, for 128 threads per 2048 points.  2000 products,
+  // kernel / five launches: N = 4096 on Dif4/1024 1.07, on Dif8/512 1.13; 8192 1.12 and 1.13;
+  // 16384 1.12 and 1.16.  With fewer both are uneven (300 of N = 8192: 0.95 and 0.82).
+  const long per_sm = (long)count / sm_count();
+  const bool large = plan->cluster == 0 && plan->lv.nlevels > 0 && plan->N >= 4096 && plan->N <= 16384 &&
+                     per_sm >= (plan->N == 16384 ? 2 : 4);
+  if (!ok || (plan->N >= 32768 && plan->cluster == 0) || few_unsplit || few_mid || large)
+    return {ProductRoute::kFive, ls, 0, ok && large};
+  return {ProductRoute::kPlain, ls};
+}
+
 }  // namespace
 
 // Products given as device items (all of the plan's N) on the largest cluster
@@ -475,12 +535,16 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   const long fill = plan->n > (size_t(1) << kBlockLog2Auto) ? (long)sm_count() / 2 : 2L * sm_count();
   // outputs that do not fill the SMs
   const bool fewer = plan->cluster == 0 && (long)count < fill;
-  // One term is a product, except where a cluster per product beats the five launches that a
-  // product takes (one of N = 8192 on Dit16/512: 48 us and 58).
-  int p0 = 0, p1 = 0;
-  const bool cluster16 = plan->lv.nlevels > 0 && algo_radix(plan->base_algo) == 16 && plan->N == 8192 &&
-                         !split2_shape(plan, count, &p0, &p1);
-  if (terms == 1 && fewer && !cluster16) return cfft_u64_product(plan, a, bhat, plan->n, out, count, stream);
+  // One term is a product where a product needs no workspace.  Else it takes the five
+  // launches below, but on radix 16 a cluster for each output where there is one (one of
+  // N = 8192 on Dit16/512: five launches 58 us, a cluster 50; on Dit16/1024 58 and 52, on
+  // Dit4/1024 37 and 40, on Dit2/1024 43 and 49).
+  bool on_cluster = false;
+  if (terms == 1 && fewer) {
+    const ProductRoute r = product_route(plan, count);
+    if (r.kind != ProductRoute::kFive) return cfft_u64_product(plan, a, bhat, plan->n, out, count, stream);
+    on_cluster = algo_radix(plan->base_algo) == 16 && r.ls0 > 0 && plan->N > (size_t(2) << kBlockLog2Auto);
+  }
   // A few outputs of a plan on a DIF base without an outer level, or with one of radix 2,
   // 4 or 8 (the external product of a blind-rotation step): every term's forward on a
   // cluster of its own, then every output's sum and inverse on one, in two launches
@@ -511,7 +575,7 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   // one CTA or cluster per output runs its terms one after the other (N = 2048 on Dit4: two
   // outputs of 8 terms 137 us, five launches 24; 75 of 6 108 and 44; 300 of 4, two CTAs per
   // SM, 106 and 93; N = 8192 on Dit8/1024: 40 of 3 101 and 90, 75 of 6 186 and 207).
-  if (fewer && terms > 1 && all + count <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
+  if (fewer && !on_cluster && all + count <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
     const cfft_status st = product_sum_unfused(plan, a, bhat, terms, out, count, s);
     if (st != CFFT_ERR_OUT_OF_MEMORY) return st;
   }
@@ -634,59 +698,20 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
   if (!plan || !a || !bhat || !out) return fail(CFFT_ERR_INVALID_ARGUMENT, "null argument");
   if (bhat_stride != 0 && bhat_stride != plan->n)
     return fail(CFFT_ERR_INVALID_ARGUMENT, "bhat_stride must be 0 or N/2");
-  bool ok = true;
-  const int ls = product_split_log2(plan, count, &ok);
   if (count == 0) return CFFT_OK;
-  // The five-launch path on a workspace from the stream-ordered allocator: N > 65536
-  // (no cluster holds it), and N >= 32768 at every batch, where it measured faster
-  // than one cluster per product (Dif8/512, CUDA events: one product 30.5 vs 74.4 us
-  // at 32768, 35.8 vs 142 at 65536; 38 products 134 vs 212 and 274 vs 423; large
-  // batches 304 vs 280 k products/s at 32768, 129 vs 102 k at 65536)
-  const bool many = (long)count >= (long)sm_count() / 2 && plan->cluster == 0;
-  // A few products whose transform has no outer level (n = base_n): one cluster per
-  // product on the base's residue classes (u64_product_split0_kernel), as does a plan
-  // forced to a cluster size.  Device time per call at N = 2048, Dif4, 4
-  // CTAs: 11.7 us for one product (one CTA: 32.2, the five launches: 13.7), 16.7 for
-  // 38 (one CTA: 34.9, five launches: 19.4)
-  if (plan->cluster >= 2 && split0_log2(plan, false) >= 1)
-    return launch_split0_product(plan, std::min(split0_log2(plan, false), ilog2((size_t)plan->cluster)), a, bhat,
-                                 bhat_stride, out, count, (cudaStream_t)stream);
-  // Base radix >= 4: up to one product per SM (N = 2048, 152 products: 25.5 us on Dif4
-  // clusters, 33.9 on one CTA each; Dif8 28.9 against 35.0); radix 2 lost there (Dif2,
-  // N = 1024, 152 products: 24.9 against 20.5 us) and keeps the SMs/2 limit.
-  const long split0_max = (plan->base_algo >= 2) ? (long)sm_count() : (long)sm_count() / 2 - 1;
-  if (plan->cluster == 0 && plan->N >= 512 && (long)count <= split0_max && split0_log2(plan) >= 1)
-    return launch_split0_product(plan, split0_log2(plan), a, bhat, bhat_stride, out, count, (cudaStream_t)stream);
-  // Likewise a plan with one outer level of radix 2, 4 or 8 over a DIF base: level 0's
-  // slices times classes of the base (u64_product_split2_kernel).  One product, Dif4
-  // on 1024 points: 13.7 us at N = 4096 (five launches 32.1), 20.9 at 8192 (34.2);
-  // 38 products: 23.3 (33.5) and 44.7 (58.8)
-  int ls0 = 0, ls1 = 0;
-  if (plan->cluster == 0 && !many && split2_shape(plan, count, &ls0, &ls1))
-    return launch_split2_product(plan, ls0, ls1, a, bhat, bhat_stride, out, count, (cudaStream_t)stream);
-  // otherwise (no cluster kernel for the base) the five launches, whose transforms
-  // split over 2-8 CTAs each
-  const bool few_unsplit = ls == 0 && plan->cluster == 0 && plan->N >= 2048 && !many;
-  // Fewer than SMs/4 products of N = 4096 or 8192 as well (one product: 34 vs 37 us at
-  // 4096, 37 vs 39 us at 8192; from SMs/4 products of N = 8192 the cluster kernel is faster)
-  const bool few_mid = plan->cluster == 0 && plan->N >= 4096 && plan->N <= 8192 &&
-                       (long)count < (long)sm_count() / 4;
-  // N = 4096 to 16384 from 4 products per SM (2 at 16384): whole transforms of 2048 points
-  // run 3 CTAs per SM with the additions on the integer pipes, where the product kernels wait
-  // for their clusters and, at N = 4096, for 128 threads per 2048 points.  2000 products,
-  // kernel / five launches: N = 4096 on Dif4/1024 1.07, on Dif8/512 1.13; 8192 1.12 and 1.13;
-  // 16384 1.12 and 1.16.  With fewer both are uneven (300 of N = 8192: 0.95 and 0.82).
-  const long per_sm = (long)count / sm_count();
-  const bool large = plan->cluster == 0 && plan->lv.nlevels > 0 && plan->N >= 4096 && plan->N <= 16384 &&
-                     per_sm >= (plan->N == 16384 ? 2 : 4);
-  if (!ok || (plan->N >= 32768 && plan->cluster == 0) || few_unsplit || few_mid || large) {
-    cudaStream_t s = (cudaStream_t)stream;
-    // `large` calls have another route: in equal parts within a small workspace
-    const size_t fit = large ? std::max<size_t>(1, kWorkspaceSmall / (plan->n * sizeof(double2))) : count;
+  cudaStream_t s = (cudaStream_t)stream;
+  const ProductRoute r = product_route(plan, count);
+  if (r.kind == ProductRoute::kSplit0)
+    return launch_split0_product(plan, r.ls0, a, bhat, bhat_stride, out, count, s);
+  if (r.kind == ProductRoute::kSplit2)
+    return launch_split2_product(plan, r.ls0, r.ls1, a, bhat, bhat_stride, out, count, s);
+  if (r.kind == ProductRoute::kFive) {
+    // with another route, in equal parts within a small workspace
+    const size_t fit = r.spare ? std::max<size_t>(1, kWorkspaceSmall / (plan->n * sizeof(double2))) : count;
     const size_t parts = (count + fit - 1) / fit, part = (count + parts - 1) / parts;
     void* z = nullptr;
-    const bool got = plan->workspace.alloc((void**)&z, part * plan->n * sizeof(double2), s) == cudaSuccess;
-    if (!got && !large) return fail(CFFT_ERR_OUT_OF_MEMORY, "u64 product workspace");
+    const bool got = plan->workspace.alloc(&z, part * plan->n * sizeof(double2), s) == cudaSuccess;
+    if (!got && !r.spare) return fail(CFFT_ERR_OUT_OF_MEMORY, "u64 product workspace");
     if (got) {
       cfft_status st = CFFT_OK;
       for (size_t c0 = 0; c0 < count && st == CFFT_OK; c0 += part) {
@@ -701,11 +726,9 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
       cudaFreeAsync(z, s);
       return st;
     }
-    cudaGetLastError();  // no workspace: the product kernels below need none
   }
-  if (ls > 0) return launch_split_product(plan, ls, a, bhat, bhat_stride, out, count, (cudaStream_t)stream);
-  return launch_product(plan, a, bhat, bhat_stride, out, count, (cudaStream_t)stream);
-
+  if (r.ls0 > 0) return launch_split_product(plan, r.ls0, a, bhat, bhat_stride, out, count, s);
+  return launch_product(plan, a, bhat, bhat_stride, out, count, s);
 }
 
 // Method::Measure for the product: every (base_algo, base_n) the reference's

@@ -123,7 +123,8 @@ def sum_case(torch, N, algo, base, count, terms):
 
 SUMS = [(2048, 2, 1024, 2, 4), (1024, 4, 512, 3, 5), (2048, 0, 1024, 75, 2), (4096, 2, 1024, 2, 4), (8192, 4, 1024, 1, 3),
         (16384, 2, 1024, 2, 3), (8192, 6, 512, 5, 2), (2048, 3, 1024, 4, 3), (2048, 7, 1024, 2, 2), (8192, 5, 1024, 40, 3),
-        (4096, 1, 512, 3, 2), (8192, 7, 512, 1, 2), (64, 1, 32, 5, 3)]
+        (4096, 1, 512, 3, 2), (8192, 7, 512, 1, 2), (64, 1, 32, 5, 3), (2048, 7, 1024, 2, 1), (4096, 1, 512, 3, 1),
+        (8192, 7, 512, 1, 1), (16384, 3, 1024, 2, 1)]
 
 
 @pytest.mark.parametrize("N,algo,base,count,terms", SUMS)
@@ -136,3 +137,24 @@ def test_u64_product_sum_without_workspace(cuda, N, algo, base, count, terms):
     with no_workspace():
         product_sum(out)
     assert cuda.equal(out, want)
+
+
+def test_u64_product_sum_of_one_term_takes_a_bounded_workspace(cuda):
+    """75 products of N = 2^21 go through parts of 1 GiB, not through 75 transforms (1.2 GiB) at once."""
+    import concrete_fft as cf
+    cf.check(cf.load().cfft_diag_set_workspace_limit(1 << 30))
+    try:
+        plan, product_sum, out = u64_large_sum(cuda)
+        product_sum()
+    finally:
+        cf.check(cf.load().cfft_diag_set_workspace_limit(0))
+
+
+def u64_large_sum(torch):
+    import concrete_fft as cf
+    N, count = 1 << 21, 75
+    plan = cf.product.U64ProductPlan(N, 2, 1024)
+    a = torch.ones((count, 1, N), dtype=torch.int64, device="cuda")
+    bhat = torch.ones((count, 1, N // 2), dtype=torch.complex128, device="cuda")
+    out = torch.empty((count, N), dtype=torch.int64, device="cuda")
+    return plan, lambda: plan.product_sum(a, bhat, out), out
