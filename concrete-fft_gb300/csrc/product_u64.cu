@@ -535,6 +535,7 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   const long fill = plan->n > (size_t(1) << kBlockLog2Auto) ? (long)sm_count() / 2 : 2L * sm_count();
   // outputs that do not fill the SMs
   const bool fewer = plan->cluster == 0 && (long)count < fill;
+  const bool room = fewer && !stream_capturing(s);  // for a workspace
   // One term is a product where a product needs no workspace.  Else it takes the five
   // launches below, but on radix 16 a cluster for each output where there is one (one of
   // N = 8192 on Dit16/512: five launches 58 us, a cluster 50; on Dit16/1024 58 and 52, on
@@ -552,7 +553,7 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   // fill the SMs with one CTA or cluster each.
   const bool dif = !(plan->base_algo & 1);
   const int s0 = dif ? split0_log2(plan) : 0;
-  if (few && dif && terms > 1 && all <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
+  if (few && room && dif && terms > 1 && all <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
     int f0 = 0, f1 = 0, i0 = 0, i1 = 0;
     const bool level = split2_shape(plan, all, &f0, &f1, kForward) && split2_shape(plan, count, &i0, &i1, kInverse);
     void* ws = nullptr;
@@ -575,7 +576,7 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   // one CTA or cluster per output runs its terms one after the other (N = 2048 on Dit4: two
   // outputs of 8 terms 137 us, five launches 24; 75 of 6 108 and 44; 300 of 4, two CTAs per
   // SM, 106 and 93; N = 8192 on Dit8/1024: 40 of 3 101 and 90, 75 of 6 186 and 207).
-  if (fewer && !on_cluster && all + count <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
+  if (room && !on_cluster && all + count <= kWorkspaceSmall / (plan->n * sizeof(double2))) {
     const cfft_status st = product_sum_unfused(plan, a, bhat, terms, out, count, s);
     if (st != CFFT_ERR_OUT_OF_MEMORY) return st;
   }
@@ -705,7 +706,7 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
     return launch_split0_product(plan, r.ls0, a, bhat, bhat_stride, out, count, s);
   if (r.kind == ProductRoute::kSplit2)
     return launch_split2_product(plan, r.ls0, r.ls1, a, bhat, bhat_stride, out, count, s);
-  if (r.kind == ProductRoute::kFive) {
+  if (r.kind == ProductRoute::kFive && !(r.spare && stream_capturing(s))) {
     // with another route, in equal parts within a small workspace
     const size_t fit = r.spare ? std::max<size_t>(1, kWorkspaceSmall / (plan->n * sizeof(double2))) : count;
     const size_t parts = (count + fit - 1) / fit, part = (count + parts - 1) / parts;

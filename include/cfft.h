@@ -296,8 +296,9 @@ cfft_status cfft_u64_product_host(const cfft_u64_product_plan* plan, const uint6
  * do not fill the SMs run all their terms at once, around a workspace of at
  * most 256 MiB: in two launches (fewer than SMs/2 outputs of a plan on a DIF
  * base without an outer level or with one of radix 2, 4 or 8) or unfused.  Up to
- * N = 16384 a sum that cannot have its workspace runs on one CTA or cluster per
- * output, its terms one after another. */
+ * N = 16384 a sum that cannot have its workspace, or whose stream is under
+ * capture, runs on one CTA or cluster per output, its terms one after another;
+ * its graph then holds no allocation, of which CUDA makes one instance only. */
 cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64_t* a, const double* bhat,
                                  size_t terms, uint64_t* out, size_t count, void* stream);
 

@@ -139,6 +139,32 @@ def test_u64_product_sum_without_workspace(cuda, N, algo, base, count, terms):
     assert cuda.equal(out, want)
 
 
+@pytest.mark.parametrize("N,algo,base,count,terms", SUMS)
+def test_u64_product_sum_captured_without_allocations(cuda, N, algo, base, count, terms):
+    plan, product_sum, want = sum_case(cuda, N, algo, base, count, terms)
+    out = want.clone()
+    for _ in run_two_instances(cuda, lambda: product_sum(out), lambda: out.fill_(-1)):
+        assert cuda.equal(out, want)
+
+
+@pytest.mark.parametrize("N,algo,base,count", [(4096, 2, 1024, 612), (8192, 5, 512, 610), (16384, 4, 1024, 305)])
+def test_u64_products_without_workspace_and_captured(cuda, N, algo, base, count):
+    import concrete_fft as cf
+    g = cuda.Generator(device="cuda").manual_seed(N)
+    plan = cf.product.U64ProductPlan(N, algo, base)
+    a = cuda.randint(-(1 << 63), (1 << 63) - 1, (count, N), generator=g, device="cuda")
+    bhat = cuda.empty((count, N // 2), dtype=cuda.complex128, device="cuda")
+    plan.prepare_operand(cuda.randint(-128, 128, (count, N), generator=g, device="cuda"), bhat)
+    want = cuda.empty_like(a)
+    plan.product(a, bhat, want)
+    out = want.clone().fill_(-1)
+    with no_workspace():
+        plan.product(a, bhat, out)
+    assert cuda.equal(out, want)
+    for _ in run_two_instances(cuda, lambda: plan.product(a, bhat, out), lambda: out.fill_(-1)):
+        assert cuda.equal(out, want)
+
+
 def test_u64_product_sum_of_one_term_takes_a_bounded_workspace(cuda):
     """75 products of N = 2^21 go through parts of 1 GiB, not through 75 transforms (1.2 GiB) at once."""
     import concrete_fft as cf
