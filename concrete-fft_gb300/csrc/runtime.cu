@@ -331,8 +331,10 @@ WorkspaceUser::WorkspaceUser() {
 WorkspaceUser::~WorkspaceUser() {
   WorkspacePools& w = workspace_pools();
   std::lock_guard<std::mutex> lk(w.mu);
-  if (--w.users == 0)
-    for (const DevicePool& p : w.pools) cudaMemPoolTrimTo(p.pool, 0);
+  if (--w.users > 0) return;
+  // destroyed rather than trimmed: what a stream still has to free goes back as well, then
+  for (const DevicePool& p : w.pools) cudaMemPoolDestroy(p.pool);
+  w.pools.clear();
 }
 
 namespace {

@@ -1,5 +1,8 @@
 """Product calls whose workspace cannot be had, or whose stream is captured: the kernels without a workspace run."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -184,3 +187,37 @@ def u64_large_sum(torch):
     bhat = torch.ones((count, 1, N // 2), dtype=torch.complex128, device="cuda")
     out = torch.empty((count, N), dtype=torch.int64, device="cuda")
     return plan, lambda: plan.product_sum(a, bhat, out), out
+
+
+LAST_PLAN = """
+import sys
+sys.path.insert(0, %r)
+import torch
+import concrete_fft as cf
+plan = cf.product.U128ProductPlan(16384)
+a = torch.ones((2000, 16384, 2), dtype=torch.int64, device="cuda")
+bhat = torch.ones((1, 4, 8192), dtype=torch.float64, device="cuda")
+out = torch.empty_like(a)
+s = torch.cuda.Stream()
+with torch.cuda.stream(s):
+    plan.product(a, bhat, out, shared_operand=True)  # a first call loads the kernels
+torch.cuda.synchronize()
+del plan
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+plan = cf.product.U128ProductPlan(16384)
+with torch.cuda.stream(s):
+    for _ in range(3):
+        plan.product(a, bhat, out, shared_operand=True)
+del plan  # with the products and the free of their workspace still to run
+torch.cuda.synchronize()
+torch.cuda.synchronize()
+assert free - torch.cuda.mem_get_info()[0] <= 32 << 20, (free, torch.cuda.mem_get_info()[0])
+"""
+
+
+def test_last_plan_gives_the_pool_back(cuda):
+    """The workspace pool goes with the last product plan, also where a stream has not run its frees yet."""
+    pkg = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "concrete-fft_gb300")
+    r = subprocess.run([sys.executable, "-c", LAST_PLAN % pkg], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
