@@ -314,14 +314,20 @@ int split_log2(const C64Plan& p, long batch, int* mode) {
   }
   int ls = 0;
   while (ls < max_ls && (batch << ls) < target) ++ls;
-  // 4 to 5 transforms per SM on radix 2 or 4: whole, a fifth on some SMs doubles their last
-  // round; two CTAs each halve it (613 forwards of 2048 points on Dif4: 69.0 us, 64.6; of
-  // 1024 32.2 and 28.4, on Dif2 36.1 and 31.4).  From 6 per SM the exchange costs as much
-  // (1000 of 2048 points: 94 and 99), at radix 8 from the start (613 of 1024: 32.4 and 36.1)
-  // but for Dif8 under an outer level (613 of 2048: 71.6 and 61.9 on 1024, 65.9 and 61.6 on
-  // 512), and at 4096 points one CTA per SM holds half a transform (613: 121 and 132)
-  const bool split_wins = p.base_algo < 4 || (p.base_algo == CFFT_DIF8 && p.lv.nlevels > 0 && log2n == kBlockLog2Auto);
-  if (ls == 0 && max_ls >= 1 && split_wins && log2n >= 9 && log2n <= kBlockLog2Auto && batch < 5L * sm_count())
+  // From 4 transforms per SM the SM with the most of them sets the time: ceil(batch / SMs)
+  // whole ones (in CTAs of p.tpc), or ceil(2 batch / SMs) halves.  Where that is less, two
+  // CTAs per transform win on radix 4, and on radix 2 without an outer level; whole / halves
+  // over 609 to 684 transforms, forward and inverse: 1024 points 1.00 to 1.18, 2048 points
+  // 1.05 to 1.11 (650 on Dif4/1024 69.3 us and 65.9).  At the same count the halves lose up to
+  // 7%, but at 512 points, where a CTA holds two transforms, they win up to 759 (radix 2 1.19
+  // to 1.43, Dif4 1.04 to 1.17, Dit4 0.98 to 1.10).  From 5 per SM the exchange costs what is
+  // left to gain.  Radix 2 under a level lost at 1024 points (0.81 to 0.95), radix 8 at 512 and
+  // 1024 (0.49 to 0.99).
+  const long sms = sm_count(), tpc = p.tpc;
+  const long whole = 2 * tpc * ((batch + tpc * sms - 1) / (tpc * sms)), halves = (2 * batch + sms - 1) / sms;
+  const bool radix4 = algo_radix(p.base_algo) == 4, radix2 = algo_radix(p.base_algo) == 2;
+  if (ls == 0 && max_ls >= 1 && (radix4 || (radix2 && p.lv.nlevels == 0)) && log2n >= 9 &&
+      log2n <= kBlockLog2Auto && batch < 5 * sms && whole - halves >= (tpc > 1 ? 0 : 1))
     ls = 1;
   return ls;
 }
