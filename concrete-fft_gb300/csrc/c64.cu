@@ -272,8 +272,8 @@ int split_log2(const C64Plan& p, long batch, int* mode) {
         // both directions (with one cluster more than fit, some SMs run two CTAs)
         const size_t part = p.n >> (ls0 + ls1);
         const int threads = (int)std::min<size_t>(256, std::max<size_t>(32, 2 * part / (size_t)(1 << lr)));
-        const void* f = c64_split_kernel_ptr(p.base_algo, true, ls0 + ls1, 1 + ls0);
-        const void* i = c64_split_kernel_ptr(p.base_algo, false, ls0 + ls1, 1 + ls0);
+        const void* f = c64_split_kernel_ptr(p.base_algo, true, ls0 + ls1, 1 + ls0, true);
+        const void* i = c64_split_kernel_ptr(p.base_algo, false, ls0 + ls1, 1 + ls0, true);
         if (f && i && batch <= spread_clusters(f, threads, 16) && batch <= spread_clusters(i, threads, 16)) break;
         ls1 = 0;
       }
@@ -334,7 +334,6 @@ int split_log2(const C64Plan& p, long batch, int* mode) {
 
 cfft_status launch_split(const C64Plan& p, bool fwd, int ls, int mode, long nsub, cudaStream_t stream,
                          double2* data) {
-  const void* fn = c64_split_kernel_ptr(p.base_algo, fwd, ls, mode);
   const size_t part = p.n >> ls;
   const size_t smem = 2 * part * sizeof(double2);
   // one thread per butterfly of a pass over the part (more would idle at the barriers);
@@ -342,12 +341,14 @@ cfft_status launch_split(const C64Plan& p, bool fwd, int ls, int mode, long nsub
   // halves (radix 16 at every size: a whole butterfly takes 126 registers, and one warp
   // per CTA was slower, 84 against 70 us for 1024 transforms of 1024 points on 2 CTAs)
   const int R = algo_radix(p.base_algo);
-  int few = half_butterflies(nsub << ls, part / (size_t)R);
+  const bool few = half_butterflies(nsub << ls, part / (size_t)R);
+  // (the one-level kernels where the CTA has two threads per butterfly)
+  const void* fn = c64_split_kernel_ptr(p.base_algo, fwd, ls, mode, few && (mode < 2 || 2 * part / (size_t)R <= 256));
   const bool halves = (p.base_algo & 1) == 0 && (R == 16 || few);
   const int threads = (int)std::min<size_t>(256, std::max<size_t>(32, (halves ? 2 : 1) * part / (size_t)R));
   DevLevels L = p.dlv;
   const double2* w = fwd ? p.d_w : p.d_winv;
-  void* args[] = {&data, &L, (void*)&w, &few};
+  void* args[] = {&data, &L, (void*)&w};
   if ((nsub << ls) > 0x7fffffffL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   const int grid = (int)(nsub << ls);
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),

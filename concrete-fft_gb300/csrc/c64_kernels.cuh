@@ -192,7 +192,8 @@ constexpr int kProdThreads = 128;
 // N = 256 on Dif16: 49 us on the integer pipes, 25; one of N = 1024 on Dit8: 37 and 25).
 const void* c64_kernel(int algo, bool fwd, bool few);
 // one transform over 2^ls CTAs (split.cuh); mode 0 no outer levels, 1 with levels
-const void* c64_split_kernel_ptr(int algo, bool fwd, int ls, int mode);
+// (few: as half_butterflies gives it for the parts)
+const void* c64_split_kernel_ptr(int algo, bool fwd, int ls, int mode, bool few);
 const void* u64_product_kernel_ptr(int algo, bool few);
 const void* u64_prepare_kernel_ptr(int algo, bool few);
 const void* u64_product_sum_kernel_ptr(int algo, bool reg_acc, bool few);

@@ -89,16 +89,11 @@ constexpr int kAddsSplit = R == 16 ? 0 : 6;
 // additions of a butterfly of radix 8, or of the outer level of a one-level kernel, are a
 // longer chain than its FP64 ones (one N = 16384 product on Dif4/1024: 30.2 us, 27.5 with
 // the radix-8 level on the FP64 pipe; 512 points x 64 on Dit8: 13.0 and 11.0).  kAddsFew is
-// for the DIT passes; core_split chooses by the launch's kind (half butterflies: few).
+// for the DIT passes of the split kernels.
 template <int R>
 constexpr int kAddsFew = R >= 8 ? 0 : 6;
 template <int R, bool FWD, int E>
 struct Core;
-template <int R, bool FWD>
-__device__ __forceinline__ void core_split(c64* v, bool few) {
-  if (few) Core<R, FWD, 0>::run(v);
-  else Core<R, FWD, kAddsSplit<R>>::run(v);
-}
 
 constexpr double kFrac1Sqrt2 = 0.70710678118654752440;
 constexpr double kH1X = 0.9238795325112867;    // cos(-pi/8)

@@ -20,16 +20,16 @@ const void* c64_kernel(int algo, bool fwd, bool few) {
     default: return nullptr;
   }
 }
-const void* c64_split_kernel_ptr(int algo, bool fwd, int ls, int mode) {
+const void* c64_split_kernel_ptr(int algo, bool fwd, int ls, int mode, bool few) {
   switch (algo) {
-    case 0: return split_ptr<0>(fwd, ls, mode);
-    case 1: return split_ptr<1>(fwd, ls, mode);
-    case 2: return split_ptr<2>(fwd, ls, mode);
-    case 3: return split_ptr<3>(fwd, ls, mode);
-    case 4: return split_ptr<4>(fwd, ls, mode);
-    case 5: return split_ptr<5>(fwd, ls, mode);
-    case 6: return split_ptr<6>(fwd, ls, mode);
-    case 7: return split_ptr<7>(fwd, ls, mode);
+    case 0: return split_ptr<0>(fwd, ls, mode, few);
+    case 1: return split_ptr<1>(fwd, ls, mode, few);
+    case 2: return split_ptr<2>(fwd, ls, mode, few);
+    case 3: return split_ptr<3>(fwd, ls, mode, few);
+    case 4: return split_ptr<4>(fwd, ls, mode, few);
+    case 5: return split_ptr<5>(fwd, ls, mode, few);
+    case 6: return split_ptr<6>(fwd, ls, mode, few);
+    case 7: return split_ptr<7>(fwd, ls, mode, few);
     default: return nullptr;
   }
 }

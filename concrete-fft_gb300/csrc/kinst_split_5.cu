@@ -3,5 +3,5 @@
 #include "split.cuh"
 
 namespace cfft {
-template const void* split_ptr<5>(bool, int, int);
+template const void* split_ptr<5>(bool, int, int, bool);
 }  // namespace cfft

@@ -3,7 +3,7 @@
 #include "split_product.cuh"
 
 namespace cfft {
-template const void* split_product_ptr<0>(int, bool);
-template const void* split0_product_ptr<0>(int, int);
-template const void* split2_product_ptr<0>(int, int, int);
+template const void* split_product_ptr<0>(int, bool, bool);
+template const void* split0_product_ptr<0>(int, int, bool);
+template const void* split2_product_ptr<0>(int, int, int, bool);
 }  // namespace cfft

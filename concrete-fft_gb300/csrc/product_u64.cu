@@ -236,7 +236,6 @@ cfft_status launch_split_product(const cfft_u64_product_plan* plan, int ls, cons
                                  const cfft_product_item* items = nullptr, int terms = 1) {
   const size_t part = plan->n >> ls;
   const bool big = part > 2048;  // 4096 points per CTA: one CTA per SM, 512 threads
-  const void* fn = u64_product_split_ptr(plan->base_algo, ls, big);
   const size_t smem = 2 * (plan->n >> ls) * sizeof(double2);
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   DevLevels L = plan->dlv;
@@ -246,9 +245,11 @@ cfft_status launch_split_product(const cfft_u64_product_plan* plan, int ls, cons
   // (shared memory allows 3 CTAs per SM), 512 for 4096 (one CTA per SM)
   const int threads = part <= 1024 ? 128 : (part <= 2048 ? kSplitProdThreads : kSplitProdThreadsBig);
   const int grid = (int)(count << ls);
-  int few = half_butterflies(grid, std::min<size_t>((size_t)threads, part / (size_t)algo_radix(plan->base_algo)));
+  const bool few =
+      half_butterflies(grid, std::min<size_t>((size_t)threads, part / (size_t)algo_radix(plan->base_algo)));
+  const void* fn = u64_product_split_ptr(plan->base_algo, ls, big, few);
   void* args[] = {(void*)&a, (void*)&bh, &stride, (void*)&out, &terms, (void*)&items, &L, (void*)&plan->d_w,
-                  (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw, &few};
+                  (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw};
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),
                                stream);
 }
@@ -270,17 +271,18 @@ int split0_log2(const cfft_u64_product_plan* p, bool fast = true) {
   return ls;
 }
 
-// Threads per CTA of the class-split product kernels (`ctas` CTAs of `part` points).  DIF:
-// two threads per butterfly of a pass (half butterflies) in small launches, DIT: one; at
-// least a thread per two points for the elementwise steps (radix 16 has few butterflies per
-// pass).  Larger DIF launches take one thread per butterfly, which is how the kernel tells
-// them apart.  Sums in one launch (kSum) always have a thread per two points, for their
-// accumulators.
-int split_product_threads(int algo, size_t part, long ctas, int phase) {
+// Threads per CTA of the class-split product kernels (`ctas` CTAs of `part` points), and
+// which instance.  DIF: two threads per butterfly of a pass (half butterflies) in small
+// launches, DIT: one; at least a thread per two points for the elementwise steps (radix 16
+// has few butterflies per pass).  Larger DIF launches take one thread per butterfly, and so
+// does a part too large for two threads each.  Sums in one launch (kSum) always have a
+// thread per two points, for their accumulators.
+int split_product_threads(int algo, size_t part, long ctas, int phase, bool* few) {
   const size_t radix = size_t(2) << (algo / 2);
   const size_t full = part / radix;
-  size_t want = std::max(((algo & 1) ? 1 : 2) * full, part / 2);
-  if (!(algo & 1) && radix < 16 && phase != kSum && !half_butterflies(ctas, full)) want = full;
+  const bool one = (algo & 1) || radix == 16 || phase == kSum, half = half_butterflies(ctas, full);
+  *few = one || (half && 2 * full <= 256);
+  const size_t want = one || half ? std::max(((algo & 1) ? 1 : 2) * full, part / 2) : full;
   return (int)std::min<size_t>(256, std::max<size_t>(32, want));
 }
 
@@ -291,11 +293,12 @@ cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, con
                                   const cfft_product_item* items = nullptr, int phase = kWhole, int terms = 1,
                                   double2* ws = nullptr) {
   const int algo = plan->base_algo;
-  const void* fn = u64_product_split0_ptr(algo, ls, phase);
+  const size_t part = plan->n >> ls;
+  bool few = false;
+  const int threads = split_product_threads(algo, part, (long)(count << ls), phase, &few);
+  const void* fn = u64_product_split0_ptr(algo, ls, phase, few);
   if (!fn) return fail(CFFT_ERR_INVALID_SIZE, "no cluster product kernel for this base and cluster size");
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
-  const size_t part = plan->n >> ls;
-  const int threads = split_product_threads(algo, part, (long)(count << ls), phase);
   const size_t smem = 3 * part * sizeof(double2);
   const int grid = (int)(count << ls);
   DevLevels L = plan->dlv;
@@ -310,9 +313,10 @@ cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, con
 
 // Launch shape of u64_product_split2_kernel with 2^ls1 classes: threads per CTA
 // and shared memory (three buffers of the CTA's part of the base).
-void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, int phase, int* threads, size_t* smem) {
+void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, int phase, int* threads, size_t* smem,
+                         bool* few) {
   const size_t part = p->base_n >> ls1;
-  *threads = split_product_threads(p->base_algo, part, ctas, phase);
+  *threads = split_product_threads(p->base_algo, part, ctas, phase, few);
   *smem = 3 * part * sizeof(double2);
 }
 
@@ -335,12 +339,13 @@ bool split2_shape(const cfft_u64_product_plan* p, size_t count, int* ls0, int* l
     int l1 = std::min(max_ls - l0, lr);
     while (l1 > 0 && (log2m - l1 < 6 || log2m - l1 - lr < 5)) --l1;
     if (l1 < 1) return false;
-    const void* fn = u64_product_split2_ptr(p->base_algo, l0, l1, phase);
+    int threads = 0;
+    size_t smem = 0;
+    bool small = false;
+    split2_launch_shape(p, l1, (long)(count << (l0 + l1)), phase, &threads, &smem, &small);
+    const void* fn = u64_product_split2_ptr(p->base_algo, l0, l1, phase, small);
     if (!fn) continue;
     if (l0 + l1 > 3) {  // every product's 16-CTA cluster resident at once, one CTA per SM
-      int threads = 0;
-      size_t smem = 0;
-      split2_launch_shape(p, l1, (long)(count << (l0 + l1)), phase, &threads, &smem);
       // the terms of a sum may take two rounds of clusters: two outputs of 4 terms, N = 16384
       const long rounds = phase == kForward ? 2 : 1;
       if ((long)count > rounds * spread_clusters(fn, threads, 16)) continue;
@@ -356,13 +361,14 @@ cfft_status launch_split2_product(const cfft_u64_product_plan* plan, int ls0, in
                                   const double* bhat, size_t bhat_stride, uint64_t* out, size_t count,
                                   cudaStream_t stream, const cfft_product_item* items = nullptr, int phase = kWhole,
                                   int terms = 1, double2* ws = nullptr) {
-  const void* fn = u64_product_split2_ptr(plan->base_algo, ls0, ls1, phase);
-  if (!fn) return fail(CFFT_ERR_INVALID_SIZE, "no one-level cluster product kernel for this shape");
   const int ls = ls0 + ls1;
-  if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   int threads = 0;
   size_t smem = 0;
-  split2_launch_shape(plan, ls1, (long)(count << ls), phase, &threads, &smem);
+  bool few = false;
+  split2_launch_shape(plan, ls1, (long)(count << ls), phase, &threads, &smem, &few);
+  const void* fn = u64_product_split2_ptr(plan->base_algo, ls0, ls1, phase, few);
+  if (!fn) return fail(CFFT_ERR_INVALID_SIZE, "no one-level cluster product kernel for this shape");
+  if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
   const int grid = (int)(count << ls);
   DevLevels L = plan->dlv;
   long stride = (long)bhat_stride;

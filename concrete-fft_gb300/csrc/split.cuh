@@ -39,9 +39,16 @@
 
 namespace cfft {
 
+// The kernels below are compiled twice.  FEW: for launches of about one warp per SM
+// sub-partition (half_butterflies), with every addition on the FP64 pipe (E = 0) and, for
+// the DIF algorithms, two threads per butterfly.  Otherwise: one thread per butterfly and
+// most additions on the integer pipes.  The host chooses: both in one kernel, chosen as it
+// runs, cost a single N = 8192 product on Dif8/1024 22.7 us against 20.8, a 64-point
+// forward on Dif2 5.9 against 5.4.
+
 // Passes 1 .. npass-1 and the end butterfly of a DIF transform of 2^log2n
 // points, run on one residue class mod 2^LS compacted to 2^(log2n - LS) points.
-template <int R, bool FWD, int E = kAddsSplit<R>>
+template <int R, bool FWD, int E>
 __device__ __forceinline__ FlatBuf dif_after_first(int log2n, int ls, FlatBuf x, FlatBuf y,
                                                    const double2* __restrict__ wb, int tid, int nth) {
   constexpr int LR = Log2<R>::v;
@@ -53,20 +60,20 @@ __device__ __forceinline__ FlatBuf dif_after_first(int log2n, int ls, FlatBuf x,
   const int log2c = log2n - ls;
   FlatBuf cur = x, oth = y;
   for (int i = 1; i < npass; ++i) {
-    stockham_pass<R, FWD, false, E, true>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
+    stockham_pass<R, FWD, false, E, E == 0>(log2c, i * LR - ls, 1, cur, oth, wb, tid, nth, ls);
     __syncthreads();
     const FlatBuf t = cur;
     cur = oth;
     oth = t;
   }
-  end_dispatch<R, FWD, E, true>(lm, log2c, 1, cur, tid, nth);
+  end_dispatch<R, FWD, E, E == 0>(lm, log2c, 1, cur, tid, nth);
   __syncthreads();
   return cur;
 }
 
 // The end butterfly and passes npass-1 .. 1 of a DIT transform, on one
 // residue class mod 2^LS (compacted), i.e. everything but the s = 1 pass.
-template <int R, bool FWD, int E = kAddsFew<R>>
+template <int R, bool FWD, int E>
 __device__ __forceinline__ FlatBuf dit_before_last(int log2n, int ls, FlatBuf x, FlatBuf y,
                                                    const double2* __restrict__ wb, int tid, int nth) {
   constexpr int LR = Log2<R>::v;
@@ -139,19 +146,19 @@ __device__ __forceinline__ void level0_last(double2* g, int lm, double2* const* 
 // input k (of R), and each output (p*R + k) is stored into the part of its
 // residue class mod S (distributed shared memory), compacted.  Every thread
 // calls before_store() once, before its first store (warp-uniformly): a
-// cluster barrier's wait there overlaps the barrier with the loads.  With
+// cluster barrier's wait there overlaps the barrier with the loads.  With E = 0 and
 // twice as many threads as butterflies (a multiple of 32), the butterflies are
 // split into halves as in stockham_pass.
 struct NoWait {
   __device__ void operator()() const {}
 };
-template <int R, bool FWD, int LS, int E = kAddsSplit<R>, class Load, class Wait = NoWait>
+template <int R, bool FWD, int LS, int E, class Load, class Wait = NoWait>
 __device__ __forceinline__ void first_pass_scatter(Load load, int per, int p0, int pstep, double2* const* part,
                                                    const double2* __restrict__ wb, int tid, int nth,
                                                    Wait before_store = Wait{}) {
   constexpr int LR = Log2<R>::v;
   constexpr int S = 1 << LS;
-  if (nth >= 2 * per && (per & 31) == 0) {
+  if (E == 0 && nth >= 2 * per && (per & 31) == 0) {
     if (tid >= 2 * per) {
       before_store();
     } else {
@@ -212,6 +219,9 @@ __device__ __forceinline__ void dif_first_scatter(const double2* g, int lper, in
 // MODE 1: unordered with outer levels (forward: first, inverse: last).
 // One transform per S consecutive CTAs; w is the plan's forward table
 // (forward) or inverse table (inverse).
+// FEW keeps the additions on the FP64 pipe (one forward of 16384 points on Dit2/1024: 27.4 us
+// on the integer pipes, 24.1; one of 256 points on Dif8, too few butterflies for halves:
+// 11.0 and 10.2).
 template <int ALGO, bool FWD, int LS, int MODE, bool FEW>
 __device__ __forceinline__ void c64_split(double2* data, const DevLevels& L, const double2* __restrict__ w) {
   constexpr int R = AlgoInfo<ALGO>::R;
@@ -337,16 +347,26 @@ __device__ __forceinline__ void c64_split(double2* data, const DevLevels& L, con
     cl.sync();
   }
 }
-// few: about one warp per SM sub-partition (half_butterflies), where the additions stay on
-// the FP64 pipe (one forward of 16384 points on Dit2/1024: 27.4 us on the integer pipes, 24.1;
-// one of 256 points on Dif8, too few butterflies for halves: 11.0 and 10.2).
+
+template <int ALGO, bool FWD, int LS, int MODE, bool FEW>
+__global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels L, const double2* __restrict__ w) {
+  c64_split<ALGO, FWD, LS, MODE, FEW>(data, L, w);
+}
+// FEW on radix 2 to 8, with the registers it asks for: held to 64 by its own choice, the
+// compiler spilled some of these kernels (one 2048-point inverse on Dif2/1024 12.2 us, 11.3).
 template <int ALGO, bool FWD, int LS, int MODE>
-__global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels L, const double2* __restrict__ w,
-                                                        int few) {
-  constexpr int R = AlgoInfo<ALGO>::R;
-  constexpr bool kSame = MODE == 0 && (R == 16 || (AlgoInfo<ALGO>::DIT && R == 8));  // FP64 pipe in both
-  if (kSame || few) c64_split<ALGO, FWD, LS, MODE, true>(data, L, w);
-  else c64_split<ALGO, FWD, LS, MODE, false>(data, L, w);
+__global__ void __launch_bounds__(256, 1) c64_split_few_kernel(double2* data, DevLevels L,
+                                                              const double2* __restrict__ w) {
+  c64_split<ALGO, FWD, LS, MODE, true>(data, L, w);
+}
+// The larger launches with levels, held to 3 CTAs of 256 threads per SM by registers, DIT
+// inverses to 4 (75 forwards of 8192 points on Dif2/512: 57 us at 80 registers, 64 at 98; 300
+// inverses of 2048 on Dit2/1024: 37.6 at 64 registers, 41.2 at 72).  Radix 16 needs more (300
+// forwards of 4096 on Dif16/1024: 98 us, 115 at 80) and stays with the kernel above.
+template <int ALGO, bool FWD, int LS>
+__global__ void __launch_bounds__(256, AlgoInfo<ALGO>::DIT && !FWD && LS < 3 ? 4 : 3)
+    c64_split_levels_kernel(double2* data, DevLevels L, const double2* __restrict__ w) {
+  c64_split<ALGO, FWD, LS, 1, false>(data, L, w);
 }
 
 // An unordered transform with exactly one outer level, of radix R0 = 2^LS0 <= 4,
@@ -364,9 +384,11 @@ __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels
 // level 0's butterflies, reading point i of every slice from the CTA that
 // holds its class.  The same operations on the same values as the one-CTA
 // kernel, in place.
-template <int ALGO, bool FWD, int LS0, int LS1>
-__global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevels L, const double2* __restrict__ w) {
+template <int ALGO, bool FWD, int LS0, int LS1, bool FEW>
+__global__ void __launch_bounds__(256, 1) c64_split2_kernel(double2* data, DevLevels L, const double2* __restrict__ w) {
   constexpr int R = AlgoInfo<ALGO>::R;
+  constexpr int E = FEW ? 0 : kAddsSplit<R>;
+  constexpr int E0 = FEW ? 0 : kAddsSplit<(1 << LS0)>;
   constexpr int LR = Log2<R>::v;
   constexpr int R0 = 1 << LS0;
   constexpr int S1 = 1 << LS1;
@@ -392,7 +414,6 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
   const int lpp = lq - LS1;
   const int pp = 1 << lpp;
   const int cnt = m >> LS;  // level-0 butterflies per CTA
-  const bool few = nth >= 2 * pp;  // a small launch, in half butterflies
   const int i0 = c * cnt;
   double2* part[S1];
   if constexpr (FWD) {
@@ -412,7 +433,7 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
       c64 v[R0];
 #pragma unroll
       for (int k = 0; k < R0; ++k) v[k] = b == tid ? v0[k] : ld(g + (k << log2m) + i);
-      core_split<R0, true>(v, few);
+      Core<R0, true, E0>::run(v);
       const double2* twl = wl + (R0 - 1) * i - 1;
       const int p = i & ((1 << lq) - 1);
       const int dst = ((i >> lq) << lpp) + (p & (pp - 1));
@@ -424,10 +445,10 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
       }
     }
     cl.sync();  // every staging buffer is complete; every read of the transform is done
-    first_pass_scatter<R, true, LS1>([&](int k, int b, int) { return ld(ys + (k << lpp) + b); }, pp, c1 * pp, 1,
+    first_pass_scatter<R, true, LS1, E>([&](int k, int b, int) { return ld(ys + (k << lpp) + b); }, pp, c1 * pp, 1,
                                      part, wb, tid, nth);
     cl.sync();  // every part is complete
-    const FlatBuf r = dif_after_first<R, true>(log2m, LS1, FlatBuf{xs}, FlatBuf{ys}, wb, tid, nth);
+    const FlatBuf r = dif_after_first<R, true, E>(log2m, LS1, FlatBuf{xs}, FlatBuf{ys}, wb, tid, nth);
     double2* gs = g + ((long)s0 << log2m) + c1;
     for (int j = tid; j < (1 << log2c); j += nth) gs[j << LS1] = r.p[j];
   } else {
@@ -440,10 +461,10 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
     for (int j = tid; j < (1 << log2c); j += nth) xs[j] = gs[j << LS1];
     __syncthreads();
     cl.barrier_wait(std::move(token));
-    first_pass_scatter<R, false, LS1>([&](int k, int b, int) { return ld(xs + (k << lpp) + b); }, pp, c1, S1, part,
+    first_pass_scatter<R, false, LS1, E>([&](int k, int b, int) { return ld(xs + (k << lpp) + b); }, pp, c1, S1, part,
                                       wb, tid, nth);
     cl.sync();  // every part is complete; every read of the transform is done
-    const FlatBuf sv = dif_after_first<R, false>(log2m, LS1, FlatBuf{ys}, FlatBuf{xs}, wb, tid, nth);
+    const FlatBuf sv = dif_after_first<R, false, E>(log2m, LS1, FlatBuf{ys}, FlatBuf{xs}, wb, tid, nth);
     cl.sync();  // every slice is complete
     for (int b = tid; b < cnt; b += nth) {
       const int i = i0 + b;
@@ -455,7 +476,7 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
 #pragma unroll
       for (int k = 1; k < R0; ++k)
         v[k] = cmul(ldg(twl + k), ld(cl.map_shared_rank(sv.p, (unsigned)((slot<R0>(k) << LS1) + cls)) + at));
-      core_split<R0, false>(v, few);
+      Core<R0, false, E0>::run(v);
 #pragma unroll
       for (int k = 0; k < R0; ++k) st(g + (k << log2m) + i, v[k]);
     }
@@ -463,21 +484,33 @@ __global__ void __launch_bounds__(256) c64_split2_kernel(double2* data, DevLevel
   }
 }
 
-// Kernel pointer for (ALGO, direction, LS, MODE); nullptr where S = 2^LS
+// Kernel pointer for (ALGO, direction, LS, MODE, FEW); nullptr where S = 2^LS
 // exceeds the radix that is split.
-template <int A, int LS>
+template <int A, int LS, bool FEW>
 const void* split_ptr_ls(bool fwd, int mode) {
+  constexpr int R = AlgoInfo<A>::R;
+  // without levels, radix 16 and DIT radix 8 run the FP64 pipe alone at every size
+  constexpr bool kOne = R == 16 || (AlgoInfo<A>::DIT && R == 8);
   if (mode == 0) {
-    if constexpr (LS <= Log2<AlgoInfo<A>::R>::v)
-      return fwd ? (const void*)c64_split_kernel<A, true, LS, 0> : (const void*)c64_split_kernel<A, false, LS, 0>;
-    else
+    if constexpr (LS > Log2<R>::v)
       return nullptr;
+    else if constexpr (FEW && !kOne)
+      return fwd ? (const void*)c64_split_few_kernel<A, true, LS, 0> : (const void*)c64_split_few_kernel<A, false, LS, 0>;
+    else
+      return fwd ? (const void*)c64_split_kernel<A, true, LS, 0, kOne>
+                 : (const void*)c64_split_kernel<A, false, LS, 0, kOne>;
   }
-  return fwd ? (const void*)c64_split_kernel<A, true, LS, 1> : (const void*)c64_split_kernel<A, false, LS, 1>;
+  if constexpr (R == 16)
+    return fwd ? (const void*)c64_split_kernel<A, true, LS, 1, FEW>
+               : (const void*)c64_split_kernel<A, false, LS, 1, FEW>;
+  else if constexpr (FEW)
+    return fwd ? (const void*)c64_split_few_kernel<A, true, LS, 1> : (const void*)c64_split_few_kernel<A, false, LS, 1>;
+  else
+    return fwd ? (const void*)c64_split_levels_kernel<A, true, LS> : (const void*)c64_split_levels_kernel<A, false, LS>;
 }
 // Mode 2 (R0 = 2), 3 (R0 = 4) and 4 (R0 = 8): c64_split2_kernel with S1 = 2^ls / R0,
 // for DIF bases with S1 <= R and R0 * S1 <= 8, or 16 (4 x 4 and 8 x 2).
-template <int A, int LS0>
+template <int A, int LS0, bool FEW>
 const void* split2_ptr(bool fwd, int ls) {
   if constexpr (AlgoInfo<A>::DIT) {
     return nullptr;
@@ -488,37 +521,43 @@ const void* split2_ptr(bool fwd, int ls) {
       return nullptr;
     } else {
       if (ls1 == 1)
-        return fwd ? (const void*)c64_split2_kernel<A, true, LS0, 1> : (const void*)c64_split2_kernel<A, false, LS0, 1>;
+        return fwd ? (const void*)c64_split2_kernel<A, true, LS0, 1, FEW>
+                   : (const void*)c64_split2_kernel<A, false, LS0, 1, FEW>;
     }
     if constexpr (LS0 <= 2 && LRA >= 2) {
       if (ls1 == 2)
-        return fwd ? (const void*)c64_split2_kernel<A, true, LS0, 2> : (const void*)c64_split2_kernel<A, false, LS0, 2>;
+        return fwd ? (const void*)c64_split2_kernel<A, true, LS0, 2, FEW>
+                   : (const void*)c64_split2_kernel<A, false, LS0, 2, FEW>;
     }
     return nullptr;
   }
 }
-template <int A>
-const void* split_ptr(bool fwd, int ls, int mode) {
-  if (mode == 2) return split2_ptr<A, 1>(fwd, ls);
-  if (mode == 3) return split2_ptr<A, 2>(fwd, ls);
-  if (mode == 4) return split2_ptr<A, 3>(fwd, ls);
+template <int A, bool FEW>
+const void* split_ptr_few(bool fwd, int ls, int mode) {
+  if (mode == 2) return split2_ptr<A, 1, FEW>(fwd, ls);
+  if (mode == 3) return split2_ptr<A, 2, FEW>(fwd, ls);
+  if (mode == 4) return split2_ptr<A, 3, FEW>(fwd, ls);
   switch (ls) {
-    case 1: return split_ptr_ls<A, 1>(fwd, mode);
-    case 2: return split_ptr_ls<A, 2>(fwd, mode);
-    case 3: return split_ptr_ls<A, 3>(fwd, mode);
+    case 1: return split_ptr_ls<A, 1, FEW>(fwd, mode);
+    case 2: return split_ptr_ls<A, 2, FEW>(fwd, mode);
+    case 3: return split_ptr_ls<A, 3, FEW>(fwd, mode);
     default: return nullptr;
   }
 }
+template <int A>
+const void* split_ptr(bool fwd, int ls, int mode, bool few) {
+  return few ? split_ptr_few<A, true>(fwd, ls, mode) : split_ptr_few<A, false>(fwd, ls, mode);
+}
 
 #ifndef CFFT_KERNEL_INSTANCE  // instantiated in kinst_split_<A>.cu, one unit per algorithm
-extern template const void* split_ptr<0>(bool, int, int);
-extern template const void* split_ptr<1>(bool, int, int);
-extern template const void* split_ptr<2>(bool, int, int);
-extern template const void* split_ptr<3>(bool, int, int);
-extern template const void* split_ptr<4>(bool, int, int);
-extern template const void* split_ptr<5>(bool, int, int);
-extern template const void* split_ptr<6>(bool, int, int);
-extern template const void* split_ptr<7>(bool, int, int);
+extern template const void* split_ptr<0>(bool, int, int, bool);
+extern template const void* split_ptr<1>(bool, int, int, bool);
+extern template const void* split_ptr<2>(bool, int, int, bool);
+extern template const void* split_ptr<3>(bool, int, int, bool);
+extern template const void* split_ptr<4>(bool, int, int, bool);
+extern template const void* split_ptr<5>(bool, int, int, bool);
+extern template const void* split_ptr<6>(bool, int, int, bool);
+extern template const void* split_ptr<7>(bool, int, int, bool);
 #endif
 
 }  // namespace cfft

@@ -83,10 +83,12 @@ constexpr int kSplit0Acc = 2;
 // all); out: N u64 per output.  When `items` is not null (terms = 1), product
 // p takes its three pointers from items[p] instead.  Requires L.nlevels >= 1,
 // 2^L.log2r[0] >= S and n/S <= kSplitAcc x blockDim.x.
-template <int ALGO, int LS, bool FEW>
-__device__ __forceinline__ void u64_product_split(
+// FEW keeps the additions on the FP64 pipe (one N = 2048 product on Dit8/512: 39.4 us on the
+// integer pipes, 26.4); parts of 4096 points, one CTA of 16 warps per SM, never do.
+template <int ALGO, int LS, int MAXT, bool FEW>
+__global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
-    int terms, const cfft_product_item* __restrict__ items, const DevLevels& L, const double2* __restrict__ w,
+    int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
     const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -183,17 +185,6 @@ __device__ __forceinline__ void u64_product_split(
   }
   cl.sync();  // no CTA exits while a peer reads its shared memory
 }
-// few: about one warp per SM sub-partition (half_butterflies), where the additions stay on
-// the FP64 pipe (one N = 2048 product on Dit8/512: 39.4 us on the integer pipes, 26.4).
-template <int ALGO, int LS, int MAXT>
-__global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
-    const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
-    int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
-    const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw, int few) {
-  // (parts of 4096 points, one CTA of 16 warps per SM, are not told apart)
-  if (MAXT == kSplitProdThreads && few) u64_product_split<ALGO, LS, true>(a, bhat, bhat_stride, out, terms, items, L, w, winv, tw, itw);
-  else u64_product_split<ALGO, LS, false>(a, bhat, bhat_stride, out, terms, items, L, w, winv, tw, itw);
-}
 
 // One product per cluster of S = 2^LS CTAs (S <= the base radix R) when the
 // N/2-point transform has no outer level (n = base_n, e.g. N = 2048 on a
@@ -230,13 +221,14 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
 // Shared memory: three buffers of n/S points.  Requires L.nlevels == 0,
 // S <= R, n >= R*S and, for kSum, n/S <= kSplit0Acc x blockDim.x.
 enum ProductPhase { kWhole = 0, kForward = 1, kInverse = 2, kSum = 3 };
-template <int ALGO, int LS, int PHASE>
-__global__ void __launch_bounds__(256) u64_product_split0_kernel(
+template <int ALGO, int LS, int PHASE, bool FEW>
+__global__ void __launch_bounds__(256, 1) u64_product_split0_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
     int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
     const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw,
     double2* __restrict__ ws) {
   constexpr int R = AlgoInfo<ALGO>::R;
+  constexpr int E = FEW ? 0 : kAddsSplit<R>;
   constexpr int LR = Log2<R>::v;
   constexpr int S = 1 << LS;
   namespace cg = cooperative_groups;
@@ -290,10 +282,10 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
         }
         __syncthreads();
         cl.barrier_wait(std::move(token));
-        first_pass_scatter<R, true, LS>([&](int k, int b, int) { return ld(y + (k << lpc) + b); }, per, c * per, 1,
+        first_pass_scatter<R, true, LS, E>([&](int k, int b, int) { return ld(y + (k << lpc) + b); }, per, c * per, 1,
                                         peer_x, wf, tid, nth);
         cl.sync();  // every part's x is complete
-        const FlatBuf r = dif_after_first<R, true>(log2n, LS, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
+        const FlatBuf r = dif_after_first<R, true, E>(log2n, LS, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
         if constexpr (PHASE == kForward) {
           double2* o = ws + (g << log2n) + c;
           for (int j = tid; j < (1 << log2c); j += nth)
@@ -332,10 +324,10 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
       cl.barrier_wait(std::move(token));
     }
     __syncthreads();
-    first_pass_scatter<R, false, LS>([&](int k, int b, int) { return ld(src + (k << lpc) + b); }, per, c, S, peer_z,
+    first_pass_scatter<R, false, LS, E>([&](int k, int b, int) { return ld(src + (k << lpc) + b); }, per, c, S, peer_z,
                                      wi, tid, nth);
     cl.sync();  // every part's z is complete (no peer memory is touched after this)
-    const FlatBuf s = dif_after_first<R, false>(log2n, LS, FlatBuf{z}, FlatBuf{x}, wi, tid, nth);
+    const FlatBuf s = dif_after_first<R, false, E>(log2n, LS, FlatBuf{z}, FlatBuf{x}, wi, tid, nth);
     for (int j = tid; j < (1 << log2c); j += nth) {
       const int jg = (j << LS) + c;
       const c64 t = cmul(ldg(itw + jg), ld(s.p + j));
@@ -426,13 +418,15 @@ __global__ void __launch_bounds__(256) u64_product_split0_kernel(
 // per output, or as one (kSum), as u64_product_split0_kernel.  Requires
 // L.nlevels == 1, 2^L.log2r[0] == R0, S1 <= the base radix R, m >= R*S1 and, for
 // kSum, m/S1 <= kSplit0Acc x blockDim.x.
-template <int ALGO, int LS0, int LS1, int PHASE>
-__global__ void __launch_bounds__(256) u64_product_split2_kernel(
+template <int ALGO, int LS0, int LS1, int PHASE, bool FEW>
+__global__ void __launch_bounds__(256, 1) u64_product_split2_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
     int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
     const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw,
     double2* __restrict__ ws) {
   constexpr int R = AlgoInfo<ALGO>::R;
+  constexpr int E = FEW ? 0 : kAddsSplit<R>;
+  constexpr int E0 = FEW ? 0 : kAddsSplit<(1 << LS0)>;
   constexpr int LR = Log2<R>::v;
   constexpr int R0 = 1 << LS0;
   constexpr int S1 = 1 << LS1;
@@ -472,7 +466,6 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
     peer_z[j] = cl.map_shared_rank(z, (unsigned)((s0 << LS1) + j));
   }
   const int cnt = m >> LS;
-  const bool few = nth >= 2 * pp;  // a small launch, in half butterflies
   const int i0 = c * cnt;
   const double2* src = y;  // input of the inverse's first pass
   if constexpr (PHASE != kInverse) {
@@ -507,7 +500,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
     } else {
       load_l0(i, v);
     }
-    core_split<R0, true>(v, few);
+    Core<R0, true, E0>::run(v);
     const double2* twl = wl + (R0 - 1) * i - 1;
     const int p = i & ((1 << lq) - 1);
     const int dst = (((i >> lq) << lpp) + (p & (pp - 1)));
@@ -521,12 +514,12 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
   cl.sync();  // every staging buffer is complete
 
   // 2. the base's first pass on this slice, butterflies [c1*pp, (c1+1)*pp)
-  first_pass_scatter<R, true, LS1>([&](int k, int b, int) { return ld(y + (k << lpp) + b); }, pp, c1 * pp, 1, peer_x,
+  first_pass_scatter<R, true, LS1, E>([&](int k, int b, int) { return ld(y + (k << lpp) + b); }, pp, c1 * pp, 1, peer_x,
                                    wf, tid, nth);
   cl.sync();  // every part's x is complete
 
   // 3. the later passes, the pointwise product, the inverse's first pass
-  const FlatBuf r = dif_after_first<R, true>(log2m, LS1, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
+  const FlatBuf r = dif_after_first<R, true, E>(log2m, LS1, FlatBuf{x}, FlatBuf{y}, wf, tid, nth);
   const double2* bs = tbp + ((long)s0 << log2m) + c1;
   if constexpr (PHASE == kForward) {
     double2* o = ws + (g << log2n) + ((long)s0 << log2m) + c1;
@@ -565,12 +558,12 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
     cl.barrier_wait(std::move(token));
   }
   __syncthreads();
-  first_pass_scatter<R, false, LS1>([&](int k, int b, int) { return ld(src + (k << lpp) + b); }, pp, c1, S1, peer_z,
+  first_pass_scatter<R, false, LS1, E>([&](int k, int b, int) { return ld(src + (k << lpp) + b); }, pp, c1, S1, peer_z,
                                     wi, tid, nth);
   cl.sync();  // every part's z is complete
 
   // 4. the rest of the base inverse
-  const FlatBuf sv = dif_after_first<R, false>(log2m, LS1, FlatBuf{z}, FlatBuf{x}, wi, tid, nth);
+  const FlatBuf sv = dif_after_first<R, false, E>(log2m, LS1, FlatBuf{z}, FlatBuf{x}, wi, tid, nth);
   cl.sync();  // every slice's inverse is complete
 
   // 5. level 0 inverse on butterflies [c*m/S, (c+1)*m/S), untwisted and rounded
@@ -584,7 +577,7 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
 #pragma unroll
     for (int k = 1; k < R0; ++k)
       v[k] = cmul(ldg(twl + k), ld(cl.map_shared_rank(sv.p, (unsigned)((slot<R0>(k) << LS1) + cls)) + at));
-    core_split<R0, false>(v, few);
+    Core<R0, false, E0>::run(v);
 #pragma unroll
     for (int k = 0; k < R0; ++k) {
       const int j = (k << log2m) + i;
@@ -596,77 +589,87 @@ __global__ void __launch_bounds__(256) u64_product_split2_kernel(
   cl.sync();  // no CTA exits while a peer reads its shared memory
 }
 
-// Kernel pointers of base algorithm A (big: the 512-thread variant, for parts of 4096 points).
-template <int A>
-const void* split_product_ptr(int ls, bool big) {
-  if (big) {
-    switch (ls) {
-      case 1: return (const void*)u64_product_split_kernel<A, 1, kSplitProdThreadsBig>;
-      case 2: return (const void*)u64_product_split_kernel<A, 2, kSplitProdThreadsBig>;
-      case 3: return (const void*)u64_product_split_kernel<A, 3, kSplitProdThreadsBig>;
-      default: return nullptr;
-    }
-  }
+// Kernel pointers of base algorithm A (big: the 512-thread variant, for parts of 4096 points;
+// few: the FEW instances).
+template <int A, int MAXT, bool FEW>
+const void* split_product_ptr_t(int ls) {
   switch (ls) {
-    case 1: return (const void*)u64_product_split_kernel<A, 1, kSplitProdThreads>;
-    case 2: return (const void*)u64_product_split_kernel<A, 2, kSplitProdThreads>;
-    case 3: return (const void*)u64_product_split_kernel<A, 3, kSplitProdThreads>;
+    case 1: return (const void*)u64_product_split_kernel<A, 1, MAXT, FEW>;
+    case 2: return (const void*)u64_product_split_kernel<A, 2, MAXT, FEW>;
+    case 3: return (const void*)u64_product_split_kernel<A, 3, MAXT, FEW>;
     default: return nullptr;
   }
 }
+template <int A>
+const void* split_product_ptr(int ls, bool big, bool few) {
+  return big   ? split_product_ptr_t<A, kSplitProdThreadsBig, false>(ls)
+         : few ? split_product_ptr_t<A, kSplitProdThreads, true>(ls)
+               : split_product_ptr_t<A, kSplitProdThreads, false>(ls);
+}
 
-template <int A, int PHASE>
+template <int A, int PHASE, bool FEW>
 const void* split0_product_ptr_t(int ls) {
   constexpr int LRA = Log2<AlgoInfo<A>::R>::v;
   switch (ls) {
-    case 1: return (const void*)u64_product_split0_kernel<A, 1, PHASE>;
-    case 2: if constexpr (LRA >= 2) return (const void*)u64_product_split0_kernel<A, 2, PHASE>; else return nullptr;
-    case 3: if constexpr (LRA >= 3) return (const void*)u64_product_split0_kernel<A, 3, PHASE>; else return nullptr;
+    case 1: return (const void*)u64_product_split0_kernel<A, 1, PHASE, FEW>;
+    case 2: if constexpr (LRA >= 2) return (const void*)u64_product_split0_kernel<A, 2, PHASE, FEW>; else return nullptr;
+    case 3: if constexpr (LRA >= 3) return (const void*)u64_product_split0_kernel<A, 3, PHASE, FEW>; else return nullptr;
     default: return nullptr;
   }
 }
-// phase: kWhole, or a phase of a sum (DIF bases only)
+// phase: kWhole, or a phase of a sum (DIF bases only).  DIT and radix-16 kernels and sums in
+// one launch have one instance.
 template <int A>
-const void* split0_product_ptr(int ls, int phase) {
-  if (phase == kWhole) return split0_product_ptr_t<A, kWhole>(ls);
-  if constexpr (AlgoInfo<A>::DIT) return nullptr;
+const void* split0_product_ptr(int ls, int phase, bool few) {
+  constexpr bool kTwo = !AlgoInfo<A>::DIT && AlgoInfo<A>::R < 16;
+  if (phase == kWhole)
+    return few || !kTwo ? split0_product_ptr_t<A, kWhole, true>(ls) : split0_product_ptr_t<A, kWhole, !kTwo>(ls);
+  if constexpr (AlgoInfo<A>::DIT)
+    return nullptr;
   else
-    return phase == kForward   ? split0_product_ptr_t<A, kForward>(ls)
-           : phase == kInverse ? split0_product_ptr_t<A, kInverse>(ls)
-                               : split0_product_ptr_t<A, kSum>(ls);
+    return phase == kSum       ? split0_product_ptr_t<A, kSum, true>(ls)
+           : phase == kForward ? (few || !kTwo ? split0_product_ptr_t<A, kForward, true>(ls)
+                                               : split0_product_ptr_t<A, kForward, !kTwo>(ls))
+                               : (few || !kTwo ? split0_product_ptr_t<A, kInverse, true>(ls)
+                                               : split0_product_ptr_t<A, kInverse, !kTwo>(ls));
 }
 
-// (R0, S1) = (2, 2), (2, 4), (4, 2) for DIF bases with S1 <= R
-template <int A, int PHASE>
+// (R0, S1) = (2, 2), (2, 4), (4, 2) and, in 16-CTA clusters, (4, 4) and (8, 2), for DIF bases
+// with S1 <= R
+template <int A, int PHASE, bool FEW>
 const void* split2_product_ptr_t(int ls0, int ls1) {
   if constexpr (AlgoInfo<A>::DIT) {
     return nullptr;
   } else {
     constexpr int LRA = Log2<AlgoInfo<A>::R>::v;
-    if (ls0 == 1 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 1, 1, PHASE>;
-    if (ls0 == 2 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 2, 1, PHASE>;
+    if (ls0 == 1 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 1, 1, PHASE, FEW>;
+    if (ls0 == 2 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 2, 1, PHASE, FEW>;
     if constexpr (LRA >= 2) {
-      if (ls0 == 1 && ls1 == 2) return (const void*)u64_product_split2_kernel<A, 1, 2, PHASE>;
-      // 16-CTA clusters
-      if (ls0 == 2 && ls1 == 2) return (const void*)u64_product_split2_kernel<A, 2, 2, PHASE>;
-      if (ls0 == 3 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 3, 1, PHASE>;
+      if (ls0 == 1 && ls1 == 2) return (const void*)u64_product_split2_kernel<A, 1, 2, PHASE, FEW>;
+      if (ls0 == 2 && ls1 == 2) return (const void*)u64_product_split2_kernel<A, 2, 2, PHASE, FEW>;
+      if (ls0 == 3 && ls1 == 1) return (const void*)u64_product_split2_kernel<A, 3, 1, PHASE, FEW>;
     }
     return nullptr;
   }
 }
 template <int A>
-const void* split2_product_ptr(int ls0, int ls1, int phase) {
-  return phase == kWhole     ? split2_product_ptr_t<A, kWhole>(ls0, ls1)
-         : phase == kForward ? split2_product_ptr_t<A, kForward>(ls0, ls1)
-         : phase == kInverse ? split2_product_ptr_t<A, kInverse>(ls0, ls1)
-                             : split2_product_ptr_t<A, kSum>(ls0, ls1);
+const void* split2_product_ptr(int ls0, int ls1, int phase, bool few) {
+  constexpr bool kTwo = AlgoInfo<A>::R < 16;
+  const bool f = few || !kTwo;
+  return phase == kSum       ? split2_product_ptr_t<A, kSum, true>(ls0, ls1)
+         : phase == kWhole   ? (f ? split2_product_ptr_t<A, kWhole, true>(ls0, ls1)
+                                  : split2_product_ptr_t<A, kWhole, !kTwo>(ls0, ls1))
+         : phase == kForward ? (f ? split2_product_ptr_t<A, kForward, true>(ls0, ls1)
+                                  : split2_product_ptr_t<A, kForward, !kTwo>(ls0, ls1))
+                             : (f ? split2_product_ptr_t<A, kInverse, true>(ls0, ls1)
+                                  : split2_product_ptr_t<A, kInverse, !kTwo>(ls0, ls1));
 }
 
 #ifndef CFFT_KERNEL_INSTANCE  // instantiated in kinst_split_prod_<A>.cu, one unit per algorithm
-#define CFFT_EXTERN_SPLIT_PRODUCT(A)                              \
-  extern template const void* split_product_ptr<A>(int, bool);    \
-  extern template const void* split0_product_ptr<A>(int, int);    \
-  extern template const void* split2_product_ptr<A>(int, int, int);
+#define CFFT_EXTERN_SPLIT_PRODUCT(A)                                  \
+  extern template const void* split_product_ptr<A>(int, bool, bool);  \
+  extern template const void* split0_product_ptr<A>(int, int, bool);  \
+  extern template const void* split2_product_ptr<A>(int, int, int, bool);
 CFFT_EXTERN_SPLIT_PRODUCT(0)
 CFFT_EXTERN_SPLIT_PRODUCT(1)
 CFFT_EXTERN_SPLIT_PRODUCT(2)
@@ -677,26 +680,27 @@ CFFT_EXTERN_SPLIT_PRODUCT(6)
 CFFT_EXTERN_SPLIT_PRODUCT(7)
 #undef CFFT_EXTERN_SPLIT_PRODUCT
 
-inline const void* u64_product_split_ptr(int algo, int ls, bool big) {
-  const void* (*const of[8])(int, bool) = {split_product_ptr<0>, split_product_ptr<1>, split_product_ptr<2>,
-                                           split_product_ptr<3>, split_product_ptr<4>, split_product_ptr<5>,
-                                           split_product_ptr<6>, split_product_ptr<7>};
-  return of[algo](ls, big);
+inline const void* u64_product_split_ptr(int algo, int ls, bool big, bool few) {
+  const void* (*const of[8])(int, bool, bool) = {split_product_ptr<0>, split_product_ptr<1>, split_product_ptr<2>,
+                                                 split_product_ptr<3>, split_product_ptr<4>, split_product_ptr<5>,
+                                                 split_product_ptr<6>, split_product_ptr<7>};
+  return of[algo](ls, big, few);
 }
 // the kernel for plans without an outer level; nullptr where S = 2^ls exceeds the
 // radix, or a phase of a sum on a DIT base
-inline const void* u64_product_split0_ptr(int algo, int ls, int phase) {
-  const void* (*const of[8])(int, int) = {split0_product_ptr<0>, split0_product_ptr<1>, split0_product_ptr<2>,
-                                          split0_product_ptr<3>, split0_product_ptr<4>, split0_product_ptr<5>,
-                                          split0_product_ptr<6>, split0_product_ptr<7>};
-  return of[algo](ls, phase);
+inline const void* u64_product_split0_ptr(int algo, int ls, int phase, bool few) {
+  const void* (*const of[8])(int, int, bool) = {split0_product_ptr<0>, split0_product_ptr<1>, split0_product_ptr<2>,
+                                                split0_product_ptr<3>, split0_product_ptr<4>, split0_product_ptr<5>,
+                                                split0_product_ptr<6>, split0_product_ptr<7>};
+  return of[algo](ls, phase, few);
 }
 // the one-level kernel (DIF bases only); nullptr where the shape is not instantiated
-inline const void* u64_product_split2_ptr(int algo, int ls0, int ls1, int phase) {
-  const void* (*const of[8])(int, int, int) = {split2_product_ptr<0>, split2_product_ptr<1>, split2_product_ptr<2>,
-                                               split2_product_ptr<3>, split2_product_ptr<4>, split2_product_ptr<5>,
-                                               split2_product_ptr<6>, split2_product_ptr<7>};
-  return of[algo](ls0, ls1, phase);
+inline const void* u64_product_split2_ptr(int algo, int ls0, int ls1, int phase, bool few) {
+  const void* (*const of[8])(int, int, int, bool) = {split2_product_ptr<0>, split2_product_ptr<1>,
+                                                     split2_product_ptr<2>, split2_product_ptr<3>,
+                                                     split2_product_ptr<4>, split2_product_ptr<5>,
+                                                     split2_product_ptr<6>, split2_product_ptr<7>};
+  return of[algo](ls0, ls1, phase, few);
 }
 #endif
 
