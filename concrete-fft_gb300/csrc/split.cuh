@@ -352,10 +352,15 @@ template <int ALGO, bool FWD, int LS, int MODE, bool FEW>
 __global__ void __launch_bounds__(256) c64_split_kernel(double2* data, DevLevels L, const double2* __restrict__ w) {
   c64_split<ALGO, FWD, LS, MODE, FEW>(data, L, w);
 }
-// FEW on radix 2 to 8, with the registers it asks for: held to 64 by its own choice, the
-// compiler spilled some of these kernels (one 2048-point inverse on Dif2/1024 12.2 us, 11.3).
+// Registers for three CTAs of 256 threads per SM, two under a radix-8 level: by its own choice
+// the compiler held some of the FEW instances to 64 and spilled (one 2048-point inverse on
+// Dif2/1024 12.2 us, 11.7), and at two per SM the 320 CTAs of 40 outputs of N = 8192 on
+// Dif8/1024 take a round more (3 terms each: 75.5 us, 65.8).  Radix 16 is left to that choice
+// (0): 75 products of N = 4096 on Dif16/1024 33 us, 78 with all the registers it asks for.
+template <int ALGO, bool FEW, int LS0 = 0>
+constexpr int kFewCtas = !FEW || AlgoInfo<ALGO>::DIT || AlgoInfo<ALGO>::R == 16 ? 0 : LS0 == 3 ? 2 : 3;
 template <int ALGO, bool FWD, int LS, int MODE>
-__global__ void __launch_bounds__(256, 1) c64_split_few_kernel(double2* data, DevLevels L,
+__global__ void __launch_bounds__(256, 3) c64_split_few_kernel(double2* data, DevLevels L,
                                                               const double2* __restrict__ w) {
   c64_split<ALGO, FWD, LS, MODE, true>(data, L, w);
 }
@@ -385,7 +390,8 @@ __global__ void __launch_bounds__(256, AlgoInfo<ALGO>::DIT && !FWD && LS < 3 ? 4
 // holds its class.  The same operations on the same values as the one-CTA
 // kernel, in place.
 template <int ALGO, bool FWD, int LS0, int LS1, bool FEW>
-__global__ void __launch_bounds__(256, 1) c64_split2_kernel(double2* data, DevLevels L, const double2* __restrict__ w) {
+__global__ void __launch_bounds__(256, kFewCtas<ALGO, FEW, LS0>)
+    c64_split2_kernel(double2* data, DevLevels L, const double2* __restrict__ w) {
   constexpr int R = AlgoInfo<ALGO>::R;
   constexpr int E = FEW ? 0 : kAddsSplit<R>;
   constexpr int E0 = FEW ? 0 : kAddsSplit<(1 << LS0)>;
