@@ -1678,7 +1678,9 @@ def measure_latency(torch, cf, local, world, cpu=True, cpu_seconds=0.5, profile_
             plan.prepare_operand(torch.from_numpy(b_np).cuda(), bh)
             out = torch.empty((2, N), dtype=torch.int64, device="cuda")
             row = {"plan": "%s/%d" % (ALGO_NAMES[int(algo)], base),
-                   "auto_us": graph_device_us(torch, lambda: plan.product_sum(a, bh, out))}
+                   "captured_without_workspace_us": graph_device_us(torch, lambda: plan.product_sum(a, bh, out))}
+            plan.set_graph_workspace(True)  # the route of uncaptured calls
+            row["auto_us"] = graph_device_us(torch, lambda: plan.product_sum(a, bh, out))
             ok = out.clone()
             plan.set_cluster_size(1)
             row["one_cta_per_output_us"] = graph_device_us(torch, lambda: plan.product_sum(a, bh, out))

@@ -112,6 +112,8 @@ _SIGS = [
     ("cfft_u64_untwist_round", c_int, [vp, vp, vp, c_size, vp]),
     ("cfft_u64_product_fft", vp, [vp]),
     ("cfft_u64_fourier_mul_monomial", c_int, [vp, ctypes.c_ulonglong, vp, c_size, vp]),
+    ("cfft_u64_product_set_graph_workspace", c_int, [vp, c_int]),
+    ("cfft_u128_product_set_graph_workspace", c_int, [vp, c_int]),
     ("cfft_u64_product_set_int_adds", c_int, [vp, c_int]),
     ("cfft_u64_product_set_cluster_size", c_int, [vp, c_int]),
     ("cfft_u64_product_int_adds", c_int, [vp]),

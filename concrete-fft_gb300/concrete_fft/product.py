@@ -61,6 +61,11 @@ class U64ProductPlan:
         """CTAs per product: 0 automatic, 1 one CTA, 2/4/8 a thread-block cluster; results unchanged."""
         check(self._lib.cfft_u64_product_set_cluster_size(self._h, int(ctas)))
 
+    def set_graph_workspace(self, on):
+        """Whether calls captured in a CUDA graph may allocate workspaces (faster, but CUDA then makes one
+        instance of the graph at a time) where kernels without one serve; results unchanged."""
+        check(self._lib.cfft_u64_product_set_graph_workspace(self._h, int(bool(on))))
+
     def product_unfused(self, a, bhat, out, z):
         """The same product as five separate launches (fold+twist, the N/2-point unordered
         forward transform, pointwise product, inverse transform, untwist+round): the plain
@@ -109,6 +114,10 @@ class U128ProductPlan:
         if getattr(self, "_h", None):
             self._lib.cfft_u128_product_plan_destroy(self._h)
             self._h = None
+
+    def set_graph_workspace(self, on):
+        """As U64ProductPlan.set_graph_workspace, for N = 4096 and 8192."""
+        check(self._lib.cfft_u128_product_set_graph_workspace(self._h, int(bool(on))))
 
     def prepare_operand(self, b, bhat4):
         count = B.batch_of(b, self.N, 8)

@@ -585,6 +585,7 @@ struct cfft_f128_plan {
 
 struct cfft_u128_product_plan {
   size_t N = 0;
+  bool graph_workspace = false;  // captured calls may allocate where the fused kernel serves
   WorkspaceUser workspace;
   cfft_f128_plan f;
 };
@@ -1056,10 +1057,10 @@ cfft_status cfft_u128_product(const cfft_u128_product_plan* p, const uint64_t* a
   // N = 4096: 1001 us fused, 908 as five launches; 200 of N = 8192: 1272 and 790; 1024
   // of N = 2048: 838 and 853).  The workspace is at most what the pool keeps: larger
   // batches go through it in parts.  N up to 8192 runs fused where no workspace can be had and, but
-  // for the few, where the stream is captured (stream_capturing).
+  // for the few, where the stream is captured (stream_capturing) and the plan not told so.
   const bool fused_fits = p->f.n <= (size_t(1) << kF128SmemLog2);
   if (!fused_fits || (few && p->f.n >= 512) ||
-      (p->f.n >= 2048 && !stream_capturing((cudaStream_t)stream))) {
+      (p->f.n >= 2048 && (p->graph_workspace || !stream_capturing((cudaStream_t)stream)))) {
     cudaStream_t s = (cudaStream_t)stream;
     const int log2n = ilog2(p->f.n);
     const size_t part = std::min(count, std::max<size_t>(1, kWorkspaceKeep / (32 * p->f.n)));
@@ -1104,6 +1105,12 @@ cfft_status cfft_u128_product(const cfft_u128_product_plan* p, const uint64_t* a
   u128_product_kernel<<<grid, threads, smem, (cudaStream_t)stream>>>(
       a, bhat4, (long)bhat_stride, out, (long)count, log2n, p->f.tw());
   CFFT_CHECK_LAUNCH();
+  return CFFT_OK;
+}
+
+cfft_status cfft_u128_product_set_graph_workspace(cfft_u128_product_plan* p, int on) {
+  if (!p || (on != 0 && on != 1)) return fail(CFFT_ERR_INVALID_ARGUMENT, "graph workspace must be 0 or 1");
+  p->graph_workspace = on == 1;
   return CFFT_OK;
 }
 

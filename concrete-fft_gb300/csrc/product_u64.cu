@@ -40,6 +40,7 @@ struct cfft_u64_product_plan {
   double2 *d_w = nullptr, *d_winv = nullptr, *d_tw = nullptr, *d_itw = nullptr;
   int emu = 0;  // eighths of the butterfly additions issued on the integer pipe
   int cluster = 0;  // CTAs per product: 0 automatic, 1 one CTA, 2/4/8 a cluster of that size
+  bool graph_workspace = false;  // captured calls may allocate where kernels without a workspace serve
 };
 
 namespace cfft {
@@ -379,6 +380,12 @@ cfft_status launch_split2_product(const cfft_u64_product_plan* plan, int ls0, in
                                stream, phase == kForward || phase == kInverse);
 }
 
+// Whether a call that has another route may take a workspace: not into a graph that the
+// caller has not allowed it in (stream_capturing).
+bool may_allocate(const cfft_u64_product_plan* plan, cudaStream_t s) {
+  return plan->graph_workspace || !stream_capturing(s);
+}
+
 // Where the products of a call run.
 struct ProductRoute {
   enum Kind {
@@ -541,7 +548,7 @@ cfft_status cfft_u64_product_sum(const cfft_u64_product_plan* plan, const uint64
   const long fill = plan->n > (size_t(1) << kBlockLog2Auto) ? (long)sm_count() / 2 : 2L * sm_count();
   // outputs that do not fill the SMs
   const bool fewer = plan->cluster == 0 && (long)count < fill;
-  const bool room = fewer && !stream_capturing(s);  // for a workspace
+  const bool room = fewer && may_allocate(plan, s);
   // One term is a product where a product needs no workspace.  Else it takes the five
   // launches below, but on radix 16 a cluster for each output where there is one (one of
   // N = 8192 on Dit16/512: five launches 58 us, a cluster 50; on Dit16/1024 58 and 52, on
@@ -622,6 +629,12 @@ cfft_status cfft_u64_product_set_cluster_size(cfft_u64_product_plan* plan, int c
   if (!plan || !(ctas == 0 || ctas == 1 || ctas == 2 || ctas == 4 || ctas == 8))
     return fail(CFFT_ERR_INVALID_ARGUMENT, "cluster size must be 0 (automatic), 1, 2, 4 or 8");
   plan->cluster = ctas;
+  return CFFT_OK;
+}
+
+cfft_status cfft_u64_product_set_graph_workspace(cfft_u64_product_plan* plan, int on) {
+  if (!plan || (on != 0 && on != 1)) return fail(CFFT_ERR_INVALID_ARGUMENT, "graph workspace must be 0 or 1");
+  plan->graph_workspace = on == 1;
   return CFFT_OK;
 }
 
@@ -712,7 +725,7 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
     return launch_split0_product(plan, r.ls0, a, bhat, bhat_stride, out, count, s);
   if (r.kind == ProductRoute::kSplit2)
     return launch_split2_product(plan, r.ls0, r.ls1, a, bhat, bhat_stride, out, count, s);
-  if (r.kind == ProductRoute::kFive && !(r.spare && stream_capturing(s))) {
+  if (r.kind == ProductRoute::kFive && (!r.spare || may_allocate(plan, s))) {
     // with another route, in equal parts within a small workspace
     const size_t fit = r.spare ? std::max<size_t>(1, kWorkspaceSmall / (plan->n * sizeof(double2))) : count;
     const size_t parts = (count + fit - 1) / fit, part = (count + parts - 1) / parts;

@@ -41,17 +41,21 @@ def run_two_instances(torch, call, wipe):
         finally:
             end = cu.cuStreamEndCapture(s, ctypes.byref(graph))
         ok(end, "end")
-        execs = [ctypes.c_void_p(), ctypes.c_void_p()]
-        for e in execs:
-            ok(cu.cuGraphInstantiateWithFlags(ctypes.byref(e), graph, ctypes.c_ulonglong(0)), "instance")
-        for e in execs:
-            wipe()
-            ok(cu.cuGraphLaunch(e, s), "launch")
-            stream.synchronize()
-            yield
-        for e in execs:
-            ok(cu.cuGraphExecDestroy(e), "destroy")
-        ok(cu.cuGraphDestroy(graph), "destroy")
+        execs = []
+        try:
+            for _ in range(2):
+                e = ctypes.c_void_p()
+                ok(cu.cuGraphInstantiateWithFlags(ctypes.byref(e), graph, ctypes.c_ulonglong(0)), "instance")
+                execs.append(e)
+            for e in execs:
+                wipe()
+                ok(cu.cuGraphLaunch(e, s), "launch")
+                stream.synchronize()
+                yield
+        finally:
+            for e in execs:
+                cu.cuGraphExecDestroy(e)
+            cu.cuGraphDestroy(graph)
 
 
 def u128_case(torch, N, count):
@@ -187,6 +191,42 @@ def u64_large_sum(torch):
     bhat = torch.ones((count, 1, N // 2), dtype=torch.complex128, device="cuda")
     out = torch.empty((count, N), dtype=torch.int64, device="cuda")
     return plan, lambda: plan.product_sum(a, bhat, out), out
+
+
+@pytest.mark.parametrize("case", ["sum", "sum_unfused", "products", "u128"])
+def test_graph_workspace_on_request(cuda, case):
+    """Captured calls of a plan that allows it take the workspace routes: the same bits, in one instance."""
+    torch = cuda
+    if case.startswith("sum"):
+        plan, call, want = sum_case(torch, *((2048, 2, 1024, 2, 4) if case == "sum" else (2048, 3, 1024, 4, 3)))
+    elif case == "u128":
+        plan, call, want = u128_case(torch, 4096, 80)
+        call(want)
+    else:
+        import concrete_fft as cf
+        plan = cf.product.U64ProductPlan(4096, 2, 1024)
+        a = torch.randint(-(1 << 63), (1 << 63) - 1, (612, 4096), device="cuda")
+        bhat = torch.randn((612, 2048), dtype=torch.complex128, device="cuda")
+        want = torch.empty_like(a)
+        plan.product(a, bhat, want)
+
+        def call(out):
+            plan.product(a, bhat, out)
+    plan.set_graph_workspace(True)
+    out = want.clone()
+    with pytest.raises(AssertionError, match="instance"):  # the second one, as CUDA documents it
+        for _ in run_two_instances(torch, lambda: call(out), lambda: out.fill_(-1)):
+            pass
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(out)
+    for _ in range(2):
+        out.fill_(-1)
+        graph.replay()
+        assert torch.equal(out, want)
+    plan.set_graph_workspace(False)
+    for _ in run_two_instances(torch, lambda: call(out), lambda: out.fill_(-1)):
+        assert torch.equal(out, want)
 
 
 LAST_PLAN = """
