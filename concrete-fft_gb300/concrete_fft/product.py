@@ -28,7 +28,7 @@ class U64ProductPlan:
             self._h = None
 
     def set_int_adds(self, eighths):
-        """Kept with the plan (0..8): the kernels choose the integer-pipe share of the additions themselves."""
+        """0: every addition on the FP64 pipe; 1..8: most on the integer pipes; never set: by the launch."""
         check(self._lib.cfft_u64_product_set_int_adds(self._h, int(eighths)))
 
     def int_adds(self):

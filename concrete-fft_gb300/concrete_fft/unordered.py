@@ -49,7 +49,7 @@ class Plan:
         return FftAlgo(a.value), b.value
 
     def set_int_adds(self, eighths):
-        """Kept with the plan (0..8): the kernels choose the integer-pipe share of the additions themselves."""
+        """0: every addition on the FP64 pipe; 1..8: most on the integer pipes; never set: by the launch."""
         check(self._lib.cfft_unordered_set_int_adds(self._h, int(eighths)))
 
     def set_cluster_size(self, ctas):

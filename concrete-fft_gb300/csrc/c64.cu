@@ -136,7 +136,7 @@ struct C64Plan {
   int d0 = 0;        // first level handled in shared memory
   int threads = 128;  // CTA size of the shared-memory kernel
   int tpc = 1;       // sub-transforms per CTA
-  int emu = 0;       // eighths of the butterfly additions issued on the integer pipe
+  int int_adds = kIntAddsAuto;  // cfft_*_set_int_adds
   int cluster = 0;   // CTAs per transform: 0 automatic, 1 one CTA, 2/4/8 a cluster of that size
   bool block_set = false;  // block size chosen by the caller (no per-call change)
 };
@@ -193,15 +193,14 @@ void free_plan(C64Plan& p) {
   p.d_w = p.d_winv = p.d_mono = nullptr;
 }
 
-int emu_level(const C64Plan& p) { return emu_level_for(p.base_algo, p.emu); }
-
 cfft_status launch_smem(const C64Plan& p, bool fwd, int blocks, size_t smem, cudaStream_t stream, double2* data,
                         int nsub, const double2* w) {
   DevLevels L = p.dlv;
   int tpc = p.tpc, d0 = p.d0;
   void* args[] = {&data, &nsub, &tpc, &L, &d0, (void*)&w};
   const size_t pass = ((size_t)p.tpc << p.lv.log2n[p.d0]) / (size_t)algo_radix(p.base_algo);  // butterflies per CTA
-  const void* fn = c64_kernel(p.base_algo, fwd, half_butterflies(blocks, std::min(pass, (size_t)p.threads)));
+  const bool few = half_butterflies(blocks, std::min(pass, (size_t)p.threads));
+  const void* fn = c64_kernel(p.base_algo, fwd, fp64_additions(p.int_adds, few));
   return launch_kernel(fn, blocks, p.threads, args, spread_smem(fn, blocks, p.threads, 1, smem), stream, true);
 }
 
@@ -343,7 +342,8 @@ cfft_status launch_split(const C64Plan& p, bool fwd, int ls, int mode, long nsub
   const int R = algo_radix(p.base_algo);
   const bool few = half_butterflies(nsub << ls, part / (size_t)R);
   // (the one-level kernels where the CTA has two threads per butterfly)
-  const void* fn = c64_split_kernel_ptr(p.base_algo, fwd, ls, mode, few && (mode < 2 || 2 * part / (size_t)R <= 256));
+  const void* fn = c64_split_kernel_ptr(
+      p.base_algo, fwd, ls, mode, fp64_additions(p.int_adds, few && (mode < 2 || 2 * part / (size_t)R <= 256)));
   const bool halves = (p.base_algo & 1) == 0 && (R == 16 || few);
   const int threads = (int)std::min<size_t>(256, std::max<size_t>(32, (halves ? 2 : 1) * part / (size_t)R));
   DevLevels L = p.dlv;
@@ -356,7 +356,7 @@ cfft_status launch_split(const C64Plan& p, bool fwd, int ls, int mode, long nsub
 }
 
 cfft_status launch_level(bool fwd, double2* data, long total, int log2r, int log2nl, const double2* wl, int nsm,
-                         cudaStream_t stream) {
+                         int int_adds, cudaStream_t stream) {
   // fewer butterflies than 256 per SM: smaller CTAs, so that the level's FP64 work
   // spreads over the SMs (one forward of 16384 points on Dif8/512, a radix-8 level
   // in global memory, then 8 sub-transforms on clusters: 15.2 us with 256-thread
@@ -367,7 +367,7 @@ cfft_status launch_level(bool fwd, double2* data, long total, int log2r, int log
   void* args[] = {&data, &total, &log2r, &log2nl, (void*)&wl};
   // with about one warp per SM sub-partition the additions stay on the FP64 pipe (one
   // forward of 16384 points on Dif8/512: 13.9 us on the integer pipes, 12.7)
-  const bool few = half_butterflies(1, (size_t)total);
+  const bool few = fp64_additions(int_adds, half_butterflies(1, (size_t)total));
   const void* fn = few ? (fwd ? (const void*)c64_level_kernel<true, 0> : (const void*)c64_level_kernel<false, 0>)
                        : (fwd ? (const void*)c64_level_kernel<true, kAddsBatch>
                               : (const void*)c64_level_kernel<false, kAddsBatch>);
@@ -447,7 +447,7 @@ cfft_status run_plan(const C64Plan& plan, double* buf, size_t batch, bool fwd, c
         cfft_status st = launch_level(fwd, data, ((long)batch << log2n) >> plan.lv.log2r[l], plan.lv.log2r[l],
                                       plan.lv.log2n[l],
                                       fwd ? plan.d_w + plan.lv.w_off[l] : plan.d_winv + plan.lv.winv_off[l], nsm,
-                                      stream);
+                                      plan.int_adds, stream);
         if (st != CFFT_OK) return st;
       }
       if (fwd) return launch_split(sub, true, sls, smode, nsub, stream, data);
@@ -477,7 +477,7 @@ cfft_status run_plan(const C64Plan& plan, double* buf, size_t batch, bool fwd, c
   if (fwd) {
     for (int l = 0; l < p.d0; ++l) {
       cfft_status st = launch_level(true, data, ((long)batch << log2n) >> p.lv.log2r[l], p.lv.log2r[l],
-                                    p.lv.log2n[l], p.d_w + p.lv.w_off[l], nsm, stream);
+                                    p.lv.log2n[l], p.d_w + p.lv.w_off[l], nsm, p.int_adds, stream);
       if (st != CFFT_OK) return st;
     }
     cfft_status st = launch_smem(p, true, blocks, smem, stream, data, (int)nsub, p.d_w);
@@ -487,7 +487,7 @@ cfft_status run_plan(const C64Plan& plan, double* buf, size_t batch, bool fwd, c
     if (st != CFFT_OK) return st;
     for (int l = p.d0 - 1; l >= 0; --l) {
       st = launch_level(false, data, ((long)batch << log2n) >> p.lv.log2r[l], p.lv.log2r[l], p.lv.log2n[l],
-                        p.d_winv + p.lv.winv_off[l], nsm, stream);
+                        p.d_winv + p.lv.winv_off[l], nsm, p.int_adds, stream);
       if (st != CFFT_OK) return st;
     }
   }
@@ -691,7 +691,6 @@ cfft_status cfft_ordered_plan_create_measure(size_t n, double seconds, cfft_orde
     if (st == CFFT_OK) {
       (*out)->p.threads = tv.threads;
       (*out)->p.tpc = tv.tpc;
-      (*out)->p.emu = tv.emu;
     }
     return st;
   }
@@ -705,7 +704,7 @@ cfft_status cfft_ordered_plan_create_measure(size_t n, double seconds, cfft_orde
   if (st == CFFT_OK) {
     tune_launch((*out)->p, scratch, batch, seconds);
     const C64Plan& p = (*out)->p;
-    tune_store(0, n, TuneVal{p.base_algo, p.base_n, p.threads, p.tpc, p.emu});
+    tune_store(0, n, TuneVal{p.base_algo, p.base_n, p.threads, p.tpc, 0});
   }
   if (scratch) cudaFree(scratch);
   return st;
@@ -739,10 +738,10 @@ cfft_status cfft_ordered_inv_host(const cfft_ordered_plan* plan, double* buf, si
 
 cfft_status cfft_ordered_set_int_adds(cfft_ordered_plan* plan, int eighths) {
   if (!plan || eighths < 0 || eighths > 8) return fail(CFFT_ERR_INVALID_ARGUMENT, "eighths must be in 0..8");
-  plan->p.emu = eighths;
+  plan->p.int_adds = eighths;
   return CFFT_OK;
 }
-int cfft_ordered_int_adds(const cfft_ordered_plan* plan) { return plan ? emu_level(plan->p) : -1; }
+int cfft_ordered_int_adds(const cfft_ordered_plan* plan) { return plan ? int_adds_of(plan->p.int_adds) : -1; }
 
 cfft_status cfft_ordered_set_cluster_size(cfft_ordered_plan* plan, int ctas) {
   if (!plan || !(ctas == 0 || ctas == 1 || ctas == 2 || ctas == 4 || ctas == 8))
@@ -776,10 +775,10 @@ size_t cfft_unordered_block_points(const cfft_unordered_plan* plan) {
 
 cfft_status cfft_unordered_set_int_adds(cfft_unordered_plan* plan, int eighths) {
   if (!plan || eighths < 0 || eighths > 8) return fail(CFFT_ERR_INVALID_ARGUMENT, "eighths must be in 0..8");
-  plan->p.emu = eighths;
+  plan->p.int_adds = eighths;
   return CFFT_OK;
 }
-int cfft_unordered_int_adds(const cfft_unordered_plan* plan) { return plan ? emu_level(plan->p) : -1; }
+int cfft_unordered_int_adds(const cfft_unordered_plan* plan) { return plan ? int_adds_of(plan->p.int_adds) : -1; }
 
 cfft_status cfft_unordered_plan_create(size_t n, cfft_algo base_algo, size_t base_n, cfft_unordered_plan** out) {
   if (!out) return fail(CFFT_ERR_INVALID_ARGUMENT, "null output pointer");
@@ -815,7 +814,6 @@ cfft_status cfft_unordered_plan_create_measure(size_t n, double seconds, cfft_un
     if (st == CFFT_OK) {
       (*out)->p.threads = tv.threads;
       (*out)->p.tpc = tv.tpc;
-      (*out)->p.emu = tv.emu;
     }
     return st;
   }
@@ -858,7 +856,7 @@ cfft_status cfft_unordered_plan_create_measure(size_t n, double seconds, cfft_un
   if (st == CFFT_OK) {
     tune_launch((*out)->p, scratch, batch, seconds);
     const C64Plan& p = (*out)->p;
-    tune_store(1, n, TuneVal{p.base_algo, p.base_n, p.threads, p.tpc, p.emu});
+    tune_store(1, n, TuneVal{p.base_algo, p.base_n, p.threads, p.tpc, 0});
   }
   cudaFree(scratch);
   return st;

@@ -38,7 +38,7 @@ struct cfft_u64_product_plan {
   LevelDesc lv{};
   DevLevels dlv{};
   double2 *d_w = nullptr, *d_winv = nullptr, *d_tw = nullptr, *d_itw = nullptr;
-  int emu = 0;  // eighths of the butterfly additions issued on the integer pipe
+  int int_adds = kIntAddsAuto;  // cfft_u64_product_set_int_adds
   int cluster = 0;  // CTAs per product: 0 automatic, 1 one CTA, 2/4/8 a cluster of that size
   bool graph_workspace = false;  // captured calls may allocate where kernels without a workspace serve
 };
@@ -179,6 +179,7 @@ cfft_status product_sum_unfused(const cfft_u64_product_plan* plan, const uint64_
 // idle lanes leave of an integer addition costs more than the FP64 one (1500 products of
 // N = 256 on Dit16: 78.6 us, 66.8; of N = 1024, a full warp: 110 and 121).
 bool few_warps(const cfft_u64_product_plan* plan, long ctas, size_t points) {
+  if (plan->int_adds != kIntAddsAuto) return plan->int_adds == 0;
   const size_t radix = (size_t)algo_radix(plan->base_algo), pass = std::min<size_t>(kProdThreads, points / radix);
   if (radix == 16 && pass < 32) return true;
   const long per_sm = std::max<long>(1, (long)((size_t(227) << 10) / (2 * points * sizeof(double2))));
@@ -248,7 +249,7 @@ cfft_status launch_split_product(const cfft_u64_product_plan* plan, int ls, cons
   const int grid = (int)(count << ls);
   const bool few =
       half_butterflies(grid, std::min<size_t>((size_t)threads, part / (size_t)algo_radix(plan->base_algo)));
-  const void* fn = u64_product_split_ptr(plan->base_algo, ls, big, few);
+  const void* fn = u64_product_split_ptr(plan->base_algo, ls, big, fp64_additions(plan->int_adds, few));
   void* args[] = {(void*)&a, (void*)&bh, &stride, (void*)&out, &terms, (void*)&items, &L, (void*)&plan->d_w,
                   (void*)&plan->d_winv, (void*)&plan->d_tw, (void*)&plan->d_itw};
   return launch_kernel_cluster(fn, grid, threads, 1 << ls, args, spread_smem(fn, grid, threads, 1 << ls, smem),
@@ -278,11 +279,12 @@ int split0_log2(const cfft_u64_product_plan* p, bool fast = true) {
 // has few butterflies per pass).  Larger DIF launches take one thread per butterfly, and so
 // does a part too large for two threads each.  Sums in one launch (kSum) always have a
 // thread per two points, for their accumulators.
-int split_product_threads(int algo, size_t part, long ctas, int phase, bool* few) {
+int split_product_threads(const cfft_u64_product_plan* plan, size_t part, long ctas, int phase, bool* few) {
+  const int algo = plan->base_algo;
   const size_t radix = size_t(2) << (algo / 2);
   const size_t full = part / radix;
   const bool one = (algo & 1) || radix == 16 || phase == kSum, half = half_butterflies(ctas, full);
-  *few = one || (half && 2 * full <= 256);
+  *few = one || fp64_additions(plan->int_adds, half && 2 * full <= 256);
   const size_t want = one || half ? std::max(((algo & 1) ? 1 : 2) * full, part / 2) : full;
   return (int)std::min<size_t>(256, std::max<size_t>(32, want));
 }
@@ -296,7 +298,7 @@ cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, con
   const int algo = plan->base_algo;
   const size_t part = plan->n >> ls;
   bool few = false;
-  const int threads = split_product_threads(algo, part, (long)(count << ls), phase, &few);
+  const int threads = split_product_threads(plan, part, (long)(count << ls), phase, &few);
   const void* fn = u64_product_split0_ptr(algo, ls, phase, few);
   if (!fn) return fail(CFFT_ERR_INVALID_SIZE, "no cluster product kernel for this base and cluster size");
   if ((count << ls) > 0x7fffffffUL) return fail(CFFT_ERR_INVALID_SIZE, "batch too large");
@@ -317,7 +319,7 @@ cfft_status launch_split0_product(const cfft_u64_product_plan* plan, int ls, con
 void split2_launch_shape(const cfft_u64_product_plan* p, int ls1, long ctas, int phase, int* threads, size_t* smem,
                          bool* few) {
   const size_t part = p->base_n >> ls1;
-  *threads = split_product_threads(p->base_algo, part, ctas, phase, few);
+  *threads = split_product_threads(p, part, ctas, phase, few);
   *smem = 3 * part * sizeof(double2);
 }
 
@@ -640,11 +642,11 @@ cfft_status cfft_u64_product_set_graph_workspace(cfft_u64_product_plan* plan, in
 
 cfft_status cfft_u64_product_set_int_adds(cfft_u64_product_plan* plan, int eighths) {
   if (!plan || eighths < 0 || eighths > 8) return fail(CFFT_ERR_INVALID_ARGUMENT, "eighths must be in 0..8");
-  plan->emu = eighths;
+  plan->int_adds = eighths;
   return CFFT_OK;
 }
 int cfft_u64_product_int_adds(const cfft_u64_product_plan* plan) {
-  return plan ? emu_level_for(plan->base_algo, plan->emu) : -1;
+  return plan ? int_adds_of(plan->int_adds) : -1;
 }
 
 cfft_status cfft_u64_product_plan_create(size_t N, cfft_algo base_algo, size_t base_n, cfft_u64_product_plan** out) {
@@ -768,7 +770,6 @@ cfft_status cfft_u64_product_plan_create_measure(size_t N, double seconds, cfft_
   TuneVal tv;
   if (tune_lookup(2, N, &tv)) {  // measured before on this GPU model
     cfft_status st = cfft_u64_product_plan_create(N, (cfft_algo)tv.algo, tv.base_n, out);
-    if (st == CFFT_OK) (*out)->emu = tv.emu;
     return st;
   }
   std::vector<size_t> bases;

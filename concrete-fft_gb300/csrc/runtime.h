@@ -53,6 +53,14 @@ inline bool half_butterflies(long ctas, size_t butterflies) {
   return ctas * (long)((butterflies + 31) / 32) * 4 < 5L * 4 * sm_count();
 }
 
+// Which instance of a kernel a plan's launch takes: additions on the FP64 pipe (true) or
+// most of them on the integer pipes.  int_adds: the plan's cfft_*_set_int_adds, or
+// kIntAddsAuto; few: the launch's own choice, as half_butterflies or one like it gives it.
+constexpr int kIntAddsAuto = -1;
+constexpr int kIntAddsShare = 6;  // eighths that the integer instances move (kAddsBatch)
+inline bool fp64_additions(int int_adds, bool few) { return int_adds == kIntAddsAuto ? few : int_adds == 0; }
+inline int int_adds_of(int int_adds) { return int_adds == kIntAddsAuto ? kIntAddsShare : int_adds; }
+
 // Launch a kernel through its pointer, raising its dynamic shared-memory limit
 // the first time it is used with more than 48 KiB.  `pdl`: programmatic stream
 // serialization (the kernel may start while the previous one drains; it must

@@ -62,7 +62,7 @@ cfft_status cfft_tune_save(const char* path) {
   for (const auto& kv : cfft::g_table) {
     const auto& v = kv.second;
     f << std::get<0>(kv.first) << '\t' << std::get<1>(kv.first) << '\t' << std::get<2>(kv.first) << '\t' << v.algo
-      << '\t' << v.base_n << '\t' << v.threads << '\t' << v.tpc << '\t' << v.emu << '\n';
+      << '\t' << v.base_n << '\t' << v.threads << '\t' << v.tpc << '\t' << v.int_adds << '\n';
   }
   return f ? CFFT_OK : cfft::fail_status(CFFT_ERR_INVALID_ARGUMENT, "write failed");
 }

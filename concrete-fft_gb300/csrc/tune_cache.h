@@ -13,7 +13,7 @@ struct TuneVal {
   uint64_t base_n;
   int threads;
   int tpc;
-  int emu;
+  int int_adds;  // written as 0 and not read: the launches choose
 };
 
 bool tune_lookup(int kind, uint64_t n, TuneVal* v);

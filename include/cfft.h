@@ -102,9 +102,11 @@ cfft_status cfft_ordered_inv_host(const cfft_ordered_plan* plan, double* buf, si
  * reference).  GB300 issues FP64 at 1/64 of its integer rate, so the kernels
  * run three in four of a butterfly's additions as exact IEEE additions on the
  * integer pipes, and none in launches of about a warp per SM sub-partition.
- * That share is the kernels' own: `eighths` (0..8, checked) is kept with the
- * plan and its saved tuning and given back, and changes neither speed nor
- * results. */
+ * `eighths` 0 keeps every addition of the plan's launches on the FP64 pipe, 1 to
+ * 8 moves the kernels' own share at every launch size; a plan that was not set
+ * chooses by the launch.  Results are bit-identical for every value.  The getter
+ * gives back what was set, 6 for a plan that was not.  (Some cluster kernels, of
+ * radix 16 and DIT products, come in one form.) */
 cfft_status cfft_ordered_set_int_adds(cfft_ordered_plan* plan, int eighths);
 int cfft_ordered_int_adds(const cfft_ordered_plan* plan);
 

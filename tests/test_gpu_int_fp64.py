@@ -113,3 +113,77 @@ def test_one_cta_kernels_with_few_and_many_warps(cuda, oracle, algo, N):
         d = torch.from_numpy(x.copy()).cuda()
         fft.fwd(d)
         assert np.array_equal(d.cpu().numpy().view(np.uint64), oracle.ordered_fwd(algo, x).view(np.uint64)), count
+
+
+@pytest.mark.parametrize("algo", range(8))
+def test_set_int_adds_chooses_the_instance(cuda, algo):
+    """0 and 8 run the FP64-pipe and the integer instance of every kernel on the same data: the same bits,
+    at small and large launches alike."""
+    import concrete_fft as cf
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(algo)
+
+    def same(x, y):
+        return torch.equal(x.view(torch.int64), y.view(torch.int64))
+
+    for n, base, batch in ((64, 64, 1), (1024, 1024, 1), (1024, 1024, 700), (2048, 512, 3), (4096, 1024, 400),
+                           (1 << 16, 1024, 1), (1 << 16, 512, 9)):
+        plan = cf.unordered.Plan(n, cf.unordered.Method.UserProvided(algo, base))
+        assert plan.int_adds() == 6
+        x = torch.randn((batch, n, 2), dtype=torch.float64, device="cuda", generator=g)
+        res = []
+        for adds in (None, 0, 8):
+            if adds is not None:
+                plan.set_int_adds(adds)
+                assert plan.int_adds() == adds
+            f = x.clone()
+            plan.fwd(torch.view_as_complex(f))
+            i = f.clone()
+            plan.inv(torch.view_as_complex(i))
+            res.append((f, i))
+        for f, i in res[1:]:
+            assert same(f, res[0][0]) and same(i, res[0][1]), (n, batch)
+    for N, base, count, terms in ((256, 128, 700, 1), (2048, 1024, 2, 4), (2048, 1024, 900, 1), (8192, 1024, 1, 1),
+                                  (8192, 512, 100, 2), (16384, 1024, 60, 1)):
+        plan = cf.product.U64ProductPlan(N, algo, base)
+        assert plan.int_adds() == 6
+        a = torch.randint(-(1 << 63), (1 << 63) - 1, (count, terms, N), generator=g, device="cuda")
+        b = torch.randint(-128, 128, (count * terms, N), generator=g, device="cuda")
+        res = []
+        for adds in (None, 0, 8):
+            if adds is not None:
+                plan.set_int_adds(adds)
+            bhat = torch.empty((count, terms, N // 2, 2), dtype=torch.float64, device="cuda")
+            plan.prepare_operand(b, bhat)
+            out = torch.empty((count, N), dtype=torch.int64, device="cuda")
+            plan.product_sum(a, torch.view_as_complex(bhat), out)
+            if terms == 1:
+                p = torch.empty_like(out)
+                plan.product(a.reshape(count, N), bhat, p)
+                assert torch.equal(p, out)
+            res.append((bhat, out))
+        for bhat, out in res[1:]:
+            assert same(bhat, res[0][0]) and torch.equal(out, res[0][1]), (N, count)
+
+
+def test_set_int_adds_changes_the_time(cuda):
+    """8192 products of N = 2048 are bound by the FP64 pipe when every addition stays on it (1.5 times)."""
+    import concrete_fft as cf
+    torch = cuda
+    N, count = 2048, 8192
+    plan = cf.product.U64ProductPlan(N, 2, 1024)
+    a = torch.randint(-(1 << 63), (1 << 63) - 1, (count, N), device="cuda")
+    bhat = torch.randn((count, N // 2), dtype=torch.complex128, device="cuda")
+    out = torch.empty_like(a)
+    ms = {}
+    for adds in (0, 8, 0, 8):
+        plan.set_int_adds(adds)
+        plan.product(a, bhat, out)
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        for _ in range(5):
+            plan.product(a, bhat, out)
+        e1.record()
+        e1.synchronize()
+        ms[adds] = min(ms.get(adds, 1e9), e0.elapsed_time(e1))
+    assert ms[0] > 1.2 * ms[8]
