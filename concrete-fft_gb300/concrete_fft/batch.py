@@ -1,4 +1,4 @@
-"""Mixed-size transforms in one persistent launch (cfft_batch_* of include/cfft.h)."""
+"""Mixed-size transforms in a few persistent launches (cfft_batch_* of include/cfft.h)."""
 import ctypes
 
 import numpy as np
@@ -43,7 +43,7 @@ class Batch:
         return FftAlgo(a.value), b.value, t.value
 
     def run(self, data, stream=None):
-        """One persistent launch over every item, in place on the device buffer `data`."""
+        """Every item in a few persistent launches, in place on the device buffer `data`."""
         if not B.is_device(data):
             raise TypeError("batch data must be a CUDA tensor")
         s = B.stream_of(data) if stream is None else ctypes.c_void_p(stream)

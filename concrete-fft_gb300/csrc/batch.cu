@@ -321,8 +321,8 @@ cfft_status finalize(cfft_batch* b) {
   return st;
 }
 
-// FP64 instructions (DADD/DMUL/DFMA) of one unordered transform of 2^log2n points
-// with the given base: the outer levels' radix-r butterflies plus r - 1 twiddle
+// FP64 operations (additions, products, FMAs) of one unordered transform of 2^log2n points
+// with the given base, wherever they run: the outer levels' radix-r butterflies plus r - 1 twiddle
 // products each, the base's radix-R passes likewise, and its end butterfly.
 double fp64_ops_per_point(int log2n, int base_log2, int algo) {
   auto core = [](int r) { return r == 2 ? 4.0 : r == 4 ? 16.0 : r == 8 ? 56.0 : 168.0; };
@@ -343,9 +343,9 @@ double fp64_ops_per_point(int log2n, int base_log2, int algo) {
 }
 
 // Times candidate schedules of one size class on a synthetic homogeneous batch.
-// The class runs at the FP64 roof, so among candidates timed within 3% of the
-// fastest (short timings are that noisy) the one with the fewest FP64
-// instructions per point wins, and the time decides between equal counts.
+// Among candidates timed within 3% of the fastest (short timings are that noisy)
+// the one with the fewest FP64 operations per point wins, so that the choice
+// does not hang on the noise, and the time decides between equal counts.
 cfft_status tune_class(cfft_batch* b, size_t ci, double seconds) {
   ClassHost& c = b->classes[ci];
   const int log2n = c.key.log2n;

@@ -297,7 +297,8 @@ int split_log2(const C64Plan& p, long batch, int* mode) {
   if (min_ls > 0) {
     // transforms above one CTA's shared memory: a cluster of 8 SMs beats the global-level
     // path (all SMs, several launches) only up to 8192 points and for small batches
-    // (batch 1 fwd+inv, additions on the FP64 pipe as such launches keep them: 37 vs 47 us at 8192, 70 vs 72 at 16384, 131 vs 123 at 32768)
+    // (batch 1 fwd+inv, additions on the FP64 pipe as such launches keep them: 37 vs 47 us
+    // at 8192, 70 vs 72 at 16384, 131 vs 123 at 32768)
     if (log2n > 13 || (batch << max_ls) >= target) return 0;
     return max_ls;
   }

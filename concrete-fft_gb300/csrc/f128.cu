@@ -642,9 +642,10 @@ cfft_status run_f128_tw(size_t n, const F128Tw& tw, double* re0, double* re1, do
   const int log2n = ilog2(n);
   // a small batch of 64..2048 points: one transform per cluster, two warps per 32
   // butterflies, every CTA on an SM of its own: up to 8 CTAs of 128 points up to 1024
-  // points, 16 CTAs (a non-portable cluster size, when such a cluster fits) at 2048.  fwd+inv, one transform, with every addition on the FP64 pipe: 24.9 us at 64 points (one CTA, a thread per
-  // butterfly: 43.6), 42.1 at 512 (75.8), 46.7 at 1024 (85.2), 51.7 at 2048 (93.6 over
-  // global stages).  From SMs/2 CTAs on the block path is as fast.  4096 points take
+  // points, 16 CTAs (a non-portable cluster size, when such a cluster fits) at 2048.
+  // fwd+inv, one transform, with every addition on the FP64 pipe: 24.9 us at 64 points
+  // (one CTA, a thread per butterfly: 43.6), 42.1 at 512 (75.8), 46.7 at 1024 (85.2), 51.7
+  // at 2048 (93.6 over global stages).  From SMs/2 CTAs on the block path is as fast.  4096 points take
   // the half-butterfly stages below (one forward 51.9 us on a 16-CTA cluster, whose 16
   // SMs' FP64 pipes bind it)
   if (!one_kernel && block_log2 == 0 && log2n >= 6 && log2n <= 11) {

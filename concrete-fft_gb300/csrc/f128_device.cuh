@@ -331,42 +331,6 @@ __device__ __forceinline__ void f128_stages_smem(F128Arrays s, int log2n, int lo
 }
 
 // ---------------------------------------------------------------- integers
-// (double)(__int128)v, round to nearest even, on the integer pipe.
-__device__ __forceinline__ double i128_to_f64_rne(uint64_t lo, uint64_t hi) {
-  const bool neg = (hi >> 63) != 0;
-  if (neg) {  // magnitude of the two's complement value
-    lo = ~lo;
-    hi = ~hi;
-    lo += 1;
-    if (lo == 0) hi += 1;
-  }
-  if (hi == 0 && lo == 0) return 0.0;
-  int lz;
-  uint64_t top, rest;  // top: normalised leading 64 bits, rest: sticky source
-  if (hi != 0) {
-    lz = __clzll((long long)hi);
-    top = lz == 0 ? hi : ((hi << lz) | (lo >> (64 - lz)));
-    rest = lz == 0 ? lo : (lo << lz);
-  } else {
-    const int l2 = __clzll((long long)lo);
-    lz = 64 + l2;
-    top = lo << l2;
-    rest = 0;
-  }
-  uint64_t m = top >> 11;
-  const uint64_t r = top & 0x7ff;
-  uint64_t e = (uint64_t)(1023 + 127 - lz);
-  const bool sticky = rest != 0;
-  if (r > 0x400 || (r == 0x400 && (sticky || (m & 1)))) {
-    m += 1;
-    if (m == (1ull << 53)) {
-      m >>= 1;
-      e += 1;
-    }
-  }
-  return __longlong_as_double((long long)((neg ? 0x8000000000000000ull : 0ull) | (e << 52) | (m & 0xfffffffffffffull)));
-}
-
 // One u128 coefficient (lo, hi, read as i128) -> f128: xh = the nearest double, xl =
 // the nearest double to the remainder (src/fft128/mod.rs:2006-2016 pattern), without
 // going back from xh to an integer: the remainder is the bits that xh's rounding

@@ -60,9 +60,7 @@ __device__ __forceinline__ uint32_t round_with_error(uint64_t V, uint32_t e, uin
   const uint32_t rem = Nl & 0x7ffu;
   const uint32_t up = (rem + 0x3ffu + (l & 1u)) >> 11;
   const uint32_t x = e - (f << 20);  // exponent of the result less one, in place
-  uint32_t c;
   asm("add.cc.u32 %0, %0, %3;\n\taddc.u32 %1, %1, %2;" : "+r"(l), "+r"(h) : "r"(x + sign), "r"(up));
-  (void)c;
   // unit of bit 0 of N: 2^-11 of the last place of a result of exponent x + 1
   return small_times_ulp((int)rem - (int)(up << 11), x + (1u << 20) - (11u << 20), sign);
 }

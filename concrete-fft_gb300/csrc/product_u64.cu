@@ -755,12 +755,14 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
 
 // Method::Measure for the product: every (base_algo, base_n) the reference's
 // unordered measurement considers for n = N/2 (src/unordered.rs:553-640: the
-// ordered algorithms at n when n <= 256, else bases 512 and 1024), timed on
-// the fused product kernel itself over a batch that fills every SM.  Several
-// candidates run at the FP64 roof within noise of each other; among those
-// within 2% of the fastest a DIF base is taken, whose few-product cluster
-// kernels are the faster ones (one N = 4096 product: 13.7 us on Dif4/1024, 31
-// us on the five launches that DIT bases take).
+// ordered algorithms at n when n <= 256, else bases 512 and 1024), timed over
+// a batch that fills every SM, on the route that such a batch takes: the
+// fused kernel below N = 4096, the five launches from there.  The ranking is
+// for full batches; smaller ones run other kernels, which are not timed.
+// Several candidates come within noise of each other; among those within 2%
+// of the fastest a DIF base is taken, whose few-product cluster kernels are
+// the faster ones (one N = 4096 product: 12.8 us on Dif4/1024, 33 us on the
+// five launches that DIT bases take).
 cfft_status cfft_u64_product_plan_create_measure(size_t N, double seconds, cfft_u64_product_plan** out) {
   if (!out) return fail(CFFT_ERR_INVALID_ARGUMENT, "null output pointer");
   *out = nullptr;

@@ -250,11 +250,14 @@ cfft_status cfft_f128_sincospi(double x_hi, double x_lo, double* sin_out2, doubl
  * untwist, exact rounding back to the integer ring.
  *
  * u64: coefficients are read as i64, rounded with floor(x + 1/2) and reduced
- * mod 2^64.  N a power of two, 64 <= N <= 2^29: one CTA per product up to
- * N = 8192, a thread-block cluster of 2..16 CTAs per product up to 16384 (and
- * for small batches, see cfft_u64_product_set_cluster_size), and from 32768
- * the five-launch path on a workspace from the stream-ordered allocator (a
- * forced cluster size keeps clusters up to 65536).  bhat
+ * mod 2^64.  N a power of two, 64 <= N <= 2^29.  Small batches run a thread-block
+ * cluster of 2..16 CTAs per product (see cfft_u64_product_set_cluster_size), or
+ * the five steps as launches where the base has no cluster kernel; larger ones one
+ * CTA per product up to N = 4096 and a cluster per product at 8192 and 16384.  From
+ * 4 products per SM (2 at 16384) at N = 4096 to 16384, and always from 32768, the
+ * five launches run around a stream-ordered workspace: at most 256 MiB up to 16384,
+ * where a call that cannot have it takes the kernels without one; N/2 c64 per
+ * product from 32768 (a forced cluster size keeps clusters up to 65536).  bhat
  * holds N/2 c64 per operand in the plan's permuted order; `bhat_stride` is 0
  * (one operand shared by all products) or N/2 (one operand per product). */
 typedef struct cfft_u64_product_plan cfft_u64_product_plan;
@@ -500,8 +503,8 @@ cfft_status cfft_u128_product_host(const cfft_u128_product_plan* plan, const uin
                                    size_t bhat_stride, uint64_t* out, size_t count);
 
 /* ============================================ mixed-size batch (persistent) ====
- * Many c64 transforms of different sizes and kinds in a few persistent kernels
- * launch (no counterpart in the reference, whose plans transform one buffer of
+ * Many c64 transforms of different sizes and kinds in a few persistent kernel
+ * launches (no counterpart in the reference, whose plans transform one buffer of
  * one size per call).  Items live anywhere in one device buffer; each is the
  * transform the matching ordered::Plan / unordered::Plan would compute, with
  * the schedule below, and its result is bit-identical to that plan's. */
@@ -509,7 +512,7 @@ typedef struct cfft_batch_item {
   uint64_t offset;     /* first point of the item in the buffer (c64 units) */
   uint32_t log2n;      /* size 2^log2n: ordered 1..10, unordered 1..16 */
   uint32_t kind;       /* 0: ordered::Plan, 1: unordered::Plan */
-  uint32_t direction;  /* 1: fwd, 2: inv, 3: fwd then inv (one shared-memory residency) */
+  uint32_t direction;  /* 1: fwd, 2: inv, 3: fwd then inv (up to 2048 points without leaving the SM) */
   uint32_t reserved;   /* must be 0 */
 } cfft_batch_item;
 typedef struct cfft_batch cfft_batch;
@@ -523,14 +526,15 @@ size_t cfft_batch_units(const cfft_batch* batch);
 /* The schedule chosen for one size class. */
 cfft_status cfft_batch_schedule(const cfft_batch* batch, uint32_t kind, uint32_t log2n, uint32_t direction,
                                 cfft_algo* base_algo, size_t* base_n, uint32_t* per_unit);
-/* One persistent launch over every item, in place on `data`.  On a non-NULL
- * stream the launch is captured into a CUDA graph on first use (per stream and
- * buffer) and replayed afterwards.  Runs of one batch must not overlap. */
+/* One persistent launch over the items up to 2048 points and the sub-transforms of
+ * larger ones, and one per outer level of these before and after it, in place on
+ * `data`.  On a non-NULL stream the launches are captured into a CUDA graph on first
+ * use (per stream and buffer) and replayed afterwards.  Runs of one batch must not overlap. */
 cfft_status cfft_batch_run(cfft_batch* batch, double* data, void* stream);
 /* The batch from host memory and back (no counterpart in the reference): the
  * items, in offset order, are split into about 16 chunks of equal size; each
  * chunk's points are copied host -> device into `dev` (same layout as `host`),
- * transformed by a persistent launch over the chunk's items, and copied back,
+ * transformed by such launches over the chunk's items, and copied back,
  * the chunks pipelined over three internal streams so that copies overlap
  * transforms.  Ordered after prior work on `stream`; later work on `stream`
  * waits for it.  Only the point ranges of items are copied.  `host` should be
