@@ -30,6 +30,7 @@ ALGO_NAMES = ["Dif2", "Dit2", "Dif4", "Dit4", "Dif8", "Dit8", "Dif16", "Dit16"]
 BASE_SEED = 2  # the workload's index in the benchmark table
 BYTES_PER_PRODUCT = 3 * N_POLY * 8  # A + Bhat + out: 16 KiB each
 METRIC = "N=2048 negacyclic u64 polymul/s"
+LINE_MAX = 2200  # characters of the default line
 
 
 def fp64_ops_per_transform(n, base_n, algo):
@@ -469,9 +470,7 @@ def run_gb300(args):
                      "algorithmic_bytes_per_launch": BYTES_PER_PRODUCT * count,
                      "fp64": {"achieved_ops_per_s": fp64_achieved, "peak_ops_per_s": fp64_peak,
                               "frac": fp64_achieved / fp64_peak, "ops_per_product": fp64_ops,
-                              "microbenchmark_rates": rates,
-                              "note": "the algorithm's FP64 operations against the best DFMA/DADD/DMUL/mix issue rate, "
-                                      "measured live; three additions in four run on the integer pipes, so above 1"}},
+                              "microbenchmark_rates": rates}},
         "plain_path": plain,
         "cpu_baseline": cpu,
         "accuracy": accuracy,
@@ -480,9 +479,36 @@ def run_gb300(args):
                 "copy_only_gbs": copy_gbs},
         "clocks": clk.summary(),
         "gpu_launches": args.steps,
-        "configs": configs,
     }
-    print(json.dumps(line))
+    print_headline(line, dict(line, configs=configs))
+
+
+def short(v, digits=7):
+    """v with its numbers rounded to `digits` significant ones."""
+    if isinstance(v, dict):
+        return {k: short(x, digits) for k, x in v.items()}
+    if isinstance(v, list):
+        return [short(x, digits) for x in v]
+    return float("%.*g" % (digits, v)) if isinstance(v, float) else v
+
+
+def print_headline(line, detail):
+    """The benchmark's one line on stdout, short enough to survive in the tail of a log (LINE_MAX):
+    the headline with its checks, and a value for each further configuration.  Everything that was
+    measured goes to stderr before it, as one JSON object."""
+    print(json.dumps(detail), file=sys.stderr, flush=True)
+    line = short(line)
+    configs = detail.get("configs") or {}
+    rows = {"configs": {k: short(v.get("value", "error" if "error" in v else "in the detail"), 5)
+                        for k, v in configs.items()}} if configs else {}
+    out = json.dumps(dict(line, **rows))
+    for key in ("plain_path", "cpu_baseline", "accuracy"):  # the longest, whole in the detail
+        if len(out) <= LINE_MAX:
+            break
+        line[key] = {k: v for k, v in (line.get(key) or {}).items()
+                     if isinstance(v, (int, float)) or isinstance(v, str) and len(v) <= 12} or None
+        out = json.dumps(dict(line, **rows))
+    print(out, flush=True)
 
 
 # ---------------------------------------------------------------- other workloads
