@@ -33,10 +33,17 @@ METRIC = "N=2048 negacyclic u64 polymul/s"
 LINE_MAX = 2200  # characters of the default line
 
 
-def fp64_ops_per_transform(n, base_n, algo):
-    """FP64 instructions (DADD/DMUL/DFMA, one each) of one unordered transform
-    of n points with the given base, counted from the butterfly code."""
-    core = {2: 4, 4: 16, 8: 56, 16: 168}
+# FP64 operations of the radix-R butterfly cores, and how many of them the throughput kernels
+# leave on the FP64 pipe: of the additions, which come in sum/difference pairs, three pairs in
+# four run on the integer pipes (all of a radix-2 core's, half of radix 16's); products stay.
+CORE_OPS = {2: 4, 4: 16, 8: 56, 16: 168}
+CORE_ISSUED = {2: 0, 4: 4, 8: 16, 16: 96}
+
+
+def fp64_ops_per_transform(n, base_n, algo, core=CORE_OPS):
+    """FP64 operations (additions, products and FMAs, one each) of one unordered transform
+    of n points with the given base, counted from the butterfly code; core=CORE_ISSUED: the
+    instructions that the FP64 pipe executes for them."""
     ops = 0
     m = n
     while m > base_n:  # outer levels: core + (r-1) twiddle products of 4 ops
@@ -53,9 +60,16 @@ def fp64_ops_per_transform(n, base_n, algo):
     return ops
 
 
-def fp64_ops_per_product(N, base_n, algo):
+def fp64_ops_per_product(N, base_n, algo, core=CORE_OPS):
     n = N // 2
-    return 2 * fp64_ops_per_transform(n, base_n, algo) + 3 * 4 * n  # twist, pointwise, untwist
+    return 2 * fp64_ops_per_transform(n, base_n, algo, core) + 3 * 4 * n  # twist, pointwise, untwist
+
+
+def fp64_roof(ops, issued, seconds, peak):
+    """The FP64 pipe's share: the algorithm's operations a second, the instructions issued to the
+    pipe for them, and these against the best measured issue rate."""
+    return {"algorithm_ops_per_s": ops / seconds, "issued_per_s": issued / seconds, "peak_per_s": peak,
+            "frac": issued / seconds / peak}
 
 
 class ClockSampler:
@@ -421,7 +435,7 @@ def run_gb300(args):
     rates = fp64_rates(cf)
     fp64_peak = max(rates.values())
     fp64_ops = fp64_ops_per_product(N_POLY, base_n, int(algo))
-    fp64_achieved = fp64_ops * count / per_launch_s
+    fp64_issued = fp64_ops_per_product(N_POLY, base_n, int(algo), CORE_OPS if int_adds == 0 else CORE_ISSUED)
 
     del z, out_plain, ha, hout
     # the other benchmark configurations, each with its own clocks, roofline, e2e, accuracy and
@@ -468,9 +482,7 @@ def run_gb300(args):
                      "frac": achieved_gbs / peaks.get("hbm_gbs"), "peak_kind": peak_kind,
                      "traffic": traffic.get("dram_bytes_per_launch") if traffic else None,
                      "algorithmic_bytes_per_launch": BYTES_PER_PRODUCT * count,
-                     "fp64": {"achieved_ops_per_s": fp64_achieved, "peak_ops_per_s": fp64_peak,
-                              "frac": fp64_achieved / fp64_peak, "ops_per_product": fp64_ops,
-                              "microbenchmark_rates": rates}},
+                     "fp64": fp64_roof(fp64_ops * count, fp64_issued * count, per_launch_s, fp64_peak)},
         "plain_path": plain,
         "cpu_baseline": cpu,
         "accuracy": accuracy,
@@ -480,7 +492,9 @@ def run_gb300(args):
         "clocks": clk.summary(),
         "gpu_launches": args.steps,
     }
-    print_headline(line, dict(line, configs=configs))
+    detail = dict(line, fp64={"ops_per_product": fp64_ops, "issued_per_product": fp64_issued,
+                              "microbenchmark_rates": rates}, configs=configs)
+    print_headline(line, detail)
 
 
 def short(v, digits=7):
@@ -761,6 +775,7 @@ def measure_ordered(torch, cf, steps, warmup, local, world, full=False, cpu_seco
     ms1g20, _ = timed(torch, graph20.replay, reps20, min(warmup, 4), local, world, restore1, 4)
     per = ms256 * 1e-3 / steps
     ops = 256 * 2 * fp64_ops_ordered(1024, int(algo))
+    issued = 256 * 2 * fp64_ops_per_transform(1024, 1024, int(algo), CORE_ISSUED)
     peak = fp64_peak(cf)
     peaks, peak_kind = measured_peaks()
     bytes_step = 256 * 2 * 32768  # each of the 512 calls reads and writes 16 KiB
@@ -788,9 +803,7 @@ def measure_ordered(torch, cf, steps, warmup, local, world, full=False, cpu_seco
                      "frac": bytes_step / per / 1e9 / peaks["hbm_gbs"], "peak_kind": peak_kind,
                      "traffic": prof.get("dram_bytes_per_launch"),
                      "algorithmic_bytes_per_launch": 256 * 32768,
-                     "fp64": {"achieved_ops_per_s": ops / per, "peak_ops_per_s": peak, "frac": ops / per / peak,
-                              "ops_per_transform": fp64_ops_ordered(1024, int(algo)),
-                              "note": "the algorithm's operations; additions also run on the integer pipes"}},
+                     "fp64": dict(fp64_roof(ops, issued, per, peak), ops_per_transform=fp64_ops_ordered(1024, int(algo)))},
         "e2e": {"value": e2e, "unit": "transforms/s", "h2d_bytes_per_step": 2 * 256 * 1024 * 16,
                 "d2h_bytes_per_step": 2 * 256 * 1024 * 16, "steps": e2e_steps,
                 "path": "cfft_ordered_fwd_host / _inv_host on a page-locked buffer, in place"},
@@ -910,7 +923,7 @@ def mixed_items(cf, count, seed):
 def measure_mixed(torch, cf, steps, warmup, local, world, count=100000, tune_seconds=0.0005, seed=3,
                   cpu_seconds=3.0, cpu=True, e2e_steps=3):
     """100,000 c64 transforms, sizes 2^k with k uniform in 8..16, half ordered and half unordered,
-    forward then inverse, one persistent launch per step (CUDA graph replay)."""
+    forward then inverse, persistent launches in one CUDA graph per step."""
     import numpy as np
     po = _oracle()
     items, log2n, kind, sizes, offs, rng = mixed_items(cf, count, seed)
@@ -956,7 +969,7 @@ def measure_mixed(torch, cf, steps, warmup, local, world, count=100000, tune_sec
     transforms = 2 * count
     value = world * transforms * steps / (ms * 1e-3)
     per_launch = ms * 1e-3 / steps
-    ops = 0
+    ops = issued = 0
     sched = {}
     for k in range(8, 17):
         for kd in (0, 1):
@@ -966,6 +979,7 @@ def measure_mixed(torch, cf, steps, warmup, local, world, count=100000, tune_sec
             algo, base, tpc = b.schedule(kd, k, 3)
             sched["%s%d" % ("o" if kd == 0 else "u", k)] = [algo.name, base, tpc]
             ops += int(sel.sum()) * 2 * fp64_ops_per_transform(1 << k, base, int(algo))
+            issued += int(sel.sum()) * 2 * fp64_ops_per_transform(1 << k, base, int(algo), CORE_ISSUED)
     peak = fp64_peak(cf)
     bytes_alg = total * 32 * 2  # forward and inverse each read and write every point
     peaks, peak_kind = measured_peaks()
@@ -985,7 +999,7 @@ def measure_mixed(torch, cf, steps, warmup, local, world, count=100000, tune_sec
         "metric": "mixed-size c64 transforms/s (100k items, n=2^8..2^16, fwd then inv)", "value": value,
         "unit": "transforms/s", "steps": steps, "warmup": warmup, "ms_per_step": ms / steps,
         "higher_is_better": True, "dtype": "f64",
-        "config": {"workload": "mixed batch, %d items, %d points, one persistent launch per step (graph)"
+        "config": {"workload": "mixed batch, %d items, %d points, persistent launches in one graph per step"
                                % (count, total),
                    "schedule": sched, "units": b.units(), "tune_seconds_total": tune_s,
                    "ordered_items": int((kind == 0).sum()), "l2": "23 GB of data > L2"},
@@ -993,8 +1007,7 @@ def measure_mixed(torch, cf, steps, warmup, local, world, count=100000, tune_sec
                      "unit": "GB/s", "frac": bytes_alg / per_launch / 1e9 / peaks["hbm_gbs"], "peak_kind": peak_kind,
                      "traffic": (prof.get("dram_bytes_per_point") * total) if prof.get("dram_bytes_per_point") else None,
                      "algorithmic_bytes_per_launch": bytes_alg,
-                     "fp64": {"achieved_ops_per_s": ops / per_launch, "peak_ops_per_s": peak,
-                              "frac": ops / per_launch / peak, "note": "the algorithm's operations; additions also run on the integer pipes"}},
+                     "fp64": fp64_roof(ops, issued, per_launch, peak)},
         "e2e": {"value": world * transforms * e2e_steps / e2e_s, "unit": "transforms/s",
                 "h2d_bytes_per_step": total * 16, "d2h_bytes_per_step": total * 16, "steps": e2e_steps,
                 "path": "cfft_batch_run_host from page-locked host memory, 16 pipelined chunks"},
@@ -1125,11 +1138,10 @@ def measure_u128(torch, cf, steps, warmup, local, world, full=False, cpu_seconds
     v = by_n[1024]["products_per_s"]
     fp64 = None
     if prof.get("fp64_thread_inst_per_product"):
-        ach = prof["fp64_thread_inst_per_product"] * v
-        fp64 = {"achieved_ops_per_s": ach, "peak_ops_per_s": peak, "frac": ach / peak,
-                "ops_per_product": prof["fp64_thread_inst_per_product"],
-                "note": "DADD/DFMA/DMUL of the algorithm per product (N=1024); its error-free sums and cross "
-                        "products run on the integer pipes, so above 1"}
+        fp64 = dict(fp64_roof(prof["fp64_thread_inst_per_product"] * v,
+                              prof["fp64_issued_thread_inst_per_product"] * v, 1.0, peak),
+                    note="DADD/DFMA/DMUL of the algorithm per product (N=1024), and those issued: the error-free "
+                         "sums and cross products run on the integer pipes")
     # fft128::Plan itself at n = 512 (batch 4096 and batch 1), GPU and the host's restatement
     plans128 = {}
     for n, batch in (((512, 4096), (2048, 1024), (4096, 512), (16384, 128)) if full else ((512, 4096),)):
@@ -1594,6 +1606,8 @@ def run_product_sum(args):
     n = N // 2
     ops = groups * (T * (fp64_ops_per_transform(n, 1024, 2) + 4 * n + 4 * n + 2 * n) - 2 * n
                     + fp64_ops_per_transform(n, 1024, 2) + 4 * n)
+    issued = ops - groups * (T + 1) * (fp64_ops_per_transform(n, 1024, 2)
+                                       - fp64_ops_per_transform(n, 1024, 2, CORE_ISSUED))
     peak = fp64_peak(cf)
     peaks, peak_kind = measured_peaks()
     alg_bytes = groups * T * N * 8 + groups * T * n * 16 + groups * N * 8  # A and Bhat read, sums written
@@ -1609,7 +1623,7 @@ def run_product_sum(args):
                      "frac": alg_bytes / per / 1e9 / peaks["hbm_gbs"], "peak_kind": peak_kind,
                      "traffic": (profiled_traffic("u64_product_sum_n2048") or {}).get("dram_bytes_per_launch"),
                      "algorithmic_bytes_per_launch": alg_bytes,
-                     "fp64": {"achieved_ops_per_s": ops / per, "peak_ops_per_s": peak, "frac": ops / per / peak}},
+                     "fp64": fp64_roof(ops, issued, per, peak)},
         "clocks": clocks, "gpu_launches": args.steps,
     }))
 
@@ -1737,7 +1751,7 @@ def measure_latency(torch, cf, local, world, cpu=True, cpu_seconds=0.5, profile_
             rows["u128_product_N%d" % N] = row
         clk.mark(t0, time.time())
     return {"rows": rows, "clocks": clk.summary(),
-            "gpu": "device time per call: 20 calls captured in a CUDA graph, replayed 10 times from the inputs, CUDA events",
+            "gpu": "device time per call: 20 calls captured in a CUDA graph, replayed 10 times, CUDA events",
             "cpu": "the restated reference pipeline on one host core with the plan's algorithm, per product over "
                    "calls of 32 products (8 for u128), so that the plan's set-up is spread as for a prepared plan"}
 
@@ -1783,7 +1797,7 @@ def run_u64_large(args):
         ms_u, _ = timed(torch, lambda: plan.product_unfused(a, bhat, out2, z), max(3, args.steps // 4), 2, local,
                         world)
         per = ms * 1e-3 / args.steps
-        ops = fp64_ops_per_product(N, 1024, int(cf.FftAlgo.Dif4)) * count
+        ops = fp64_ops_per_product(N, 1024, int(cf.FftAlgo.Dif4), CORE_ISSUED) * count
         rows[N] = {"products_per_s": world * count / per, "fp64_frac": ops / per / peak,
                    "cluster_products_per_s": world * count * args.steps / (ms_c * 1e-3),
                    "unfused_products_per_s": world * count * max(3, args.steps // 4) / (ms_u * 1e-3),
@@ -1871,7 +1885,7 @@ def main():
     ap.add_argument("--base-algo", default=None, help="fix the base algorithm (e.g. Dif4) instead of measuring")
     ap.add_argument("--base-n", type=int, default=1024)
     ap.add_argument("--int-adds", type=int, default=None,
-                    help="eighths of butterfly additions on the integer pipe (default: the plan's tuned value)")
+                    help="eighths of butterfly additions on the integer pipe (0: none; 1-8: the kernels' share; default: by the size of the launch)")
     ap.add_argument("--profile-case", action="store_true",
                     help="small fixed case for ncu: 1 warm-up + 1 launch, no timing")
     ap.add_argument("--rate", type=float, default=20000.0)

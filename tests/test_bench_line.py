@@ -20,7 +20,7 @@ def test_line_is_short_and_whole(capsys):
                 "ms_per_step": third / 1e7, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
                 "dtype": "f64", "data": "synthetic (seeded numpy PCG64)"}
     line = dict(contract, config={"workload": "w" * 120, "l2": "inputs 384 MiB > L2 (no flush needed)"},
-                roofline={"frac": third, "fp64": {"frac": third}},
+                roofline={"frac": third, "fp64": b.fp64_roof(3.0, 2.0, third, third)},
                 plain_path={"note": "x" * 400, "value": third}, cpu_baseline={"sample": "y" * 400, "value": third},
                 accuracy={"bound": "z" * 1600, "worst_bits": third, "ok": True},
                 e2e={"value": third, "h2d_bytes_per_step": 1, "d2h_bytes_per_step": 1},
@@ -36,3 +36,12 @@ def test_line_is_short_and_whole(capsys):
     assert got["configs"]["config_0"] == 3333300.0 and got["configs"]["failed"] == "error"
     assert json.loads(err)["configs"] == configs and json.loads(err)["value"] == third
 
+
+def test_issued_fp64_instructions():
+    """8192 products of N = 2048 on Dif4 executed 12.66 M FP64 warp instructions: the counted ones and
+    the conversions of fold and round."""
+    b = _bench()
+    issued = b.fp64_ops_per_product(2048, 1024, 2, b.CORE_ISSUED) * 8192 / 32
+    assert 0.9 * 12.66e6 < issued < 12.66e6
+    for algo in range(8):
+        assert b.fp64_ops_per_transform(2048, 512, algo, b.CORE_ISSUED) < b.fp64_ops_per_transform(2048, 512, algo)
