@@ -187,3 +187,38 @@ def test_set_int_adds_changes_the_time(cuda):
         e1.synchronize()
         ms[adds] = min(ms.get(adds, 1e9), e0.elapsed_time(e1))
     assert ms[0] > 1.2 * ms[8]
+
+
+def _same_or_nan(got, want):
+    """The same bits, or NaN in both (whose sign and payload IEEE 754 leaves open)."""
+    import numpy as np
+    g, w = got.view(np.uint64).ravel(), want.view(np.uint64).ravel()
+    nan = np.isnan(got.view(np.float64).ravel()) & np.isnan(want.view(np.float64).ravel())
+    return bool(np.all((g == w) | nan))
+
+
+@pytest.mark.parametrize("kind", ["infinities", "nans", "near_overflow", "overflowing"])
+@pytest.mark.parametrize("algo", range(8))
+def test_transforms_of_infinities_and_overflow(cuda, oracle, algo, kind):
+    """Infinities, NaNs and values at the top of the range through transforms of both instances."""
+    import concrete_fft as cf
+    import numpy as np
+    torch = cuda
+    rng = np.random.default_rng(algo)
+    for n, batch in ((256, 1), (1024, 200), (512, 700)):
+        x = rng.uniform(-1, 1, (batch, n)) + 1j * rng.uniform(-1, 1, (batch, n))
+        p = np.arange(batch) % n
+        if kind == "infinities":
+            x.real[np.arange(batch), p] = np.where(p % 2, np.inf, -np.inf)
+        elif kind == "nans":
+            x.imag[np.arange(batch), p] = np.nan
+        elif kind == "near_overflow":  # sums just below the largest double
+            x = x * 2.0 ** (1023 - n.bit_length())
+        else:
+            x = x * 2.0 ** 1022
+        plan = cf.ordered.Plan(n, cf.ordered.Method.UserProvided(algo))
+        d = torch.from_numpy(x.copy()).cuda()
+        plan.fwd(d)
+        with np.errstate(all="ignore"):
+            f = oracle.ordered_fwd(algo, x)
+        assert _same_or_nan(d.cpu().numpy(), f), (n, batch)

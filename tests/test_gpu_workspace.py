@@ -229,6 +229,28 @@ def test_graph_workspace_on_request(cuda, case):
         assert torch.equal(out, want)
 
 
+def test_workspace_calls_on_two_streams_at_once(cuda):
+    """Sums in two launches, unfused sums and large products interleaved on two streams: every call has a
+    workspace of its own."""
+    torch = cuda
+    cases = [sum_case(torch, *c) for c in ((2048, 2, 1024, 2, 4), (2048, 3, 1024, 40, 3), (16384, 2, 1024, 2, 3))]
+    plan, product, want = u128_case(torch, 4096, 80)
+    product(want)
+    cases.append((plan, product, want))
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = [[want.clone().fill_(-1) for _, _, want in cases] for _ in streams]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for k, (_, call, _) in enumerate(cases):
+            for s, out in zip(streams, outs):
+                with torch.cuda.stream(s):
+                    call(out[k])
+    torch.cuda.synchronize()
+    for out in outs:
+        for (_, _, want), o in zip(cases, out):
+            assert torch.equal(o, want)
+
+
 LAST_PLAN = """
 import sys
 sys.path.insert(0, %r)
