@@ -316,18 +316,23 @@ int split_log2(const C64Plan& p, long batch, int* mode) {
   while (ls < max_ls && (batch << ls) < target) ++ls;
   // From 4 transforms per SM the SM with the most of them sets the time: ceil(batch / SMs)
   // whole ones (in CTAs of p.tpc), or ceil(2 batch / SMs) halves.  Where that is less, two
-  // CTAs per transform win on radix 4, and on radix 2 without an outer level; whole / halves
-  // over 609 to 684 transforms, forward and inverse: 1024 points 1.00 to 1.18, 2048 points
-  // 1.05 to 1.11 (650 on Dif4/1024 69.3 us and 65.9).  At the same count the halves lose up to
-  // 7%, but at 512 points, where a CTA holds two transforms, they win up to 759 (radix 2 1.19
-  // to 1.43, Dif4 1.04 to 1.17, Dit4 0.98 to 1.10).  From 5 per SM the exchange costs what is
-  // left to gain.  Radix 2 under a level lost at 1024 points (0.81 to 0.95), radix 8 at 512 and
-  // 1024 (0.49 to 0.99).
+  // CTAs per transform win on radix 4, on radix 2 without an outer level, and on DIF radix 8
+  // where a half's pass has four warps of butterflies, one per SM sub-partition; whole / halves
+  // over 609 to 684 transforms, forward and inverse: radix 2 and 4 at 1024 points 1.00 to 1.18,
+  // at 2048 points 1.05 to 1.11 (650 on Dif4/1024 69.3 us and 65.9), Dif8 at 2048 points 0.98 to
+  // 1.16 (613 on base 512 74.8 us and 69.9), with two warps at 1024 points 0.85 to 0.99, one at
+  // 512 0.79 to 0.86.  At the same count the halves lose up to 7% (11% on Dif8), but at 512
+  // points, where a CTA holds two transforms, radix 2 and 4 win up to 759 (radix 2 1.19 to
+  // 1.43, Dif4 1.04 to 1.17, Dit4 0.98 to 1.10).  From 5 per SM the exchange costs what is left
+  // to gain.  Radix 2 under a level lost at 1024 points (0.81 to 0.95); DIT radix 8 (0.6 to
+  // 0.78) and radix 16 have no additions on the integer pipes in the split kernels.
   const long sms = sm_count(), tpc = p.tpc;
   const long whole = 2 * tpc * ((batch + tpc * sms - 1) / (tpc * sms)), halves = (2 * batch + sms - 1) / sms;
-  const bool radix4 = algo_radix(p.base_algo) == 4, radix2 = algo_radix(p.base_algo) == 2;
-  if (ls == 0 && max_ls >= 1 && (radix4 || (radix2 && p.lv.nlevels == 0)) && log2n >= 9 &&
-      log2n <= kBlockLog2Auto && batch < 5 * sms && whole - halves >= (tpc > 1 ? 0 : 1))
+  const size_t radix = (size_t)algo_radix(p.base_algo);
+  const bool wins = radix == 4 || (radix == 2 && p.lv.nlevels == 0) ||
+                    (p.base_algo == CFFT_DIF8 && p.n / 2 / radix >= 128);
+  if (ls == 0 && max_ls >= 1 && wins && log2n >= 9 && log2n <= kBlockLog2Auto && batch < 5 * sms &&
+      whole - halves >= (tpc > 1 ? 0 : 1))
     ls = 1;
   return ls;
 }
