@@ -221,8 +221,13 @@ __global__ void __launch_bounds__(MAXT) u64_product_split_kernel(
 // Shared memory: three buffers of n/S points.  Requires L.nlevels == 0,
 // S <= R, n >= R*S and, for kSum, n/S <= kSplit0Acc x blockDim.x.
 enum ProductPhase { kWhole = 0, kForward = 1, kInverse = 2, kSum = 3 };
+// CTAs of 256 threads per SM by registers.  kSum keeps its accumulator besides: 2 outputs of
+// 4 terms of N = 2048 on Dif4/1024 28.5 us at two per SM, 31.4 at three; on Dif8/1024 40.5 and
+// 41.3.
+template <int ALGO, bool FEW, int PHASE, int LS0 = 0>
+constexpr int kProductCtas = PHASE == kSum && AlgoInfo<ALGO>::R < 16 ? 2 : kFewCtas<ALGO, FEW, LS0>;
 template <int ALGO, int LS, int PHASE, bool FEW>
-__global__ void __launch_bounds__(256, kFewCtas<ALGO, FEW>) u64_product_split0_kernel(
+__global__ void __launch_bounds__(256, kProductCtas<ALGO, FEW, PHASE>) u64_product_split0_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
     int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
     const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw,
@@ -419,7 +424,7 @@ __global__ void __launch_bounds__(256, kFewCtas<ALGO, FEW>) u64_product_split0_k
 // L.nlevels == 1, 2^L.log2r[0] == R0, S1 <= the base radix R, m >= R*S1 and, for
 // kSum, m/S1 <= kSplit0Acc x blockDim.x.
 template <int ALGO, int LS0, int LS1, int PHASE, bool FEW>
-__global__ void __launch_bounds__(256, kFewCtas<ALGO, FEW, LS0>) u64_product_split2_kernel(
+__global__ void __launch_bounds__(256, kProductCtas<ALGO, FEW, PHASE, LS0>) u64_product_split2_kernel(
     const uint64_t* __restrict__ a, const double2* __restrict__ bhat, long bhat_stride, uint64_t* __restrict__ out,
     int terms, const cfft_product_item* __restrict__ items, DevLevels L, const double2* __restrict__ w,
     const double2* __restrict__ winv, const double2* __restrict__ tw, const double2* __restrict__ itw,
