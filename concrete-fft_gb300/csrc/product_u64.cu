@@ -728,8 +728,9 @@ cfft_status cfft_u64_product(const cfft_u64_product_plan* plan, const uint64_t* 
   if (r.kind == ProductRoute::kSplit2)
     return launch_split2_product(plan, r.ls0, r.ls1, a, bhat, bhat_stride, out, count, s);
   if (r.kind == ProductRoute::kFive && (!r.spare || may_allocate(plan, s))) {
-    // with another route, in equal parts within a small workspace
-    const size_t fit = r.spare ? std::max<size_t>(1, kWorkspaceSmall / (plan->n * sizeof(double2))) : count;
+    // in equal parts within what the pool keeps, or a small workspace where there is another route
+    const size_t fit =
+        std::max<size_t>(1, (r.spare ? kWorkspaceSmall : kWorkspaceKeep) / (plan->n * sizeof(double2)));
     const size_t parts = (count + fit - 1) / fit, part = (count + parts - 1) / parts;
     void* z = nullptr;
     const bool got = plan->workspace.alloc(&z, part * plan->n * sizeof(double2), s) == cudaSuccess;

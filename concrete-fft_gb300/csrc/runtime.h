@@ -145,7 +145,8 @@ void* mapped_host_range(const void* p, size_t bytes);
 // capture, as cudaMallocAsync is.  A plan holds a WorkspaceUser; cudaFreeAsync frees.
 // Larger batches go through parts of kWorkspaceKeep, so that these do not come from the
 // device again each time (a pool of 256 MiB under parts of 1 GiB, waited for: 1000 sums of 4
-// terms of N = 32768 7.35 ms, 5.63; 9000 u128 products of N = 4096 15.2 ms, 14.4.  Parts of 256 MiB
+// terms of N = 32768 7.35 ms, 5.63; 9000 u128 products of N = 4096 15.2 ms, 14.4; 6000 u64
+// products of N = 32768, all at once before, 15.0 ms, 12.3.  Parts of 256 MiB
 // instead took 5.75 and 14.6 ms, and 2.5% more where nothing waits: 1100 u128 products of
 // N = 16384 8.34 ms, 8.13).
 constexpr unsigned long long kWorkspaceKeep = 1ull << 30;

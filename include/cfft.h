@@ -256,8 +256,9 @@ cfft_status cfft_f128_sincospi(double x_hi, double x_lo, double* sin_out2, doubl
  * CTA per product up to N = 4096 and a cluster per product at 8192 and 16384.  From
  * 4 products per SM (2 at 16384) at N = 4096 to 16384, and always from 32768, the
  * five launches run around a stream-ordered workspace: at most 256 MiB up to 16384,
- * where a call that cannot have it takes the kernels without one; N/2 c64 per
- * product from 32768 (a forced cluster size keeps clusters up to 65536).  bhat
+ * where a call that cannot have it takes the kernels without one; at most 1 GiB, or
+ * one product at a time, from 32768 (a forced cluster size keeps clusters up to
+ * 65536).  bhat
  * holds N/2 c64 per operand in the plan's permuted order; `bhat_stride` is 0
  * (one operand shared by all products) or N/2 (one operand per product). */
 typedef struct cfft_u64_product_plan cfft_u64_product_plan;

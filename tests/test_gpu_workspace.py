@@ -251,6 +251,28 @@ def test_workspace_calls_on_two_streams_at_once(cuda):
             assert torch.equal(o, want)
 
 
+def test_u64_products_go_through_parts_of_the_pool(cuda):
+    """130 products of N = 2^20 need 1.02 GiB at once: they run in two parts of at most 1 GiB, with the same bits."""
+    import concrete_fft as cf
+    torch = cuda
+    N, count = 1 << 20, 130
+    g = torch.Generator(device="cuda").manual_seed(3)
+    plan = cf.product.U64ProductPlan(N, 2, 1024)
+    a = torch.randint(-(1 << 63), (1 << 63) - 1, (count, N), generator=g, device="cuda")
+    bhat = torch.empty((1, N // 2), dtype=torch.complex128, device="cuda")
+    plan.prepare_operand(torch.randint(-128, 128, (1, N), generator=g, device="cuda"), bhat)
+    out = torch.empty_like(a)
+    cf.check(cf.load().cfft_diag_set_workspace_limit(1 << 30))
+    try:
+        plan.product(a, bhat, out, True)
+    finally:
+        cf.check(cf.load().cfft_diag_set_workspace_limit(0))
+    for r in (0, 64, 65, 129):
+        one = torch.empty((1, N), dtype=torch.int64, device="cuda")
+        plan.product(a[r:r + 1].contiguous(), bhat, one, True)
+        assert torch.equal(out[r], one[0]), r
+
+
 LAST_PLAN = """
 import sys
 sys.path.insert(0, %r)
