@@ -43,23 +43,25 @@ struct EngClass {
   int log2n;  // log2(N/2); 0 when the size is not configured
 };
 
-template <int ALGO>
-__device__ void engine_product(const EngClass& C, const cfft_product_item& it, double2* x, double2* y,
-                               double2* __restrict__ ws, int tid, int nth) {
+// E: the share of the additions on the integer pipes (cfft_device.cuh).  The instances are
+// functions of their own: inlined together, products of N = 8192 and more lost 3 to 5%.
+template <int ALGO, int E>
+__device__ __noinline__ void engine_product(const EngClass& C, const cfft_product_item& it, double2* x, double2* y,
+                                            double2* __restrict__ ws, int tid, int nth) {
   const int log2n = C.log2n, n = 1 << log2n;
   const uint64_t* a = it.a;
   const double2* bh = (const double2*)it.bhat;
   uint64_t* out = it.out;
-  if (C.d0 == 0) {
+  if (E == 0 || C.d0 == 0) {  // (E = 0: sizes that shared memory holds)
     for (int j = tid; j < n; j += nth) {
       const c64 v{i64_to_f64_rne((int64_t)__ldcs(a + j)), i64_to_f64_rne((int64_t)__ldcs(a + j + n))};
       st(x + j, cmul(ldg(C.tw + j), v));
     }
     __syncthreads();
-    double2* r = unordered_smem<true, kAddsBatch, ALGO>(C.L, 0, 1, x, y, C.w, tid, nth);
+    double2* r = unordered_smem<true, E, ALGO>(C.L, 0, 1, x, y, C.w, tid, nth);
     for (int k = tid; k < n; k += nth) st(r + k, cmul(ldg(bh + k), ld(r + k)));
     __syncthreads();
-    double2* s = unordered_smem<false, kAddsBatch, ALGO>(C.L, 0, 1, r, r == x ? y : x, C.winv, tid, nth);
+    double2* s = unordered_smem<false, E, ALGO>(C.L, 0, 1, r, r == x ? y : x, C.winv, tid, nth);
     for (int j = tid; j < n; j += nth) {
       const c64 t = cmul(ldg(C.itw + j), ld(s + j));
       __stcs(out + j, round_half_up_mod64(t.re));
@@ -74,7 +76,7 @@ __device__ void engine_product(const EngClass& C, const cfft_product_item& it, d
   }
   __syncthreads();
   for (int l = 0; l < C.d0; ++l) {
-    outer_level<true, kAddsBatch>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), ws, C.w + C.L.w_off[l], tid, nth);
+    outer_level<true, E>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), ws, C.w + C.L.w_off[l], tid, nth);
     __syncthreads();
   }
   const int log2sub = C.L.log2n[C.d0], m = 1 << log2sub;
@@ -82,16 +84,16 @@ __device__ void engine_product(const EngClass& C, const cfft_product_item& it, d
     double2* gc = ws + ((long)c << log2sub);
     for (int i = tid; i < m; i += nth) x[i] = gc[i];
     __syncthreads();
-    double2* r = unordered_smem<true, kAddsBatch, ALGO>(C.L, C.d0, 1, x, y, C.w, tid, nth);
+    double2* r = unordered_smem<true, E, ALGO>(C.L, C.d0, 1, x, y, C.w, tid, nth);
     const double2* bc = bh + ((long)c << log2sub);
     for (int k = tid; k < m; k += nth) st(r + k, cmul(ldg(bc + k), ld(r + k)));
     __syncthreads();
-    double2* s = unordered_smem<false, kAddsBatch, ALGO>(C.L, C.d0, 1, r, r == x ? y : x, C.winv, tid, nth);
+    double2* s = unordered_smem<false, E, ALGO>(C.L, C.d0, 1, r, r == x ? y : x, C.winv, tid, nth);
     for (int i = tid; i < m; i += nth) gc[i] = s[i];
     __syncthreads();
   }
   for (int l = C.d0 - 1; l >= 0; --l) {
-    outer_level<false, kAddsBatch>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), ws, C.winv + C.L.winv_off[l], tid,
+    outer_level<false, E>(C.L.log2r[l], C.L.log2n[l], 1 << (log2n - C.L.log2n[l]), ws, C.winv + C.L.winv_off[l], tid,
                           nth);
     __syncthreads();
   }
@@ -122,8 +124,12 @@ __global__ void __launch_bounds__(kEngThreads, 2) product_engine_kernel(const En
     if (i >= count) break;
     const cfft_product_item it = items[i];
     const EngClass C = classes[it.log2N];
-    if (C.algo == 2) engine_product<2>(C, it, x, y, ws, tid, nth);
-    else engine_product<4>(C, it, x, y, ws, tid, nth);
+    // Dif8 (N = 64, 256, 1024) has at most two warps in a pass, a chain that integer additions
+    // lengthen (one of N = 1024: 39.0 us, 25.0 on the FP64 pipe; 1000: 128 and 102; one of
+    // N = 64 24.6 and 14.8).  Of Dif4 only N = 128 would gain (14.4 and 12.9), and a third
+    // instance costs one product of N = 8192 107 -> 112 us
+    if (C.algo == 4) engine_product<4, 0>(C, it, x, y, ws, tid, nth);
+    else engine_product<2, kAddsBatch>(C, it, x, y, ws, tid, nth);
   }
 }
 
